@@ -363,7 +363,12 @@ __global__ void k_untranspose_rows(const T* __restrict__ in, uint32_t V, int n, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// tasks: item i of a list index (begin[i], begin[i+1]) split into pieces of <= kTaskEdges edges
+// tasks: item i of a list index (begin[i], begin[i+1]) split into pieces of <= kTaskEdges edges.
+// A task is one 16-byte record, so that a warp knows its edges, its vertex and where its result
+// goes after a single load (which it issues one task ahead):
+//   x  first edge, low 32 bits          z  vertex whose row the task reduces into
+//   y  first edge, bits 32..39 in 0..7  w  slot of a list cut into several tasks, or kNoSlot
+//      edges of the task << 8
 struct TaskLoad {
     const uint64_t* begin;
     __device__ uint32_t operator()(uint64_t i) const {
@@ -372,134 +377,151 @@ struct TaskLoad {
     }
 };
 struct TaskEpi {
-    uint32_t* t_item;
-    uint32_t* t_part;
-    uint32_t* heavy_slot;     // per item
-    uint32_t* heavy_item;     // per slot
+    uint4* rec;
+    const uint64_t* begin;
+    const uint32_t* item_vertex;  // null: the item index is the vertex
+    uint32_t* heavy_vertex;       // per slot
     uint32_t* nheavy;
     __device__ void operator()(uint64_t i, uint64_t excl, uint32_t cnt) const {
-        for (uint32_t p = 0; p < cnt; ++p) {
-            t_item[excl + p] = (uint32_t)i;
-            t_part[excl + p] = p;
-        }
+        if (!cnt) return;
+        const uint32_t v = item_vertex ? item_vertex[i] : (uint32_t)i;
         uint32_t slot = kNoSlot;
         if (cnt > 1) {
             slot = atomicAdd(nheavy, 1u);
-            heavy_item[slot] = (uint32_t)i;
+            heavy_vertex[slot] = v;
         }
-        heavy_slot[i] = slot;
+        const uint64_t b = begin[i], e = begin[i + 1];
+        for (uint32_t p = 0; p < cnt; ++p) {
+            const uint64_t e0 = b + (uint64_t)p * kTaskEdges;
+            const uint32_t len = (uint32_t)(e - e0 < kTaskEdges ? e - e0 : kTaskEdges);
+            rec[excl + p] = make_uint4((uint32_t)e0, (uint32_t)(e0 >> 32) | (len << 8), v, slot);
+        }
     }
 };
+__device__ __forceinline__ uint64_t task_begin(const uint4& t) { return ((uint64_t)(t.y & 0xFFu) << 32) | t.x; }
+__device__ __forceinline__ uint32_t task_len(const uint4& t) { return t.y >> 8; }
 
 struct RowTasks {
-    DevBuf item, part, heavy_slot, heavy_item, counts;
+    DevBuf rec, heavy_vertex, counts;
     uint64_t ntasks = 0;
     uint32_t nheavy = 0;
-    uint64_t nitems = 0;
-    const uint64_t* begin = nullptr;
 };
 
-static int make_tasks(eg_graph* g, RowTasks& t, const uint64_t* begin, uint64_t nitems) {
-    // upper bound on tasks: items + E / kTaskEdges
-    const uint64_t cap = nitems + g->E / kTaskEdges + 2;
-    EG_TRY(t.item.reserve(sizeof(uint32_t) * cap));
-    EG_TRY(t.part.reserve(sizeof(uint32_t) * cap));
-    EG_TRY(t.heavy_slot.reserve(sizeof(uint32_t) * (nitems + 1)));
-    EG_TRY(t.heavy_item.reserve(sizeof(uint32_t) * (g->E / kTaskEdges + 2)));
+static int make_tasks(eg_graph* g, RowTasks& t, const uint64_t* begin, uint64_t nitems, const uint32_t* item_vertex) {
+    // upper bound on tasks: non-empty items + E / kTaskEdges
+    const uint64_t cap = std::min<uint64_t>(nitems, g->E) + g->E / kTaskEdges + 2;
+    EG_TRY(t.rec.reserve(sizeof(uint4) * cap));
+    EG_TRY(t.heavy_vertex.reserve(sizeof(uint32_t) * (g->E / kTaskEdges + 2)));
     EG_TRY(t.counts.reserve(32));
     EG_CUDA(cudaMemsetAsync(t.counts.ptr, 0, 32, g->stream));
     uint64_t* d_total = t.counts.as<uint64_t>();
     uint32_t* d_nheavy = reinterpret_cast<uint32_t*>(t.counts.as<uint64_t>() + 1);
-    TaskEpi ep{t.item.as<uint32_t>(), t.part.as<uint32_t>(), t.heavy_slot.as<uint32_t>(), t.heavy_item.as<uint32_t>(),
-               d_nheavy};
+    TaskEpi ep{t.rec.as<uint4>(), begin, item_vertex, t.heavy_vertex.as<uint32_t>(), d_nheavy};
     EG_TRY(launch_scan(g, TaskLoad{begin}, ep, nitems, d_total, "row_tasks"));
     uint64_t h[2] = {0, 0};
     EG_CUDA(cudaMemcpyAsync(h, t.counts.ptr, 16, cudaMemcpyDeviceToHost, g->stream));
     EG_CUDA(cudaStreamSynchronize(g->stream));
     t.ntasks = nitems ? h[0] : 0;
     t.nheavy = (uint32_t)(h[1] & 0xFFFFFFFFu);
-    t.nitems = nitems;
-    t.begin = begin;
     return EG_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
-// row kernels: warp per task, lane l owns columns 2l, 2l+1 of a 64-column row (float2)
+// row kernels: one warp per task, 64-column rows of 256 bytes
 struct RowArgs {
-    const uint32_t* t_item;
-    const uint32_t* t_part;
+    const uint4* rec;
     uint64_t ntasks;
-    const uint32_t* heavy_slot;
-    const uint32_t* item_vertex;  // null: item index is the vertex
-    const uint64_t* begin;        // list offsets per item (item i: [begin[i], begin[i+1]))
     const uint32_t* adj;
     const float* w;               // per-edge weight (normalised for PPR, raw for SSSP)
 };
 
-// PPR forward: y[v] = (1-a) * sum_{u in in(v)} wn_uv * x[u]
-// rows gathered together per warp in the row sweeps (independent 256-byte loads in flight).  The
-// PPR adjoint at 2^22/2^26, K = 50: 717 ms one row at a time, 650 ms at 4, 575 ms at 8, 616 ms at 16
-// (78 registers); the forward 176 ms at 4, 174 ms at 8
-constexpr int kRowGather = 8;
+// The PPR sweeps read a 256-byte row per edge: one warp per task, the two half-warps take alternate
+// edges, lane c of a half owns columns 4c..4c+3 (one 16-byte load per row and lane).  A step is
+// 2 * kRowPairs edges: their ids and weights are loaded one edge per lane, while the previous step's
+// rows are reduced, and handed round by shuffles.
+// Both sweeps are bound by the row gathers (256 E bytes a sweep, mostly out of L2).  Rows are asked
+// to stay in L2 (half of them evict-last), ids, weights and results pass through evict-first.
+// 1 M vertices, 16 M edges: the forward sweep 0.61 ms with one 8-byte column pair per lane and
+// default caching, 0.66 ms with half-warp rows alone, 0.64 streaming ids and results, 0.53 ms with
+// the rows kept as well (7.8 TB/s of rows); the adjoint sweep 1.05 -> 0.76 ms.  8 rows per half-warp
+// at 4 CTAs per SM (64 registers): 4 rows 0.56, 16 rows 0.81 ms.
+constexpr int kRowPairs = 8;
+constexpr uint32_t kRowStep = 2 * kRowPairs;
 
-__global__ void __launch_bounds__(256) k_row_spmm(RowArgs a, const float2* __restrict__ x, float2* __restrict__ y,
-                                                   float2* __restrict__ heavy_acc, float scale) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ float4 half_sum(float4 v) {  // the two half-warps' partial rows
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+    v.z += __shfl_xor_sync(0xffffffffu, v.z, 16);
+    v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
+    return v;
+}
+
+// a task's finished row: stored, or added to its list's accumulator when the list has several tasks
+__device__ __forceinline__ void row_out(const uint4& rec, float4 acc, uint32_t lane, float4* __restrict__ y,
+                                        float4* __restrict__ heavy_acc, float scale) {
+    acc = half_sum(acc);
+    if (lane >= 16) return;
+    if (rec.w == kNoSlot)
+        __stcs(y + (uint64_t)rec.z * 16 + lane, make_float4(scale * acc.x, scale * acc.y, scale * acc.z, scale * acc.w));
+    else
+        atomicAdd(heavy_acc + (uint64_t)rec.w * 16 + lane, acc);
+}
+
+// PPR forward: y[v] = (1-a) * sum_{u in in(v)} wn_uv * x[u]
+__global__ void __launch_bounds__(256, 4) k_row_spmm(RowArgs a, const float4* __restrict__ x, float4* __restrict__ y,
+                                                  float4* __restrict__ heavy_acc, float scale) {
+    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t t = warp; t < a.ntasks; t += nwarps) {
-        const uint32_t it = a.t_item[t];
-        const uint64_t lb = a.begin[it], le = a.begin[it + 1];
-        const uint64_t e0 = lb + (uint64_t)a.t_part[t] * kTaskEdges;
-        const uint64_t e1 = e0 + kTaskEdges < le ? e0 + kTaskEdges : le;
-        float2 acc = make_float2(0.f, 0.f);
-        uint64_t e = e0;
-        for (; e + kRowGather <= e1; e += kRowGather) {
-            uint32_t u[kRowGather];
-            float wv[kRowGather];
+    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
+    for (; t < a.ntasks; t += nwarps) {
+        const uint4 rec = nxt;
+        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
+        const uint64_t e0 = task_begin(rec);
+        const uint32_t n = task_len(rec);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t u = lane < n ? __ldcs(a.adj + e0 + lane) : 0u;
+        float w = lane < n ? __ldcs(a.w + e0 + lane) : 0.f;
+        for (uint32_t eb = 0; eb < n; eb += 32) {
+            const uint32_t k = eb + 32 + lane;
+            const uint32_t u2 = k < n ? __ldcs(a.adj + e0 + k) : 0u;
+            const float w2 = k < n ? __ldcs(a.w + e0 + k) : 0.f;
+            const uint32_t left = n - eb < 32 ? n - eb : 32;
+            for (uint32_t s = 0; s < left; s += kRowStep) {
+                float4 r[kRowPairs];
+                float wj[kRowPairs];
 #pragma unroll
-            for (int j = 0; j < kRowGather; ++j) {
-                u[j] = __ldg(a.adj + e + j);
-                wv[j] = __ldg(a.w + e + j);
+                for (int j = 0; j < kRowPairs; ++j) {
+                    const uint32_t i = s + 2 * j + half;
+                    const uint32_t uj = __shfl_sync(0xffffffffu, u, i & 31);
+                    wj[j] = __shfl_sync(0xffffffffu, w, i & 31);
+                    r[j] = i < left ? ld_keep(x + (uint64_t)uj * 16 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < kRowPairs; ++j) {
+                    acc.x = fmaf(wj[j], r[j].x, acc.x);
+                    acc.y = fmaf(wj[j], r[j].y, acc.y);
+                    acc.z = fmaf(wj[j], r[j].z, acc.z);
+                    acc.w = fmaf(wj[j], r[j].w, acc.w);
+                }
             }
-            float2 r[kRowGather];
-#pragma unroll
-            for (int j = 0; j < kRowGather; ++j) r[j] = __ldcg(x + (uint64_t)u[j] * 32 + lane);
-#pragma unroll
-            for (int j = 0; j < kRowGather; ++j) {
-                acc.x = fmaf(wv[j], r[j].x, acc.x);
-                acc.y = fmaf(wv[j], r[j].y, acc.y);
-            }
+            u = u2;
+            w = w2;
         }
-        for (; e < e1; ++e) {
-            const uint32_t u = __ldg(a.adj + e);
-            const float wv = __ldg(a.w + e);
-            const float2 r = __ldcg(x + (uint64_t)u * 32 + lane);
-            acc.x = fmaf(wv, r.x, acc.x);
-            acc.y = fmaf(wv, r.y, acc.y);
-        }
-        const uint32_t v = a.item_vertex ? a.item_vertex[it] : it;
-        const uint32_t slot = a.heavy_slot[it];
-        if (slot == kNoSlot) {
-            y[(uint64_t)v * 32 + lane] = make_float2(scale * acc.x, scale * acc.y);
-        } else {
-            atomicAdd(&heavy_acc[(uint64_t)slot * 32 + lane].x, acc.x);
-            atomicAdd(&heavy_acc[(uint64_t)slot * 32 + lane].y, acc.y);
-        }
+        row_out(rec, acc, lane, y, heavy_acc, scale);
     }
 }
 
-__global__ void k_row_heavy_finish(const uint32_t* __restrict__ heavy_item, const uint32_t* __restrict__ item_vertex,
-                                   uint32_t nheavy, float2* __restrict__ heavy_acc, float2* __restrict__ y, float scale) {
+__global__ void k_row_heavy_finish(const uint32_t* __restrict__ heavy_vertex, uint32_t nheavy,
+                                   float4* __restrict__ heavy_acc, float4* __restrict__ y, float scale) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t slot = i >> 5;
-    const int lane = threadIdx.x & 31;
+    const uint64_t slot = i >> 4;
+    const uint32_t c = threadIdx.x & 15;
     if (slot >= nheavy) return;
-    const uint32_t it = heavy_item[slot];
-    const uint32_t v = item_vertex ? item_vertex[it] : it;
-    const float2 a = heavy_acc[slot * 32 + lane];
-    heavy_acc[slot * 32 + lane] = make_float2(0.f, 0.f);
-    y[(uint64_t)v * 32 + lane] = make_float2(scale * a.x, scale * a.y);
+    const uint32_t v = heavy_vertex[slot];
+    const float4 a = heavy_acc[slot * 16 + c];
+    heavy_acc[slot * 16 + c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    y[(uint64_t)v * 16 + c] = make_float4(scale * a.x, scale * a.y, scale * a.z, scale * a.w);
 }
 
 // y[seed_s][s] += a
@@ -538,71 +560,77 @@ __global__ void k_row_of(const uint64_t* __restrict__ off, uint32_t V, uint32_t*
 // ---- adjoint sweep over the CSR: for a source row u,
 //   lam_out[u] = (1-a) * sum_{v in out(u)} wn_uv * lam_in[v]
 //   gA[e]     += (1-a) * <x_k[u], lam_in[v]>      (per CSR edge e = (u, v))
-__global__ void __launch_bounds__(256) k_row_adjoint(RowArgs a, const float2* __restrict__ lam_in,
-                                                      const float2* __restrict__ xk, float2* __restrict__ lam_out,
-                                                      float2* __restrict__ heavy_acc, float* __restrict__ gA,
-                                                      float scale) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+// One step's dot products <x_k[u], lam[v]>, kRowPairs per half-warp, are summed over its 16 lanes by
+// halving: at each stage a lane hands half of its partial sums to its partner and keeps the other
+// half, so eight products take 8 shuffles (one at a time: 32); lanes with an even c end up with one
+// product each, in the order of dot_slot.
+__device__ __forceinline__ float dot_scatter(float (&d)[kRowPairs], uint32_t c) {
+    static_assert(kRowPairs == 8, "the three halving stages below leave one product of eight per lane pair");
+#pragma unroll
+    for (int o = 8, m = 4; o >= 2; o >>= 1, m >>= 1) {
+        const bool up = (c & o) != 0;
+#pragma unroll
+        for (int j = 0; j < m; ++j) {
+            const float give = up ? d[j] : d[j + m], keep = up ? d[j + m] : d[j];
+            d[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+}
+__device__ __forceinline__ uint32_t dot_slot(uint32_t c) { return c >> 1; }  // which of the eight lane c holds
+
+__global__ void __launch_bounds__(256, 4) k_row_adjoint(RowArgs a, const float4* __restrict__ lam_in,
+                                                     const float4* __restrict__ xk, float4* __restrict__ lam_out,
+                                                     float4* __restrict__ heavy_acc, float* __restrict__ gA,
+                                                     float scale) {
+    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t t = warp; t < a.ntasks; t += nwarps) {
-        const uint32_t u = a.t_item[t];  // CSR items are vertices
-        const uint64_t lb = a.begin[u], le = a.begin[u + 1];
-        const uint64_t e0 = lb + (uint64_t)a.t_part[t] * kTaskEdges;
-        const uint64_t e1 = e0 + kTaskEdges < le ? e0 + kTaskEdges : le;
-        const float2 xu = __ldcg(xk + (uint64_t)u * 32 + lane);
-        float2 acc = make_float2(0.f, 0.f);
-        uint64_t e = e0;
-        // kRowGather edges at a time: their rows are gathered together (as in k_row_spmm), and the
-        // first kRowGather lanes hold their gA entries; each dot product is summed over the warp
-        // in the same order as for a single edge, so the result does not depend on the grouping
-        for (; e + kRowGather <= e1; e += kRowGather) {
-            uint32_t v[kRowGather];
-            float wv[kRowGather];
+    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
+    for (; t < a.ntasks; t += nwarps) {
+        const uint4 rec = nxt;  // the task's vertex is the source u
+        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
+        const uint64_t e0 = task_begin(rec);
+        const uint32_t n = task_len(rec);
+        const float4 xu = __ldcg(xk + (uint64_t)rec.z * 16 + c);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t v = lane < n ? __ldcs(a.adj + e0 + lane) : 0u;
+        float w = lane < n ? __ldcs(a.w + e0 + lane) : 0.f;
+        for (uint32_t eb = 0; eb < n; eb += 32) {
+            const uint32_t k = eb + 32 + lane;
+            const uint32_t v2 = k < n ? __ldcs(a.adj + e0 + k) : 0u;
+            const float w2 = k < n ? __ldcs(a.w + e0 + k) : 0.f;
+            const uint32_t left = n - eb < 32 ? n - eb : 32;
+            for (uint32_t s = 0; s < left; s += kRowStep) {
+                // the edge whose product this lane will hold, and its gA entry
+                const uint32_t mine = s + 2 * dot_slot(c) + half;
+                const bool have = !(c & 1) && mine < left;
+                float* g = gA + e0 + eb + mine;
+                const float g_old = have ? *g : 0.f;
+                float4 l[kRowPairs];
+                float wj[kRowPairs], d[kRowPairs];
 #pragma unroll
-            for (int j = 0; j < kRowGather; ++j) {
-                v[j] = __ldg(a.adj + e + j);
-                wv[j] = __ldg(a.w + e + j);
+                for (int j = 0; j < kRowPairs; ++j) {
+                    const uint32_t i = s + 2 * j + half;
+                    const uint32_t vj = __shfl_sync(0xffffffffu, v, i & 31);
+                    wj[j] = __shfl_sync(0xffffffffu, w, i & 31);
+                    l[j] = i < left ? ld_keep(lam_in + (uint64_t)vj * 16 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int j = 0; j < kRowPairs; ++j) {
+                    acc.x = fmaf(wj[j], l[j].x, acc.x);
+                    acc.y = fmaf(wj[j], l[j].y, acc.y);
+                    acc.z = fmaf(wj[j], l[j].z, acc.z);
+                    acc.w = fmaf(wj[j], l[j].w, acc.w);
+                    d[j] = fmaf(xu.x, l[j].x, xu.y * l[j].y) + fmaf(xu.z, l[j].z, xu.w * l[j].w);
+                }
+                const float dot = dot_scatter(d, c);
+                if (have) *g = fmaf(scale, dot, g_old);
             }
-            const float g_old = lane < kRowGather ? gA[e + lane] : 0.f;
-            float2 l[kRowGather];
-#pragma unroll
-            for (int j = 0; j < kRowGather; ++j) l[j] = __ldcg(lam_in + (uint64_t)v[j] * 32 + lane);
-            float d[kRowGather];
-#pragma unroll
-            for (int j = 0; j < kRowGather; ++j) {
-                acc.x = fmaf(wv[j], l[j].x, acc.x);
-                acc.y = fmaf(wv[j], l[j].y, acc.y);
-                d[j] = fmaf(xu.x, l[j].x, xu.y * l[j].y);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                for (int j = 0; j < kRowGather; ++j) d[j] += __shfl_xor_sync(0xffffffffu, d[j], o);
-            }
-            float dl = d[0];
-#pragma unroll
-            for (int j = 1; j < kRowGather; ++j) dl = lane == j ? d[j] : dl;
-            if (lane < kRowGather) gA[e + lane] = fmaf(scale, dl, g_old);
+            v = v2;
+            w = w2;
         }
-        for (; e < e1; ++e) {
-            const uint32_t v = __ldg(a.adj + e);
-            const float wv = __ldg(a.w + e);
-            const float2 l = __ldcg(lam_in + (uint64_t)v * 32 + lane);
-            acc.x = fmaf(wv, l.x, acc.x);
-            acc.y = fmaf(wv, l.y, acc.y);
-            float d = fmaf(xu.x, l.x, xu.y * l.y);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (lane == 0) gA[e] = fmaf(scale, d, gA[e]);
-        }
-        const uint32_t slot = a.heavy_slot[u];
-        if (slot == kNoSlot) {
-            lam_out[(uint64_t)u * 32 + lane] = make_float2(scale * acc.x, scale * acc.y);
-        } else {
-            atomicAdd(&heavy_acc[(uint64_t)slot * 32 + lane].x, acc.x);
-            atomicAdd(&heavy_acc[(uint64_t)slot * 32 + lane].y, acc.y);
-        }
+        row_out(rec, acc, lane, lam_out, heavy_acc, scale);
     }
 }
 
@@ -620,70 +648,107 @@ __global__ void k_weight_grad(const uint64_t* __restrict__ off, uint32_t V, cons
     }
 }
 
-// lam_K = dL/dx_K given in [V][64]; nothing else to seed
 // ---- batched SSSP: in place, skipping sources whose row did not change in the last sweep --------
-__global__ void __launch_bounds__(256) k_row_sssp(RowArgs a, float2* __restrict__ dist,
-                                                   const uint8_t* __restrict__ changed_prev,
-                                                   uint8_t* __restrict__ changed_next, int* __restrict__ any) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+// One warp per task; the two half-warps take alternate edges and lane c of a half owns columns
+// 4c..4c+3 (one 16-byte load of a 256-byte row).  The sweep is bound by the latency of the chain
+// record -> ids -> changed bits -> rows, so the next task's record is loaded one task ahead, the
+// destination's row together with the ids, and up to kSsspRows rows are in flight per warp; sources
+// that did not change (one bit each, cached in L1: the bits do not change during a sweep) are
+// squeezed out first, their ids and weights queueing up in shared memory, so the row loads stay full
+// when few sources are active.  A destination with a single task is written by this warp alone and
+// stored plainly; cut lists (and items of several partitions that share a vertex) take the minimum
+// with atomics.  64 graphs of 1k-500k vertices, 93 M edges, 64 sources, 24 sweeps: 107 ms with one
+// row per warp load, byte flags and separate item / offset arrays, 47 ms so (10.8 E row gathers:
+// 5.5 TB/s); 6 CTAs per SM with 8 rows (40 registers) take 47.0 ms, 4 with 16 rows 47.5, 5 with 8
+// rows 52, 3 with 16 rows 53, 2 with 32 rows 72.
+constexpr int kSsspRows = 8;
+
+__global__ void __launch_bounds__(256, 6) k_row_sssp(RowArgs a, float4* __restrict__ dist,
+                                                  const uint32_t* __restrict__ changed_prev,
+                                                  uint32_t* __restrict__ changed_next, int shared_vertex,
+                                                  int* __restrict__ any) {
+    __shared__ uint2 s_act[8][64];
+    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
+    uint2* act = s_act[threadIdx.x >> 5];
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t t = warp; t < a.ntasks; t += nwarps) {
-        const uint32_t it = a.t_item[t];
-        const uint64_t lb = a.begin[it], le = a.begin[it + 1];
-        const uint64_t e0 = lb + (uint64_t)a.t_part[t] * kTaskEdges;
-        const uint64_t e1 = e0 + kTaskEdges < le ? e0 + kTaskEdges : le;
-        float2 best = make_float2(1e9f, 1e9f);
-        // 32 in-edges per step: ids, weights and "source changed" flags are loaded one per lane,
-        // then the rows of the changed sources are gathered four at a time (min is exact, so the
-        // order does not matter)
-        for (uint64_t eb = e0; eb < e1; eb += 32) {
-            const uint64_t e = eb + lane;
+    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
+    bool any_lowered = false;
+    for (; t < a.ntasks; t += nwarps) {
+        const uint4 rec = nxt;
+        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
+        const uint64_t e0 = task_begin(rec);
+        const uint32_t n = task_len(rec), v = rec.z;
+        const float4 dv = __ldcg(dist + (uint64_t)v * 16 + c);
+        float4 best = make_float4(1e9f, 1e9f, 1e9f, 1e9f);
+        uint32_t queued = 0;  // active sources waiting in act (the same in every lane)
+        for (uint32_t eb = 0; eb < n; eb += 32) {
+            const uint32_t k = eb + lane;
             uint32_t u = 0;
-            float wv = 0.f;
             bool ch = false;
-            if (e < e1) {
-                u = __ldg(a.adj + e);
-                wv = __ldg(a.w + e);
-                ch = __ldcg(changed_prev + u) != 0;
+            if (k < n) {
+                u = __ldg(a.adj + e0 + k);
+                ch = (__ldg(changed_prev + (u >> 5)) >> (u & 31)) & 1u;
             }
-            unsigned m = __ballot_sync(0xffffffffu, ch);
-            while (m) {  // m is the same in every lane
-                int sl[4];
+            const unsigned m = __ballot_sync(0xffffffffu, ch);
+            if (ch) {
+                act[queued + __popc(m & ((1u << lane) - 1u))] =
+                    make_uint2(u, __float_as_uint(__ldg(a.w + e0 + k)));
+            }
+            queued += __popc(m);
+            if (queued <= 32 && eb + 32 < n) continue;  // room for another 32
+            __syncwarp();
+            for (uint32_t b = 0; b < queued; b += kSsspRows) {
+                float4 r[kSsspRows / 2];
+                float w[kSsspRows / 2];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sl[j] = m ? __ffs(m) - 1 : -1;
-                    if (m) m &= m - 1;
-                }
-                float2 r[4];
-                float wj[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (sl[j] >= 0) {
-                        const uint32_t uj = __shfl_sync(0xffffffffu, u, sl[j]);
-                        wj[j] = __shfl_sync(0xffffffffu, wv, sl[j]);
-                        r[j] = __ldcg(dist + (uint64_t)uj * 32 + lane);
+                for (int j = 0; j < kSsspRows / 2; ++j) {
+                    const uint32_t i = b + 2 * j + half;
+                    if (i < queued) {
+                        const uint2 x = act[i];
+                        w[j] = __uint_as_float(x.y);
+                        r[j] = __ldcg(dist + (uint64_t)x.x * 16 + c);
+                    } else {
+                        w[j] = 0.f;
+                        r[j] = make_float4(1e9f, 1e9f, 1e9f, 1e9f);
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (sl[j] >= 0) {
-                        best.x = fminf(best.x, r[j].x + wj[j]);  // toolkits/sssp.cpp:55: relax_dist = msg + w
-                        best.y = fminf(best.y, r[j].y + wj[j]);
-                    }
+                for (int j = 0; j < kSsspRows / 2; ++j) {  // toolkits/sssp.cpp:55: relax_dist = msg + w
+                    best.x = fminf(best.x, r[j].x + w[j]);
+                    best.y = fminf(best.y, r[j].y + w[j]);
+                    best.z = fminf(best.z, r[j].z + w[j]);
+                    best.w = fminf(best.w, r[j].w + w[j]);
                 }
+            }
+            queued = 0;
+            __syncwarp();
+        }
+        best.x = fminf(best.x, __shfl_xor_sync(0xffffffffu, best.x, 16));
+        best.y = fminf(best.y, __shfl_xor_sync(0xffffffffu, best.y, 16));
+        best.z = fminf(best.z, __shfl_xor_sync(0xffffffffu, best.z, 16));
+        best.w = fminf(best.w, __shfl_xor_sync(0xffffffffu, best.w, 16));
+        bool lowered = best.x < dv.x || best.y < dv.y || best.z < dv.z || best.w < dv.w;
+        if (half == 0 && lowered) {
+            float4* row = dist + (uint64_t)v * 16 + c;
+            if (rec.w == kNoSlot && !shared_vertex) {
+                __stcg(row, make_float4(fminf(best.x, dv.x), fminf(best.y, dv.y), fminf(best.z, dv.z),
+                                        fminf(best.w, dv.w)));
+            } else {
+                int* p = reinterpret_cast<int*>(row);  // distances are >= 0: ordered like their bits
+                lowered = false;
+                if (best.x < dv.x) lowered |= best.x < __int_as_float(atomicMin(p, __float_as_int(best.x)));
+                if (best.y < dv.y) lowered |= best.y < __int_as_float(atomicMin(p + 1, __float_as_int(best.y)));
+                if (best.z < dv.z) lowered |= best.z < __int_as_float(atomicMin(p + 2, __float_as_int(best.z)));
+                if (best.w < dv.w) lowered |= best.w < __int_as_float(atomicMin(p + 3, __float_as_int(best.w)));
             }
         }
-        const uint32_t v = a.item_vertex[it];
-        float2* dv = dist + (uint64_t)v * 32 + lane;
-        bool lowered = false;
-        if (best.x < __ldcg(&dv->x)) lowered |= best.x < __int_as_float(atomicMin(reinterpret_cast<int*>(&dv->x), __float_as_int(best.x)));
-        if (best.y < __ldcg(&dv->y)) lowered |= best.y < __int_as_float(atomicMin(reinterpret_cast<int*>(&dv->y), __float_as_int(best.y)));
-        if (__any_sync(0xffffffffu, lowered) && lane == 0) {
-            changed_next[v] = 1;
-            *any = 1;
+        if (__any_sync(0xffffffffu, lowered && half == 0)) {
+            if (lane == 0) atomicOr(changed_next + (v >> 5), 1u << (v & 31));
+            any_lowered = true;
         }
     }
+    if (any_lowered && lane == 0) *any = 1;
 }
 
 __global__ void k_fill_f32_rows(float* p, uint64_t n, float v) {
@@ -717,6 +782,7 @@ struct BatchState {
     DevBuf persist;  // persistent traversal: per-level counts, barrier words, error flag
     DevBuf wr0, wr1;  // frontier words in renumbered order (pull gathers through renumbered sources)
     RowTasks csc_tasks, csr_tasks;
+    unsigned spmm_grid = 0;
     bool csc_ready = false, csr_ready = false;
     // captured MS-BFS level loop and the shapes it was captured for
     void* graph_exec = nullptr;
@@ -1446,29 +1512,26 @@ static int ensure_tasks(eg_graph* g, bool csr) {
     BatchState& b = bstate(g);
     if (csr) {
         if (!b.csr_ready) {
-            EG_TRY(make_tasks(g, b.csr_tasks, g->csr_off.as<uint64_t>(), g->V));
+            EG_TRY(make_tasks(g, b.csr_tasks, g->csr_off.as<uint64_t>(), g->V, nullptr));
             b.csr_ready = true;
         }
     } else if (!b.csc_ready) {
-        EG_TRY(make_tasks(g, b.csc_tasks, g->cidx.as<uint64_t>(), g->ncompressed - 1));
+        EG_TRY(make_tasks(g, b.csc_tasks, g->cidx.as<uint64_t>(), g->ncompressed - 1, g->cvert.as<uint32_t>()));
         b.csc_ready = true;
     }
     return EG_OK;
 }
 
-static unsigned row_grid(eg_graph* g) { return (unsigned)g->num_sms * 8u; }
+// resident CTAs of 256 threads of a row kernel over the whole GPU: its warps take tasks by stride
+static int resident_grid(eg_graph* g, const void* fn, unsigned* grid) {
+    int per_sm = 0;
+    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
+    *grid = (unsigned)g->num_sms * (unsigned)std::max(per_sm, 1);
+    return EG_OK;
+}
 
-static RowArgs row_args(const RowTasks& t, const uint32_t* item_vertex, const uint32_t* adj, const float* w) {
-    RowArgs a;
-    a.t_item = t.item.as<uint32_t>();
-    a.t_part = t.part.as<uint32_t>();
-    a.ntasks = t.ntasks;
-    a.heavy_slot = t.heavy_slot.as<uint32_t>();
-    a.item_vertex = item_vertex;
-    a.begin = t.begin;
-    a.adj = adj;
-    a.w = w;
-    return a;
+static RowArgs row_args(const RowTasks& t, const uint32_t* adj, const float* w) {
+    return RowArgs{t.rec.as<uint4>(), t.ntasks, adj, w};
 }
 
 // weights in CSR and CSC order, row-normalised by the source's out-weight sum
@@ -1503,15 +1566,14 @@ static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
     const uint64_t V = g->V;
     const RowTasks& t = b.csc_tasks;
     EG_CUDA(cudaMemsetAsync(y, 0, 256 * V, g->stream));
-    RowArgs a = row_args(t, g->cvert.as<uint32_t>(), g->csc_adj.as<uint32_t>(), b.wn_csc.as<float>());
+    RowArgs a = row_args(t, g->csc_adj.as<uint32_t>(), b.wn_csc.as<float>());
     Timed tm(&g->prof, g->stream, "ppr_spmm");
-    k_row_spmm<<<row_grid(g), 256, 0, g->stream>>>(a, reinterpret_cast<const float2*>(x), reinterpret_cast<float2*>(y),
-                                                  b.heavy.as<float2>(), 1.0f - alpha);
+    k_row_spmm<<<b.spmm_grid, 256, 0, g->stream>>>(a, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y),
+                                                  b.heavy.as<float4>(), 1.0f - alpha);
     EG_CHECK_LAUNCH("k_row_spmm");
     if (t.nheavy) {
-        k_row_heavy_finish<<<(unsigned)((t.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
-            t.heavy_item.as<uint32_t>(), g->cvert.as<uint32_t>(), t.nheavy, b.heavy.as<float2>(),
-            reinterpret_cast<float2*>(y), 1.0f - alpha);
+        k_row_heavy_finish<<<(unsigned)((t.nheavy * 16ull + 255) / 256), 256, 0, g->stream>>>(
+            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<float4>(), reinterpret_cast<float4*>(y), 1.0f - alpha);
         EG_CHECK_LAUNCH("k_row_heavy_finish");
     }
     k_ppr_teleport<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, y, alpha);
@@ -1544,6 +1606,7 @@ static int ppr_common(eg_graph* g, const float* w_in, const uint32_t* seeds, int
     EG_CUDA(cudaMemsetAsync(b.heavy.ptr, 0, b.heavy.bytes, g->stream));
     EG_TRY(b.rows0.reserve(256 * V + 256));
     EG_TRY(b.rows1.reserve(256 * V + 256));
+    EG_TRY(resident_grid(g, (const void*)k_row_spmm, &b.spmm_grid));
     return prepare_ppr_weights(g, wd);
 }
 
@@ -1702,7 +1765,9 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     }
     EG_CUDA(cudaMemsetAsync(b.gA.ptr, 0, 4 * E, g->stream));
     const RowTasks& tr = b.csr_tasks;
-    RowArgs ar = row_args(tr, nullptr, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
+    unsigned adjoint_grid = 0;
+    EG_TRY(resident_grid(g, (const void*)k_row_adjoint, &adjoint_grid));
+    RowArgs ar = row_args(tr, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
     float* seg = b.seg.as<float>();
     for (int cp = (K - 1) / C; cp >= 0 && K > 0; --cp) {
         const int k0 = cp * C, k1 = std::min(K, k0 + C);
@@ -1715,14 +1780,14 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
             EG_CUDA(cudaMemsetAsync(lam2, 0, row, g->stream));
             {
                 Timed tm(&g->prof, g->stream, "ppr_adjoint");
-                k_row_adjoint<<<row_grid(g), 256, 0, g->stream>>>(
-                    ar, reinterpret_cast<const float2*>(lam), reinterpret_cast<const float2*>(seg + (size_t)(k - k0) * 64 * V),
-                    reinterpret_cast<float2*>(lam2), b.heavy.as<float2>(), b.gA.as<float>(), 1.0f - alpha);
+                k_row_adjoint<<<adjoint_grid, 256, 0, g->stream>>>(
+                    ar, reinterpret_cast<const float4*>(lam), reinterpret_cast<const float4*>(seg + (size_t)(k - k0) * 64 * V),
+                    reinterpret_cast<float4*>(lam2), b.heavy.as<float4>(), b.gA.as<float>(), 1.0f - alpha);
                 EG_CHECK_LAUNCH("k_row_adjoint");
             }
             if (tr.nheavy) {
-                k_row_heavy_finish<<<(unsigned)((tr.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
-                    tr.heavy_item.as<uint32_t>(), nullptr, tr.nheavy, b.heavy.as<float2>(), reinterpret_cast<float2*>(lam2),
+                k_row_heavy_finish<<<(unsigned)((tr.nheavy * 16ull + 255) / 256), 256, 0, g->stream>>>(
+                    tr.heavy_vertex.as<uint32_t>(), tr.nheavy, b.heavy.as<float4>(), reinterpret_cast<float4*>(lam2),
                     1.0f - alpha);
                 EG_CHECK_LAUNCH("k_row_heavy_finish");
             }
@@ -1746,10 +1811,10 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-__global__ void k_sssp_init_entries(const uint2* ent, uint32_t n, float* dist, uint8_t* changed) {
+__global__ void k_sssp_init_entries(const uint2* ent, uint32_t n, float* dist, uint32_t* changed) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         dist[(uint64_t)ent[i].x * 64 + ent[i].y] = 0.f;
-        changed[ent[i].x] = 1;
+        atomicOr(changed + (ent[i].x >> 5), 1u << (ent[i].x & 31));
     }
 }
 
@@ -1759,29 +1824,33 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
     BatchState& b = bstate(g);
     const uint64_t V = g->V;
     EG_TRY(b.rows0.reserve(256 * V + 256));
-    EG_TRY(b.ch0.reserve(V + 64));
-    EG_TRY(b.ch1.reserve(V + 64));
+    const size_t ch_bytes = 4 * (V / 32 + 1);  // one bit per vertex: changed in the last sweep
+    EG_TRY(b.ch0.reserve(ch_bytes));
+    EG_TRY(b.ch1.reserve(ch_bytes));
     EG_TRY(b.flag.reserve(16));
     float* dist = b.rows0.as<float>();
     {
         Timed t(&g->prof, g->stream, "sssp_batch_init");
         k_fill_f32_rows<<<grid_for(64 * V, 256, 152u * 16u), 256, 0, g->stream>>>(dist, 64 * V, 1e9f);
         EG_CHECK_LAUNCH("k_fill_f32_rows");
-        EG_CUDA(cudaMemsetAsync(b.ch0.ptr, 0, V, g->stream));
+        EG_CUDA(cudaMemsetAsync(b.ch0.ptr, 0, ch_bytes, g->stream));
         k_sssp_init_entries<<<std::max(1u, std::min<unsigned>((n_entries + 255) / 256, 4096u)), 256, 0, g->stream>>>(
-            b.entries.as<uint2>(), n_entries, dist, b.ch0.as<uint8_t>());
+            b.entries.as<uint2>(), n_entries, dist, b.ch0.as<uint32_t>());
         EG_CHECK_LAUNCH("k_sssp_init_entries");
     }
-    RowArgs a = row_args(b.csc_tasks, g->cvert.as<uint32_t>(), g->csc_adj.as<uint32_t>(), g->csc_w.as<float>());
-    uint8_t* prev = b.ch0.as<uint8_t>();
-    uint8_t* nxt = b.ch1.as<uint8_t>();
+    unsigned grid = 0;
+    EG_TRY(resident_grid(g, (const void*)k_row_sssp, &grid));
+    RowArgs a = row_args(b.csc_tasks, g->csc_adj.as<uint32_t>(), g->csc_w.as<float>());
+    uint32_t* prev = b.ch0.as<uint32_t>();
+    uint32_t* nxt = b.ch1.as<uint32_t>();
     int sweeps = 0;
     while (true) {
-        EG_CUDA(cudaMemsetAsync(nxt, 0, V, g->stream));
+        EG_CUDA(cudaMemsetAsync(nxt, 0, ch_bytes, g->stream));
         EG_CUDA(cudaMemsetAsync(b.flag.ptr, 0, 4, g->stream));
         {
             Timed t(&g->prof, g->stream, "sssp_batch_sweep");
-            k_row_sssp<<<row_grid(g), 256, 0, g->stream>>>(a, reinterpret_cast<float2*>(dist), prev, nxt, b.flag.as<int>());
+            k_row_sssp<<<grid, 256, 0, g->stream>>>(a, reinterpret_cast<float4*>(dist), prev, nxt,
+                                                          g->partitions > 1, b.flag.as<int>());
             EG_CHECK_LAUNCH("k_row_sssp");
         }
         ++sweeps;

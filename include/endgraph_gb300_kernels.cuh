@@ -52,6 +52,13 @@ __device__ __forceinline__ unsigned long long ld_keep(const unsigned long long* 
     asm volatile("ld.global.cg.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(a), "l"(l2_keep_policy()));
     return v;
 }
+__device__ __forceinline__ float4 ld_keep(const float4* a) {
+    float4 v;
+    asm volatile("ld.global.cg.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(a), "l"(l2_keep_policy()));
+    return v;
+}
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;

@@ -1,0 +1,89 @@
+"""GPU: the 64-column row engine (batched SSSP, personalised PageRank and its adjoint) on lists whose
+lengths sit at the edges of its blocking: rows gathered together, edges per warp step, edges per
+task, and lists cut into several tasks."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 40, 63, 64, 65, 96, 511, 512, 513, 1024, 1025, 3000]
+
+
+def _fans(seed, V=4096):
+    """Destination i < len(LENGTHS) has LENGTHS[i] in-edges and source 1000 + i as many out-edges;
+    a random sparse graph connects the rest.  Vertices from 4000 on have no edges at all."""
+    rng = np.random.default_rng(seed)
+    src, dst = [], []
+    for i, n in enumerate(LENGTHS):
+        src += [rng.integers(100, 4000, n), np.full(n, 1000 + i)]
+        dst += [np.full(n, i), rng.integers(0, 4000, n)]
+    src.append(rng.integers(0, 4000, 6000))
+    dst.append(rng.integers(0, 4000, 6000))
+    src, dst = (np.concatenate(x).astype(np.uint32) for x in (src, dst))
+    p = rng.permutation(len(src))
+    return src[p], dst[p], V
+
+
+@pytest.mark.parametrize("P", [1, 2])
+@pytest.mark.parametrize("n", [1, 5, 64])
+def test_sssp_batch_list_lengths(eg_lib, P, n):
+    import endgraph_gb300 as eg
+    src, dst, V = _fans(n)
+    w = np.random.default_rng(n + 1).random(len(src)).astype(np.float32)
+    csr = oracle.build_csr(src, dst, w, V, np.array([0, V], np.uint32))
+    sources = np.concatenate([[1000 + len(LENGTHS) - 1, 4050], src[:62]]).astype(np.uint32)[:n]
+    with eg.Graph(partitions=P) as g:
+        g.load_directed(eg.pack_edges(src, dst, w), V)
+        dist = g.sssp_batch(sources)
+    for s in range(n):
+        ref = oracle.sssp(csr["off"][0], csr["adj"], csr["w"], V, int(sources[s]))
+        assert np.array_equal(dist[s].view(np.uint32), ref.view(np.uint32)), s
+
+
+def _ppr64(src, dst, w, V, seeds, alpha, K):
+    """K unrolled iterations in FP64, differentiable in w (torch, CPU)."""
+    import torch
+    s, d = torch.from_numpy(src.astype(np.int64)), torch.from_numpy(dst.astype(np.int64))
+    a = w / torch.zeros(V, dtype=torch.float64).index_add(0, s, w)[s]
+    e = torch.zeros((V, len(seeds)), dtype=torch.float64)
+    e[torch.from_numpy(seeds.astype(np.int64)), torch.arange(len(seeds))] = 1.0
+    x = e
+    for _ in range(K):
+        x = alpha * e + (1 - alpha) * torch.zeros_like(x).index_add(0, d, a[:, None] * x[s])
+    return x.t()
+
+
+@pytest.mark.parametrize("n,K", [(2, 1), (2, 2), (7, 5), (64, 9)])
+def test_ppr_and_adjoint_list_lengths(eg_lib, n, K):
+    """Seeds include a vertex without in-edges, one without any edges, and the longest lists; the
+    tolerances are those of the other FP64 comparisons of these operators: 1e-6 (relative L1) for
+    the scores, 1e-4 (relative L2) for the gradient."""
+    import torch
+
+    import endgraph_gb300 as eg
+    src, dst, V = _fans(n + K)
+    no_in = np.setdiff1d(src, dst)
+    assert len(no_in)
+    seeds = np.concatenate([[no_in[0], 4050, len(LENGTHS) - 1, 1000 + len(LENGTHS) - 1], src[:60]]).astype(np.uint32)[:n]
+    rng = np.random.default_rng(K)
+    w = rng.uniform(0.5, 1.5, len(src)).astype(np.float32)
+    tgt = rng.random((n, V)).astype(np.float32) / V
+    alpha = 0.15
+    with eg.Graph() as g:
+        g.load_directed_with_ids(eg.pack_edges(src, dst), V)
+        for _ in range(2):  # a second call reuses the buffers
+            x = g.ppr(w, seeds, alpha, K)
+            dw = g.ppr_backward(w, seeds, 2 * (x - tgt), alpha, K)
+        other = np.roll(seeds, 1) if n > 2 else seeds[::-1].copy()  # other seeds on the same buffers
+        x2 = g.ppr(w, other, alpha, K)
+        dw2 = g.ppr_backward(w, other, 2 * (x2 - tgt), alpha, K)
+    for sd, xg, dg in ((seeds, x, dw), (other, x2, dw2)):
+        wt = torch.tensor(w, dtype=torch.float64, requires_grad=True)
+        ref = _ppr64(src, dst, wt, V, sd, alpha, K)
+        ref.backward(torch.from_numpy((2 * (xg - tgt)).astype(np.float64)))
+        r = ref.detach().numpy()
+        assert np.abs(xg - r).sum() / np.abs(r).sum() <= 1e-6
+        gr = wt.grad.numpy()
+        assert np.linalg.norm(dg - gr) / np.linalg.norm(gr) <= 1e-4
