@@ -524,24 +524,75 @@ __global__ void k_row_heavy_finish(const uint32_t* __restrict__ heavy_vertex, ui
     y[(uint64_t)v * 16 + c] = make_float4(scale * a.x, scale * a.y, scale * a.z, scale * a.w);
 }
 
-// y[seed_s][s] += a
-__global__ void k_ppr_teleport(const uint32_t* seeds, int n, float* y, float alpha) {
+// y[seed_s][s] = (the sweep's value, 0 for a seed without in-edges) + a: the sweeps write only rows
+// with in-edges, so that a row without them keeps what the buffer held
+__global__ void k_ppr_teleport(const uint32_t* seeds, int n, const uint32_t* __restrict__ indeg, float* y, float alpha) {
     const int s = threadIdx.x;
-    if (s < n) atomicAdd(y + (uint64_t)seeds[s] * 64 + s, alpha);
+    if (s >= n) return;
+    const uint32_t v = seeds[s];
+    float* p = y + (uint64_t)v * 64 + s;
+    *p = (indeg[v] ? *p : 0.f) + alpha;
 }
 __global__ void k_ppr_init(const uint32_t* seeds, int n, float* x) {
     const int s = threadIdx.x;
     if (s < n) x[(uint64_t)seeds[s] * 64 + s] = 1.0f;
 }
-
-// normalised weights: wn[e] = w[eid[e]] / s[src], s[u] = sum of u's out-weights
-__global__ void k_out_weight_sums(const uint64_t* __restrict__ csr_off, const float* __restrict__ csr_eid,
-                                  const float* __restrict__ w_in, uint32_t V, float* __restrict__ s) {
-    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < V; u += (uint64_t)gridDim.x * blockDim.x) {
-        double acc = 0;
-        for (uint64_t e = csr_off[u]; e < csr_off[u + 1]; ++e) acc += w_in[__float_as_uint(csr_eid[e])];
-        s[u] = (float)acc;
+// zero the rows that no sweep writes (deg = 0) in nbuf consecutive row arrays
+__global__ void __launch_bounds__(256) k_zero_rows(const uint32_t* __restrict__ deg, uint64_t V, float4* __restrict__ rows,
+                                                   int nbuf) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V * 16; i += stride) {
+        if (deg[i >> 4]) continue;
+        for (int b = 0; b < nbuf; ++b) __stcs(rows + (uint64_t)b * V * 16 + i, make_float4(0.f, 0.f, 0.f, 0.f));
     }
+}
+
+__device__ __forceinline__ double warp_sum_f64(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Row normalisation and its gradient: one warp per CSR task (<= 512 edges of one source), so that a
+// hub's list is spread over warps.  A list of one task is finished by its warp; of a longer one the
+// FP64 partial sums meet in heavy[slot] and its tasks are finished by a second pass (heavy = 1).
+// Bound by the random 4-byte reads of the input-ordered weights; one thread per source took 10.5 ms
+// for 1 M sources and 16 M edges (a hub's list in one thread), a warp per task 0.3 ms.
+//
+// s[u] = sum of u's out-weights; wn[e] = w[eid[e]] / s[u] (null: not wanted)
+__global__ void __launch_bounds__(256) k_out_weights(const uint4* __restrict__ tasks, uint64_t ntasks,
+                                                     const float* __restrict__ eid, const float* __restrict__ w_in,
+                                                     float* __restrict__ s, float* __restrict__ wn,
+                                                     double* __restrict__ heavy, int finish_heavy) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
+        const uint4 rec = __ldg(tasks + t);
+        if (finish_heavy && rec.w == kNoSlot) continue;
+        const uint64_t e0 = task_begin(rec);
+        const uint32_t n = task_len(rec);
+        float sum;
+        if (finish_heavy) {
+            sum = s[rec.z];
+        } else {
+            double acc = 0;
+            for (uint32_t k = lane; k < n; k += 32) acc += w_in[__float_as_uint(__ldg(eid + e0 + k))];
+            acc = warp_sum_f64(acc);
+            sum = (float)acc;
+            if (lane == 0) {
+                if (rec.w == kNoSlot) s[rec.z] = sum;
+                else atomicAdd(heavy + rec.w, acc);
+            }
+            if (rec.w != kNoSlot) continue;
+        }
+        if (wn)
+            for (uint32_t k = lane; k < n; k += 32) wn[e0 + k] = w_in[__float_as_uint(__ldg(eid + e0 + k))] / sum;
+    }
+}
+__global__ void k_heavy_out_sums(const uint32_t* __restrict__ heavy_vertex, uint32_t nheavy,
+                                 const double* __restrict__ heavy, float* __restrict__ s) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nheavy) s[heavy_vertex[i]] = (float)heavy[i];
 }
 __global__ void k_gather_norm_w(const uint32_t* __restrict__ nbr_is_src, const float* __restrict__ eid,
                                 const float* __restrict__ w_in, const float* __restrict__ s, uint64_t E,
@@ -550,11 +601,6 @@ __global__ void k_gather_norm_w(const uint32_t* __restrict__ nbr_is_src, const f
         const uint32_t id = __float_as_uint(eid[e]);
         wn[e] = w_in[id] / s[nbr_is_src[e]];
     }
-}
-// CSR positions: the source of position e is the row it sits in
-__global__ void k_row_of(const uint64_t* __restrict__ off, uint32_t V, uint32_t* __restrict__ row) {
-    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < V; u += (uint64_t)gridDim.x * blockDim.x)
-        for (uint64_t e = off[u]; e < off[u + 1]; ++e) row[e] = (uint32_t)u;
 }
 
 // ---- adjoint sweep over the CSR: for a source row u,
@@ -635,16 +681,32 @@ __global__ void __launch_bounds__(256, 4) k_row_adjoint(RowArgs a, const float4*
 }
 
 // dL/dw_e = (gA_e - sum_{e' in row(u)} wn_e' gA_e') / s_u, scattered to the input edge order
-__global__ void k_weight_grad(const uint64_t* __restrict__ off, uint32_t V, const float* __restrict__ wn,
-                              const float* __restrict__ gA, const float* __restrict__ s,
-                              const float* __restrict__ eid, float* __restrict__ dw) {
-    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < V; u += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = off[u], e1 = off[u + 1];
-        if (b == e1) continue;
+__global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ tasks, uint64_t ntasks,
+                                                     const float* __restrict__ wn, const float* __restrict__ gA,
+                                                     const float* __restrict__ s, const float* __restrict__ eid,
+                                                     float* __restrict__ dw, double* __restrict__ heavy,
+                                                     int finish_heavy) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
+        const uint4 rec = __ldg(tasks + t);
+        if (finish_heavy && rec.w == kNoSlot) continue;
+        const uint64_t e0 = task_begin(rec);
+        const uint32_t n = task_len(rec);
         double dot = 0;
-        for (uint64_t e = b; e < e1; ++e) dot += (double)wn[e] * gA[e];
-        const float inv = 1.0f / s[u];
-        for (uint64_t e = b; e < e1; ++e) dw[__float_as_uint(eid[e])] = (float)(((double)gA[e] - dot) * inv);
+        if (finish_heavy) {
+            dot = heavy[rec.w];
+        } else {
+            for (uint32_t k = lane; k < n; k += 32) dot += (double)wn[e0 + k] * gA[e0 + k];
+            dot = warp_sum_f64(dot);
+            if (rec.w != kNoSlot) {
+                if (lane == 0) atomicAdd(heavy + rec.w, dot);
+                continue;
+            }
+        }
+        const float inv = 1.0f / s[rec.z];
+        for (uint32_t k = lane; k < n; k += 32)
+            dw[__float_as_uint(__ldg(eid + e0 + k))] = (float)(((double)gA[e0 + k] - dot) * inv);
     }
 }
 
@@ -776,13 +838,14 @@ int expand_with_ids(eg_graph* g, const uint8_t* rec8_dev, uint64_t E) {
 
 // ---------------------------------------------------------------------------------------------
 struct BatchState {
-    DevBuf a64, b64, c64, lev, rows0, rows1, heavy, tmp_out, seeds, wn_csc, wn_csr, s_out, gA, row_of, ck, seg;
+    DevBuf a64, b64, c64, lev, rows0, rows1, heavy, tmp_out, seeds, wn_csc, wn_csr, s_out, gA, heavy_sum, ck, seg;
     DevBuf ch0, ch1, flag, level_cnt, entries, n_entries, bm0, bm1, alive, ms_seg;
     DevBuf cap;      // captured level loop: per-level direction decisions and frontier edge counts
     DevBuf persist;  // persistent traversal: per-level counts, barrier words, error flag
     DevBuf wr0, wr1;  // frontier words in renumbered order (pull gathers through renumbered sources)
     RowTasks csc_tasks, csr_tasks;
     unsigned spmm_grid = 0;
+    size_t device_bytes = 0;  // the GPU's memory
     bool csc_ready = false, csr_ready = false;
     // captured MS-BFS level loop and the shapes it was captured for
     void* graph_exec = nullptr;
@@ -1534,38 +1597,46 @@ static RowArgs row_args(const RowTasks& t, const uint32_t* adj, const float* w) 
     return RowArgs{t.rec.as<uint4>(), t.ntasks, adj, w};
 }
 
-// weights in CSR and CSC order, row-normalised by the source's out-weight sum
-static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev) {
+// weights in CSC order (and, for the adjoint, in CSR order), row-normalised by the source's out-weight sum
+static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev, bool want_csr) {
     BatchState& b = bstate(g);
     const uint64_t E = g->E, V = g->V;
+    const RowTasks& t = b.csr_tasks;
     EG_TRY(b.wn_csc.reserve(4 * E + 64));
-    EG_TRY(b.wn_csr.reserve(4 * E + 64));
+    if (want_csr) EG_TRY(b.wn_csr.reserve(4 * E + 64));
     EG_TRY(b.s_out.reserve(4 * V + 64));
-    EG_TRY(b.row_of.reserve(4 * E + 64));
-    const unsigned gv = grid_for(V, 256, 152u * 16u), ge = grid_for(E, 256, 152u * 16u);
-    Timed t(&g->prof, g->stream, "ppr_weights");
-    k_out_weight_sums<<<gv, 256, 0, g->stream>>>(g->csr_off.as<uint64_t>(), g->csr_w.as<float>(), w_in_dev, (uint32_t)V,
-                                                 b.s_out.as<float>());
-    EG_CHECK_LAUNCH("k_out_weight_sums");
+    EG_TRY(b.heavy_sum.reserve(8ull * t.nheavy + 64));
+    const unsigned grid = (unsigned)g->num_sms * 8u;
+    const float* eid = g->csr_w.as<float>();
+    float* wn = want_csr ? b.wn_csr.as<float>() : nullptr;
+    Timed tm(&g->prof, g->stream, "ppr_weights");
+    if (t.nheavy) EG_CUDA(cudaMemsetAsync(b.heavy_sum.ptr, 0, 8ull * t.nheavy, g->stream));
+    if (g->partitions > 1) EG_CUDA(cudaMemsetAsync(b.s_out.ptr, 0, 4 * V, g->stream));  // sources without a task
+    k_out_weights<<<grid, 256, 0, g->stream>>>(t.rec.as<uint4>(), t.ntasks, eid, w_in_dev, b.s_out.as<float>(), wn,
+                                               b.heavy_sum.as<double>(), 0);
+    EG_CHECK_LAUNCH("k_out_weights");
+    if (t.nheavy) {
+        k_heavy_out_sums<<<(t.nheavy + 255) / 256, 256, 0, g->stream>>>(
+            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy_sum.as<double>(), b.s_out.as<float>());
+        EG_CHECK_LAUNCH("k_heavy_out_sums");
+        if (wn) {
+            k_out_weights<<<grid, 256, 0, g->stream>>>(t.rec.as<uint4>(), t.ntasks, eid, w_in_dev, b.s_out.as<float>(),
+                                                       wn, nullptr, 1);
+            EG_CHECK_LAUNCH("k_out_weights");
+        }
+    }
     // CSC: the neighbour is the source
-    k_gather_norm_w<<<ge, 256, 0, g->stream>>>(g->csc_adj.as<uint32_t>(), g->csc_w.as<float>(), w_in_dev,
-                                               b.s_out.as<float>(), E, b.wn_csc.as<float>());
-    EG_CHECK_LAUNCH("k_gather_norm_w");
-    // CSR: the source is the row
-    k_row_of<<<gv, 256, 0, g->stream>>>(g->csr_off.as<uint64_t>(), (uint32_t)V, b.row_of.as<uint32_t>());
-    EG_CHECK_LAUNCH("k_row_of");
-    k_gather_norm_w<<<ge, 256, 0, g->stream>>>(b.row_of.as<uint32_t>(), g->csr_w.as<float>(), w_in_dev,
-                                               b.s_out.as<float>(), E, b.wn_csr.as<float>());
+    k_gather_norm_w<<<grid_for(E, 256, 152u * 16u), 256, 0, g->stream>>>(
+        g->csc_adj.as<uint32_t>(), g->csc_w.as<float>(), w_in_dev, b.s_out.as<float>(), E, b.wn_csc.as<float>());
     EG_CHECK_LAUNCH("k_gather_norm_w");
     return EG_OK;
 }
 
-// one forward step: y = a*e + (1-a) A^T x
+// one forward step: y = a*e + (1-a) A^T x.  Rows of y without in-edges are zero already (the caller
+// cleared them once), except the seeds' entries, which k_ppr_teleport sets.
 static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
     BatchState& b = bstate(g);
-    const uint64_t V = g->V;
     const RowTasks& t = b.csc_tasks;
-    EG_CUDA(cudaMemsetAsync(y, 0, 256 * V, g->stream));
     RowArgs a = row_args(t, g->csc_adj.as<uint32_t>(), b.wn_csc.as<float>());
     Timed tm(&g->prof, g->stream, "ppr_spmm");
     k_row_spmm<<<b.spmm_grid, 256, 0, g->stream>>>(a, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y),
@@ -1576,13 +1647,13 @@ static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
             t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<float4>(), reinterpret_cast<float4*>(y), 1.0f - alpha);
         EG_CHECK_LAUNCH("k_row_heavy_finish");
     }
-    k_ppr_teleport<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, y, alpha);
+    k_ppr_teleport<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, g->indeg.as<uint32_t>(), y, alpha);
     EG_CHECK_LAUNCH("k_ppr_teleport");
     return EG_OK;
 }
 
 static int ppr_common(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float alpha, int K, int where,
-                      const float** w_dev) {
+                      bool adjoint, const float** w_dev) {
     if (!g->built_csc || !g->built_csr) { set_error("eg_ppr: graph not built"); return EG_ERR_STATE; }
     if (!g->weighted || !g->edge_ids) {
         set_error("eg_ppr: load the graph with eg_load_directed_with_ids (per-edge ids select the weights)");
@@ -1607,7 +1678,7 @@ static int ppr_common(eg_graph* g, const float* w_in, const uint32_t* seeds, int
     EG_TRY(b.rows0.reserve(256 * V + 256));
     EG_TRY(b.rows1.reserve(256 * V + 256));
     EG_TRY(resident_grid(g, (const void*)k_row_spmm, &b.spmm_grid));
-    return prepare_ppr_weights(g, wd);
+    return prepare_ppr_weights(g, wd, adjoint);
 }
 
 // one seed: the scalar chunked pull (4-byte gathers of x[src] times the normalised weight)
@@ -1683,7 +1754,7 @@ static int run_ppr_single(eg_graph* g, uint32_t seed, float alpha, int K, float*
 
 int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float alpha, int K, float* out, int where) {
     const float* wd = nullptr;
-    EG_TRY(ppr_common(g, w_in, seeds, n, alpha, K, where, &wd));
+    EG_TRY(ppr_common(g, w_in, seeds, n, alpha, K, where, false, &wd));
     BatchState& b = bstate(g);
     const uint64_t V = g->V;
     if (n == 1 && g->partitions == 1) {
@@ -1695,6 +1766,7 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
     float* x = b.rows0.as<float>();
     float* y = b.rows1.as<float>();
     EG_CUDA(cudaMemsetAsync(x, 0, 256 * V, g->stream));
+    EG_CUDA(cudaMemsetAsync(y, 0, 256 * V, g->stream));
     k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, x);
     EG_CHECK_LAUNCH("k_ppr_init");
     for (int k = 0; k < K; ++k) {
@@ -1718,33 +1790,70 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
     return EG_OK;
 }
 
+// Checkpoint stride of the adjoint: the smallest one whose iterates fit an eighth of the GPU's memory
+// (all of x_0 .. x_{K-1} at stride 1, which recomputes nothing; else K / C checkpoints and a segment
+// of C), at most ceil(sqrt(K)).  1 M vertices, K = 50: stride 1 keeps 12.8 GB and runs 99 forward
+// sweeps in a forward and an adjoint, stride 8 keeps 4 GB and runs 143.
+static uint64_t ppr_rows_kept(int K, int C) { return C == 1 ? (uint64_t)K : (uint64_t)((K + C - 1) / C) + C; }
+static int ppr_stride(int K, uint64_t row, uint64_t budget) {
+    const int most = std::max(1, (int)ceil(sqrt((double)std::max(K, 1))));
+    int C = 1;
+    while (C < most && ppr_rows_kept(K, C) * row > budget) ++C;
+    return C;
+}
+
+static int zero_rows(eg_graph* g, const uint32_t* deg, float* rows, int nbuf) {
+    if (nbuf < 1) return EG_OK;
+    k_zero_rows<<<grid_for(16ull * g->V, 256, (unsigned)g->num_sms * 16u), 256, 0, g->stream>>>(
+        deg, g->V, reinterpret_cast<float4*>(rows), nbuf);
+    EG_CHECK_LAUNCH("k_zero_rows");
+    return EG_OK;
+}
+
 // adjoint of K forward steps from x_0 = e_seed; dL/dx_K given as [n][V]; dL/dw in input edge order
 int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float alpha, int K,
                      const float* dl_dx, float* dl_dw, int where) {
     const float* wd = nullptr;
-    EG_TRY(ppr_common(g, w_in, seeds, n, alpha, K, where, &wd));
+    EG_TRY(ppr_common(g, w_in, seeds, n, alpha, K, where, true, &wd));
     if (!dl_dx || !dl_dw) { set_error("eg_ppr_backward: need dL/dx and the dL/dw output"); return EG_ERR_INVALID; }
     BatchState& b = bstate(g);
     const uint64_t V = g->V, E = g->E, Ein = g->E_input;
-    const int C = std::max(1, (int)ceil(sqrt((double)std::max(K, 1))));  // checkpoint stride
-    const int ncp = K / C + 1;
     const size_t row = 256 * V;
-    EG_TRY(b.ck.reserve(row * ncp + 256));
-    EG_TRY(b.seg.reserve(row * (C + 1) + 256));
+    if (!b.device_bytes) {
+        size_t free_bytes = 0;
+        EG_CUDA(cudaMemGetInfo(&free_bytes, &b.device_bytes));
+    }
+    int C = ppr_stride(K, row, b.device_bytes / 8);
+    while (true) {
+        int st = b.ck.reserve(row * ((std::max(K, 1) + C - 1) / C) + 256);
+        if (st == EG_OK && C > 1) st = b.seg.reserve(row * C + 256);
+        if (st == EG_OK) break;
+        const int most = ppr_stride(K, row, 0);  // the GPU is fuller than that: the fewest rows
+        if (C == most) return st;
+        C = most;
+    }
     EG_TRY(b.gA.reserve(4 * E + 64));
-    // forward with checkpoints x_0, x_C, x_2C, ...
+    // forward with checkpoints x_0, x_C, x_2C, ... up to the last one before x_K
     float* ck = b.ck.as<float>();
+    float* seg = b.seg.as<float>();
+    const uint32_t* indeg = g->indeg.as<uint32_t>();
+    const uint32_t* outdeg = g->outdeg.as<uint32_t>();
     EG_CUDA(cudaMemsetAsync(ck, 0, row, g->stream));
     k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, ck);
     EG_CHECK_LAUNCH("k_ppr_init");
-    {
+    if (C == 1) {
+        EG_TRY(zero_rows(g, indeg, ck + 64 * V, K - 1));
+        for (int k = 0; k + 1 < K; ++k) EG_TRY(ppr_step(g, ck + 64 * V * k, ck + 64 * V * (k + 1), alpha, n));
+    } else {
+        EG_TRY(zero_rows(g, indeg, seg, C));
         float* x = b.rows0.as<float>();
         float* y = b.rows1.as<float>();
         EG_CUDA(cudaMemcpyAsync(x, ck, row, cudaMemcpyDeviceToDevice, g->stream));
-        for (int k = 0; k < K; ++k) {
+        EG_CUDA(cudaMemsetAsync(y, 0, row, g->stream));
+        for (int k = 0; k < (K - 1) / C * C; ++k) {
             EG_TRY(ppr_step(g, x, y, alpha, n));
             std::swap(x, y);
-            if ((k + 1) % C == 0 && (k + 1) / C < ncp)
+            if ((k + 1) % C == 0)
                 EG_CUDA(cudaMemcpyAsync(reinterpret_cast<char*>(ck) + row * ((k + 1) / C), x, row, cudaMemcpyDeviceToDevice,
                                         g->stream));
         }
@@ -1768,20 +1877,23 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     unsigned adjoint_grid = 0;
     EG_TRY(resident_grid(g, (const void*)k_row_adjoint, &adjoint_grid));
     RowArgs ar = row_args(tr, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
-    float* seg = b.seg.as<float>();
+    // the sweeps write only rows with out-edges; the others are zero from lambda_{K-1} on
+    EG_TRY(zero_rows(g, outdeg, lam2, 1));
     for (int cp = (K - 1) / C; cp >= 0 && K > 0; --cp) {
         const int k0 = cp * C, k1 = std::min(K, k0 + C);
-        // recompute x_k0 .. x_{k1-1} into the segment buffer
-        EG_CUDA(cudaMemcpyAsync(seg, reinterpret_cast<char*>(ck) + row * cp, row, cudaMemcpyDeviceToDevice, g->stream));
-        for (int k = k0 + 1; k < k1; ++k)
-            EG_TRY(ppr_step(g, seg + (size_t)(k - 1 - k0) * 64 * V, seg + (size_t)(k - k0) * 64 * V, alpha, n));
+        const float* xs = ck + 64 * V * cp;  // x_k0 .. x_{k1-1}
+        if (C > 1) {  // recomputed into the segment buffer
+            EG_CUDA(cudaMemcpyAsync(seg, xs, row, cudaMemcpyDeviceToDevice, g->stream));
+            for (int k = k0 + 1; k < k1; ++k)
+                EG_TRY(ppr_step(g, seg + (size_t)(k - 1 - k0) * 64 * V, seg + (size_t)(k - k0) * 64 * V, alpha, n));
+            xs = seg;
+        }
         for (int k = k1 - 1; k >= k0; --k) {
             // lam holds lambda_{k+1}; gA += (1-a) <x_k[u], lam[v]>; lam2 = (1-a) A lam
-            EG_CUDA(cudaMemsetAsync(lam2, 0, row, g->stream));
             {
                 Timed tm(&g->prof, g->stream, "ppr_adjoint");
                 k_row_adjoint<<<adjoint_grid, 256, 0, g->stream>>>(
-                    ar, reinterpret_cast<const float4*>(lam), reinterpret_cast<const float4*>(seg + (size_t)(k - k0) * 64 * V),
+                    ar, reinterpret_cast<const float4*>(lam), reinterpret_cast<const float4*>(xs + (size_t)(k - k0) * 64 * V),
                     reinterpret_cast<float4*>(lam2), b.heavy.as<float4>(), b.gA.as<float>(), 1.0f - alpha);
                 EG_CHECK_LAUNCH("k_row_adjoint");
             }
@@ -1791,6 +1903,7 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
                     1.0f - alpha);
                 EG_CHECK_LAUNCH("k_row_heavy_finish");
             }
+            if (k == K - 1) EG_TRY(zero_rows(g, outdeg, lam, 1));  // dL/dx_K itself is no longer needed
             std::swap(lam, lam2);
         }
     }
@@ -1800,11 +1913,18 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
         EG_TRY(b.tmp_out.reserve(4 * Ein + 64));
         dw = b.tmp_out.as<float>();
     }
-    EG_CUDA(cudaMemsetAsync(dw, 0, 4 * Ein, g->stream));
-    k_weight_grad<<<grid_for(V, 256, 152u * 16u), 256, 0, g->stream>>>(g->csr_off.as<uint64_t>(), (uint32_t)V,
-                                                                       b.wn_csr.as<float>(), b.gA.as<float>(),
-                                                                       b.s_out.as<float>(), g->csr_w.as<float>(), dw);
-    EG_CHECK_LAUNCH("k_weight_grad");
+    // every input edge sits in one CSR position; with several partitions only the first one's are tasks
+    if (g->partitions > 1) EG_CUDA(cudaMemsetAsync(dw, 0, 4 * Ein, g->stream));
+    if (tr.nheavy) EG_CUDA(cudaMemsetAsync(b.heavy_sum.ptr, 0, 8ull * tr.nheavy, g->stream));
+    {
+        Timed tm(&g->prof, g->stream, "ppr_weight_grad");
+        for (int heavy = 0; heavy <= (tr.nheavy ? 1 : 0); ++heavy) {
+            k_weight_grad<<<(unsigned)g->num_sms * 8u, 256, 0, g->stream>>>(
+                tr.rec.as<uint4>(), tr.ntasks, b.wn_csr.as<float>(), b.gA.as<float>(), b.s_out.as<float>(),
+                g->csr_w.as<float>(), dw, b.heavy_sum.as<double>(), heavy);
+            EG_CHECK_LAUNCH("k_weight_grad");
+        }
+    }
     if (where != EG_DEVICE) EG_CUDA(cudaMemcpyAsync(dl_dw, dw, 4 * Ein, cudaMemcpyDeviceToHost, g->stream));
     EG_CUDA(cudaStreamSynchronize(g->stream));
     return EG_OK;
