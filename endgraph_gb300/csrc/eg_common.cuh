@@ -117,6 +117,8 @@ struct EngineState {
     DevBuf pr_new_id;      // u32 per vertex: position in out-degree-class order (PageRank gathers)
     DevBuf pr_adj;         // u32 per CSC edge: the source renumbered through pr_new_id
     DevBuf pr_cnt, pr_off; // class counts per vertex tile and their exclusive scan
+    DevBuf pieces0, pieces1;  // {vertex, piece} queues of the persistent traversals (eg_persist.cu)
+    DevBuf persist;           // their state words
     uint64_t pull_nsplit = 0;
     uint64_t pull_nchunks = 0;
     bool pull_ready = false;
@@ -249,6 +251,7 @@ bool want_relabel(const eg_graph* g);
 int setup_relabel(eg_graph* g);
 int run_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
 int run_sssp(eg_graph* g, uint32_t root, float* dist, int where);
+int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where);
 int run_cc(eg_graph* g, uint32_t* label, int where);
 int run_msbfs(eg_graph* g, const uint32_t* roots, int n, uint8_t* levels, int where, uint64_t* edges);
 int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float alpha, int K, float* out, int where);

@@ -913,6 +913,8 @@ int run_sssp(eg_graph* g, uint32_t root, float* dist, int where) {
     if (!g->built_csr) { set_error("eg_sssp: CSR not built"); return EG_ERR_STATE; }
     if (!g->weighted) { set_error("eg_sssp: graph has no edge weights (load 12-byte records)"); return EG_ERR_STATE; }
     if (root >= g->V) { set_error("eg_sssp: root %u >= V %u", root, g->V); return EG_ERR_INVALID; }
+    // one partition: every step inside one persistent launch (its queues count pieces in 32 bits)
+    if (g->partitions == 1 && g->V < (1u << 31) && g->E < (1ull << 38)) return run_sssp_persistent(g, root, dist, where);
     EG_TRY(ensure_engine(g));
     const uint32_t V = g->V;
     EngineState& s = g->eng;

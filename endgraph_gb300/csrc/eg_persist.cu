@@ -1,0 +1,418 @@
+// eg_persist.cu — single-source traversals as one persistent cooperative launch: every level (or
+// near/far step) runs inside the kernel between bounded grid barriers, so that a step costs a barrier
+// instead of several launches and a host round trip.
+//
+// The frontier is a queue of list pieces {vertex, first edge, edges}, at most kPiece edges each, so
+// that a hub's list is spread over the GPU without a scan over the frontier.  Warps take pieces by
+// stride (piece i goes to warp i mod warps: the pieces of one hub lie next to each other in the
+// queue), up to 32 at a time, and walk their edges together: a warp prefix sum of the lengths, kIlp
+// edges per lane in flight.  Activated vertices are queued in shared memory and leave with one
+// reservation of the global queue per CTA and step (with one per warp, all meeting in one L2 word, and
+// with the lowered distance's old value awaited, an SSSP of 50,021 vertices and 800,017 edges took
+// 0.60 ms instead of 0.37, one of 2^22 and 2^26 5.6 instead of 3.8).  Per edge the walk is bound by
+// the latency of its gathers at 32 warps per SM (64 registers): 2 edges per lane in flight are 10-20 %
+// slower, 6 spill.
+#include <math.h>
+#include <string.h>
+
+#include <algorithm>
+
+#include "eg_pull.cuh"
+
+namespace eg {
+
+constexpr uint32_t kPiece = 256;          // edges per queue entry
+constexpr int kIlp = 4;
+constexpr int kPersistThreads = 1024;
+constexpr uint32_t kStepsPerLaunch = 4096;  // then the host launches again: a kernel always ends
+
+// what one step left behind, read by every CTA after the barrier that ends the step
+struct alignas(16) StepSlot {
+    uint32_t n;         // queue entries appended
+    uint32_t min_bits;  // SSSP split: smallest parked distance
+    uint32_t parked;    // SSSP split: vertices still parked
+    uint32_t pad;
+};
+
+struct PersistState {
+    unsigned bar_count, bar_gen;
+    int err;
+    uint32_t step;       // steps done so far
+    StepSlot slot[4];    // step k reads slot k & 3, fills slot (k + 1) & 3 and clears slot (k + 2) & 3
+    float thr, delta;    // SSSP near/far threshold and its step
+    float weight_sum;    // sampled weights
+    uint32_t done;
+    unsigned long long edges;  // edges of the pieces walked
+    uint32_t pushes, splits;
+};
+
+// one grid barrier; *out gets the slot the finished step filled.  False: a wait gave up.
+__device__ __forceinline__ bool step_barrier(PersistState* st, const StepSlot* slot, StepSlot* s_slot) {
+    if (!grid_sync_bounded(&st->bar_count, &st->bar_gen, &st->err)) return false;
+    if (threadIdx.x == 0) {
+        const uint4 x = __ldcg(reinterpret_cast<const uint4*>(slot));
+        *s_slot = StepSlot{x.x, x.y, x.z, x.w};
+    }
+    __syncthreads();
+    return true;
+}
+
+__device__ __forceinline__ uint32_t warp_incl(uint32_t x) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    return x;
+}
+
+// The CTA's share of the next queue: entries gather in shared memory and go out together (flush);
+// what does not fit goes to the global queue directly.
+constexpr uint32_t kLocalQueue = 2048;
+struct LocalQueue {
+    uint4 e[kLocalQueue];
+    uint32_t n;      // reserved
+    uint32_t valid;  // reservations from here on did not fit
+    uint32_t base;
+};
+
+__device__ __forceinline__ uint4 piece(uint32_t v, uint64_t beg, uint64_t end) {
+    const uint32_t len = (uint32_t)(end - beg < kPiece ? end - beg : kPiece);
+    return make_uint4(v, (uint32_t)beg, (uint32_t)(beg >> 32), len);
+}
+
+// every lane appends the pieces of its K vertices' lists [beg[j], end[j]) (empty: none)
+template <int K>
+__device__ __forceinline__ void append_pieces(LocalQueue& lq, const uint32_t (&v)[K], const uint64_t (&beg)[K],
+                                              const uint64_t (&end)[K], uint4* q_out, uint32_t* n_out) {
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int j = 0; j < K; ++j) cnt += (uint32_t)((end[j] - beg[j] + kPiece - 1) / kPiece);
+    if (!__any_sync(0xffffffffu, cnt != 0)) return;
+    const uint32_t incl = warp_incl(cnt);
+    uint32_t at = 0, direct = 0;
+    if ((threadIdx.x & 31) == 31) {
+        at = atomicAdd(&lq.n, incl);
+        direct = at + incl > kLocalQueue;
+        if (direct) {
+            atomicMin(&lq.valid, at);
+            at = atomicAdd(n_out, incl);
+        }
+    }
+    direct = __shfl_sync(0xffffffffu, direct, 31);
+    at = __shfl_sync(0xffffffffu, at, 31) + incl - cnt;
+    uint4* out = direct ? q_out : lq.e;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+        for (uint64_t b = beg[j]; b < end[j]; b += kPiece) out[at++] = piece(v[j], b, end[j]);
+}
+
+// by the whole CTA, before the barrier that ends the step
+__device__ __forceinline__ void flush_pieces(LocalQueue& lq, uint4* q_out, uint32_t* n_out) {
+    __syncthreads();
+    const uint32_t n = min(lq.n, lq.valid);
+    if (threadIdx.x == 0) lq.base = n ? atomicAdd(n_out, n) : 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) q_out[lq.base + i] = lq.e[i];
+    if (threadIdx.x == 0) {
+        lq.n = 0;
+        lq.valid = 0xFFFFFFFFu;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// SSSP (toolkits/sssp.cpp:52-64) with the near/far split of SsspOp: a lowered vertex below the
+// threshold joins the next queue (once per step: its stamp holds the step that queued it), one
+// above it is parked in the far bitmap.  When the queue runs empty a split step raises the
+// threshold and moves the parked vertices below it.  Every relaxation is an exact float add and a
+// minimum, so the fixpoint does not depend on the order.
+struct SsspPersistArgs {
+    uint64_t V, E, nwords;
+    const uint64_t* off;
+    const uint32_t* adj;
+    const float* w;
+    float* dist;
+    uint32_t* stamp;
+    unsigned long long* far_bm;
+    uint4* q[2];
+    uint32_t root;
+    float delta;        // > 0: given; 0: plain sweeps; < 0: -delta x the sampled mean weight
+    int resume;         // continue from the state an earlier launch left
+    PersistState* st;
+};
+
+constexpr uint32_t kWeightSamples = 65536;
+
+__global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPersistArgs a) {
+    __shared__ StepSlot s_slot;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    LocalQueue& lq = *reinterpret_cast<LocalQueue*>(s_raw);
+    if (threadIdx.x == 0) {
+        lq.n = 0;
+        lq.valid = 0xFFFFFFFFu;
+    }
+    PersistState* st = a.st;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t warp = (uint32_t)(tid >> 5), nwarps = (uint32_t)(stride >> 5);
+    unsigned long long my_edges = 0;
+    uint32_t step = 0, pushes = 0, splits = 0;
+    float thr, delta;
+    if (!a.resume) {
+        for (uint64_t v = tid; v < a.V; v += stride) {
+            a.dist[v] = v == a.root ? 0.f : 1e9f;
+            a.stamp[v] = 0u;
+        }
+        for (uint64_t i = tid; i < a.nwords; i += stride) a.far_bm[i] = 0ull;
+        if (a.delta < 0.f) {  // mean of a strided sample of the weights
+            const uint64_t every = max(a.E / kWeightSamples, (uint64_t)1);
+            float acc = 0.f;
+            for (uint64_t i = tid; i < kWeightSamples && i * every < a.E; i += stride) acc += a.w[i * every];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0 && acc != 0.f) atomicAdd(&st->weight_sum, acc);
+        }
+        if (tid < 32) {  // the root's pieces
+            const uint64_t b = a.off[a.root], z = a.off[(uint64_t)a.root + 1];
+            const uint32_t np = (uint32_t)((z - b + kPiece - 1) / kPiece);
+            for (uint32_t p = lane; p < np; p += 32) a.q[0][p] = piece(a.root, b + (uint64_t)p * kPiece, z);
+            if (lane == 0) st->slot[0].n = np;
+        }
+        if (!step_barrier(st, &st->slot[0], &s_slot)) return;
+        delta = a.delta;
+        if (delta < 0.f) {
+            const uint64_t every = max(a.E / kWeightSamples, (uint64_t)1);
+            const uint64_t taken = min((uint64_t)kWeightSamples, (a.E + every - 1) / every);
+            const float mean_w = taken ? __ldcg(&st->weight_sum) / (float)taken : 0.f;
+            delta = -delta * mean_w;
+        }
+        thr = delta > 0.f ? delta : INFINITY;
+    } else {
+        step = __ldcg(&st->step);
+        thr = __ldcg(&st->thr);
+        delta = __ldcg(&st->delta);
+        if (threadIdx.x == 0) s_slot = st->slot[step & 3];
+        __syncthreads();
+    }
+    const bool split = delta > 0.f;
+    const uint32_t first = step;
+    bool done = false;
+    uint32_t last_kind = 0;  // 0: push, 1: split
+    while (step - first < kStepsPerLaunch) {
+        const uint32_t n = s_slot.n;
+        StepSlot* out = &st->slot[(step + 1) & 3];
+        uint4* q_out = a.q[(step + 1) & 1];
+        const uint32_t mark = step + 1;
+        if (n == 0) {
+            if (!split || (last_kind == 1 && s_slot.parked == 0)) {
+                done = true;
+                break;
+            }
+            // after an empty split: jump to the nearest parked distance
+            const float from = last_kind == 1 ? fmaxf(thr, __uint_as_float(s_slot.min_bits)) : thr;
+            thr = from + delta > from ? from + delta : nextafterf(from, INFINITY);
+        }
+        __syncthreads();  // s_slot has been read
+        if (tid == 0) {
+            StepSlot* clear = &st->slot[(step + 2) & 3];
+            clear->n = 0;
+            clear->min_bits = 0x7F800000u;  // +inf
+            clear->parked = 0;
+        }
+        if (n) {
+            const uint4* q = a.q[step & 1];
+            for (uint32_t base = 0; base < n; base += 32 * nwarps) {
+                const uint64_t idx = (uint64_t)base + (uint64_t)lane * nwarps + warp;
+                uint64_t beg = 0;
+                uint32_t len = 0;
+                float du = 0.f;
+                if (idx < n) {
+                    const uint4 e = __ldcg(q + idx);
+                    du = __ldcg(a.dist + e.x);
+                    beg = ((uint64_t)e.z << 32) | e.y;
+                    len = e.w;
+                }
+                const uint32_t incl = warp_incl(len);
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                if (lane == 0) my_edges += total;
+                beg -= incl - len;  // rank r of the warp's edges sits at beg + r of its owner
+                for (uint32_t r0 = 0; r0 < total; r0 += 32 * kIlp) {
+                    uint32_t x[kIlp];
+                    float nd[kIlp];
+                    uint64_t lb[kIlp], le[kIlp];
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) {
+                        const uint32_t r = r0 + 32 * j + lane;
+                        uint32_t o = 0;  // the first lane whose inclusive prefix exceeds r
+#pragma unroll
+                        for (int b = 16; b > 0; b >>= 1) {
+                            const uint32_t p = __shfl_sync(0xffffffffu, incl, o + b - 1);
+                            if (p <= r) o += b;
+                        }
+                        const uint64_t pos = __shfl_sync(0xffffffffu, beg, o) + r;
+                        const float od = __shfl_sync(0xffffffffu, du, o);
+                        x[j] = r < total ? __ldg(a.adj + pos) : 0u;
+                        nd[j] = r < total ? od + __ldg(a.w + pos) : INFINITY;  // toolkits/sssp.cpp:55
+                    }
+                    float old[kIlp];
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) old[j] = __ldcg(a.dist + x[j]);
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) {
+                        lb[j] = le[j] = 0;
+                        if (nd[j] < old[j]) {
+                            // whoever lowers x further in this step passes the same test and queues x too,
+                            // so the minimum's old value is not needed
+                            atomicMin(reinterpret_cast<int*>(a.dist + x[j]), __float_as_int(nd[j]));
+                            const unsigned long long bit = 1ull << (x[j] & 63);
+                            unsigned long long* fw = a.far_bm + (x[j] >> 6);
+                            if (split && !(nd[j] < thr)) {
+                                if (!(__ldcg(fw) & bit)) atomicOr(fw, bit);
+                            } else {
+                                const uint32_t prev = atomicExch(a.stamp + x[j], mark);
+                                const uint64_t b = __ldg(a.off + x[j]), z = __ldg(a.off + (uint64_t)x[j] + 1);
+                                if (split && (__ldcg(fw) & bit)) atomicAnd(fw, ~bit);  // queued: no longer parked
+                                if (prev != mark) {
+                                    lb[j] = b;
+                                    le[j] = z;
+                                }
+                            }
+                        }
+                    }
+                    append_pieces<kIlp>(lq, x, lb, le, q_out, &out->n);
+                }
+            }
+            ++pushes;
+            last_kind = 0;
+        } else {
+            unsigned int mn = 0x7F800000u, left = 0;
+            for (uint64_t base = tid & ~31ull; base < a.nwords; base += stride) {
+                const uint64_t wi = base + lane;
+                const unsigned long long word = wi < a.nwords ? __ldcg(a.far_bm + wi) : 0ull;
+                unsigned long long move = 0;
+                for (unsigned long long x = word; x; x &= x - 1) {
+                    const int b = __ffsll((long long)x) - 1;
+                    const float d = __ldcg(a.dist + wi * 64 + b);
+                    if (d < thr) {
+                        move |= 1ull << b;
+                    } else {
+                        ++left;
+                        mn = min(mn, __float_as_uint(d));
+                    }
+                }
+                if (move) a.far_bm[wi] = word & ~move;
+                while (__any_sync(0xffffffffu, move != 0)) {
+                    const uint32_t v[1] = {move ? (uint32_t)(wi * 64 + (uint64_t)(__ffsll((long long)move) - 1)) : 0u};
+                    const uint64_t b[1] = {move ? __ldg(a.off + v[0]) : 0ull};
+                    const uint64_t z[1] = {move ? __ldg(a.off + (uint64_t)v[0] + 1) : 0ull};
+                    move &= move - 1;
+                    append_pieces<1>(lq, v, b, z, q_out, &out->n);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                left += __shfl_xor_sync(0xffffffffu, left, o);
+            }
+            if (lane == 0 && left) {
+                atomicMin(&out->min_bits, mn);
+                atomicAdd(&out->parked, left);
+            }
+            ++splits;
+            last_kind = 1;
+        }
+        ++step;
+        flush_pieces(lq, q_out, &out->n);
+        if (!step_barrier(st, out, &s_slot)) return;
+    }
+    if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
+    if (tid == 0) {  // every CTA leaves the loop at the same step
+        st->step = step;
+        st->thr = thr;
+        st->delta = delta;
+        st->done = done ? 1u : 0u;
+        st->pushes += pushes;
+        st->splits += splits;
+    }
+}
+
+// The automatic threshold step, in mean weights.  A step costs a barrier and some L2 round trips
+// (6.5 us) however few edges it relaxes, so graphs whose vertex arrays sit in L2 take steps so wide
+// that R-MAT distances need one or two phases; larger ones gain more from relaxing less.  Times in
+// ms with 0.7 / 3 / 100 x mean weight / mean degree: 20 k vertices, 300 k edges 1.14 / 0.51 / 0.28; 200 k,
+// 4 M 1.99 / 0.87 / 0.56; 1 M, 8 M 1.42 / 1.07 / 0.88; 2 M, 64 M 4.4 / 2.9 / 3.7; 4 M, 20 M 1.8 / 2.4 / 3.1; 4 M,
+// 67 M 3.8 / 3.8 / 5.4 (a tenth of the mean weight is 1.6 to 3.2 of these units there).
+static float auto_delta(uint64_t V, uint64_t E) {
+    const float deg = (float)std::max((double)E / (double)V, 1.0);
+    if (V <= (1u << 20)) return 100.f / deg;
+    if (V <= (1u << 23)) return 0.1f;
+    return 0.7f / deg;
+}
+
+// one CTA per this many edges, up to one per SM: fewer CTAs meet sooner at a barrier, but 2,048 was
+// no slower than 4,096 or 8,192 from 20 k edges on (0.134 / 0.142 / 0.159 ms at 2 k vertices, 20 k edges)
+constexpr uint64_t kEdgesPerCta = 2048;
+
+int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
+    const uint64_t V = g->V, E = g->E;
+    EngineState& s = g->eng;
+    EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
+    EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * (std::min(V, E) + E / kPiece + 64)));
+    EG_TRY(s.persist.reserve(sizeof(PersistState)));
+    float* d_dist = dist;
+    if (where != EG_DEVICE || !dist) {
+        EG_TRY(s.vals0.reserve(sizeof(float) * (V + 1)));
+        d_dist = s.vals0.as<float>();
+    }
+    SsspPersistArgs a;
+    a.V = V;
+    a.E = E;
+    a.nwords = V / 64 + 1;
+    a.off = g->csr_off.as<uint64_t>();
+    a.adj = g->csr_adj.as<uint32_t>();
+    a.w = g->csr_w.as<float>();
+    a.dist = d_dist;
+    a.stamp = s.vals1.as<uint32_t>();
+    a.far_bm = s.bm_visit.as<unsigned long long>();
+    a.q[0] = s.pieces0.as<uint4>();
+    a.q[1] = s.pieces1.as<uint4>();
+    a.root = root;
+    a.delta = g->sssp_delta >= 0 ? (float)((double)g->sssp_delta * 1e-6) : -auto_delta(V, E);
+    a.st = s.persist.as<PersistState>();
+    const size_t smem = sizeof(LocalQueue);
+    EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms, E / kEdgesPerCta));
+    static_assert(sizeof(PersistState) <= 256, "the state is read back through the 256-byte pinned block");
+    PersistState* h = reinterpret_cast<PersistState*>(s.host_words);
+    EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(PersistState), g->stream));
+    for (a.resume = 0;; a.resume = 1) {
+        void* kargs[] = {&a};
+        {
+            Timed t(&g->prof, g->stream, "sssp_persistent");
+            EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
+                                                g->stream));
+            EG_CHECK_LAUNCH("k_sssp_persistent");
+        }
+        EG_CUDA(cudaMemcpyAsync(h, a.st, sizeof(PersistState), cudaMemcpyDeviceToHost, g->stream));
+        EG_CUDA(cudaStreamSynchronize(g->stream));
+        if (h->err) {
+            set_error("eg_sssp: a bounded grid barrier gave up");
+            return EG_ERR_TIMEOUT;
+        }
+        if (h->done) break;
+    }
+    g->last_edges_processed = h->edges;
+    g->last_iterations = (int)h->pushes;
+    g->last_pushes = (int)h->pushes;
+    g->last_pulls = 0;
+    if (dist && where != EG_DEVICE) {
+        EG_CUDA(cudaMemcpyAsync(dist, d_dist, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
+        EG_CUDA(cudaStreamSynchronize(g->stream));
+    }
+    return EG_OK;
+}
+
+}  // namespace eg

@@ -194,7 +194,8 @@ enum {
     EG_OPT_BATCH_WIDTH = 5,        /* roots per bit-parallel pass of eg_bfs_many, 1..64 */
     EG_OPT_SSSP_DELTA = 6,         /* eg_sssp near/far step in millionths of a weight unit; 0 = plain
                                       Bellman-Ford sweeps (the reference's order), -1 = automatic
-                                      (0.7 x mean weight / mean out-degree; the default) */
+                                      (a fraction of the mean weight that depends on V and on the
+                                      mean out-degree; the default) */
     EG_OPT_PR_RELABEL = 7,         /* eg_pagerank gathers through a copy of the CSC source ids
                                       renumbered by out-degree class, high degrees first, so that
                                       the values most gathered share cache lines; the same values

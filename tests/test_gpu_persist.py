@@ -1,0 +1,64 @@
+"""GPU: the single-source traversals that run every step inside one persistent launch, on the shapes
+their queues and barriers are cut by: lists at the edges of a queue piece, hubs of many pieces,
+traversals deeper than one launch, and thresholds that a step cannot move."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _sssp_ref(src, dst, w, V, root):
+    csr = oracle.build_csr(src, dst, w, V, np.array([0, V], np.uint32))
+    return oracle.sssp(csr["off"][0], csr["adj"], csr["w"], V, root)
+
+
+def _check_sssp(src, dst, w, V, roots, deltas=(-1,)):
+    import endgraph_gb300 as eg
+    src, dst, w = src.astype(np.uint32), dst.astype(np.uint32), w.astype(np.float32)
+    refs = {r: _sssp_ref(src, dst, w, V, r) for r in roots}
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst, w), V)
+        for delta in deltas:
+            g.set_option(eg.EG_OPT_SSSP_DELTA, delta)
+            for r in roots:
+                d = g.sssp(r)
+                assert np.array_equal(d.view(np.uint32), refs[r].view(np.uint32)), (delta, r)
+
+
+@pytest.mark.parametrize("deg", [1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 8193, 70000])
+def test_sssp_piece_edges(eg_lib, deg):
+    """A root of `deg` out-edges whose neighbours fan out again, over a small random graph."""
+    V = 80_000
+    rng = np.random.default_rng(deg)
+    nbr = rng.choice(V - 1, deg, replace=False) + 1
+    src = np.concatenate([np.zeros(deg, np.int64), rng.integers(0, V, 200_000)])
+    dst = np.concatenate([nbr, rng.integers(0, V, 200_000)])
+    _check_sssp(src, dst, rng.random(len(src)), V, [0, int(nbr[0])], deltas=(-1, 0, 3000))
+
+
+def test_sssp_deeper_than_one_launch(eg_lib):
+    """A chain of 10,000 vertices: more steps than one launch makes; and a root without edges."""
+    n = 10_000
+    rng = np.random.default_rng(1)
+    perm = rng.permutation(n)
+    _check_sssp(perm[:-1], perm[1:], rng.random(n - 1), n + 1, [int(perm[0]), n], deltas=(-1, 0))
+
+
+def test_sssp_threshold_below_float_resolution(eg_lib):
+    """Distances so large that adding the threshold step changes nothing: phases still advance.
+    Zero weights, equal weights and weights of very different sizes."""
+    V = 3000
+    rng = np.random.default_rng(2)
+    src, dst = rng.integers(0, V, 20_000), rng.integers(0, V, 20_000)
+    w = rng.choice(np.array([0.0, 1e-6, 1.0, 3e7]), 20_000)
+    _check_sssp(src, dst, w, V, [int(src[0]), int(src[1])], deltas=(-1, 0, 1))
+
+
+@pytest.mark.parametrize("V,E", [(1, 1), (2, 5), (33, 64), (1025, 8191), (4097, 8193), (40_000, 1_300_000)])
+def test_sssp_grid_sizes(eg_lib, V, E):
+    """From one CTA to the whole GPU."""
+    rng = np.random.default_rng(V)
+    src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
+    _check_sssp(src, dst, rng.random(E), V, [int(src[0])], deltas=(-1, 0, 20_000))

@@ -87,3 +87,38 @@ def test_ppr_and_adjoint_list_lengths(eg_lib, n, K):
         assert np.abs(xg - r).sum() / np.abs(r).sum() <= 1e-6
         gr = wt.grad.numpy()
         assert np.linalg.norm(dg - gr) / np.linalg.norm(gr) <= 1e-4
+
+
+def test_ppr_adjoint_checkpoint_stride(eg_lib):
+    """Iterates that do not fit an eighth of the GPU's memory (80 of 512 MiB) are kept at a stride and
+    recomputed in between."""
+    import torch
+
+    import endgraph_gb300 as eg
+    V, E, n, K, alpha = 1 << 21, 1 << 20, 2, 80, 0.15
+    gen = torch.Generator("cuda").manual_seed(3)
+    # edges among the first 2^17 vertices only: in-lists and iterates that differ from one step to the next
+    rec = torch.randint(0, 1 << 17, (E, 2), generator=gen, device="cuda", dtype=torch.int32)
+    seeds = rec[:n, 0].cpu().numpy().astype(np.uint32)
+    w = torch.rand(E, generator=gen, device="cuda") + 0.5
+    dl = torch.rand((n, V), generator=gen, device="cuda")
+    with eg.Graph() as g:
+        g.load_directed_with_ids(rec, V)
+        dw = torch.empty(E, device="cuda")
+        g.ppr_backward(w, seeds, dl, alpha, K, dl_dw=dw)
+    s, d, wt = rec[:, 0].long(), rec[:, 1].long(), w.double()
+    tot = torch.zeros(V, dtype=torch.float64, device="cuda").index_add(0, s, wt)
+    a = wt / tot[s]
+    e = torch.zeros((V, n), dtype=torch.float64, device="cuda")
+    e[torch.from_numpy(seeds.astype(np.int64)).cuda(), torch.arange(n, device="cuda")] = 1.0
+    xs = [e]
+    for _ in range(K - 1):
+        xs.append(alpha * e + (1 - alpha) * torch.zeros_like(e).index_add(0, d, a[:, None] * xs[-1][s]))
+    lam = dl.double().t().contiguous()
+    ga = torch.zeros(E, dtype=torch.float64, device="cuda")
+    for k in range(K - 1, -1, -1):
+        ga += (1 - alpha) * (xs[k][s] * lam[d]).sum(1)
+        lam = (1 - alpha) * torch.zeros_like(lam).index_add(0, s, a[:, None] * lam[d])
+    dot = torch.zeros(V, dtype=torch.float64, device="cuda").index_add(0, s, a * ga)
+    ref = (ga - dot[s]) / tot[s]
+    assert float((dw.double() - ref).norm() / ref.norm()) <= 1e-4
