@@ -251,6 +251,7 @@ bool want_relabel(const eg_graph* g);
 int setup_relabel(eg_graph* g);
 int run_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
 int run_sssp(eg_graph* g, uint32_t root, float* dist, int where);
+int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
 int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where);
 int run_cc(eg_graph* g, uint32_t* label, int where);
 int run_msbfs(eg_graph* g, const uint32_t* roots, int n, uint8_t* levels, int where, uint64_t* edges);

@@ -775,6 +775,9 @@ int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int whe
 int run_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached) {
     if (!g->built_csr) { set_error("eg_bfs: CSR not built"); return EG_ERR_STATE; }
     if (root >= g->V) { set_error("eg_bfs: root %u >= V %u", root, g->V); return EG_ERR_INVALID; }
+    // one partition: every level inside one persistent launch (its queues count pieces in 32 bits)
+    if (g->partitions == 1 && g->V < (1u << 31) && g->E < (1ull << 38) && !(g->use_cuda_graph & 2))
+        return run_bfs_persistent(g, root, level, parent, where, reached);
     EG_TRY(ensure_engine(g));
     const uint32_t V = g->V;
     EngineState& s = g->eng;

@@ -23,7 +23,11 @@ namespace eg {
 
 constexpr uint32_t kPiece = 256;          // edges per queue entry
 constexpr int kIlp = 4;
-constexpr int kPersistThreads = 1024;
+// two CTAs of 512 threads at 64 registers: a BFS of 2^25 / 2^29 takes 1.61 ms (mean of 16 roots)
+// against 1.66 with one CTA of 1,024, 1.70 with three of 512 (42 registers), 1.75 with two of 768 and
+// 1.87 with two of 1,024; one of 2^22 / 2^26 0.29 against 0.30 / 0.28 / 0.29 / 0.32
+constexpr int kPersistThreads = 512;
+constexpr int kPersistCtas = 2;
 constexpr uint32_t kStepsPerLaunch = 4096;  // then the host launches again: a kernel always ends
 
 // what one step left behind, read by every CTA after the barrier that ends the step
@@ -46,13 +50,12 @@ struct PersistState {
     uint32_t pushes, splits;
 };
 
-// one grid barrier; *out gets the slot the finished step filled.  False: a wait gave up.
-__device__ __forceinline__ bool step_barrier(PersistState* st, const StepSlot* slot, StepSlot* s_slot) {
+// one grid barrier; *s_slot gets the slot the finished step filled.  False: a wait gave up.
+template <class State, class Slot>
+__device__ __forceinline__ bool step_barrier(State* st, const Slot* slot, Slot* s_slot) {
     if (!grid_sync_bounded(&st->bar_count, &st->bar_gen, &st->err)) return false;
-    if (threadIdx.x == 0) {
-        const uint4 x = __ldcg(reinterpret_cast<const uint4*>(slot));
-        *s_slot = StepSlot{x.x, x.y, x.z, x.w};
-    }
+    if (threadIdx.x < sizeof(Slot) / 16)
+        reinterpret_cast<uint4*>(s_slot)[threadIdx.x] = __ldcg(reinterpret_cast<const uint4*>(slot) + threadIdx.x);
     __syncthreads();
     return true;
 }
@@ -67,14 +70,31 @@ __device__ __forceinline__ uint32_t warp_incl(uint32_t x) {
     return x;
 }
 
-// The CTA's share of the next queue: entries gather in shared memory and go out together (flush);
-// what does not fit goes to the global queue directly.
+// the first lane whose inclusive prefix exceeds rank r (lane 31 for ranks past the last)
+__device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t r) {
+    uint32_t o = 0;
+#pragma unroll
+    for (int b = 16; b > 0; b >>= 1) {
+        const uint32_t p = __shfl_sync(0xffffffffu, incl, o + b - 1);
+        if (p <= r) o += b;
+    }
+    return o;
+}
+
+// The CTA's share of the next queue: entries gather in shared memory and go out together (flush).
+// What does not fit goes to the global queue in blocks of kQueueBlock entries that one warp reserves
+// at a time (a reservation per warp and 128 edges made a push level of 2.7 M activations 0.38 ms
+// long); the rest of a warp's last block is filled with empty pieces.
 constexpr uint32_t kLocalQueue = 2048;
+constexpr uint32_t kQueueBlock = 256;
 struct LocalQueue {
     uint4 e[kLocalQueue];
     uint32_t n;      // reserved
     uint32_t valid;  // reservations from here on did not fit
     uint32_t base;
+};
+struct WarpBlock {  // the warp's block of the global queue, the same in every lane
+    uint32_t pos = 0, end = 0;
 };
 
 __device__ __forceinline__ uint4 piece(uint32_t v, uint64_t beg, uint64_t end) {
@@ -84,32 +104,54 @@ __device__ __forceinline__ uint4 piece(uint32_t v, uint64_t beg, uint64_t end) {
 
 // every lane appends the pieces of its K vertices' lists [beg[j], end[j]) (empty: none)
 template <int K>
-__device__ __forceinline__ void append_pieces(LocalQueue& lq, const uint32_t (&v)[K], const uint64_t (&beg)[K],
-                                              const uint64_t (&end)[K], uint4* q_out, uint32_t* n_out) {
+__device__ __forceinline__ void append_pieces(LocalQueue& lq, WarpBlock& wb, const uint32_t (&v)[K],
+                                              const uint64_t (&beg)[K], const uint64_t (&end)[K], uint4* q_out,
+                                              uint32_t* n_out) {
     uint32_t cnt = 0;
 #pragma unroll
     for (int j = 0; j < K; ++j) cnt += (uint32_t)((end[j] - beg[j] + kPiece - 1) / kPiece);
     if (!__any_sync(0xffffffffu, cnt != 0)) return;
     const uint32_t incl = warp_incl(cnt);
-    uint32_t at = 0, direct = 0;
-    if ((threadIdx.x & 31) == 31) {
-        at = atomicAdd(&lq.n, incl);
-        direct = at + incl > kLocalQueue;
-        if (direct) {
+    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t at = kLocalQueue;
+    if ((threadIdx.x & 31) == 31 && *(volatile uint32_t*)&lq.valid == 0xFFFFFFFFu) {
+        at = atomicAdd(&lq.n, tot);
+        if (at + tot > kLocalQueue) {
             atomicMin(&lq.valid, at);
-            at = atomicAdd(n_out, incl);
+            at = kLocalQueue;
         }
     }
-    direct = __shfl_sync(0xffffffffu, direct, 31);
-    at = __shfl_sync(0xffffffffu, at, 31) + incl - cnt;
-    uint4* out = direct ? q_out : lq.e;
+    at = __shfl_sync(0xffffffffu, at, 31);
+    uint32_t k = incl - cnt;  // this lane's first entry among the warp's
+    if (at < kLocalQueue) {
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            for (uint64_t b = beg[j]; b < end[j]; b += kPiece) lq.e[at + k++] = piece(v[j], b, end[j]);
+        return;
+    }
+    const uint32_t room = wb.end - wb.pos;
+    uint32_t fresh = 0, block = 0;
+    if (tot > room) {
+        block = tot - room > kQueueBlock ? tot - room : kQueueBlock;
+        if ((threadIdx.x & 31) == 31) fresh = atomicAdd(n_out, block);
+        fresh = __shfl_sync(0xffffffffu, fresh, 31);
+    }
 #pragma unroll
     for (int j = 0; j < K; ++j)
-        for (uint64_t b = beg[j]; b < end[j]; b += kPiece) out[at++] = piece(v[j], b, end[j]);
+        for (uint64_t b = beg[j]; b < end[j]; b += kPiece, ++k)
+            q_out[k < room ? wb.pos + k : fresh + (k - room)] = piece(v[j], b, end[j]);
+    if (tot > room) {
+        wb.pos = fresh + (tot - room);
+        wb.end = fresh + block;
+    } else {
+        wb.pos += tot;
+    }
 }
 
 // by the whole CTA, before the barrier that ends the step
-__device__ __forceinline__ void flush_pieces(LocalQueue& lq, uint4* q_out, uint32_t* n_out) {
+__device__ __forceinline__ void flush_pieces(LocalQueue& lq, WarpBlock& wb, uint4* q_out, uint32_t* n_out) {
+    for (uint32_t i = wb.pos + (threadIdx.x & 31); i < wb.end; i += 32) q_out[i] = make_uint4(0, 0, 0, 0);
+    wb.pos = wb.end = 0;
     __syncthreads();
     const uint32_t n = min(lq.n, lq.valid);
     if (threadIdx.x == 0) lq.base = n ? atomicAdd(n_out, n) : 0u;
@@ -119,6 +161,12 @@ __device__ __forceinline__ void flush_pieces(LocalQueue& lq, uint4* q_out, uint3
         lq.n = 0;
         lq.valid = 0xFFFFFFFFu;
     }
+}
+
+// entries a queue has to hold: every vertex's pieces and the blocks' empty ends
+static uint64_t queue_entries(const eg_graph* g) {
+    return std::min<uint64_t>(g->V, g->E) + g->E / kPiece +
+           (uint64_t)g->num_sms * kPersistCtas * (kPersistThreads / 32) * kQueueBlock + 64;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -144,10 +192,11 @@ struct SsspPersistArgs {
 
 constexpr uint32_t kWeightSamples = 65536;
 
-__global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPersistArgs a) {
+__global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persistent(SsspPersistArgs a) {
     __shared__ StepSlot s_slot;
     extern __shared__ __align__(16) unsigned char s_raw[];
     LocalQueue& lq = *reinterpret_cast<LocalQueue*>(s_raw);
+    WarpBlock wb;
     if (threadIdx.x == 0) {
         lq.n = 0;
         lq.valid = 0xFFFFFFFFu;
@@ -245,12 +294,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPers
 #pragma unroll
                     for (int j = 0; j < kIlp; ++j) {
                         const uint32_t r = r0 + 32 * j + lane;
-                        uint32_t o = 0;  // the first lane whose inclusive prefix exceeds r
-#pragma unroll
-                        for (int b = 16; b > 0; b >>= 1) {
-                            const uint32_t p = __shfl_sync(0xffffffffu, incl, o + b - 1);
-                            if (p <= r) o += b;
-                        }
+                        const uint32_t o = warp_owner(incl, r);
                         const uint64_t pos = __shfl_sync(0xffffffffu, beg, o) + r;
                         const float od = __shfl_sync(0xffffffffu, du, o);
                         x[j] = r < total ? __ldg(a.adj + pos) : 0u;
@@ -281,7 +325,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPers
                             }
                         }
                     }
-                    append_pieces<kIlp>(lq, x, lb, le, q_out, &out->n);
+                    append_pieces<kIlp>(lq, wb, x, lb, le, q_out, &out->n);
                 }
             }
             ++pushes;
@@ -308,7 +352,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPers
                     const uint64_t b[1] = {move ? __ldg(a.off + v[0]) : 0ull};
                     const uint64_t z[1] = {move ? __ldg(a.off + (uint64_t)v[0] + 1) : 0ull};
                     move &= move - 1;
-                    append_pieces<1>(lq, v, b, z, q_out, &out->n);
+                    append_pieces<1>(lq, wb, v, b, z, q_out, &out->n);
                 }
             }
 #pragma unroll
@@ -324,7 +368,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_sssp_persistent(SsspPers
             last_kind = 1;
         }
         ++step;
-        flush_pieces(lq, q_out, &out->n);
+        flush_pieces(lq, wb, q_out, &out->n);
         if (!step_barrier(st, out, &s_slot)) return;
     }
     if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
@@ -360,7 +404,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EngineState& s = g->eng;
     EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
     EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
-    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * (std::min(V, E) + E / kPiece + 64)));
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
     EG_TRY(s.persist.reserve(sizeof(PersistState)));
     float* d_dist = dist;
     if (where != EG_DEVICE || !dist) {
@@ -384,7 +428,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     a.st = s.persist.as<PersistState>();
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms, E / kEdgesPerCta));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
     static_assert(sizeof(PersistState) <= 256, "the state is read back through the 256-byte pinned block");
     PersistState* h = reinterpret_cast<PersistState*>(s.host_words);
     EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(PersistState), g->stream));
@@ -410,6 +454,396 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     g->last_pulls = 0;
     if (dist && where != EG_DEVICE) {
         EG_CUDA(cudaMemcpyAsync(dist, d_dist, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
+        EG_CUDA(cudaStreamSynchronize(g->stream));
+    }
+    return EG_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// BFS (toolkits/bfs.cpp:52-76): a push level claims unreached vertices through the level array; a
+// dense level gives every compressed in-list of an unreached vertex a thread that looks at its first
+// kBfsHead in-edges, then the warp walks what its 32 lists have left together, and lists longer than
+// that are cut into segments that a second half of the level spreads over the GPU.  The frontier is
+// "level == this level": no bitmaps to keep or clear.  Means of 16 roots, against the level loop driven
+// from the host that it replaces (kernels per level, bitmaps, counters read back): 100,003 vertices,
+// 1,000,003 edges 0.33 -> 0.09 ms; 2^22, 2^26 0.41 -> 0.26; 2^25, 2^29 2.11 -> 1.29, most of it where the
+// first dense level finds few parents in the lists' heads (5.04 -> 1.89 ms: the rest of a list was one
+// warp's).  A dense level is bound by its gathers: rounds of four in-edges, up to 12, take 1.29 ms, up
+// to 8 1.34, up to 4 1.44, eight at once 1.54.
+constexpr uint32_t kBfsHead = 12;
+constexpr uint32_t kBfsSeg = 1024;
+constexpr uint32_t kUnreached = 0xFFFFFFFFu;
+
+struct alignas(16) BfsSlot {
+    uint32_t n;               // queue entries appended
+    uint32_t verts;           // vertices reached
+    unsigned long long act;   // their out-edges
+    uint32_t nseg;            // segments of the dense level
+    uint32_t pad[3];
+};
+
+struct BfsPersistState {
+    unsigned bar_count, bar_gen;
+    int err;
+    uint32_t step, done, pushes, pulls, pad;
+    BfsSlot slot[4];  // as PersistState::slot
+    unsigned long long reached, edges;
+};
+
+struct BfsPersistArgs {
+    uint64_t V, nitems;
+    const uint64_t* off;
+    const uint32_t* adj;
+    const uint32_t* csc_adj;
+    const uint64_t* cidx;
+    const uint32_t* cvert;
+    uint32_t* level;
+    uint32_t* parent;  // null: not wanted
+    uint4* q[2];
+    unsigned long long* seg;  // (segment << 32) | compressed entry
+    uint32_t root;
+    int direction, has_csc;
+    unsigned long long dense_min;
+    int resume;
+    BfsPersistState* st;
+};
+
+__global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persistent(BfsPersistArgs a) {
+    __shared__ BfsSlot s_slot;
+    __shared__ uint32_t s_verts;
+    __shared__ unsigned long long s_act;
+    __shared__ uint32_t s_par[kPersistThreads];
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    LocalQueue& lq = *reinterpret_cast<LocalQueue*>(s_raw);
+    WarpBlock wb;
+    if (threadIdx.x == 0) {
+        lq.n = 0;
+        lq.valid = 0xFFFFFFFFu;
+        s_verts = 0;
+        s_act = 0;
+    }
+    BfsPersistState* st = a.st;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t warp = (uint32_t)(tid >> 5), nwarps = (uint32_t)(stride >> 5);
+    uint32_t step = 0, pushes = 0, pulls = 0;
+    unsigned long long reached = 0, edges = 0;
+    if (!a.resume) {
+        for (uint64_t v = tid; v < a.V; v += stride) {
+            a.level[v] = v == a.root ? 0u : kUnreached;
+            if (a.parent) a.parent[v] = v == a.root ? (uint32_t)v : (uint32_t)a.V;
+        }
+        if (tid < 32) {  // the root's pieces
+            const uint64_t b = a.off[a.root], z = a.off[(uint64_t)a.root + 1];
+            const uint32_t np = (uint32_t)((z - b + kPiece - 1) / kPiece);
+            for (uint32_t p = lane; p < np; p += 32) a.q[0][p] = piece(a.root, b + (uint64_t)p * kPiece, z);
+            if (lane == 0) {
+                st->slot[0].n = np;
+                st->slot[0].verts = 1;
+                st->slot[0].act = z - b;
+            }
+        }
+        if (!step_barrier(st, &st->slot[0], &s_slot)) return;
+        reached = 1;
+        edges = s_slot.act;
+    } else {
+        step = __ldcg(&st->step);
+        if (threadIdx.x < sizeof(BfsSlot) / 16)
+            reinterpret_cast<uint4*>(&s_slot)[threadIdx.x] =
+                __ldcg(reinterpret_cast<const uint4*>(&st->slot[step & 3]) + threadIdx.x);
+        __syncthreads();
+        reached = __ldcg(&st->reached);
+        edges = __ldcg(&st->edges);
+    }
+    const uint32_t first = step;
+    while (s_slot.verts > 0 && step - first < kStepsPerLaunch) {
+        const uint32_t n = s_slot.n;
+        const bool dense = a.direction == 2 || (a.direction == 0 && a.has_csc && s_slot.act >= a.dense_min);
+        BfsSlot* out = &st->slot[(step + 1) & 3];
+        uint4* q_out = a.q[(step + 1) & 1];
+        const uint32_t lvl = step;  // the frontier's level
+        uint32_t my_verts = 0;
+        unsigned long long my_act = 0;
+        __syncthreads();  // s_slot has been read
+        if (tid == 0) {
+            BfsSlot* clear = &st->slot[(step + 2) & 3];
+            clear->n = clear->verts = clear->nseg = 0;
+            clear->act = 0;
+        }
+        // hand the step's totals and the gathered queue entries over; false: a barrier gave up
+        auto end_phase = [&]() -> bool {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                my_verts += __shfl_xor_sync(0xffffffffu, my_verts, o);
+                my_act += __shfl_xor_sync(0xffffffffu, my_act, o);
+            }
+            if (lane == 0 && my_verts) {
+                atomicAdd(&s_verts, my_verts);
+                atomicAdd(&s_act, my_act);
+            }
+            my_verts = 0;
+            my_act = 0;
+            flush_pieces(lq, wb, q_out, &out->n);
+            if (threadIdx.x == 0 && s_verts) {
+                atomicAdd(&out->verts, s_verts);
+                atomicAdd(&out->act, s_act);
+                s_verts = 0;
+                s_act = 0;
+            }
+            return step_barrier(st, out, &s_slot);
+        };
+        if (!dense) {
+            const uint4* q = a.q[step & 1];
+            for (uint32_t base = 0; base < n; base += 32 * nwarps) {
+                const uint64_t idx = (uint64_t)base + (uint64_t)lane * nwarps + warp;
+                uint64_t beg = 0;
+                uint32_t len = 0, u = 0;
+                if (idx < n) {
+                    const uint4 e = __ldcg(q + idx);
+                    u = e.x;
+                    beg = ((uint64_t)e.z << 32) | e.y;
+                    len = e.w;
+                }
+                const uint32_t incl = warp_incl(len);
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                beg -= incl - len;
+                for (uint32_t r0 = 0; r0 < total; r0 += 32 * kIlp) {
+                    uint32_t x[kIlp], par[kIlp];
+                    uint64_t lb[kIlp], le[kIlp];
+                    bool open[kIlp];
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) {
+                        const uint32_t r = r0 + 32 * j + lane;
+                        const uint32_t o = warp_owner(incl, r);
+                        const uint64_t pos = __shfl_sync(0xffffffffu, beg, o) + r;
+                        par[j] = __shfl_sync(0xffffffffu, u, o);
+                        x[j] = r < total ? __ldg(a.adj + pos) : a.root;
+                    }
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) open[j] = __ldcg(a.level + x[j]) == kUnreached;
+#pragma unroll
+                    for (int j = 0; j < kIlp; ++j) {
+                        lb[j] = le[j] = 0;
+                        if (open[j]) {
+                            const uint32_t old = atomicCAS(a.level + x[j], kUnreached, lvl + 1);
+                            const uint64_t b = __ldg(a.off + x[j]), z = __ldg(a.off + (uint64_t)x[j] + 1);
+                            if (old == kUnreached) {
+                                if (a.parent) a.parent[x[j]] = par[j];
+                                lb[j] = b;
+                                le[j] = z;
+                                ++my_verts;
+                                my_act += z - b;
+                            }
+                        }
+                    }
+                    append_pieces<kIlp>(lq, wb, x, lb, le, q_out, &out->n);
+                }
+            }
+            ++pushes;
+            if (!end_phase()) return;
+        } else {
+            // a list's vertex is loaded two rounds ahead, its level and bounds one round ahead
+            uint64_t i = tid;
+            uint32_t v1 = i < a.nitems ? __ldg(a.cvert + i) : kUnreached;
+            uint32_t v2 = i + stride < a.nitems ? __ldg(a.cvert + i + stride) : kUnreached;
+            bool open1 = v1 < a.V && __ldcg(a.level + v1) == kUnreached;
+            uint64_t p1 = i < a.nitems ? __ldg(a.cidx + i) : 0, e1 = i < a.nitems ? __ldg(a.cidx + i + 1) : 0;
+            for (uint64_t base = tid & ~31ull; base < a.nitems; base += stride, i += stride) {
+                const uint32_t v = v1;
+                const bool open = open1;
+                uint64_t p = p1;
+                const uint64_t e = e1;
+                uint32_t par = kUnreached, len = 0, nsg = 0;
+                v1 = v2;
+                v2 = i + 2 * stride < a.nitems ? __ldg(a.cvert + i + 2 * stride) : kUnreached;
+                open1 = v1 < a.V && __ldcg(a.level + v1) == kUnreached;
+                if (i + stride < a.nitems) {
+                    p1 = __ldg(a.cidx + i + stride);
+                    e1 = __ldg(a.cidx + i + stride + 1);
+                }
+                if (open) {
+                    const uint64_t h = e - p > kBfsHead ? p + kBfsHead : e;
+                    for (uint64_t x = p; x < h && par == kUnreached; x += 4) {
+                        uint32_t u[4];
+                        bool hit[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) u[j] = x + j < h ? __ldg(a.csc_adj + x + j) : a.root;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) hit[j] = x + j < h && __ldcg(a.level + u[j]) == lvl;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (hit[j]) par = u[j];
+                    }
+                    if (par == kUnreached && e > h) {
+                        p = h;
+                        if (e - h <= kBfsSeg) len = (uint32_t)(e - h);
+                        else nsg = (uint32_t)((e - h + kBfsSeg - 1) / kBfsSeg);
+                    }
+                }
+                // the rest of the warp's lists, walked together
+                const uint32_t incl = warp_incl(len);
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                if (total) {
+                    uint32_t* found = s_par + (threadIdx.x & ~31u);
+                    found[lane] = kUnreached;
+                    __syncwarp();
+                    const uint64_t beg = p - (incl - len);
+                    for (uint32_t r0 = 0; r0 < total; r0 += 32 * kIlp) {
+                        uint32_t u[kIlp], o[kIlp];
+                        bool want[kIlp];
+#pragma unroll
+                        for (int j = 0; j < kIlp; ++j) {
+                            const uint32_t r = r0 + 32 * j + lane;
+                            o[j] = warp_owner(incl, r);
+                            const uint64_t pos = __shfl_sync(0xffffffffu, beg, o[j]) + r;
+                            want[j] = r < total && *(volatile uint32_t*)(found + o[j]) == kUnreached;
+                            u[j] = want[j] ? __ldg(a.csc_adj + pos) : a.root;
+                        }
+#pragma unroll
+                        for (int j = 0; j < kIlp; ++j)
+                            if (want[j] && __ldcg(a.level + u[j]) == lvl) *(volatile uint32_t*)(found + o[j]) = u[j];
+                    }
+                    __syncwarp();
+                    if (len) par = found[lane];
+                    __syncwarp();
+                }
+                const uint32_t sincl = warp_incl(nsg);
+                const uint32_t stot = __shfl_sync(0xffffffffu, sincl, 31);
+                if (stot) {
+                    uint32_t at = 0;
+                    if (lane == 31) at = atomicAdd(&out->nseg, stot);
+                    at = __shfl_sync(0xffffffffu, at, 31) + sincl - nsg;
+                    for (uint32_t k = 0; k < nsg; ++k) a.seg[at + k] = ((unsigned long long)k << 32) | (uint32_t)i;
+                }
+                const uint32_t vv[1] = {v};
+                uint64_t lb[1] = {0}, le[1] = {0};
+                if (open && par != kUnreached) {  // this lane owns v's only list
+                    a.level[v] = lvl + 1;
+                    if (a.parent) a.parent[v] = par;
+                    lb[0] = __ldg(a.off + v);
+                    le[0] = __ldg(a.off + (uint64_t)v + 1);
+                    ++my_verts;
+                    my_act += le[0] - lb[0];
+                }
+                append_pieces<1>(lq, wb, vv, lb, le, q_out, &out->n);
+            }
+            ++pulls;
+            if (!end_phase()) return;
+            const uint32_t nseg = s_slot.nseg;
+            if (nseg) {  // long lists, a warp per segment; the first segment to find a parent claims
+                __syncthreads();  // s_slot has been read
+                for (uint32_t t = warp; t < nseg; t += nwarps) {
+                    const unsigned long long ent = __ldcg(a.seg + t);
+                    const uint32_t i = (uint32_t)ent;
+                    const uint32_t v = __ldg(a.cvert + i);
+                    const uint64_t e = __ldg(a.cidx + i + 1);
+                    uint64_t p = __ldg(a.cidx + i) + kBfsHead + (ent >> 32) * kBfsSeg;
+                    const uint64_t pe = p + kBfsSeg < e ? p + kBfsSeg : e;
+                    const uint32_t vv[1] = {v};
+                    uint64_t lb[1] = {0}, le[1] = {0};
+                    for (; p < pe; p += 32 * kIlp) {
+                        if (__shfl_sync(0xffffffffu, __ldcg(a.level + v), 0) != kUnreached) break;
+                        uint32_t cand = kUnreached;
+#pragma unroll
+                        for (int j = 0; j < kIlp; ++j) {
+                            const uint64_t x = p + 32 * j + lane;
+                            const uint32_t u = x < pe ? __ldg(a.csc_adj + x) : a.root;
+                            if (x < pe && __ldcg(a.level + u) == lvl) cand = u;
+                        }
+                        const unsigned m = __ballot_sync(0xffffffffu, cand != kUnreached);
+                        if (!m) continue;
+                        const uint32_t par = __shfl_sync(0xffffffffu, cand, __ffs(m) - 1);
+                        if (lane == 0 && atomicCAS(a.level + v, kUnreached, lvl + 1) == kUnreached) {
+                            if (a.parent) a.parent[v] = par;
+                            lb[0] = __ldg(a.off + v);
+                            le[0] = __ldg(a.off + (uint64_t)v + 1);
+                            ++my_verts;
+                            my_act += le[0] - lb[0];
+                        }
+                        break;
+                    }
+                    append_pieces<1>(lq, wb, vv, lb, le, q_out, &out->n);
+                }
+                if (!end_phase()) return;
+            }
+        }
+        reached += s_slot.verts;
+        edges += s_slot.act;
+        ++step;
+    }
+    if (tid == 0) {  // every CTA leaves the loop at the same step
+        st->step = step;
+        st->done = s_slot.verts == 0 ? 1u : 0u;
+        st->reached = reached;
+        st->edges = edges;
+        st->pushes += pushes;
+        st->pulls += pulls;
+    }
+}
+
+int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached) {
+    const uint64_t V = g->V, E = g->E;
+    EngineState& s = g->eng;
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
+    EG_TRY(s.persist.reserve(sizeof(BfsPersistState)));
+    BfsPersistArgs a;
+    a.level = level;
+    a.parent = parent;
+    if (where != EG_DEVICE || !level) {
+        EG_TRY(s.vals0.reserve(sizeof(uint32_t) * (V + 1)));
+        a.level = s.vals0.as<uint32_t>();
+    }
+    if (where != EG_DEVICE && parent) {
+        EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
+        a.parent = s.vals1.as<uint32_t>();
+    }
+    a.V = V;
+    a.nitems = g->built_csc ? g->ncompressed - 1 : 0;
+    if (g->built_csc) EG_TRY(s.bu_seg.reserve(sizeof(unsigned long long) * (2 * (E / kBfsSeg) + 2)));
+    a.off = g->csr_off.as<uint64_t>();
+    a.adj = g->csr_adj.as<uint32_t>();
+    a.csc_adj = g->csc_adj.as<uint32_t>();
+    a.cidx = g->cidx.as<uint64_t>();
+    a.cvert = g->cvert.as<uint32_t>();
+    a.q[0] = s.pieces0.as<uint4>();
+    a.q[1] = s.pieces1.as<uint4>();
+    a.seg = s.bu_seg.as<unsigned long long>();
+    a.root = root;
+    a.direction = g->bfs_direction;
+    a.has_csc = g->built_csc ? 1 : 0;
+    a.dense_min = E / (uint64_t)g->dense_div;
+    a.st = s.persist.as<BfsPersistState>();
+    const size_t smem = sizeof(LocalQueue);
+    EG_CUDA(cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
+    static_assert(sizeof(BfsPersistState) <= 256, "the state is read back through the 256-byte pinned block");
+    BfsPersistState* h = reinterpret_cast<BfsPersistState*>(s.host_words);
+    EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(BfsPersistState), g->stream));
+    for (a.resume = 0;; a.resume = 1) {
+        void* kargs[] = {&a};
+        {
+            Timed t(&g->prof, g->stream, "bfs_persistent");
+            EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
+                                                g->stream));
+            EG_CHECK_LAUNCH("k_bfs_persistent");
+        }
+        EG_CUDA(cudaMemcpyAsync(h, a.st, sizeof(BfsPersistState), cudaMemcpyDeviceToHost, g->stream));
+        EG_CUDA(cudaStreamSynchronize(g->stream));
+        if (h->err) {
+            set_error("eg_bfs: a bounded grid barrier gave up");
+            return EG_ERR_TIMEOUT;
+        }
+        if (h->done) break;
+    }
+    g->last_edges_processed = h->edges;  // sum of out-degrees of the reached vertices
+    g->last_iterations = (int)h->step;
+    g->last_pushes = (int)h->pushes;
+    g->last_pulls = (int)h->pulls;
+    if (reached) *reached = h->reached;
+    if (where != EG_DEVICE) {
+        if (level) EG_CUDA(cudaMemcpyAsync(level, a.level, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
+        if (parent) EG_CUDA(cudaMemcpyAsync(parent, a.parent, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
         EG_CUDA(cudaStreamSynchronize(g->stream));
     }
     return EG_OK;

@@ -62,3 +62,80 @@ def test_sssp_grid_sizes(eg_lib, V, E):
     rng = np.random.default_rng(V)
     src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
     _check_sssp(src, dst, rng.random(E), V, [int(src[0])], deltas=(-1, 0, 20_000))
+
+
+def _check_bfs(src, dst, V, roots, directions=(0, 1, 2), divisors=(20,)):
+    import endgraph_gb300 as eg
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    deg = np.diff(csr["off"][0].astype(np.int64))
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        for root in roots:
+            ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, root)
+            for direction in directions:
+                g.set_option(eg.EG_OPT_BFS_DIRECTION, direction)
+                for div in divisors:
+                    g.set_option(eg.EG_OPT_DENSE_DIVISOR, div)
+                    lv, par = g.bfs(root)
+                    assert np.array_equal(lv, ref), (root, direction, div)
+                    assert oracle.bfs_check_parents(csr["off"][0], csr["adj"], V, root, lv, par) == 0
+                    run = g.last_run()
+                    assert run["edges"] == int(deg[ref != oracle.UNREACHED].sum())
+                    assert run["iterations"] == int(ref[ref != oracle.UNREACHED].max()) + 1
+                    assert run["iterations"] == run["push"] + run["pull"]
+
+
+@pytest.mark.parametrize("deg", [1, 4, 5, 31, 33, 127, 129, 255, 256, 257, 1027, 1028, 1029, 5000, 70000])
+def test_bfs_list_edges(eg_lib, deg):
+    """A vertex whose out-list and in-list have `deg` entries: pieces of the queue, the dense level's
+    first in-edges, the warp's walk and the segments.  Its in-neighbours are reached late or not at
+    all, so that whole lists are read in vain."""
+    V = 80_000
+    rng = np.random.default_rng(deg)
+    hub, nbr = 7, rng.choice(V - 10, deg, replace=False) + 10
+    back = rng.choice(V - 10, deg, replace=False) + 10
+    src = np.concatenate([np.full(deg, hub), back, rng.integers(10, V // 2, 120_000)])
+    dst = np.concatenate([nbr, np.full(deg, hub), rng.integers(10, V // 2, 120_000)])
+    _check_bfs(src, dst, V, [hub, int(back[0]), int(src[-1])], divisors=(1, 20, 1 << 30))
+
+
+def test_bfs_deeper_than_one_launch(eg_lib):
+    """A chain of 9,000 vertices in every direction mode, and a root without edges."""
+    n = 9_000
+    perm = np.random.default_rng(4).permutation(n)
+    _check_bfs(perm[:-1], perm[1:], n + 1, [int(perm[0]), int(perm[n // 2])], directions=(0, 1))
+    _check_bfs(perm[:-1], perm[1:], n + 1, [int(perm[n - 300]), n])
+
+
+@pytest.mark.parametrize("V,E", [(1, 1), (2, 5), (33, 64), (1025, 8191), (4097, 8193), (40_000, 1_300_000)])
+def test_bfs_grid_sizes(eg_lib, V, E):
+    rng = np.random.default_rng(V)
+    src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
+    _check_bfs(src, dst, V, [int(src[0]), 0])
+
+
+def test_bfs_outputs_on_the_device(eg_lib):
+    """Level and parent arrays of the caller are written in place; either may be left out."""
+    import torch
+
+    import endgraph_gb300 as eg
+    V, E = 5000, 40_000
+    rng = np.random.default_rng(8)
+    src, dst = rng.integers(0, V, E).astype(np.uint32), rng.integers(0, V, E).astype(np.uint32)
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    root = int(src[0])
+    ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, root)
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        level = torch.full((V + 16,), 77, dtype=torch.int32, device="cuda")
+        parent = torch.full((V + 16,), 78, dtype=torch.int32, device="cuda")
+        g.bfs(root, level=level[5:5 + V], parent=parent[3:3 + V])
+        lv, par = level.cpu().numpy(), parent.cpu().numpy()
+        assert (lv[:5] == 77).all() and (lv[5 + V:] == 77).all() and (par[:3] == 78).all() and (par[3 + V:] == 78).all()
+        assert np.array_equal(lv[5:5 + V].view(np.uint32), ref)
+        assert oracle.bfs_check_parents(csr["off"][0], csr["adj"], V, root, lv[5:5 + V].view(np.uint32).copy(),
+                                        par[3:3 + V].view(np.uint32).copy()) == 0
+        level.fill_(0)
+        g.bfs(root, level=level[:V], want_parent=False)
+        assert np.array_equal(level[:V].cpu().numpy().view(np.uint32), ref)
