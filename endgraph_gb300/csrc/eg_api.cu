@@ -180,8 +180,6 @@ int eg_sssp_graphs(eg_graph* g, const uint32_t* sources, int sources_per_graph, 
 }  // extern "C"
 
 namespace eg {
-static int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric);
-
 int load_edges_impl(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int edge_bytes, int symmetric, int where,
                     bool validate) {
     if (E > 0 && !edges) {
@@ -202,8 +200,17 @@ int load_edges_impl(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int 
     return EG_OK;
 }
 
+bool direct_records(const eg_graph* g, const void* edges, int where) {
+    if (where != EG_DEVICE || ((uintptr_t)edges & 15u)) return false;
+    cudaPointerAttributes at{};
+    const bool ok = cudaPointerGetAttributes(&at, edges) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+                    at.device == g->device;
+    cudaGetLastError();
+    return ok;
+}
+
 // argument checks, state reset and the record buffer of a new edge list
-static int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric) {
+int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric) {
     if (edge_bytes != 8 && edge_bytes != 12) {
         set_error("eg_load_edges: edge_bytes must be 8 ({src,dst}) or 12 ({src,dst,float})");
         return EG_ERR_INVALID;
@@ -768,6 +775,14 @@ int eg_load_directed(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int
     if (where == EG_HOST && E >= eg::kPipelinedLoadMin && edges) {
         EG_TRY(check_graph(g, "eg_load_directed"));
         return eg::load_build_pipelined(g, edges, E, V, edge_bytes);
+    }
+    if (g && edges && E) {
+        EG_TRY(check_graph(g, "eg_load_directed"));
+        if (g->build_launch && direct_records(g, edges, where)) {
+            EG_TRY(prepare_load(g, E, V, edge_bytes, 0));
+            // the one-launch build copies, checks and counts the records in one pass
+            if (persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0, edges);
+        }
     }
     EG_TRY(eg_load_edges(g, edges, E, V, edge_bytes, 0, where));
     return eg_build(g, 1, 1);

@@ -2125,13 +2125,18 @@ int load_graph_batch(eg_graph* g, const void* edges, int rec, const uint64_t* eo
         return EG_ERR_INVALID;
     }
     const uint64_t E = eo[G];
-    EG_TRY(load_edges_impl(g, edges, E, (uint32_t)voff[G], rec, 0, where, false));
+    // the one-launch build reads the caller's device records itself
+    EG_TRY(prepare_load(g, E, (uint32_t)voff[G], rec, 0));
+    const bool one_launch = g->build_launch && persistent_build_fits(g);
+    const bool direct = one_launch && edges && direct_records(g, edges, where);
+    if (!direct) EG_TRY(load_edges_impl(g, edges, E, (uint32_t)voff[G], rec, 0, where, false));
     EG_TRY(g->d_batch_voff.reserve(8 * (G + 1)));
     EG_TRY(g->tmp64.reserve(8 * (G + 1)));
     EG_CUDA(cudaMemcpyAsync(g->d_batch_voff.ptr, voff.data(), 8 * (G + 1), cudaMemcpyHostToDevice, g->stream));
     EG_CUDA(cudaMemcpyAsync(g->tmp64.ptr, eo.data(), 8 * (G + 1), cudaMemcpyHostToDevice, g->stream));
-    if (g->build_launch && persistent_build_fits(g)) {  // ids moved to the union inside the one launch
-        EG_TRY(build_persistent(g, g->tmp64.as<uint64_t>(), g->d_batch_voff.as<uint64_t>(), (uint32_t)G));
+    if (one_launch) {  // ids moved to the union inside the one launch
+        EG_TRY(build_persistent(g, g->tmp64.as<uint64_t>(), g->d_batch_voff.as<uint64_t>(), (uint32_t)G,
+                                direct ? edges : nullptr));
         g->batch_voff = voff;
         g->batch_eoff = eo;
         return EG_OK;

@@ -818,7 +818,7 @@ static int build_single(eg_graph* g, const UploadParts* up) {
 // The one-partition bucketed build in one cooperative launch: every phase of build_single and of
 // the index kernels of build_structures, separated by bounded grid barriers (grid_sync_bounded),
 // with one 1,024-thread CTA per SM taking pass-A and pass-B blocks by stride, pass-C buckets by
-// ticket and the scans as contiguous ranges.  A graph batch's ids are moved to the union first.
+// ticket and the scans as contiguous ranges.  A graph batch's ids are moved to the union in pass A.
 constexpr int kPersistBuildMaxCtas = 1024;
 
 struct BuildWords {
@@ -830,13 +830,20 @@ struct BuildWords {
     uint64_t tot[kPersistBuildMaxCtas];  // per-CTA sums of a grid scan
 };
 
-struct PersistBuildArgs {
-    uint8_t* edges;
-    uint64_t E;
-    uint32_t V;
+// Where the records come from: a caller's device buffer, or the handle's own list
+struct RecordSource {
+    const uint8_t* in;
+    uint8_t* out;          // the handle's list (may be `in`)
     const uint64_t* eoff;  // graph batch: record offsets (G + 1), null for one graph
     const uint64_t* voff;  // graph batch: vertex offsets (G + 1)
     uint32_t G;
+};
+
+struct PersistBuildArgs {
+    RecordSource src;
+    uint64_t E;
+    uint32_t V;
+    uint32_t* part_off;
     uint64_t chunk;
     int shift;
     uint32_t nb, nblk, LB;
@@ -942,51 +949,107 @@ __device__ bool grid_scan(Load load, Epi epi, uint64_t n, BuildWords* w, uint64_
     return true;
 }
 
-// Union ids of a graph batch: record i of graph k (eoff[k] <= i < eoff[k+1]) gets voff[k] added to
-// both ids, once they are checked against the graph's vertex count (*bad otherwise).  Loads and
-// stores go to L2 only, so that no SM holds a stale L1 line of the records for the passes that
-// read them later in the same launch.
+// Pass A of the one-launch build: one block `blk` reads its records (from the caller's buffer when it
+// is device memory), checks the ids (against V, or against the record's own graph in a batch, whose
+// ids it moves to the union), keeps them in the handle's list and counts the buckets: one read and
+// one write of the list in place of a copy, a validation pass, the batch's id move and a counting
+// pass.  Four 16-byte loads in flight per thread (12-byte records: four records in three loads).
 template <int REC>
-__device__ void relabel_union(uint8_t* edges, uint64_t E, const uint64_t* __restrict__ eoff,
-                              const uint64_t* __restrict__ voff, uint32_t G, int* bad) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+__device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t E, uint64_t chunk, int shift, uint32_t nb,
+                                                 uint32_t nblk, uint32_t* __restrict__ cnt, uint32_t V, int* bad,
+                                                 uint32_t blk, uint32_t* s_h) {
+    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) s_h[i] = 0;
+    __syncthreads();
+    const uint64_t e0 = blk * chunk;
+    const uint64_t e1 = e0 + chunk < E ? e0 + chunk : E;
+    const bool keep = r.out != r.in || r.eoff;
     bool out_of_range = false;
-    uint32_t lo = 0;  // graph of the previous record of this thread (records only move forward)
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += stride) {
-        if (lo + 1 < G && __ldg(eoff + lo + 1) <= i) {
-            uint32_t hi = G;  // last graph with eoff <= i, searched in (lo, G)
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (__ldg(eoff + mid) <= i) lo = mid; else hi = mid;
+    uint32_t lo = 0;  // graph of this thread's previous record (its records only move forward)
+    auto take = [&](uint64_t i, uint32_t& s, uint32_t& d) {
+        if (r.eoff) {
+            if (lo + 1 < r.G && __ldg(r.eoff + lo + 1) <= i) {
+                uint32_t hi = r.G;  // last graph with eoff <= i, searched in (lo, G)
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (__ldg(r.eoff + mid) <= i) lo = mid; else hi = mid;
+                }
             }
-        }
-        uint32_t* r = reinterpret_cast<uint32_t*>(edges + i * (uint64_t)REC);
-        const uint32_t s = __ldcg(r), d = __ldcg(r + 1);
-        const uint64_t base = __ldg(voff + lo), nv = __ldg(voff + lo + 1) - base;
-        if (s >= nv || d >= nv) {
+            const uint64_t base = __ldg(r.voff + lo), nv = __ldg(r.voff + lo + 1) - base;
+            if (s >= nv || d >= nv) {
+                out_of_range = true;
+                return;
+            }
+            s += (uint32_t)base;
+            d += (uint32_t)base;
+        } else if (s >= V || d >= V) {
             out_of_range = true;
-            continue;
+            return;
         }
-        __stcg(r, (uint32_t)(base + s));
-        __stcg(r + 1, (uint32_t)(base + d));
+        atomicAdd(&s_h[s >> shift], 1u);
+        atomicAdd(&s_h[nb + (d >> shift)], 1u);
+    };
+    // groups of 16 * kVec bytes: 2 records of 8 bytes, 4 of 12 (chunks are multiples of 64 records)
+    constexpr int kVec = REC == 8 ? 1 : 3, kRecs = REC == 8 ? 2 : 4, kInFlight = REC == 8 ? 4 : 2;
+    const uint4* in = reinterpret_cast<const uint4*>(r.in);
+    uint4* out = reinterpret_cast<uint4*>(r.out);
+    const uint64_t q1 = e1 / kRecs;  // whole groups
+    for (uint64_t q = e0 / kRecs + threadIdx.x; q < q1; q += (uint64_t)blockDim.x * kInFlight) {
+        uint4 x[kInFlight][kVec];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) {
+            const uint64_t g = q + (uint64_t)u * blockDim.x;
+            if (g < q1)
+#pragma unroll
+                for (int k = 0; k < kVec; ++k) x[u][k] = __ldcs(in + g * kVec + k);
+        }
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u) {
+            const uint64_t g = q + (uint64_t)u * blockDim.x;
+            if (g >= q1) break;
+            uint4(&y)[kVec] = x[u];
+            if constexpr (REC == 8) {
+                take(2 * g, y[0].x, y[0].y);
+                take(2 * g + 1, y[0].z, y[0].w);
+            } else {
+                take(4 * g, y[0].x, y[0].y);
+                take(4 * g + 1, y[0].w, y[1].x);
+                take(4 * g + 2, y[1].z, y[1].w);
+                take(4 * g + 3, y[2].y, y[2].z);
+            }
+            if (keep)
+#pragma unroll
+                for (int k = 0; k < kVec; ++k) __stcg(out + g * kVec + k, y[k]);
+        }
+    }
+    for (uint64_t e = q1 * kRecs + threadIdx.x; e < e1; e += blockDim.x) {  // the list's last records
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(r.in + e * REC);
+        uint32_t s = __ldcs(p), d = __ldcs(p + 1);
+        const uint32_t w = REC == 12 ? __ldcs(p + 2) : 0u;
+        take(e, s, d);
+        if (keep) {
+            uint32_t* o = reinterpret_cast<uint32_t*>(r.out + e * REC);
+            __stcg(o, s);
+            __stcg(o + 1, d);
+            if (REC == 12) __stcg(o + 2, w);
+        }
     }
     if (out_of_range) atomicExch(bad, 1);
+    __syncthreads();
+    // bucket-major layout: [half][bucket][block]
+    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) cnt[(uint64_t)i * nblk + blk] = s_h[i];
 }
 
 template <int REC>
 __global__ void __launch_bounds__(kBuildThreads, 1) k_build_persistent(PersistBuildArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     BuildWords* w = a.w;
-    if (a.eoff) {
-        relabel_union<REC>(a.edges, a.E, a.eoff, a.voff, a.G, &w->bad);
-        if (!build_barrier(w)) return;
-    }
-    // A: bucket counts per (half, bucket, block)
+    // A: the records in, bucket counts per (half, bucket, block)
     for (uint32_t blk = blockIdx.x; blk < a.nblk; blk += gridDim.x) {
-        bucket_hist_block<REC>(a.edges, a.E, a.chunk, a.shift, a.nb, a.nblk, a.cnt, a.V, &w->bad, blk,
-                               reinterpret_cast<uint32_t*>(s_raw));
+        load_count_block<REC>(a.src, a.E, a.chunk, a.shift, a.nb, a.nblk, a.cnt, a.V, &w->bad, blk,
+                              reinterpret_cast<uint32_t*>(s_raw));
         __syncthreads();
     }
+    if (blockIdx.x == 0 && threadIdx.x < 2) a.part_off[threadIdx.x] = threadIdx.x ? a.V : 0u;  // one partition: [0, V]
     if (!build_barrier(w)) return;
     if (*(volatile int*)&w->bad) return;  // every CTA reads the same flag after the barrier
     const uint64_t ncnt = 2ull * a.nb * a.nblk;
@@ -994,7 +1057,7 @@ __global__ void __launch_bounds__(kBuildThreads, 1) k_build_persistent(PersistBu
     if (!build_barrier(w)) return;
     // B: records bucket-sorted per half
     for (uint32_t blk = blockIdx.x; blk < a.nblk; blk += gridDim.x) {
-        bucket_scatter_block<REC, false>(a.edges, a.E, a.chunk, a.shift, a.nb, a.nblk, a.ex, a.bucketed, a.V, blk,
+        bucket_scatter_block<REC, false>(a.src.out, a.E, a.chunk, a.shift, a.nb, a.nblk, a.ex, a.bucketed, a.V, blk,
                                          s_raw);
         __syncthreads();
     }
@@ -1019,7 +1082,7 @@ bool persistent_build_fits(const eg_graph* g) {
                200ull * 1024;
 }
 
-int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G) {
+int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G, const void* src) {
     const uint32_t V = g->V;
     const uint64_t E = g->E;
     const int rec = g->edge_bytes;
@@ -1066,12 +1129,11 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
         return EG_ERR_UNSUPPORTED;
     }
     PersistBuildArgs a;
-    a.edges = g->edges.as<uint8_t>();
+    a.src = RecordSource{src ? static_cast<const uint8_t*>(src) : g->edges.as<uint8_t>(), g->edges.as<uint8_t>(), eoff, voff, G};
     a.E = E;
     a.V = V;
-    a.eoff = eoff;
-    a.voff = voff;
-    a.G = G;
+    EG_TRY(g->d_part_off.reserve(sizeof(uint32_t) * 2));
+    a.part_off = g->d_part_off.as<uint32_t>();
     a.chunk = q.chunk;
     a.shift = q.shift;
     a.nb = q.nb;
@@ -1119,13 +1181,10 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     // one partition, one sub-partition: the CPBT boundaries are [0, V]
     g->part_off.assign({0u, V});
     g->local_off.assign({0u, V});
-    EG_TRY(g->d_part_off.reserve(sizeof(uint32_t) * 2));
-    EG_CUDA(cudaMemcpyAsync(g->d_part_off.ptr, g->part_off.data(), sizeof(uint32_t) * 2, cudaMemcpyHostToDevice, g->stream));
     g->part_edges_csr.assign({0ull, E});
     g->part_edges_csc.assign({0ull, E});
     g->cstart.assign({0ull, hw.cstart[1]});
     g->ncompressed = hw.cstart[1];
-    EG_CUDA(cudaStreamSynchronize(g->stream));
     g->built_csr = g->built_csc = true;
     return EG_OK;
 }
@@ -1252,7 +1311,7 @@ int build_structures(eg_graph* g, int want_csr, int want_csc, const UploadParts*
     g->eng.pull_ready = false;
     g->eng.pr_ready = false;
 
-    if (g->build_launch && !up && persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0);
+    if (g->build_launch && !up && persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0, nullptr);
     // the bucket tables and a staging tile must fit one CTA's shared memory
     const bool bucketed =
         P == 1 && align16(20ull * plan_buckets(V, E).nb) + (uint64_t)scatter_tile(g->edge_bytes) * g->edge_bytes <=

@@ -230,7 +230,11 @@ int build_structures(eg_graph* g, int want_csr, int want_csc, const UploadParts*
 // the one-partition, one-sub-partition build as one cooperative launch; eoff / voff (device, G + 1
 // entries each, optional): a graph batch whose ids are moved to the union inside the launch
 bool persistent_build_fits(const eg_graph* g);
-int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G);
+// src (optional): device records, 16-byte aligned, that pass A copies into g->edges as it counts them
+int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G, const void* src);
+// whether pass A may read the caller's records itself: plain device memory of this GPU, 16-byte aligned
+bool direct_records(const eg_graph* g, const void* edges, int where);
+int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric);
 // eg_load_directed of host records from this many records on: upload and build pipelined
 constexpr uint64_t kPipelinedLoadMin = 1ull << 22;
 int load_build_pipelined(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int edge_bytes);

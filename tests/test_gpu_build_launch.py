@@ -152,3 +152,72 @@ def test_one_launch_build_batch_with_edgeless_graphs(eg_lib):
     base = voff[:-1].astype(np.uint64)[gid]
     _assert_oracle(one, (src.astype(np.uint64) + base).astype(np.uint32),
                    (dst.astype(np.uint64) + base).astype(np.uint32), None, int(Vs.sum()))
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("E", [1, 2, 3, 5, 63, 64, 65, 127, 129, 65_535, 65_537, 300_001])
+def test_build_from_device_records(eg_lib, weighted, E):
+    """load_directed of device records: the build reads them where they are (16-byte aligned) or after
+    a copy (a slice that is not), keeps its own list, and leaves the caller's records alone."""
+    import torch
+
+    import endgraph_gb300 as eg
+    V = 30_011
+    src, dst, w = rmat_graph(V, E, E, weights=(0.0, 1.0) if weighted else None)
+    host = eg.pack_edges(src, dst, w).view(np.int32)
+    with eg.Graph() as g:
+        for skip in (0, 1):  # 8- and 12-byte records: row 1 is not 16-byte aligned
+            buf = torch.full((E + 2, host.shape[1]), 0x7FFFFFFF, dtype=torch.int32, device="cuda")
+            rec = buf[skip:skip + E]
+            rec.copy_(torch.from_numpy(host))
+            g.load_directed(rec, V)
+            _assert_oracle(_structure(g), src, dst, w, V)
+            assert np.array_equal(rec.cpu().numpy(), host)
+            rec.fill_(0x7FFFFFFF)  # a rebuild reads the handle's own list
+            torch.cuda.synchronize()
+            g.build()
+            _assert_oracle(_structure(g), src, dst, w, V)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("at", [0, 1, 2, 3, 70_000, 150_000, 150_001])
+def test_build_from_device_records_refuses_bad_ids(eg_lib, weighted, at):
+    import torch
+
+    import endgraph_gb300 as eg
+    V, E = 30_011, 150_002
+    src, dst, w = rmat_graph(V, E, 9, weights=(0.0, 1.0) if weighted else None)
+    good = torch.from_numpy(eg.pack_edges(src, dst, w).view(np.int32)).cuda()
+    bad = good.clone()
+    bad[at, at & 1] = V
+    with eg.Graph() as g:
+        with pytest.raises(eg.EndGraphError) as e:
+            g.load_directed(bad, V)
+        assert e.value.status == 1 and "vertex id >= V" in str(e.value)
+        g.load_directed(good, V)
+        _assert_oracle(_structure(g), src, dst, w, V)
+
+
+def test_batch_from_device_records(eg_lib):
+    """A graph batch from device records: ids move to the union in the handle's list, not in the
+    caller's records; an id past its own graph is refused, also where the union would hold it."""
+    import torch
+
+    import endgraph_gb300 as eg
+    Vs, eoff, parts, src, dst, w = graph_batch(24, 5, weighted=True)
+    rec = torch.from_numpy(eg.pack_edges(src, dst, w).view(np.int32)).cuda()
+    before = rec.clone()
+    voff = np.concatenate([[0], np.cumsum(Vs)]).astype(np.uint32)
+    usrc = np.concatenate([p[0] + voff[i] for i, p in enumerate(parts)])
+    udst = np.concatenate([p[1] + voff[i] for i, p in enumerate(parts)])
+    with eg.Graph() as g:
+        for _ in range(2):
+            g.load_graph_batch(rec, eoff, Vs)
+            _assert_oracle(_structure(g), usrc, udst, w, int(voff[-1]))
+            assert torch.equal(rec, before)
+        bad = rec.clone()
+        bad[int(eoff[3]), 1] = int(Vs[3])
+        with pytest.raises(eg.EndGraphError):
+            g.load_graph_batch(bad, eoff, Vs)
+        g.load_graph_batch(rec, eoff, Vs)
+        _assert_oracle(_structure(g), usrc, udst, w, int(voff[-1]))
