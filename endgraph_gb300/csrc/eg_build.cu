@@ -291,16 +291,17 @@ __global__ void k_part_edges(const uint64_t* off, uint32_t V, int P, uint64_t E,
 
 // =============================================================================================
 // One-partition build without per-edge global atomics: a counting sort in three passes.
-//   A  per-block shared-memory histograms of the bucket (vertex >> shift) of src and of dst
-//   B  each block re-reads its edges and writes them bucket by bucket to offsets given by an
-//      exclusive scan of A's (bucket, block) counts; the 2 x nb x nblk write frontiers advance
-//      sequentially, so L2 merges the scattered record stores into full sectors
+//   A  per-block shared-memory histograms of the bucket (vertex >> shift) of src and of dst, added up
+//      per bucket; an exclusive scan of the 2 x nb totals gives every bucket its place
+//   B  tiles of records are sorted by bucket in shared memory and stored as one run per bucket, at
+//      positions taken from the bucket's cursor (one atomic per bucket and tile).  All blocks append
+//      to the same 2 x nb frontiers, so the ends of their runs meet in L2 and leave as whole
+//      sectors, whatever the number of buckets
 //   C  one CTA per bucket: shared-memory degree histogram of the bucket's vertex range, block scan
 //      (degrees and offsets written coalesced), then the scatter into the bucket's contiguous
 //      output range through shared-memory cursors
 // =============================================================================================
 constexpr int kBucketThreads = 1024;
-constexpr int kBuildThreads = 1024;
 constexpr uint32_t kMaxBucketVerts = 32768;  // 128 KiB of shared-memory counters in pass C
 constexpr int kBuildUnroll = 4;
 
@@ -309,7 +310,7 @@ constexpr int kBuildUnroll = 4;
 // One block `blk` of pass A (s_h: 2 nb shared counters)
 template <int REC>
 __device__ __forceinline__ void bucket_hist_block(const uint8_t* __restrict__ edges, uint64_t E, uint64_t chunk,
-                                                  int shift, uint32_t nb, uint32_t nblk, uint32_t* __restrict__ cnt,
+                                                  int shift, uint32_t nb, unsigned long long* __restrict__ tot,
                                                   uint32_t V, int* bad, uint32_t blk, uint32_t* s_h) {
     for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) s_h[i] = 0;
     __syncthreads();
@@ -347,16 +348,17 @@ __device__ __forceinline__ void bucket_hist_block(const uint8_t* __restrict__ ed
     }
     if (out_of_range) atomicExch(bad, 1);
     __syncthreads();
-    // bucket-major layout: [half][bucket][block]
-    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) cnt[(uint64_t)i * nblk + blk] = s_h[i];
+    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x)
+        if (s_h[i]) atomicAdd(tot + i, (unsigned long long)s_h[i]);
 }
 
 template <int REC>
 __global__ void __launch_bounds__(kBucketThreads) k_bucket_hist(const uint8_t* __restrict__ edges, uint64_t E,
-                                                                 uint64_t chunk, int shift, uint32_t nb, uint32_t nblk,
-                                                                 uint32_t* __restrict__ cnt, uint32_t V, int* bad) {
+                                                                 uint64_t chunk, int shift, uint32_t nb,
+                                                                 unsigned long long* __restrict__ tot, uint32_t V,
+                                                                 int* bad) {
     extern __shared__ uint32_t s_h[];  // [2][nb]
-    bucket_hist_block<REC>(edges, E, chunk, shift, nb, nblk, cnt, V, bad, blockIdx.x, s_h);
+    bucket_hist_block<REC>(edges, E, chunk, shift, nb, tot, V, bad, blockIdx.x, s_h);
 }
 
 // in-place exclusive scan of s[0..n) by the whole block; returns the total.  s_warp: 33 words
@@ -400,43 +402,85 @@ __device__ uint32_t block_exclusive_scan(uint32_t* s, uint32_t n, uint32_t* s_wa
     return total;
 }
 
-// B: tiles of scatter_per(REC) x 1024 edges are counting-sorted by bucket in shared memory and then
-// stored in that order, so consecutive threads store consecutive addresses of a bucket's run
-// (whole sectors instead of one partial sector per record).  The block's running base per bucket
-// starts at its exclusive (bucket, block) offset from the scan of pass A.
-constexpr int kScatterThreads = 1024;
-// 16 records per thread for 8-byte records (128 KiB tile: longer runs per bucket, fewer partial
-// sectors), 8 for 12-byte records so that the tile and the bucket tables still fit 200 KiB
-__host__ __device__ constexpr int scatter_per(int rec) { return rec == 8 ? 16 : 8; }
-__host__ __device__ constexpr int scatter_tile(int rec) { return kScatterThreads * scatter_per(rec); }
+// exclusive prefix of one value per thread over the block; *total: the block's sum
+__device__ __forceinline__ uint64_t block_excl_u64(uint64_t v, uint64_t* s_red, uint64_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint64_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) s_red[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const uint64_t x = lane < nw ? s_red[lane] : 0ull;
+        uint64_t y = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t z = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) y += z;
+        }
+        if (lane < nw) s_red[lane] = y - x;
+        if (lane == 31) s_red[32] = y;
+    }
+    __syncthreads();
+    const uint64_t r = s_red[warp] + inc - v;
+    *total = s_red[32];
+    __syncthreads();
+    return r;
+}
+
+// start[i] = tot[0] + .. + tot[i - 1] for i in [0, n], by one block
+__device__ __forceinline__ void bucket_starts(const unsigned long long* tot, uint32_t n, uint64_t* start) {
+    __shared__ uint64_t s_red[33];
+    uint64_t carry = 0;
+    for (uint32_t t0 = 0; t0 < n; t0 += blockDim.x) {
+        const uint32_t i = t0 + threadIdx.x;
+        uint64_t total;
+        const uint64_t x = block_excl_u64(i < n ? __ldcg(tot + i) : 0ull, s_red, &total);
+        if (i < n) start[i] = carry + x;
+        carry += total;
+    }
+    if (threadIdx.x == 0) start[n] = carry;
+}
+__global__ void __launch_bounds__(1024) k_bucket_starts(const unsigned long long* tot, uint32_t n, uint64_t* start) {
+    bucket_starts(tot, n, start);
+}
+
+// B: 16 records of 8 bytes per thread and tile (128 KiB), 10 of 12 bytes (120 KiB); one CTA of 1,024
+// threads per SM.  Two of 512 with half the tile took as long (4.38 against 4.41 ms at 2^25 / 2^29,
+// 1,024 buckets) and pass C longer.
+__host__ __device__ constexpr int scatter_per(int rec) { return rec == 8 ? 16 : 10; }
+__host__ __device__ constexpr uint32_t scatter_tile(int rec) { return (uint32_t)(kBucketThreads * scatter_per(rec)); }
+// shared memory of pass B: u64 positions and u32 counts per bucket, the tile
+__host__ __device__ constexpr size_t scatter_smem(int rec, uint32_t nb) {
+    return align16(12ull * nb) + (size_t)scatter_tile(rec) * rec;
+}
 
 // kCheck: skip records with an id >= V as pass A did (an upload validated in pass A); edge lists
 // validated at load leave it off
-// One block `blk` of pass B (s_raw: the bucket tables and the staging tile)
+// Tiles blockIdx.x, blockIdx.x + gridDim.x, ... (s_raw: the bucket tables and the staging tile)
 template <int REC, bool kCheck>
-__device__ __forceinline__ void bucket_scatter_block(const uint8_t* __restrict__ edges, uint64_t E, uint64_t chunk,
-                                                     int shift, uint32_t nb, uint32_t nblk,
-                                                     const uint64_t* __restrict__ excl, uint8_t* __restrict__ out,
-                                                     uint32_t V, uint32_t blk, unsigned char* s_raw) {
+__device__ __forceinline__ void bucket_scatter_tiles(const uint8_t* __restrict__ edges, uint64_t E, int shift, uint32_t nb,
+                                                     const uint64_t* __restrict__ start,
+                                                     unsigned long long* __restrict__ cursor,
+                                                     uint8_t* __restrict__ out, uint32_t V, unsigned char* s_raw) {
     constexpr int W = REC / 4;  // words per record
-    unsigned long long* s_base = reinterpret_cast<unsigned long long*>(s_raw);  // [2][nb]
-    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_base + 2 * nb);            // [nb]
-    uint32_t* s_stage = reinterpret_cast<uint32_t*>(s_raw + align16(20ull * nb));  // [tile][W]
-    __shared__ uint32_t s_warp[33];
-    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) s_base[i] = excl[(uint64_t)i * nblk + blk];
-    const uint64_t e0 = blk * chunk;
-    const uint64_t e1 = e0 + chunk < E ? e0 + chunk : E;
     constexpr int kPer = scatter_per(REC);
-    unsigned long long keep;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
-    for (uint64_t t0 = e0; t0 < e1; t0 += scatter_tile(REC)) {
-        uint32_t rec[kPer][W];
-        bool valid[kPer];
+    constexpr uint32_t kTile = scatter_tile(REC), kThreads = kBucketThreads;
+    unsigned long long* s_base = reinterpret_cast<unsigned long long*>(s_raw);      // [nb] run position - run start
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_base + nb);                    // [nb] counts, then run starts
+    uint32_t* s_stage = reinterpret_cast<uint32_t*>(s_raw + align16(12ull * nb));  // [tile][W]
+    __shared__ uint32_t s_warp[33];
+    uint32_t rec[kPer][W];
+    uint32_t valid = 0;  // bit j: record j of this thread exists
+    auto load_tile = [&](uint64_t t0) {
+        valid = 0;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
-            const uint64_t e = t0 + (uint64_t)j * blockDim.x + threadIdx.x;
-            valid[j] = e < e1;
-            if (valid[j]) {
+            const uint64_t e = t0 + (uint64_t)j * kThreads + threadIdx.x;
+            if (e < E) {
                 if (W == 2) {
                     const uint2 x = __ldcs(reinterpret_cast<const uint2*>(edges) + e);
                     rec[j][0] = x.x;
@@ -446,23 +490,46 @@ __device__ __forceinline__ void bucket_scatter_block(const uint8_t* __restrict__
 #pragma unroll
                     for (int w = 0; w < W; ++w) rec[j][w] = __ldcs(r + w);
                 }
-                if (kCheck) valid[j] = rec[j][0] < V && rec[j][1] < V;  // pass A skipped it too
+                valid |= 1u << j;
             }
+        }
+    };
+    uint64_t t0 = (uint64_t)blockIdx.x * kTile;
+    if (t0 < E) load_tile(t0);
+    for (; t0 < E; t0 += (uint64_t)gridDim.x * kTile) {
+        if (kCheck) {
+#pragma unroll
+            for (int j = 0; j < kPer; ++j)  // pass A skipped it too
+                if ((valid >> j & 1u) && (rec[j][0] >= V || rec[j][1] >= V)) valid &= ~(1u << j);
         }
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) s_cnt[i] = 0;
+            for (uint32_t i = threadIdx.x; i < nb; i += kThreads) s_cnt[i] = 0;
             __syncthreads();
             uint32_t rank[kPer];
 #pragma unroll
             for (int j = 0; j < kPer; ++j)
-                rank[j] = valid[j] ? atomicAdd(&s_cnt[rec[j][half] >> shift], 1u) : 0u;
+                rank[j] = valid >> j & 1u ? atomicAdd(&s_cnt[rec[j][half] >> shift], 1u) : 0u;
             __syncthreads();
-            // tile-local exclusive starts; s_cnt keeps the counts in a copy inside s_stage's tail
+            // the runs' places: one round trip per bucket and tile, on its way while the counts are
+            // scanned (the first two buckets of a thread, all of them up to 2,048)
+            unsigned long long* cur = cursor + (uint64_t)half * nb;
+            const uint64_t* st = start + (uint64_t)half * nb;
+            unsigned long long place[2] = {0, 0};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t b = threadIdx.x + k * kThreads;
+                const uint32_t c = b < nb ? s_cnt[b] : 0u;
+                if (c) place[k] = __ldcg(st + b) + atomicAdd(cur + b, (unsigned long long)c);
+            }
+            for (uint32_t b = threadIdx.x + 2 * kThreads; b < nb; b += kThreads) {
+                const uint32_t c = s_cnt[b];
+                if (c) s_base[b] = __ldcg(st + b) + atomicAdd(cur + b, (unsigned long long)c);
+            }
             const uint32_t n_tile = block_exclusive_scan(s_cnt, nb, s_warp);
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
-                if (valid[j]) {
+                if (valid >> j & 1u) {
                     const uint32_t slot = s_cnt[rec[j][half] >> shift] + rank[j];
                     if (W == 2) {
                         reinterpret_cast<uint2*>(s_stage)[slot] = make_uint2(rec[j][0], rec[j][1]);
@@ -472,29 +539,28 @@ __device__ __forceinline__ void bucket_scatter_block(const uint8_t* __restrict__
                     }
                 }
             }
-            __syncthreads();
-            unsigned long long* base = s_base + (size_t)half * nb;
-            for (uint32_t i = threadIdx.x; i < n_tile; i += blockDim.x) {
-                const uint32_t* r = s_stage + i * W;
-                const uint32_t b = r[half] >> shift;
-                const uint64_t pos = base[b] + (i - s_cnt[b]);
-                uint32_t* o = reinterpret_cast<uint32_t*>(out + pos * REC);
-                if (W == 2) {  // 8-byte records: one 8-byte store, kept in L2 (the next tile's run
-                               // of the same bucket completes its partial sectors)
-                    const uint2 q = *reinterpret_cast<const uint2*>(r);
-                    asm volatile("st.global.L2::cache_hint.v2.u32 [%0], {%1, %2}, %3;" ::"l"(o), "r"(q.x), "r"(q.y),
-                                 "l"(keep)
-                                 : "memory");
-                } else {
+            // the next tile's records, on their way while this tile's second half goes out
+            if (half == 1 && t0 + (uint64_t)gridDim.x * kTile < E) load_tile(t0 + (uint64_t)gridDim.x * kTile);
 #pragma unroll
-                    for (int w = 0; w < W; ++w) o[w] = r[w];
-                }
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t b = threadIdx.x + k * kThreads;
+                if (b < nb) s_base[b] = place[k] - s_cnt[b];
             }
+            for (uint32_t b = threadIdx.x + 2 * kThreads; b < nb; b += kThreads) s_base[b] -= s_cnt[b];
             __syncthreads();
-            // advance the block's running bases by this tile's counts (start[b+1] - start[b])
-            for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) {
-                const uint32_t next = b + 1 < nb ? s_cnt[b + 1] : n_tile;
-                base[b] += next - s_cnt[b];
+            if (W == 2) {
+                for (uint32_t i = threadIdx.x; i < n_tile; i += kThreads) {
+                    const uint2 q = reinterpret_cast<const uint2*>(s_stage)[i];
+                    const uint64_t pos = s_base[(half ? q.y : q.x) >> shift] + i;
+                    __stcg(reinterpret_cast<uint2*>(out) + pos, q);
+                }
+            } else {  // word by word, so that a warp's stores are contiguous
+                uint32_t* o = reinterpret_cast<uint32_t*>(out);
+                for (uint32_t i = threadIdx.x; i < n_tile * W; i += kThreads) {
+                    const uint32_t r = i / W;
+                    const uint64_t pos = s_base[s_stage[r * W + half] >> shift] + r;
+                    __stcg(o + pos * W + (i - r * W), s_stage[i]);
+                }
             }
             __syncthreads();
         }
@@ -502,12 +568,12 @@ __device__ __forceinline__ void bucket_scatter_block(const uint8_t* __restrict__
 }
 
 template <int REC, bool kCheck>
-__global__ void __launch_bounds__(kScatterThreads) k_bucket_scatter(const uint8_t* __restrict__ edges, uint64_t E,
-                                                                    uint64_t chunk, int shift, uint32_t nb, uint32_t nblk,
-                                                                    const uint64_t* __restrict__ excl,
-                                                                    uint8_t* __restrict__ out, uint32_t V) {
+__global__ void __launch_bounds__(kBucketThreads)
+    k_bucket_scatter(const uint8_t* __restrict__ edges, uint64_t E, int shift, uint32_t nb,
+                     const uint64_t* __restrict__ start, unsigned long long* __restrict__ cursor,
+                     uint8_t* __restrict__ out, uint32_t V) {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    bucket_scatter_block<REC, kCheck>(edges, E, chunk, shift, nb, nblk, excl, out, V, blockIdx.x, s_raw);
+    bucket_scatter_tiles<REC, kCheck>(edges, E, shift, nb, start, cursor, out, V, s_raw);
 }
 
 // Visit records [r0, r1) of a bucket with several loads in flight per thread.  8-byte records go
@@ -560,15 +626,13 @@ __device__ __forceinline__ void st_keep_u32(uint32_t* p, uint32_t v, unsigned lo
 
 // The bucketed records of a build come in K parts (an upload in pieces scatters each piece as it
 // lands): part k holds 2 x E_k records from record 2 * e0_k on, bucket-sorted per half, with
-// excl[k] its exclusive scan over (half, bucket, block) of nblk[k] blocks (entry 2 * nb * nblk[k]
-// the part's total).  Bucket b of half h is the union over k of
-// [2 e0_k + excl_k[(h nb + b) nblk_k], 2 e0_k + excl_k[(h nb + b + 1) nblk_k]).
+// start[k] its exclusive scan over (half, bucket).  Bucket b of half h is the union over k of
+// [2 e0_k + start_k[h nb + b], 2 e0_k + start_k[h nb + b + 1]).
 constexpr int kMaxParts = 8;
 struct BuildParts {
     int K;
     uint64_t base2[kMaxParts];          // 2 * e0_k
-    const uint64_t* excl[kMaxParts];
-    uint32_t nblk[kMaxParts];
+    const uint64_t* start[kMaxParts];
 };
 
 // C: one bucket per CTA iteration (persistent CTAs take buckets from a ticket); s_cnt: LB counters
@@ -595,10 +659,9 @@ __device__ __forceinline__ void bucket_build_loop(const uint8_t* __restrict__ re
         if (threadIdx.x == 0) {
             uint64_t r0 = 0, len = 0;
             for (int k = 0; k < parts.K; ++k) {
-                const uint64_t* ex = parts.excl[k];
-                const uint64_t nbk = parts.nblk[k];
-                const uint64_t lo = ex[((uint64_t)half * nb + b) * nbk], hi = ex[((uint64_t)half * nb + b + 1) * nbk];
-                r0 += lo - ex[(uint64_t)half * nb * nbk];  // this part's records of earlier buckets
+                const uint64_t* st = parts.start[k] + (uint64_t)half * nb;
+                const uint64_t lo = __ldcg(st + b), hi = __ldcg(st + b + 1);
+                r0 += lo - __ldcg(st);  // this part's records of earlier buckets
                 len += hi - lo;
                 s_lo[k] = parts.base2[k] + lo;
                 s_hi[k] = parts.base2[k] + hi;
@@ -634,7 +697,7 @@ __device__ __forceinline__ void bucket_build_loop(const uint8_t* __restrict__ re
 }
 
 template <int REC>
-__global__ void __launch_bounds__(kBuildThreads) k_bucket_build(const uint8_t* __restrict__ rec, BuildParts parts,
+__global__ void __launch_bounds__(kBucketThreads) k_bucket_build(const uint8_t* __restrict__ rec, BuildParts parts,
                                                                  int half, uint32_t nb, uint32_t LB, uint32_t V,
                                                                  uint32_t* __restrict__ deg, uint64_t* __restrict__ off,
                                                                  uint32_t* __restrict__ adj, float* __restrict__ wout,
@@ -645,27 +708,38 @@ __global__ void __launch_bounds__(kBuildThreads) k_bucket_build(const uint8_t* _
 
 struct BucketPlan {
     int shift;
-    uint32_t LB, nb, nblk;
-    uint64_t chunk;
+    uint32_t LB, nb;
+    size_t smem;     // the largest of the three passes
+    uint32_t nblk;   // pass A blocks
+    uint64_t chunk;  // records per pass A block
 };
 
-static BucketPlan plan_buckets(uint32_t V, uint64_t E) {
+// Buckets: about 1,024, and more while pass C's scattered stores would cover more than L2 (one
+// bucket's output per SM) and pass B's runs stay 8 records long on average.  2^25 / 2^29: 1,024 / 2,048 /
+// 4,096 buckets take 4.4 / 5.2 / 7.0 ms in pass B, 9.9 / 7.9 / 6.9 in pass C; 10.4 M / 734 M: 636 / 1,272 /
+// 2,543 buckets 5.8 / 6.2 / 7.9 and 12.9 / 10.5 / 8.8; 2^22 / 2^26, where 1,024 fit: 0.57 / 0.66 / 0.83 and
+// 0.98 / 0.89 / 0.92.  (With frontiers per block, 2^25 / 2^29 took 4.8 / 7.9 ms in pass B at 1,024 / 2,048.)
+static BucketPlan plan_buckets(uint32_t V, uint64_t E, int rec) {
     BucketPlan p;
     uint32_t lb = 256;
-    while (lb < kMaxBucketVerts && (uint64_t)lb * 1024 < V) lb <<= 1;  // aim for >= 1024 buckets
+    while (lb < kMaxBucketVerts && (uint64_t)lb * 1024 < V) lb <<= 1;
+    const uint64_t out_bytes = E * (rec - 4);  // of one structure
+    while (lb > 256 && ((uint64_t)V + lb - 1) / lb <= 1280 && out_bytes / std::max<uint64_t>(V / lb, 1) * 152 > (100ull << 20))
+        lb >>= 1;
     p.LB = lb;
     p.shift = 0;
     while ((1u << p.shift) < lb) ++p.shift;
     p.nb = (uint32_t)(((uint64_t)V + lb - 1) / lb);
+    p.smem = std::max({scatter_smem(rec, p.nb), sizeof(uint32_t) * (size_t)lb, sizeof(uint32_t) * 2 * (size_t)p.nb});
     uint64_t want = (E + 65535) / 65536;
-    p.nblk = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, 304));
+    p.nblk = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, 608));
     p.chunk = (E + p.nblk - 1) / p.nblk;
     p.chunk = (p.chunk + 63) & ~63ull;
     p.nblk = (uint32_t)std::max<uint64_t>(1, (E + p.chunk - 1) / p.chunk);
     return p;
 }
+static bool plan_fits(const BucketPlan& p) { return p.smem <= 224 * 1024; }
 
-int scan_exclusive_u32(eg_graph* g, const uint32_t* in, uint64_t n, uint64_t* out);
 
 // the handle's stream waits for part k of an upload (once the uploader has recorded its event)
 static int wait_upload_part(eg_graph* g, const UploadParts* up, int k) {
@@ -709,72 +783,65 @@ static int build_single(eg_graph* g, const UploadParts* up) {
     const int K = up ? up->K : 1;
     std::vector<uint64_t> e0(K + 1, 0);
     for (int k = 0; k <= K; ++k) e0[k] = up ? up->e0[k] : (k ? E : 0);
-    std::vector<BucketPlan> pl(K);
-    std::vector<uint64_t> co(K + 1, 0), oo(K + 1, 0);  // count / offset table positions per part
-    for (int k = 0; k < K; ++k) {
-        pl[k] = plan_buckets(V, e0[k + 1] - e0[k]);
-        co[k + 1] = co[k] + 2ull * pl[k].nb * pl[k].nblk;
-        oo[k + 1] = oo[k] + 2ull * pl[k].nb * pl[k].nblk + 1;
-    }
-    const uint32_t nb = pl[0].nb, LB = pl[0].LB;
-    const int shift = pl[0].shift;
-    EG_TRY(g->bucket_cnt.reserve(sizeof(uint32_t) * co[K]));
-    EG_TRY(g->bucket_off.reserve(sizeof(uint64_t) * oo[K]));
+    const BucketPlan whole = plan_buckets(V, E, rec);
+    const uint32_t nb = whole.nb, LB = whole.LB;
+    const int shift = whole.shift;
+    const size_t table = 2ull * nb + 2;  // words of one part's table: totals, cursors or starts
+    EG_TRY(g->bucket_cnt.reserve(sizeof(uint64_t) * table * 2 * K));
+    EG_TRY(g->bucket_off.reserve(sizeof(uint64_t) * table * K));
     EG_TRY(g->bucketed.reserve((size_t)2 * E * rec + 64));
     EG_TRY(g->scan.counter.reserve(16));
     int* bad = g->err.as<int>() + 1;
     EG_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), g->stream));
+    EG_CUDA(cudaMemsetAsync(g->bucket_cnt.ptr, 0, sizeof(uint64_t) * table * 2 * K, g->stream));
     const size_t smem_a = sizeof(uint32_t) * 2 * nb;
-    const size_t smem_b = align16(20ull * nb) + (size_t)scatter_tile(rec) * rec;  // [2][nb] u64, [nb] u32, tile
-    auto scatter_fn = [&]() -> const void* {
-        if (rec == 8) return up ? (const void*)k_bucket_scatter<8, true> : (const void*)k_bucket_scatter<8, false>;
-        return up ? (const void*)k_bucket_scatter<12, true> : (const void*)k_bucket_scatter<12, false>;
-    };
-    EG_CUDA(cudaFuncSetAttribute(scatter_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
-    if (rec == 8)
-        EG_CUDA(cudaFuncSetAttribute(k_bucket_hist<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
-    else
-        EG_CUDA(cudaFuncSetAttribute(k_bucket_hist<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    const size_t smem_b = scatter_smem(rec, nb);
+    const size_t smem_c = sizeof(uint32_t) * LB;
+    const void* fn_a = rec == 8 ? (const void*)k_bucket_hist<8> : (const void*)k_bucket_hist<12>;
+    const void* fn_b = rec == 8 ? (up ? (const void*)k_bucket_scatter<8, true> : (const void*)k_bucket_scatter<8, false>)
+                                : (up ? (const void*)k_bucket_scatter<12, true> : (const void*)k_bucket_scatter<12, false>);
+    const void* fn_c = rec == 8 ? (const void*)k_bucket_build<8> : (const void*)k_bucket_build<12>;
+    EG_CUDA(cudaFuncSetAttribute(fn_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a));
+    EG_CUDA(cudaFuncSetAttribute(fn_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+    EG_CUDA(cudaFuncSetAttribute(fn_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
+    int per_sm_b = 1, per_sm_c = 1;
+    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_b, fn_b, kBucketThreads, smem_b));
+    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, fn_c, kBucketThreads, smem_c));
     BuildParts parts{};
     parts.K = K;
     for (int k = 0; k < K; ++k) {
         if (up) EG_TRY(wait_upload_part(g, up, k));
         const uint64_t Ek = e0[k + 1] - e0[k];
         const uint8_t* src = g->edges.as<uint8_t>() + (size_t)e0[k] * rec;
-        uint32_t* cnt = g->bucket_cnt.as<uint32_t>() + co[k];
-        uint64_t* ex = g->bucket_off.as<uint64_t>() + oo[k];
+        unsigned long long* tot = g->bucket_cnt.as<unsigned long long>() + table * 2 * k;
+        unsigned long long* cursor = tot + table;
+        uint64_t* start = g->bucket_off.as<uint64_t>() + table * k;
         uint8_t* out = g->bucketed.as<uint8_t>() + (size_t)2 * e0[k] * rec;
-        const BucketPlan& q = pl[k];
+        const BucketPlan q = plan_buckets(V, Ek, rec);
         {
             Timed t(&g->prof, g->stream, "bucket_hist");
             if (rec == 8)
-                k_bucket_hist<8><<<q.nblk, kBucketThreads, smem_a, g->stream>>>(src, Ek, q.chunk, shift, nb, q.nblk, cnt,
-                                                                                 V, bad);
+                k_bucket_hist<8><<<q.nblk, kBucketThreads, smem_a, g->stream>>>(src, Ek, q.chunk, shift, nb, tot, V, bad);
             else
-                k_bucket_hist<12><<<q.nblk, kBucketThreads, smem_a, g->stream>>>(src, Ek, q.chunk, shift, nb, q.nblk,
-                                                                                  cnt, V, bad);
+                k_bucket_hist<12><<<q.nblk, kBucketThreads, smem_a, g->stream>>>(src, Ek, q.chunk, shift, nb, tot, V, bad);
             EG_CHECK_LAUNCH("k_bucket_hist");
         }
-        EG_TRY(scan_exclusive_u32(g, cnt, co[k + 1] - co[k], ex));
+        k_bucket_starts<<<1, 1024, 0, g->stream>>>(tot, 2 * nb, start);
+        EG_CHECK_LAUNCH("k_bucket_starts");
         {
             Timed t(&g->prof, g->stream, "bucket_scatter");
-            if (rec == 8 && up)
-                k_bucket_scatter<8, true><<<q.nblk, kScatterThreads, smem_b, g->stream>>>(src, Ek, q.chunk, shift, nb,
-                                                                                          q.nblk, ex, out, V);
-            else if (rec == 8)
-                k_bucket_scatter<8, false><<<q.nblk, kScatterThreads, smem_b, g->stream>>>(src, Ek, q.chunk, shift, nb,
-                                                                                           q.nblk, ex, out, V);
-            else if (up)
-                k_bucket_scatter<12, true><<<q.nblk, kScatterThreads, smem_b, g->stream>>>(src, Ek, q.chunk, shift, nb,
-                                                                                           q.nblk, ex, out, V);
-            else
-                k_bucket_scatter<12, false><<<q.nblk, kScatterThreads, smem_b, g->stream>>>(src, Ek, q.chunk, shift,
-                                                                                            nb, q.nblk, ex, out, V);
+            const uint32_t tile = scatter_tile(rec);
+            const unsigned grid = (unsigned)std::max<uint64_t>(
+                1, std::min<uint64_t>((Ek + tile - 1) / tile, (uint64_t)g->num_sms * (uint64_t)std::max(per_sm_b, 1)));
+            uint64_t Ea = Ek;
+            uint32_t nba = nb, Va = V;
+            int sh = shift;
+            void* args[] = {&src, &Ea, &sh, &nba, &start, &cursor, &out, &Va};
+            EG_CUDA(cudaLaunchKernel(fn_b, dim3(grid), dim3(kBucketThreads), args, smem_b, g->stream));
             EG_CHECK_LAUNCH("k_bucket_scatter");
         }
         parts.base2[k] = 2 * e0[k];
-        parts.excl[k] = ex;
-        parts.nblk[k] = q.nblk;
+        parts.start[k] = start;
     }
     if (up) {  // an upload validates in pass A: ids >= V stop the build here
         int h = 0;
@@ -785,30 +852,19 @@ static int build_single(eg_graph* g, const UploadParts* up) {
             return EG_ERR_INVALID;
         }
     }
-    const size_t smem_c = sizeof(uint32_t) * LB;
-    if (rec == 8) EG_CUDA(cudaFuncSetAttribute(k_bucket_build<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
-    else EG_CUDA(cudaFuncSetAttribute(k_bucket_build<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
-    int per_sm = 1;
-    if (rec == 8)
-        EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bucket_build<8>, kBuildThreads, smem_c));
-    else
-        EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bucket_build<12>, kBuildThreads, smem_c));
-    const unsigned grid = std::min<uint32_t>(nb, (uint32_t)g->num_sms * (uint32_t)std::max(per_sm, 1));
+    const unsigned grid = std::min<uint32_t>(nb, (uint32_t)g->num_sms * (uint32_t)std::max(per_sm_c, 1));
     for (int half = 0; half < 2; ++half) {
         EG_CUDA(cudaMemsetAsync(g->scan.counter.ptr, 0, 4, g->stream));
         Timed t(&g->prof, g->stream, "bucket_build");
+        const uint8_t* recs = g->bucketed.as<uint8_t>();
         uint32_t* deg = half == 0 ? g->outdeg.as<uint32_t>() : g->indeg.as<uint32_t>();
         uint64_t* off = half == 0 ? g->csr_off.as<uint64_t>() : g->csc_off.as<uint64_t>();
         uint32_t* adj = half == 0 ? g->csr_adj.as<uint32_t>() : g->csc_adj.as<uint32_t>();
         float* w = half == 0 ? g->csr_w.as<float>() : g->csc_w.as<float>();
-        if (rec == 8)
-            k_bucket_build<8><<<grid, kBuildThreads, smem_c, g->stream>>>(g->bucketed.as<uint8_t>(), parts, half, nb, LB,
-                                                                          V, deg, off, adj, w,
-                                                                          g->scan.counter.as<uint32_t>());
-        else
-            k_bucket_build<12><<<grid, kBuildThreads, smem_c, g->stream>>>(g->bucketed.as<uint8_t>(), parts, half, nb,
-                                                                           LB, V, deg, off, adj, w,
-                                                                           g->scan.counter.as<uint32_t>());
+        uint32_t* ticket = g->scan.counter.as<uint32_t>();
+        uint32_t nba = nb, LBa = LB, Va = V;
+        void* args[] = {&recs, &parts, &half, &nba, &LBa, &Va, &deg, &off, &adj, &w, &ticket};
+        EG_CUDA(cudaLaunchKernel(fn_c, dim3(grid), dim3(kBucketThreads), args, smem_c, g->stream));
         EG_CHECK_LAUNCH("k_bucket_build");
     }
     return EG_OK;
@@ -847,8 +903,9 @@ struct PersistBuildArgs {
     uint64_t chunk;
     int shift;
     uint32_t nb, nblk, LB;
-    uint32_t* cnt;
-    uint64_t* ex;
+    unsigned long long* tot;     // records per (half, bucket)
+    unsigned long long* cursor;  // records placed so far
+    uint64_t* start;
     uint8_t* bucketed;
     BuildParts parts;
     uint32_t *outdeg, *indeg;
@@ -876,35 +933,6 @@ __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t* s_red) {
     }
     __syncthreads();
     const uint64_t r = s_red[32];
-    __syncthreads();
-    return r;
-}
-
-// exclusive prefix of one value per thread over the block; *total: the block's sum
-__device__ __forceinline__ uint64_t block_excl_u64(uint64_t v, uint64_t* s_red, uint64_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint64_t inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) s_red[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        const uint64_t x = lane < nw ? s_red[lane] : 0ull;
-        uint64_t y = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t z = __shfl_up_sync(0xffffffffu, y, o);
-            if (lane >= o) y += z;
-        }
-        if (lane < nw) s_red[lane] = y - x;
-        if (lane == 31) s_red[32] = y;
-    }
-    __syncthreads();
-    const uint64_t r = s_red[warp] + inc - v;
-    *total = s_red[32];
     __syncthreads();
     return r;
 }
@@ -956,7 +984,7 @@ __device__ bool grid_scan(Load load, Epi epi, uint64_t n, BuildWords* w, uint64_
 // pass.  Four 16-byte loads in flight per thread (12-byte records: four records in three loads).
 template <int REC>
 __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t E, uint64_t chunk, int shift, uint32_t nb,
-                                                 uint32_t nblk, uint32_t* __restrict__ cnt, uint32_t V, int* bad,
+                                                 unsigned long long* __restrict__ tot, uint32_t V, int* bad,
                                                  uint32_t blk, uint32_t* s_h) {
     for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) s_h[i] = 0;
     __syncthreads();
@@ -1035,32 +1063,27 @@ __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t
     }
     if (out_of_range) atomicExch(bad, 1);
     __syncthreads();
-    // bucket-major layout: [half][bucket][block]
-    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x) cnt[(uint64_t)i * nblk + blk] = s_h[i];
+    for (uint32_t i = threadIdx.x; i < 2 * nb; i += blockDim.x)
+        if (s_h[i]) atomicAdd(tot + i, (unsigned long long)s_h[i]);
 }
 
 template <int REC>
-__global__ void __launch_bounds__(kBuildThreads, 1) k_build_persistent(PersistBuildArgs a) {
+__global__ void __launch_bounds__(kBucketThreads, 1) k_build_persistent(PersistBuildArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     BuildWords* w = a.w;
     // A: the records in, bucket counts per (half, bucket, block)
     for (uint32_t blk = blockIdx.x; blk < a.nblk; blk += gridDim.x) {
-        load_count_block<REC>(a.src, a.E, a.chunk, a.shift, a.nb, a.nblk, a.cnt, a.V, &w->bad, blk,
+        load_count_block<REC>(a.src, a.E, a.chunk, a.shift, a.nb, a.tot, a.V, &w->bad, blk,
                               reinterpret_cast<uint32_t*>(s_raw));
         __syncthreads();
     }
     if (blockIdx.x == 0 && threadIdx.x < 2) a.part_off[threadIdx.x] = threadIdx.x ? a.V : 0u;  // one partition: [0, V]
     if (!build_barrier(w)) return;
     if (*(volatile int*)&w->bad) return;  // every CTA reads the same flag after the barrier
-    const uint64_t ncnt = 2ull * a.nb * a.nblk;
-    if (!grid_scan(LoadU32{a.cnt}, EpiExclusive{a.ex}, ncnt, w, a.ex + ncnt)) return;
+    if (blockIdx.x == 0) bucket_starts(a.tot, 2 * a.nb, a.start);
     if (!build_barrier(w)) return;
     // B: records bucket-sorted per half
-    for (uint32_t blk = blockIdx.x; blk < a.nblk; blk += gridDim.x) {
-        bucket_scatter_block<REC, false>(a.src.out, a.E, a.chunk, a.shift, a.nb, a.nblk, a.ex, a.bucketed, a.V, blk,
-                                         s_raw);
-        __syncthreads();
-    }
+    bucket_scatter_tiles<REC, false>(a.src.out, a.E, a.shift, a.nb, a.start, a.cursor, a.bucketed, a.V, s_raw);
     if (!build_barrier(w)) return;
     // C: both halves (independent outputs, no barrier between them)
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_raw);
@@ -1077,9 +1100,7 @@ __global__ void __launch_bounds__(kBuildThreads, 1) k_build_persistent(PersistBu
 }
 
 bool persistent_build_fits(const eg_graph* g) {
-    return g->partitions == 1 && g->sub_partitions == 1 && g->E > 0 &&
-           align16(20ull * plan_buckets(g->V, g->E).nb) + (uint64_t)scatter_tile(g->edge_bytes) * g->edge_bytes <=
-               200ull * 1024;
+    return g->partitions == 1 && g->sub_partitions == 1 && g->E > 0 && plan_fits(plan_buckets(g->V, g->E, g->edge_bytes));
 }
 
 int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G, const void* src) {
@@ -1093,8 +1114,8 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     g->built_csr = g->built_csc = false;
     g->eng.pull_ready = false;
     g->eng.pr_ready = false;
-    const BucketPlan q = plan_buckets(V, E);
-    const uint64_t ncnt = 2ull * q.nb * q.nblk;
+    const BucketPlan q = plan_buckets(V, E, rec);
+    const size_t table = 2ull * q.nb + 2;
     const uint64_t nwords = (uint64_t)V / 64 + 1;
     EG_TRY(g->outdeg.reserve(sizeof(uint32_t) * (size_t)V));
     EG_TRY(g->indeg.reserve(sizeof(uint32_t) * (size_t)V));
@@ -1106,8 +1127,8 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
         EG_TRY(g->csr_w.reserve(sizeof(float) * (E + 32)));
         EG_TRY(g->csc_w.reserve(sizeof(float) * (E + 32)));
     }
-    EG_TRY(g->bucket_cnt.reserve(sizeof(uint32_t) * ncnt));
-    EG_TRY(g->bucket_off.reserve(sizeof(uint64_t) * (ncnt + 1)));
+    EG_TRY(g->bucket_cnt.reserve(sizeof(uint64_t) * table * 2));
+    EG_TRY(g->bucket_off.reserve(sizeof(uint64_t) * table));
     EG_TRY(g->bucketed.reserve((size_t)2 * E * rec + 64));
     EG_TRY(g->csr_bitmap.reserve(sizeof(uint64_t) * nwords));
     const uint64_t cap = std::min<uint64_t>(E, V) + 1;
@@ -1117,12 +1138,11 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     BuildWords* w = g->build_words.as<BuildWords>();
     EG_CUDA(cudaMemsetAsync(w, 0, sizeof(BuildWords), g->stream));
 
-    const size_t smem = std::max({sizeof(uint32_t) * 2 * q.nb, align16(20ull * q.nb) + (size_t)scatter_tile(rec) * rec,
-                                  sizeof(uint32_t) * (size_t)q.LB});
+    EG_CUDA(cudaMemsetAsync(g->bucket_cnt.ptr, 0, sizeof(uint64_t) * table * 2, g->stream));
     const void* fn = rec == 8 ? (const void*)k_build_persistent<8> : (const void*)k_build_persistent<12>;
-    EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem));
     int per_sm = 0;
-    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBuildThreads, smem));
+    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBucketThreads, q.smem));
     const int grid = std::min(g->num_sms * per_sm, kPersistBuildMaxCtas);
     if (grid < 1) {
         set_error("eg_build: the one-launch build does not fit an SM");
@@ -1139,14 +1159,14 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     a.nb = q.nb;
     a.nblk = q.nblk;
     a.LB = q.LB;
-    a.cnt = g->bucket_cnt.as<uint32_t>();
-    a.ex = g->bucket_off.as<uint64_t>();
+    a.tot = g->bucket_cnt.as<unsigned long long>();
+    a.cursor = a.tot + table;
+    a.start = g->bucket_off.as<uint64_t>();
     a.bucketed = g->bucketed.as<uint8_t>();
     a.parts = BuildParts{};
     a.parts.K = 1;
     a.parts.base2[0] = 0;
-    a.parts.excl[0] = a.ex;
-    a.parts.nblk[0] = q.nblk;
+    a.parts.start[0] = a.start;
     a.outdeg = g->outdeg.as<uint32_t>();
     a.indeg = g->indeg.as<uint32_t>();
     a.csr_off = g->csr_off.as<uint64_t>();
@@ -1163,7 +1183,7 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     void* kargs[] = {&a};
     {
         Timed t(&g->prof, g->stream, "build_persistent");
-        EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(kBuildThreads), kargs, smem, g->stream));
+        EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)grid), dim3(kBucketThreads), kargs, q.smem, g->stream));
         EG_CHECK_LAUNCH("k_build_persistent");
     }
     BuildWords hw;  // the flags and the index range (the per-CTA sums are not needed)
@@ -1313,9 +1333,7 @@ int build_structures(eg_graph* g, int want_csr, int want_csc, const UploadParts*
 
     if (g->build_launch && !up && persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0, nullptr);
     // the bucket tables and a staging tile must fit one CTA's shared memory
-    const bool bucketed =
-        P == 1 && align16(20ull * plan_buckets(V, E).nb) + (uint64_t)scatter_tile(g->edge_bytes) * g->edge_bytes <=
-                      200ull * 1024;
+    const bool bucketed = P == 1 && plan_fits(plan_buckets(V, E, g->edge_bytes));
     if (bucketed) {
         // one partition: both structures (and both degree arrays) from the bucketed build
         want_csr = want_csc = 1;
