@@ -210,7 +210,7 @@ bool direct_records(const eg_graph* g, const void* edges, int where) {
 }
 
 // argument checks, state reset and the record buffer of a new edge list
-int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric) {
+int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric, bool keep_list) {
     if (edge_bytes != 8 && edge_bytes != 12) {
         set_error("eg_load_edges: edge_bytes must be 8 ({src,dst}) or 12 ({src,dst,float})");
         return EG_ERR_INVALID;
@@ -237,8 +237,30 @@ int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmet
     g->edge_bytes = edge_bytes;
     g->weighted = edge_bytes == 12;
     g->symmetric = symmetric != 0;
-    EG_TRY(g->edges.reserve((size_t)total * edge_bytes + 64));
+    g->list_in_csr = !keep_list;
+    if (keep_list) EG_TRY(g->edges.reserve((size_t)total * edge_bytes + 64));
     return EG_OK;
+}
+
+// Load and build in one: the one-launch build reads the caller's device records where they are (host
+// records from the handle's buffer), checks and counts them in one pass, and takes every record both
+// ways for a symmetrised list, whose in-lists are its out-lists.  *done: false when another path has
+// to take the call (no such build, or records that cannot be read in place).
+static int load_build_direct(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int edge_bytes, int symmetric,
+                             int where, bool* done) {
+    *done = false;
+    if (!g->build_launch || !edges || !E) return EG_OK;
+    const bool host = where == EG_HOST;
+    if (!host && !direct_records(g, edges, where)) return EG_OK;
+    EG_TRY(prepare_load(g, E, V, edge_bytes, symmetric, false));
+    if (!persistent_build_fits(g)) return EG_OK;
+    *done = true;
+    if (host) {
+        EG_TRY(g->edges.reserve((size_t)E * edge_bytes + 64));
+        EG_CUDA(cudaMemcpyAsync(g->edges.ptr, edges, (size_t)E * edge_bytes, cudaMemcpyHostToDevice, g->stream));
+        if (!symmetric) g->list_in_csr = false;
+    }
+    return build_persistent(g, nullptr, nullptr, 0, host ? g->edges.ptr : edges);
 }
 
 // preload_graph_file (core/graph.hpp:1011-1084) for one rank: the whole file, read in 128 MiB
@@ -718,6 +740,7 @@ int eg_build(eg_graph* g, int want_csr, int want_csc) {
         return EG_ERR_STATE;
     }
     free_batch_state(g);
+    EG_TRY(ensure_list(g));
     return build_structures(g, want_csr, want_csc);
 }
 
@@ -737,6 +760,7 @@ int eg_load_directed_with_ids(eg_graph* g, const void* edges, uint64_t E, uint32
     g->edge_bytes = 12;
     g->weighted = 1;
     g->symmetric = 0;
+    g->list_in_csr = false;
     g->edge_ids = true;
     EG_TRY(g->edges.reserve((size_t)E * 12 + 64));
     EG_TRY(g->bucketed.reserve((size_t)E * 8 + 64));
@@ -776,20 +800,20 @@ int eg_load_directed(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int
         EG_TRY(check_graph(g, "eg_load_directed"));
         return eg::load_build_pipelined(g, edges, E, V, edge_bytes);
     }
-    if (g && edges && E) {
-        EG_TRY(check_graph(g, "eg_load_directed"));
-        if (g->build_launch && direct_records(g, edges, where)) {
-            EG_TRY(prepare_load(g, E, V, edge_bytes, 0));
-            // the one-launch build copies, checks and counts the records in one pass
-            if (persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0, edges);
-        }
-    }
+    EG_TRY(check_graph(g, "eg_load_directed"));
+    bool done = false;
+    const int st = load_build_direct(g, edges, E, V, edge_bytes, 0, where, &done);
+    if (done || st != EG_OK) return st;
     EG_TRY(eg_load_edges(g, edges, E, V, edge_bytes, 0, where));
     return eg_build(g, 1, 1);
 }
 
 int eg_load_undirected_from_directed(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int edge_bytes,
                                      int where) {
+    EG_TRY(check_graph(g, "eg_load_undirected_from_directed"));
+    bool done = false;
+    const int st = load_build_direct(g, edges, E, V, edge_bytes, 1, where, &done);
+    if (done || st != EG_OK) return st;
     EG_TRY(eg_load_edges(g, edges, E, V, edge_bytes, 1, where));
     return eg_build(g, 1, 1);
 }

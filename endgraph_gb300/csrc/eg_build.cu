@@ -460,12 +460,14 @@ __host__ __device__ constexpr size_t scatter_smem(int rec, uint32_t nb) {
 
 // kCheck: skip records with an id >= V as pass A did (an upload validated in pass A); edge lists
 // validated at load leave it off
+// sym: one set of buckets takes every record twice, as it is and reversed
 // Tiles blockIdx.x, blockIdx.x + gridDim.x, ... (s_raw: the bucket tables and the staging tile)
 template <int REC, bool kCheck>
 __device__ __forceinline__ void bucket_scatter_tiles(const uint8_t* __restrict__ edges, uint64_t E, int shift, uint32_t nb,
                                                      const uint64_t* __restrict__ start,
                                                      unsigned long long* __restrict__ cursor,
-                                                     uint8_t* __restrict__ out, uint32_t V, unsigned char* s_raw) {
+                                                     uint8_t* __restrict__ out, uint32_t V, unsigned char* s_raw,
+                                                     bool sym = false) {
     constexpr int W = REC / 4;  // words per record
     constexpr int kPer = scatter_per(REC);
     constexpr uint32_t kTile = scatter_tile(REC), kThreads = kBucketThreads;
@@ -513,8 +515,9 @@ __device__ __forceinline__ void bucket_scatter_tiles(const uint8_t* __restrict__
             __syncthreads();
             // the runs' places: one round trip per bucket and tile, on its way while the counts are
             // scanned (the first two buckets of a thread, all of them up to 2,048)
-            unsigned long long* cur = cursor + (uint64_t)half * nb;
-            const uint64_t* st = start + (uint64_t)half * nb;
+            unsigned long long* cur = cursor + (sym ? 0ull : (uint64_t)half * nb);
+            const uint64_t* st = start + (sym ? 0ull : (uint64_t)half * nb);
+            const bool swap = sym && half == 1;  // the reversed copy: keyed and stored by its own source
             unsigned long long place[2] = {0, 0};
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -532,10 +535,13 @@ __device__ __forceinline__ void bucket_scatter_tiles(const uint8_t* __restrict__
                 if (valid >> j & 1u) {
                     const uint32_t slot = s_cnt[rec[j][half] >> shift] + rank[j];
                     if (W == 2) {
-                        reinterpret_cast<uint2*>(s_stage)[slot] = make_uint2(rec[j][0], rec[j][1]);
+                        reinterpret_cast<uint2*>(s_stage)[slot] =
+                            swap ? make_uint2(rec[j][1], rec[j][0]) : make_uint2(rec[j][0], rec[j][1]);
                     } else {
+                        s_stage[slot * W] = swap ? rec[j][1] : rec[j][0];
+                        s_stage[slot * W + 1] = swap ? rec[j][0] : rec[j][1];
 #pragma unroll
-                        for (int w = 0; w < W; ++w) s_stage[slot * W + w] = rec[j][w];
+                        for (int w = 2; w < W; ++w) s_stage[slot * W + w] = rec[j][w];
                     }
                 }
             }
@@ -551,14 +557,14 @@ __device__ __forceinline__ void bucket_scatter_tiles(const uint8_t* __restrict__
             if (W == 2) {
                 for (uint32_t i = threadIdx.x; i < n_tile; i += kThreads) {
                     const uint2 q = reinterpret_cast<const uint2*>(s_stage)[i];
-                    const uint64_t pos = s_base[(half ? q.y : q.x) >> shift] + i;
+                    const uint64_t pos = s_base[(half && !sym ? q.y : q.x) >> shift] + i;
                     __stcg(reinterpret_cast<uint2*>(out) + pos, q);
                 }
             } else {  // word by word, so that a warp's stores are contiguous
                 uint32_t* o = reinterpret_cast<uint32_t*>(out);
                 for (uint32_t i = threadIdx.x; i < n_tile * W; i += kThreads) {
                     const uint32_t r = i / W;
-                    const uint64_t pos = s_base[s_stage[r * W + half] >> shift] + r;
+                    const uint64_t pos = s_base[s_stage[r * W + (sym ? 0 : half)] >> shift] + r;
                     __stcg(o + pos * W + (i - r * W), s_stage[i]);
                 }
             }
@@ -889,10 +895,11 @@ struct BuildWords {
 // Where the records come from: a caller's device buffer, or the handle's own list
 struct RecordSource {
     const uint8_t* in;
-    uint8_t* out;          // the handle's list (may be `in`)
+    uint8_t* out;          // graph batch: the handle's list, with the ids of the union (may be `in`)
     const uint64_t* eoff;  // graph batch: record offsets (G + 1), null for one graph
     const uint64_t* voff;  // graph batch: vertex offsets (G + 1)
     uint32_t G;
+    int sym;               // every record stands for itself and for its reverse
 };
 
 struct PersistBuildArgs {
@@ -979,9 +986,9 @@ __device__ bool grid_scan(Load load, Epi epi, uint64_t n, BuildWords* w, uint64_
 
 // Pass A of the one-launch build: one block `blk` reads its records (from the caller's buffer when it
 // is device memory), checks the ids (against V, or against the record's own graph in a batch, whose
-// ids it moves to the union), keeps them in the handle's list and counts the buckets: one read and
-// one write of the list in place of a copy, a validation pass, the batch's id move and a counting
-// pass.  Four 16-byte loads in flight per thread (12-byte records: four records in three loads).
+// ids it moves to the union in the handle's list) and counts the buckets: one read of the list in
+// place of a copy, a validation pass and a counting pass.  Four 16-byte loads in flight per thread
+// (12-byte records: four records in three loads).
 template <int REC>
 __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t E, uint64_t chunk, int shift, uint32_t nb,
                                                  unsigned long long* __restrict__ tot, uint32_t V, int* bad,
@@ -990,7 +997,8 @@ __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t
     __syncthreads();
     const uint64_t e0 = blk * chunk;
     const uint64_t e1 = e0 + chunk < E ? e0 + chunk : E;
-    const bool keep = r.out != r.in || r.eoff;
+    const bool keep = r.eoff != nullptr;
+    uint32_t* s_hd = r.sym ? s_h : s_h + nb;  // a symmetrised list has one set of buckets
     bool out_of_range = false;
     uint32_t lo = 0;  // graph of this thread's previous record (its records only move forward)
     auto take = [&](uint64_t i, uint32_t& s, uint32_t& d) {
@@ -1014,7 +1022,7 @@ __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t
             return;
         }
         atomicAdd(&s_h[s >> shift], 1u);
-        atomicAdd(&s_h[nb + (d >> shift)], 1u);
+        atomicAdd(&s_hd[d >> shift], 1u);
     };
     // groups of 16 * kVec bytes: 2 records of 8 bytes, 4 of 12 (chunks are multiples of 64 records)
     constexpr int kVec = REC == 8 ? 1 : 3, kRecs = REC == 8 ? 2 : 4, kInFlight = REC == 8 ? 4 : 2;
@@ -1067,6 +1075,22 @@ __device__ __forceinline__ void load_count_block(const RecordSource& r, uint64_t
         if (s_h[i]) atomicAdd(tot + i, (unsigned long long)s_h[i]);
 }
 
+// n words from one array to another by the whole grid (both 16-byte aligned)
+__device__ __forceinline__ void copy_words(const uint32_t* __restrict__ from, uint32_t* __restrict__ to, uint64_t n) {
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    constexpr int kInFlight = 4;
+    for (uint64_t q = tid; q < n / 4; q += stride * kInFlight) {
+        uint4 x[kInFlight];
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u)
+            if (q + u * stride < n / 4) x[u] = __ldcs(reinterpret_cast<const uint4*>(from) + q + u * stride);
+#pragma unroll
+        for (int u = 0; u < kInFlight; ++u)
+            if (q + u * stride < n / 4) __stcs(reinterpret_cast<uint4*>(to) + q + u * stride, x[u]);
+    }
+    for (uint64_t i = (n & ~3ull) + tid; i < n; i += stride) to[i] = from[i];
+}
+
 template <int REC>
 __global__ void __launch_bounds__(kBucketThreads, 1) k_build_persistent(PersistBuildArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -1080,23 +1104,35 @@ __global__ void __launch_bounds__(kBucketThreads, 1) k_build_persistent(PersistB
     if (blockIdx.x == 0 && threadIdx.x < 2) a.part_off[threadIdx.x] = threadIdx.x ? a.V : 0u;  // one partition: [0, V]
     if (!build_barrier(w)) return;
     if (*(volatile int*)&w->bad) return;  // every CTA reads the same flag after the barrier
-    if (blockIdx.x == 0) bucket_starts(a.tot, 2 * a.nb, a.start);
+    const bool sym = a.src.sym != 0;
+    if (blockIdx.x == 0) bucket_starts(a.tot, sym ? a.nb : 2 * a.nb, a.start);
     if (!build_barrier(w)) return;
     // B: records bucket-sorted per half
-    bucket_scatter_tiles<REC, false>(a.src.out, a.E, a.shift, a.nb, a.start, a.cursor, a.bucketed, a.V, s_raw);
+    bucket_scatter_tiles<REC, false>(a.src.eoff ? a.src.out : a.src.in, a.E, a.shift, a.nb, a.start, a.cursor, a.bucketed,
+                                     a.V, s_raw, sym);
     if (!build_barrier(w)) return;
-    // C: both halves (independent outputs, no barrier between them)
+    // C: both halves (independent outputs, no barrier between them); one when they are the same
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_raw);
     bucket_build_loop<REC>(a.bucketed, a.parts, 0, a.nb, a.LB, a.V, a.outdeg, a.csr_off, a.csr_adj, a.csr_w,
                            &w->ticket[0], s_cnt);
-    __syncthreads();  // every thread has read the last ticket of half 0 before thread 0 takes one of half 1
-    bucket_build_loop<REC>(a.bucketed, a.parts, 1, a.nb, a.LB, a.V, a.indeg, a.csc_off, a.csc_adj, a.csc_w,
-                           &w->ticket[1], s_cnt);
+    if (!sym) {
+        __syncthreads();  // every thread has read the last ticket of half 0 before thread 0 takes one of half 1
+        bucket_build_loop<REC>(a.bucketed, a.parts, 1, a.nb, a.LB, a.V, a.indeg, a.csc_off, a.csc_adj, a.csc_w,
+                               &w->ticket[1], s_cnt);
+    }
     if (!build_barrier(w)) return;
+    if (sym) {  // out-lists and in-lists of a symmetrised list are the same
+        copy_words(a.csr_adj, a.csc_adj, 2 * a.E);
+        if (REC == 12) copy_words(reinterpret_cast<const uint32_t*>(a.csr_w), reinterpret_cast<uint32_t*>(a.csc_w), 2 * a.E);
+        copy_words(a.outdeg, a.indeg, a.V);
+        copy_words(reinterpret_cast<const uint32_t*>(a.csr_off), reinterpret_cast<uint32_t*>(a.csc_off), 2 * ((uint64_t)a.V + 1));
+    }
     // outgoing_adj_bitmap and the compressed incoming index
     bitmap_words(a.outdeg, a.V, 1, a.bitmap, a.nwords);
-    grid_scan(LoadFlag{a.indeg, a.V, 1}, EpiCompress{a.csc_off, a.cvert, a.cidx, w->cstart, a.V, 1, a.indeg},
-              (uint64_t)a.V + 1, w, nullptr);
+    const uint32_t* indeg = sym ? a.outdeg : a.indeg;
+    const uint64_t* off = sym ? a.csr_off : a.csc_off;
+    grid_scan(LoadFlag{indeg, a.V, 1}, EpiCompress{off, a.cvert, a.cidx, w->cstart, a.V, 1, indeg}, (uint64_t)a.V + 1, w,
+              nullptr);
 }
 
 bool persistent_build_fits(const eg_graph* g) {
@@ -1116,6 +1152,10 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     g->eng.pr_ready = false;
     const BucketPlan q = plan_buckets(V, E, rec);
     const size_t table = 2ull * q.nb + 2;
+    // a symmetrised list straight from the caller's records: E / 2 of them
+    const bool sym = src && g->symmetric;
+    const uint64_t Erec = sym ? g->E_input : E;
+    const BucketPlan qa = plan_buckets(V, Erec, rec);  // pass A's blocks
     const uint64_t nwords = (uint64_t)V / 64 + 1;
     EG_TRY(g->outdeg.reserve(sizeof(uint32_t) * (size_t)V));
     EG_TRY(g->indeg.reserve(sizeof(uint32_t) * (size_t)V));
@@ -1129,7 +1169,7 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     }
     EG_TRY(g->bucket_cnt.reserve(sizeof(uint64_t) * table * 2));
     EG_TRY(g->bucket_off.reserve(sizeof(uint64_t) * table));
-    EG_TRY(g->bucketed.reserve((size_t)2 * E * rec + 64));
+    EG_TRY(g->bucketed.reserve((size_t)2 * Erec * rec + 64));
     EG_TRY(g->csr_bitmap.reserve(sizeof(uint64_t) * nwords));
     const uint64_t cap = std::min<uint64_t>(E, V) + 1;
     EG_TRY(g->cvert.reserve(sizeof(uint32_t) * cap));
@@ -1149,15 +1189,16 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
         return EG_ERR_UNSUPPORTED;
     }
     PersistBuildArgs a;
-    a.src = RecordSource{src ? static_cast<const uint8_t*>(src) : g->edges.as<uint8_t>(), g->edges.as<uint8_t>(), eoff, voff, G};
-    a.E = E;
+    a.src = RecordSource{src ? static_cast<const uint8_t*>(src) : g->edges.as<uint8_t>(), g->edges.as<uint8_t>(), eoff, voff, G,
+                         sym ? 1 : 0};
+    a.E = Erec;
     a.V = V;
     EG_TRY(g->d_part_off.reserve(sizeof(uint32_t) * 2));
     a.part_off = g->d_part_off.as<uint32_t>();
-    a.chunk = q.chunk;
+    a.chunk = qa.chunk;
     a.shift = q.shift;
     a.nb = q.nb;
-    a.nblk = q.nblk;
+    a.nblk = qa.nblk;
     a.LB = q.LB;
     a.tot = g->bucket_cnt.as<unsigned long long>();
     a.cursor = a.tot + table;
@@ -1210,6 +1251,43 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
 }
 
 // ---------------------------------------------------------------------------------------------
+// the handle's edge list from its CSR, for a rebuild after a build that read the caller's records
+template <int REC>
+__global__ void k_list_from_csr(const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj,
+                                const float* __restrict__ w, uint32_t V, uint64_t E, uint8_t* __restrict__ edges) {
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t lo = 0, hi = V;  // last source with off <= e
+        while (hi - lo > 1) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            if (off[mid] <= e) lo = mid; else hi = mid;
+        }
+        uint32_t* r = reinterpret_cast<uint32_t*>(edges + e * REC);
+        r[0] = lo;
+        r[1] = adj[e];
+        if (REC == 12) r[2] = __float_as_uint(w[e]);
+    }
+}
+
+int ensure_list(eg_graph* g) {
+    if (!g->list_in_csr) return EG_OK;
+    if (!g->built_csr) {
+        set_error("eg_build: no edge list (the last load failed)");
+        return EG_ERR_INVALID;
+    }
+    const uint64_t E = g->E;
+    EG_TRY(g->edges.reserve((size_t)E * g->edge_bytes + 64));
+    const unsigned grid = grid_for(E, 256, 152u * 16u);
+    if (g->edge_bytes == 8)
+        k_list_from_csr<8><<<grid, 256, 0, g->stream>>>(g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(), nullptr, g->V, E,
+                                                        g->edges.as<uint8_t>());
+    else
+        k_list_from_csr<12><<<grid, 256, 0, g->stream>>>(g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(),
+                                                         g->csr_w.as<float>(), g->V, E, g->edges.as<uint8_t>());
+    EG_CHECK_LAUNCH("k_list_from_csr");
+    g->list_in_csr = false;
+    return EG_OK;
+}
+
 int compute_degrees(eg_graph* g) {
     const uint64_t E = g->E;
     const uint32_t V = g->V;

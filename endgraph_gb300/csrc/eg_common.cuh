@@ -152,6 +152,7 @@ struct eg_graph {
     int symmetric = 0;
     eg::DevBuf edges;     // packed records as loaded (8 or 12 bytes each)
     int edge_bytes = 8;
+    bool list_in_csr = false;  // the records live in the CSR only: the build read the caller's (ensure_list)
     // degrees (u32 V)
     eg::DevBuf outdeg, indeg;
     // CPBT
@@ -230,11 +231,13 @@ int build_structures(eg_graph* g, int want_csr, int want_csc, const UploadParts*
 // the one-partition, one-sub-partition build as one cooperative launch; eoff / voff (device, G + 1
 // entries each, optional): a graph batch whose ids are moved to the union inside the launch
 bool persistent_build_fits(const eg_graph* g);
-// src (optional): device records, 16-byte aligned, that pass A copies into g->edges as it counts them
+// src (optional): device records, 16-byte aligned, read where they are; with g->symmetric they are the
+// E / 2 records before symmetrisation
 int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G, const void* src);
 // whether pass A may read the caller's records itself: plain device memory of this GPU, 16-byte aligned
 bool direct_records(const eg_graph* g, const void* edges, int where);
-int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric);
+int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric, bool keep_list = true);
+int ensure_list(eg_graph* g);  // g->edges holds the list again
 // eg_load_directed of host records from this many records on: upload and build pipelined
 constexpr uint64_t kPipelinedLoadMin = 1ull << 22;
 int load_build_pipelined(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int edge_bytes);
@@ -257,6 +260,7 @@ int run_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int w
 int run_sssp(eg_graph* g, uint32_t root, float* dist, int where);
 int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
 int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where);
+int run_cc_symmetric(eg_graph* g, uint32_t* label, int where);
 int run_cc(eg_graph* g, uint32_t* label, int where);
 int run_msbfs(eg_graph* g, const uint32_t* roots, int n, uint8_t* levels, int where, uint64_t* edges);
 int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float alpha, int K, float* out, int where);

@@ -221,3 +221,52 @@ def test_batch_from_device_records(eg_lib):
             g.load_graph_batch(bad, eoff, Vs)
         g.load_graph_batch(rec, eoff, Vs)
         _assert_oracle(_structure(g), usrc, udst, w, int(voff[-1]))
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("E", [1, 2, 3, 64, 65, 16_383, 16_385, 200_003])
+def test_symmetrised_build(eg_lib, weighted, E):
+    """load_undirected_from_directed builds both structures from one: the same lists, index, bitmap and
+    degrees as the build with one launch per pass and as the oracle on the doubled list, from host
+    and device records (aligned or not), with self loops and duplicates, and again after a rebuild."""
+    import torch
+
+    import endgraph_gb300 as eg
+    V = 20_011
+    src, dst, w = rmat_graph(V, E, E, weights=(0.0, 1.0) if weighted else None)
+    src[: E // 8], dst[: E // 8] = dst[: E // 8].copy(), dst[: E // 8].copy()  # self loops
+    src[E // 2:], dst[E // 2:] = src[: E - E // 2].copy(), dst[: E - E // 2].copy()  # duplicates
+    host = eg.pack_edges(src, dst, w)
+    s2, d2 = np.concatenate([src, dst]), np.concatenate([dst, src])
+    w2 = np.concatenate([w, w]) if weighted else None
+    buf = torch.zeros((E + 1, host.shape[1]), dtype=torch.int32, device="cuda")
+    with eg.Graph() as g:
+        g.set_option(eg.EG_OPT_BUILD_LAUNCH, 0)
+        g.load_undirected_from_directed(host, V)
+        per_pass = _structure(g)
+        g.set_option(eg.EG_OPT_BUILD_LAUNCH, 1)
+        for skip in (None, 0, 1):
+            if skip is None:
+                g.load_undirected_from_directed(host, V)
+            else:
+                buf[skip:skip + E].copy_(torch.from_numpy(host.view(np.int32)))
+                g.load_undirected_from_directed(buf[skip:skip + E], V)
+            i = g.info()
+            assert i.E == 2 * E and i.symmetric == 1
+            _assert_same(_structure(g), per_pass)
+            _assert_oracle(_structure(g), s2, d2, w2, V)
+        buf.zero_()
+        for launch in (1, 0):
+            g.set_option(eg.EG_OPT_BUILD_LAUNCH, launch)
+            g.build()
+            _assert_same(_structure(g), per_pass)
+        bad = host.copy()
+        bad[E // 2, 1] = V
+        g.set_option(eg.EG_OPT_BUILD_LAUNCH, 1)
+        for rec in (bad, torch.from_numpy(bad.view(np.int32)).cuda()):
+            with pytest.raises(eg.EndGraphError):
+                g.load_undirected_from_directed(rec, V)
+            with pytest.raises(eg.EndGraphError):
+                g.build()
+        g.load_undirected_from_directed(host, V)
+        _assert_same(_structure(g), per_pass)
