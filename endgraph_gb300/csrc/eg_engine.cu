@@ -1012,6 +1012,9 @@ int run_sssp(eg_graph* g, uint32_t root, float* dist, int where) {
 
 int run_cc(eg_graph* g, uint32_t* label, int where) {
     if (!g->built_csr || !g->built_csc) { set_error("eg_cc: CSR and CSC must be built"); return EG_ERR_STATE; }
+    // a symmetrised list in one partition: union-find (propagation along directed edges labels every
+    // vertex with the smallest one that reaches it, which is something else)
+    if (g->symmetric && g->partitions == 1 && g->V < (1u << 31) && g->E < (1ull << 38)) return run_cc_symmetric(g, label, where);
     EG_TRY(ensure_engine(g));
     EG_TRY(setup_pull(g));
     const uint32_t V = g->V;

@@ -167,7 +167,8 @@ int eg_pagerank(eg_graph* g, int iterations, float damping, float* out, int wher
 /* BFS (toolkits/bfs.cpp:22-84), push.  level[V] (0xFFFFFFFF unreached) and parent[V] (V when
  * unreached; parent[root] = root); either may be NULL.  *reached (may be NULL) = reached count. */
 int eg_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
-/* CC (toolkits/cc.cpp:22-84) on a graph loaded with eg_load_undirected_from_directed: min-label
+/* CC (toolkits/cc.cpp:22-84): the smallest vertex of each component.  A list symmetrised at load, in
+ * one partition, is labelled by union-find (eg_last_run: one iteration); any other graph by min-label
  * propagation, push/pull switched per iteration on active_edges < E/20 (core/graph.hpp:1484-1491). */
 int eg_cc(eg_graph* g, uint32_t* label, int where);
 /* SSSP (toolkits/sssp.cpp:24-84), push Bellman-Ford on float weights; unreached = 1e9. */

@@ -139,3 +139,48 @@ def test_bfs_outputs_on_the_device(eg_lib):
         level.fill_(0)
         g.bfs(root, level=level[:V], want_parent=False)
         assert np.array_equal(level[:V].cpu().numpy().view(np.uint32), ref)
+
+
+def _check_cc(src, dst, V, w=None):
+    import endgraph_gb300 as eg
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    ref = oracle.cc_labels(src, dst, V)
+    with eg.Graph() as g:
+        g.load_undirected_from_directed(eg.pack_edges(src, dst, w), V)
+        assert np.array_equal(g.cc(), ref)
+
+
+def test_cc_chain_and_components(eg_lib):
+    """Paths whose parents form long chains, several components of similar size beside a large one,
+    and vertices without edges."""
+    n = 30_000
+    _check_cc(np.arange(n - 1), np.arange(1, n), n + 5)
+    _check_cc(np.arange(1, n), np.arange(n - 1), n)
+    perm = np.random.default_rng(1).permutation(n)
+    _check_cc(perm[:-1], perm[1:], n)
+    _check_cc(perm[:-2], perm[2:], n)          # two interleaved paths
+    rng = np.random.default_rng(2)
+    part = rng.integers(0, 7, 60_000)          # seven random graphs over one id space
+    ids = [np.flatnonzero(part == k) for k in range(7)]
+    src = np.concatenate([rng.choice(i, 12_000) for i in ids])
+    dst = np.concatenate([rng.choice(i, 12_000) for i in ids])
+    _check_cc(src, dst, 60_000)
+
+
+@pytest.mark.parametrize("deg", [1, 2, 3, 255, 257, 258, 259, 514, 20_000])
+def test_cc_lists_outside_the_common_component(eg_lib, deg):
+    """A star whose hub is outside the largest component: its list goes through the queue."""
+    V = 120_000
+    rng = np.random.default_rng(deg)
+    big = rng.permutation(V - 30_000) + 30_000
+    leaves = rng.choice(29_990, deg, replace=False) + 10
+    src = np.concatenate([big[:-1], np.full(deg, 5), leaves[: deg // 2]])
+    dst = np.concatenate([big[1:], leaves, rng.permutation(leaves)[: deg // 2]])
+    _check_cc(src, dst, V)
+
+
+@pytest.mark.parametrize("V,E", [(1, 1), (2, 1), (5, 3), (1025, 700), (4097, 4096), (40_000, 900_000)])
+def test_cc_grid_sizes(eg_lib, V, E):
+    rng = np.random.default_rng(V)
+    src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
+    _check_cc(src, dst, V, rng.random(E).astype(np.float32))
