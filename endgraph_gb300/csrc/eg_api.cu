@@ -226,7 +226,7 @@ int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmet
     }
     g->built_csr = g->built_csc = false;
     g->eng.pull_ready = false;
-    g->eng.pr_ready = false;
+    g->eng.pr_ready = g->eng.pr_heads_ready = false;
     free_batch_state(g);
     g->batch_voff.clear();
     g->batch_eoff.clear();
@@ -752,7 +752,7 @@ int eg_load_directed_with_ids(eg_graph* g, const void* edges, uint64_t E, uint32
     }
     g->built_csr = g->built_csc = false;
     g->eng.pull_ready = false;
-    g->eng.pr_ready = false;
+    g->eng.pr_ready = g->eng.pr_heads_ready = false;
     free_batch_state(g);
     g->V = V;
     g->E = E;

@@ -1149,7 +1149,7 @@ int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, ui
     }
     g->built_csr = g->built_csc = false;
     g->eng.pull_ready = false;
-    g->eng.pr_ready = false;
+    g->eng.pr_ready = g->eng.pr_heads_ready = false;
     const BucketPlan q = plan_buckets(V, E, rec);
     const size_t table = 2ull * q.nb + 2;
     // a symmetrised list straight from the caller's records: E / 2 of them
@@ -1407,7 +1407,7 @@ int build_structures(eg_graph* g, int want_csr, int want_csc, const UploadParts*
     const uint64_t nwords = (uint64_t)V / 64 + 1;
     g->built_csr = g->built_csc = false;
     g->eng.pull_ready = false;
-    g->eng.pr_ready = false;
+    g->eng.pr_ready = g->eng.pr_heads_ready = false;
 
     if (g->build_launch && !up && persistent_build_fits(g)) return build_persistent(g, nullptr, nullptr, 0, nullptr);
     // the bucket tables and a staging tile must fit one CTA's shared memory

@@ -122,6 +122,11 @@ struct EngineState {
     uint64_t pull_nsplit = 0;
     uint64_t pull_nchunks = 0;
     bool pull_ready = false;
+    // one-partition PageRank sweep (eg_pagerank.cu): list-start bits, entries of blocks, boundaries of
+    // runs, degrees and places in entry order; what they were made for
+    DevBuf pr_heads, pr_item_of, pr_split, pr_deg, pr_place;
+    bool pr_heads_ready = false;
+    bool pr_heads_relabel = false;
     bool pr_ready = false;  // pr_new_id / pr_adj match the built CSC
     uint64_t* host_words = nullptr;  // pinned host block (256 bytes) for the readbacks of counters
     // single-root BFS replayed as a CUDA graph (eg_engine.cu): the instantiated graph, its state
@@ -251,6 +256,7 @@ int selftest_bounded_wait(eg_graph* g, uint32_t spin_cap);
 int selftest_grid_barrier(eg_graph* g, uint32_t spin_cap);
 int validate_edges(eg_graph* g, uint64_t E);
 int symmetrize_edges(eg_graph* g, uint64_t E);
+int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, int where);
 int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where);
 // renumbering of the CSC sources by out-degree class (eng.pr_new_id / eng.pr_adj), built once per
 // structure build and shared by the PageRank and bit-parallel BFS pull gathers
@@ -307,6 +313,35 @@ __device__ __forceinline__ bool grid_sync_bounded(unsigned* count, unsigned* gen
             }
         }
         __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// The same for kernels whose steps are a few microseconds: one counter that only grows, so that no
+// CTA resets it and advances a generation before the others can go on (40 barriers of 128 CTAs in a
+// PageRank of 65,536 / 2^20: 0.23 instead of 0.27 ms).  *count is zero at launch; `target` starts at zero in every CTA.
+__device__ __forceinline__ bool grid_sync_growing(unsigned* count, int* err, unsigned& target,
+                                                  uint32_t spin_cap = kBarrierSpinCap) {
+    __shared__ int s_ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        // release: what the CTA wrote is seen by whoever acquires a count that includes this arrival
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        int ok = 1;
+        for (uint32_t spins = 1;; ++spins) {
+            unsigned x;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(count) : "memory");
+            if ((int)(x - target) >= 0) break;
+            if (spins > spin_cap || ((spins & 63u) == 0 && *(volatile int*)err)) {
+                atomicExch(err, 1);
+                ok = 0;
+                break;
+            }
+            __nanosleep(20);
+        }
         s_ok = ok;
     }
     __syncthreads();

@@ -258,34 +258,19 @@ struct CcPushOp {  // toolkits/cc.cpp:50-60: msg = label[src]; write_min(label[d
     }
 };
 
-struct PrPullOp {  // toolkits/pagerank.cpp:64-97: sum curr[src]; next = 1-d+d*sum (/ outdeg)
+struct PrPullOp {  // toolkits/pagerank.cpp:64-97: sum curr[src] (several partitions; one: eg_pagerank.cu)
     using Acc = float;
     static constexpr bool kFilter = false;
     __device__ bool stopped() const { return false; }
     __device__ bool item_active(uint32_t) const { return true; }
     const float* curr;
-    float* next;
     float* acc;
-    const uint32_t* outdeg;
-    const uint32_t* slot;  // null: next in vertex order; else next[slot[v]] (renumbered order)
-    float base, d;
-    int divide, single;
     __device__ Acc identity() const { return 0.f; }
     __device__ Acc gather(uint32_t src, uint64_t) const { return ld_keep(curr + src); }
     __device__ Acc combine(Acc a, Acc b) const { return a + b; }
     __device__ void smem_add(Acc* slot, Acc v) const { atomicAdd(slot, v); }
-    __device__ void finish(bool ok, uint32_t v, Acc a, bool whole) const {
-        if (!ok) return;
-        if (whole && single) {
-            float x = base + d * a;
-            if (divide) {
-                uint32_t dg = outdeg[v];
-                if (dg > 0) x /= (float)dg;
-            }
-            next[slot ? slot[v] : v] = x;
-        } else {
-            atomicAdd(acc + v, a);
-        }
+    __device__ void finish(bool ok, uint32_t v, Acc a, bool) const {
+        if (ok) atomicAdd(acc + v, a);
     }
 };
 
@@ -348,21 +333,6 @@ __global__ void k_pr_zero_in(float* buf, const uint32_t* __restrict__ indeg, con
             uint32_t dg = outdeg[v];
             buf[slot ? slot[v] : v] = (divide && dg > 0) ? base / (float)dg : base;
         }
-    }
-}
-// destinations whose list crossed a chunk boundary (P == 1)
-__global__ void k_pr_split(const uint32_t* __restrict__ split, const uint32_t* __restrict__ cvert, uint64_t nsplit,
-                           float* next, float* acc, const uint32_t* __restrict__ outdeg, float base, float d, int divide,
-                           const uint32_t* __restrict__ slot) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nsplit; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t v = cvert[split[i]];
-        float x = base + d * acc[v];
-        acc[v] = 0.f;
-        if (divide) {
-            uint32_t dg = outdeg[v];
-            if (dg > 0) x /= (float)dg;
-        }
-        next[slot ? slot[v] : v] = x;
     }
 }
 // P > 1: every destination with in-edges combines its partial sums
@@ -715,6 +685,7 @@ static int build_bfs_graph(eg_graph* g) {
 int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where) {
     if (!g->built_csc) { set_error("eg_pagerank: CSC not built"); return EG_ERR_STATE; }
     if (iterations < 0) { set_error("eg_pagerank: iterations must be >= 0"); return EG_ERR_INVALID; }
+    if (g->partitions == 1 && iterations > 0 && g->E > 0) return run_pagerank_single(g, iterations, damping, out, where);
     EG_TRY(ensure_engine(g));
     EG_TRY(setup_pull(g));
     const uint32_t V = g->V;
@@ -722,7 +693,6 @@ int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int whe
     float* A = s.vals0.as<float>();
     float* B = s.vals1.as<float>();
     const float base = 1.0f - damping;
-    const int single = g->partitions == 1;
     const unsigned gv = grid_for(V, 256, 152u * 16u);
     // with renumbered gathers every vector but the final one is kept in class order
     const bool relabel = iterations > 0 && g->E > 0 && want_relabel(g);
@@ -746,21 +716,12 @@ int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int whe
                                                     slot);
             EG_CHECK_LAUNCH("k_pr_zero_in");
         }
-        PrPullOp op{curr, next, s.acc.as<float>(), g->outdeg.as<uint32_t>(), slot, base, damping, !last, single};
+        PrPullOp op{curr, s.acc.as<float>()};
         EG_TRY(launch_pull(g, op, "pr_pull", gather_adj));
         Timed t(&g->prof, g->stream, "pr_finish");
-        if (single) {
-            if (s.pull_nsplit) {
-                k_pr_split<<<grid_for(s.pull_nsplit, 256), 256, 0, g->stream>>>(
-                    s.pull_split.as<uint32_t>(), g->cvert.as<uint32_t>(), s.pull_nsplit, next, s.acc.as<float>(),
-                    g->outdeg.as<uint32_t>(), base, damping, !last, slot);
-                EG_CHECK_LAUNCH("k_pr_split");
-            }
-        } else {
-            k_pr_finish_all<<<gv, 256, 0, g->stream>>>(g->indeg.as<uint32_t>(), V, next, s.acc.as<float>(),
-                                                       g->outdeg.as<uint32_t>(), base, damping, !last, slot);
-            EG_CHECK_LAUNCH("k_pr_finish_all");
-        }
+        k_pr_finish_all<<<gv, 256, 0, g->stream>>>(g->indeg.as<uint32_t>(), V, next, s.acc.as<float>(),
+                                                   g->outdeg.as<uint32_t>(), base, damping, !last, slot);
+        EG_CHECK_LAUNCH("k_pr_finish_all");
     }
     float* result = (iterations & 1) ? B : A;
     EG_TRY(copy_out(g, out, result, sizeof(float) * (size_t)V, where));

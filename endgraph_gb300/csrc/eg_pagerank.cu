@@ -1,0 +1,376 @@
+// eg_pagerank.cu — PageRank (toolkits/pagerank.cpp:26-98) on a one-partition graph: dense pull sweeps
+// over the CSC by independent warps.
+//
+// A sweep is bound by the L1 lookups of its gathers (one per edge), so everything else is kept off
+// that path.  Where a list starts is one bit per edge, read with the ids: no entry bounds to stage,
+// no search for a thread's first entry.  A warp takes blocks of 512 edges, 8 consecutive ids per lane
+// and half block, issues its 16 gathers, and sums lists with one segmented warp scan per half block;
+// totals of lists that end in the block gather in shared memory and are finished one per lane, from
+// degrees and places in entry order that were loaded behind the gathers.  The open list is carried
+// from block to block; what a warp's run of blocks begins or ends in the middle of a list is added to
+// the list's accumulator, and a second pass over the run boundaries finishes those lists.  (Counting
+// a list's pieces, so that the last warp finishes it, made the sweep wait for the counters of the
+// hubs: 2.7 instead of 1.95 ms at 2^25 / 2^29, 2.8 with fences.)  Small graphs run every iteration in one
+// persistent launch between grid barriers.
+#include <algorithm>
+
+#include "eg_pull.cuh"
+
+namespace eg {
+
+constexpr uint32_t kPrBlock = 512;  // edges per warp step
+constexpr uint32_t kNoBoundary = 0xFFFFFFFFu;
+constexpr int kPrGroup = 8;  // consecutive edges per lane: 4 or 16 were no faster (40.3 / 40.3 against 39.4 ms of sweeps)
+
+struct PrArgs {
+    const uint32_t* adj;
+    const uint32_t* heads;    // bit e: edge e is the first of its list (one word of zeros past E)
+    const uint32_t* item_of;  // per block: compressed entry that holds its first edge
+    const uint32_t* dst;      // per entry: where its value goes in next
+    const uint32_t* deg;      // per entry: its vertex's out-degree
+    uint64_t E;
+    uint64_t nruns;           // runs of 1 << shift blocks
+    int shift;
+    const float* curr;
+    float* next;
+    float* acc;               // per run boundary: the list that crosses it first there (split)
+    const uint32_t* split;    // per run: boundary its first list's pieces meet at
+    float base, d;
+    int divide;
+};
+
+__device__ __forceinline__ float pr_value(const PrArgs& a, float sum, uint32_t deg) {  // toolkits/pagerank.cpp:80-97
+    const float x = a.base + a.d * sum;
+    return a.divide && deg > 0 ? x / (float)deg : x;
+}
+__device__ __forceinline__ void pr_write(const PrArgs& a, uint32_t item, float sum) {
+    const uint32_t to = __ldg(a.dst + item), deg = __ldg(a.deg + item);
+    a.next[to] = pr_value(a, sum, deg);
+}
+
+// one run of blocks by one warp; s_sum: kPrBlock floats of the warp's own
+__device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_sum) {
+    constexpr int G = kPrGroup, kGroups = (int)kPrBlock / (32 * G);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    const uint64_t e_begin = (run << a.shift) * kPrBlock;
+    const uint64_t e_end = min(a.E, ((run + 1) << a.shift) * kPrBlock);
+    uint32_t item = __ldg(a.item_of + (run << a.shift));
+    bool open_first = !(__ldg(a.heads + (e_begin >> 5)) & 1u);  // the first list began in an earlier run
+    float carry = 0.f;                                           // sum of the open list so far
+    for (uint64_t e0 = e_begin; e0 < e_end; e0 += kPrBlock) {
+        float val[kGroups][G];
+        uint32_t head[kGroups];
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+            const uint64_t e = e0 + (uint64_t)g * (32 * G) + lane * G;
+            uint32_t id[G];
+            if (e + G <= a.E) {
+#pragma unroll
+                for (int q = 0; q < G / 4; ++q) {
+                    const uint4 x = __ldcs(reinterpret_cast<const uint4*>(a.adj + e) + q);
+                    id[4 * q] = x.x;
+                    id[4 * q + 1] = x.y;
+                    id[4 * q + 2] = x.z;
+                    id[4 * q + 3] = x.w;
+                }
+#pragma unroll
+                for (int j = 0; j < G; ++j) val[g][j] = ld_keep(a.curr + id[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < G; ++j) val[g][j] = e + j < a.E ? ld_keep(a.curr + a.adj[e + j]) : 0.f;
+            }
+            if (G == 16) head[g] = e < a.E ? __ldcs(reinterpret_cast<const uint16_t*>(a.heads) + e / 16) : 0u;
+            else if (G == 8) head[g] = e < a.E ? __ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8) : 0u;
+            else head[g] = e < a.E ? (__ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8) >> (e & 7)) & 0xFu : 0u;
+            if (e == e_begin) head[g] &= ~1u;  // the run's first edge opens nothing new
+        }
+        // lists that end in earlier lanes (rank, per group) and in the whole block
+        uint32_t rank[kGroups], closed = 0;
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+            rank[g] = closed;
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const uint32_t b = __ballot_sync(0xffffffffu, (head[g] >> j) & 1u);
+                rank[g] += __popc(b & below);
+                closed += __popc(b);
+            }
+        }
+        const uint32_t to = lane < closed ? __ldg(a.dst + item + lane) : 0u;
+        const uint32_t deg = lane < closed ? __ldg(a.deg + item + lane) : 0u;
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+            const uint32_t f = head[g];
+            float t = 0.f, first = 0.f;
+            uint32_t k = rank[g];
+            bool seen = false;
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if ((f >> j) & 1u) {
+                    if (seen) s_sum[k] = t;
+                    else first = t;
+                    ++k;
+                    seen = true;
+                    t = 0.f;
+                }
+                t += val[g][j];
+            }
+            // the open list along the lanes: t becomes its sum up to and including this lane
+            const uint32_t m = __ballot_sync(0xffffffffu, seen);
+            const int begin = 31 - __clz(m & (below | (1u << lane)));  // last lane that opened one, or -1
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float y = __shfl_up_sync(0xffffffffu, t, o);
+                if ((int)lane - o >= max(begin, 0)) t += y;
+            }
+            if (begin < 0) t += carry;
+            float before = __shfl_up_sync(0xffffffffu, t, 1);
+            if (lane == 0) before = carry;
+            if (seen) s_sum[rank[g]] = before + first;
+            carry = __shfl_sync(0xffffffffu, t, 31);
+        }
+        __syncwarp();
+        for (uint32_t k = lane; k < closed; k += 32) {
+            const float sum = s_sum[k];
+            if (k == 0 && open_first) atomicAdd(a.acc + __ldg(a.split + run), sum);
+            else if (k < 32) a.next[to] = pr_value(a, sum, deg);
+            else pr_write(a, item + k, sum);
+        }
+        __syncwarp();
+        if (closed) open_first = false;
+        item += closed;
+    }
+    if (lane == 0) {
+        const bool ends = e_end == a.E || ((__ldg(a.heads + (e_end >> 5)) >> (e_end & 31)) & 1u);
+        if (open_first) atomicAdd(a.acc + __ldg(a.split + run), carry);
+        else if (ends) pr_write(a, item, carry);
+        else atomicAdd(a.acc + __ldg(a.split + run + 1), carry);
+    }
+}
+
+// the list that crosses the start of run r, if it began in the run before: its pieces are all in
+__device__ __forceinline__ void pr_boundary(const PrArgs& a, uint64_t r) {
+    if (__ldg(a.split + r) != (uint32_t)r) return;
+    const float sum = __ldcg(a.acc + r);
+    a.acc[r] = 0.f;  // for the next sweep
+    pr_write(a, __ldg(a.item_of + (r << a.shift)), sum);
+}
+
+// 20 iterations at 2^25 / 2^29: 6 CTAs per SM (40 registers) 38.6 ms, 5 38.9, 4 39.5, 8 (32, spilled) 47;
+// 49.5 ms with 4,096-edge CTA chunks, entry bounds in shared memory and an accumulator per entry there
+__global__ void __launch_bounds__(256, 6) k_pr_sweep(PrArgs a) {
+    __shared__ float s_sum[8][kPrBlock];
+    const uint64_t run = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (run < a.nruns) pr_run(a, run, s_sum[threadIdx.x >> 5]);
+}
+
+__global__ void k_pr_boundaries(PrArgs a) {
+    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < a.nruns; r += (uint64_t)gridDim.x * blockDim.x)
+        pr_boundary(a, r);
+}
+
+// Per entry: the bit of its first edge, its vertex's degree and (slot non-null) place; the entry of
+// each block's first edge; per run the first run boundary that its first list crosses (none
+// when the list starts with the run).
+__global__ void k_pr_setup(const uint64_t* __restrict__ cidx, const uint32_t* __restrict__ cvert, uint64_t nitems,
+                           const uint32_t* __restrict__ outdeg, const uint32_t* __restrict__ slot, int shift,
+                           uint32_t* heads, uint32_t* __restrict__ item_of, uint32_t* __restrict__ deg,
+                           uint32_t* __restrict__ place, uint32_t* __restrict__ split) {
+    const uint64_t run = (uint64_t)kPrBlock << shift;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nitems; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t s = cidx[i], e = cidx[i + 1];
+        if (e <= s) continue;
+        atomicOr(heads + (s >> 5), 1u << (s & 31));
+        for (uint64_t c = (s + kPrBlock - 1) / kPrBlock; c * kPrBlock < e; ++c) item_of[c] = (uint32_t)i;
+        const uint32_t v = cvert[i];
+        deg[i] = outdeg[v];
+        if (slot) place[i] = slot[v];
+        const uint64_t r0 = s / run + 1;
+        if (s % run == 0) split[s / run] = kNoBoundary;
+        for (uint64_t r = r0; r * run < e; ++r) split[r] = (uint32_t)r0;
+    }
+}
+
+__device__ __forceinline__ void pr_start(float* curr, const uint32_t* __restrict__ outdeg, uint64_t V,
+                                         const uint32_t* __restrict__ slot, float* acc, uint64_t nruns, uint64_t tid,
+                                         uint64_t stride) {  // pagerank.cpp:36-45
+    for (uint64_t v = tid; v < V; v += stride) {
+        const uint32_t dg = outdeg[v];
+        curr[slot ? slot[v] : v] = dg > 0 ? 1.0f / (float)dg : 1.0f;
+    }
+    for (uint64_t r = tid; r <= nruns; r += stride) acc[r] = 0.f;
+}
+// vertices without in-edges: next = 1-d (/ outdeg)
+__device__ __forceinline__ void pr_no_in(float* next, const uint32_t* __restrict__ indeg, const uint32_t* __restrict__ outdeg,
+                                         uint64_t V, float base, int divide, const uint32_t* __restrict__ slot, uint64_t tid,
+                                         uint64_t stride) {
+    for (uint64_t v = tid; v < V; v += stride) {
+        if (indeg[v]) continue;
+        const uint32_t dg = outdeg[v];
+        next[slot ? slot[v] : v] = (divide && dg > 0) ? base / (float)dg : base;
+    }
+}
+__global__ void k_pr_start(float* curr, const uint32_t* outdeg, uint64_t V, const uint32_t* slot, float* acc,
+                           uint64_t nruns) {
+    pr_start(curr, outdeg, V, slot, acc, nruns, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+             (uint64_t)gridDim.x * blockDim.x);
+}
+__global__ void k_pr_no_in(float* next, const uint32_t* indeg, const uint32_t* outdeg, uint64_t V, float base, int divide,
+                           const uint32_t* slot) {
+    pr_no_in(next, indeg, outdeg, V, base, divide, slot, blockIdx.x * (uint64_t)blockDim.x + threadIdx.x,
+             (uint64_t)gridDim.x * blockDim.x);
+}
+
+struct PrPersistArgs {
+    PrArgs pr;              // curr, next, dst and divide are set per iteration
+    uint64_t V;
+    const uint32_t *indeg, *outdeg, *cvert;
+    const uint32_t* order;  // slot of every vector but the last
+    float* vec[2];
+    float* out;             // the last vector
+    int iterations;
+    unsigned* words;        // barrier count, unused, error flag
+};
+
+constexpr int kPrPersistThreads = 512, kPrPersistCtas = 2;
+
+__global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persistent(PrPersistArgs a) {
+    __shared__ float s_sum[kPrPersistThreads / 32][kPrBlock];
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    unsigned arrived = 0;
+    auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), arrived); };
+    pr_start(a.vec[0], a.outdeg, a.V, a.order, a.pr.acc, a.pr.nruns, tid, stride);
+    for (int it = 0; it < a.iterations; ++it) {
+        if (!barrier()) return;
+        const bool last = it == a.iterations - 1;
+        PrArgs p = a.pr;
+        p.curr = a.vec[it & 1];
+        p.next = last ? a.out : a.vec[(it & 1) ^ 1];
+        if (last) p.dst = a.cvert;
+        p.divide = !last;
+        if (it < 2 || last) pr_no_in(p.next, a.indeg, a.outdeg, a.V, p.base, p.divide, last ? nullptr : a.order, tid, stride);
+        for (uint64_t run = tid >> 5; run < p.nruns; run += stride >> 5) pr_run(p, run, s_sum[threadIdx.x >> 5]);
+        if (!barrier()) return;
+        for (uint64_t r = tid; r < p.nruns; r += stride) pr_boundary(p, r);
+    }
+}
+
+// Blocks per run: few boundaries (sweeps at 2^25 / 2^29 with 1 / 4 / 8 blocks: 41.2 / 38.6 / 38.0 ms), but runs
+// enough for every resident warp several times (1 M / 16 M: 1.44 / 1.71 / 1.72).
+static int pr_shift(uint64_t E) {
+    int s = 0;
+    while (s < 3 && (E >> (10 + s)) >= 24000) ++s;
+    return s;
+}
+
+static int pr_setup(eg_graph* g, const uint32_t* order) {
+    EngineState& s = g->eng;
+    if (s.pr_heads_ready && s.pr_heads_relabel == (order != nullptr)) return EG_OK;
+    const uint64_t E = g->E, nitems = g->ncompressed - 1;
+    const size_t words = E / 32 + 2;
+    const int shift = pr_shift(E);
+    EG_TRY(s.pr_heads.reserve(4 * words + 64));
+    EG_TRY(s.pr_item_of.reserve(4 * (E / kPrBlock + 2)));
+    EG_TRY(s.pr_split.reserve(4 * ((E / kPrBlock >> shift) + 3)));
+    EG_TRY(s.pr_deg.reserve(4 * (nitems + 1)));
+    if (order) EG_TRY(s.pr_place.reserve(4 * (nitems + 1)));
+    Timed t(&g->prof, g->stream, "pr_setup");
+    EG_CUDA(cudaMemsetAsync(s.pr_heads.ptr, 0, 4 * words, g->stream));
+    k_pr_setup<<<grid_for(nitems, 256), 256, 0, g->stream>>>(
+        g->cidx.as<uint64_t>(), g->cvert.as<uint32_t>(), nitems, g->outdeg.as<uint32_t>(), order, shift,
+        s.pr_heads.as<uint32_t>(), s.pr_item_of.as<uint32_t>(), s.pr_deg.as<uint32_t>(), s.pr_place.as<uint32_t>(),
+        s.pr_split.as<uint32_t>());
+    EG_CHECK_LAUNCH("k_pr_setup");
+    s.pr_heads_ready = true;
+    s.pr_heads_relabel = order != nullptr;
+    return EG_OK;
+}
+
+int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, int where) {
+    EngineState& s = g->eng;
+    const uint64_t V = g->V, E = g->E;
+    for (DevBuf* b : {&s.vals0, &s.vals1}) EG_TRY(b->reserve(4 * (V + 1)));
+    // with renumbered gathers every vector but the final one is kept in class order
+    const bool relabel = want_relabel(g);
+    if (relabel) EG_TRY(setup_relabel(g));
+    const uint32_t* order = relabel ? s.pr_new_id.as<uint32_t>() : nullptr;
+    EG_TRY(pr_setup(g, order));
+    float* vec[2] = {s.vals0.as<float>(), s.vals1.as<float>()};
+    float* result = out && where == EG_DEVICE ? out : vec[iterations & 1];
+    // every iteration in one launch up to here: 20 iterations take 0.26 / 0.35 ms (one launch / two per
+    // iteration) at 65,536 / 2^20, 1.45 / 1.54 at 1 M / 16 M, 5.29 / 5.17 at 2^22 / 2^26
+    const bool small = E <= (1ull << 25);
+    PrArgs p;
+    p.adj = relabel ? s.pr_adj.as<uint32_t>() : g->csc_adj.as<uint32_t>();
+    p.heads = s.pr_heads.as<uint32_t>();
+    p.item_of = s.pr_item_of.as<uint32_t>();
+    p.dst = relabel ? s.pr_place.as<uint32_t>() : g->cvert.as<uint32_t>();
+    p.deg = s.pr_deg.as<uint32_t>();
+    p.E = E;
+    p.shift = pr_shift(E);
+    p.nruns = (E + (kPrBlock << p.shift) - 1) / (kPrBlock << p.shift);
+    EG_TRY(s.acc.reserve(4 * (p.nruns + 2)));
+    p.acc = s.acc.as<float>();
+    p.split = s.pr_split.as<uint32_t>();
+    const uint32_t* outdeg = g->outdeg.as<uint32_t>();
+    p.base = 1.0f - damping;
+    p.d = damping;
+    if (small) {
+        EG_TRY(s.persist.reserve(64));
+        EG_CUDA(cudaMemsetAsync(s.persist.ptr, 0, 16, g->stream));
+        PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations, s.persist.as<unsigned>()};
+        const unsigned grid = (unsigned)std::max<uint64_t>(
+            1, std::min<uint64_t>((uint64_t)g->num_sms * kPrPersistCtas, (p.nruns + kPrPersistThreads / 32 - 1) / (kPrPersistThreads / 32)));
+        void* kargs[] = {&a};
+        {
+            Timed t(&g->prof, g->stream, "pr_persistent");
+            EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_pr_persistent, dim3(grid), dim3(kPrPersistThreads), kargs, 0,
+                                                g->stream));
+            EG_CHECK_LAUNCH("k_pr_persistent");
+        }
+        EG_CUDA(cudaMemcpyAsync(s.host_words, s.persist.ptr, 16, cudaMemcpyDeviceToHost, g->stream));
+    } else {
+        const unsigned gv = grid_for(V, 256, 152u * 16u);
+        {
+            Timed t(&g->prof, g->stream, "pr_vertex");
+            k_pr_start<<<gv, 256, 0, g->stream>>>(vec[0], outdeg, V, order, p.acc, p.nruns);
+            EG_CHECK_LAUNCH("k_pr_start");
+        }
+        for (int it = 0; it < iterations; ++it) {
+            const bool last = it == iterations - 1;
+            p.curr = vec[it & 1];
+            p.next = last ? result : vec[(it & 1) ^ 1];
+            if (last) p.dst = g->cvert.as<uint32_t>();
+            p.divide = !last;
+            if (it < 2 || last) {
+                Timed t(&g->prof, g->stream, "pr_vertex");
+                k_pr_no_in<<<gv, 256, 0, g->stream>>>(p.next, g->indeg.as<uint32_t>(), outdeg, V, p.base, p.divide,
+                                                       last ? nullptr : order);
+                EG_CHECK_LAUNCH("k_pr_no_in");
+            }
+            {
+                Timed t(&g->prof, g->stream, "pr_pull");
+                k_pr_sweep<<<(unsigned)((p.nruns + 7) / 8), 256, 0, g->stream>>>(p);
+                EG_CHECK_LAUNCH("k_pr_sweep");
+            }
+            Timed t(&g->prof, g->stream, "pr_finish");
+            k_pr_boundaries<<<grid_for(p.nruns, 256), 256, 0, g->stream>>>(p);
+            EG_CHECK_LAUNCH("k_pr_boundaries");
+        }
+    }
+    if (out && where != EG_DEVICE)
+        EG_CUDA(cudaMemcpyAsync(out, result, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
+    EG_CUDA(cudaStreamSynchronize(g->stream));
+    if (small && reinterpret_cast<const int*>(s.host_words)[2]) {
+        set_error("eg_pagerank: a bounded grid barrier gave up");
+        return EG_ERR_TIMEOUT;
+    }
+    g->last_edges_processed = E * (uint64_t)iterations;
+    g->last_iterations = iterations;
+    g->last_pushes = 0;
+    g->last_pulls = iterations;
+    return EG_OK;
+}
+
+}  // namespace eg

@@ -39,7 +39,7 @@ struct alignas(16) StepSlot {
 };
 
 struct PersistState {
-    unsigned bar_count, bar_gen;
+    unsigned bar_count, bar_pad;
     int err;
     uint32_t step;       // steps done so far
     StepSlot slot[4];    // step k reads slot k & 3, fills slot (k + 1) & 3 and clears slot (k + 2) & 3
@@ -52,8 +52,8 @@ struct PersistState {
 
 // one grid barrier; *s_slot gets the slot the finished step filled.  False: a wait gave up.
 template <class State, class Slot>
-__device__ __forceinline__ bool step_barrier(State* st, const Slot* slot, Slot* s_slot) {
-    if (!grid_sync_bounded(&st->bar_count, &st->bar_gen, &st->err)) return false;
+__device__ __forceinline__ bool step_barrier(State* st, const Slot* slot, Slot* s_slot, unsigned& arrived) {
+    if (!grid_sync_growing(&st->bar_count, &st->err, arrived)) return false;
     if (threadIdx.x < sizeof(Slot) / 16)
         reinterpret_cast<uint4*>(s_slot)[threadIdx.x] = __ldcg(reinterpret_cast<const uint4*>(slot) + threadIdx.x);
     __syncthreads();
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
         lq.valid = 0xFFFFFFFFu;
     }
     PersistState* st = a.st;
+    unsigned arrived = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
             for (uint32_t p = lane; p < np; p += 32) a.q[0][p] = piece(a.root, b + (uint64_t)p * kPiece, z);
             if (lane == 0) st->slot[0].n = np;
         }
-        if (!step_barrier(st, &st->slot[0], &s_slot)) return;
+        if (!step_barrier(st, &st->slot[0], &s_slot, arrived)) return;
         delta = a.delta;
         if (delta < 0.f) {
             const uint64_t every = max(a.E / kWeightSamples, (uint64_t)1);
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
         }
         ++step;
         flush_pieces(lq, wb, q_out, &out->n);
-        if (!step_barrier(st, out, &s_slot)) return;
+        if (!step_barrier(st, out, &s_slot, arrived)) return;
     }
     if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
     if (tid == 0) {  // every CTA leaves the loop at the same step
@@ -433,6 +434,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     PersistState* h = reinterpret_cast<PersistState*>(s.host_words);
     EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(PersistState), g->stream));
     for (a.resume = 0;; a.resume = 1) {
+        if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
         void* kargs[] = {&a};
         {
             Timed t(&g->prof, g->stream, "sssp_persistent");
@@ -483,7 +485,7 @@ struct alignas(16) BfsSlot {
 };
 
 struct BfsPersistState {
-    unsigned bar_count, bar_gen;
+    unsigned bar_count, bar_pad;
     int err;
     uint32_t step, done, pushes, pulls, pad;
     BfsSlot slot[4];  // as PersistState::slot
@@ -523,6 +525,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
         s_act = 0;
     }
     BfsPersistState* st = a.st;
+    unsigned arrived = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -544,7 +547,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 st->slot[0].act = z - b;
             }
         }
-        if (!step_barrier(st, &st->slot[0], &s_slot)) return;
+        if (!step_barrier(st, &st->slot[0], &s_slot, arrived)) return;
         reached = 1;
         edges = s_slot.act;
     } else {
@@ -591,7 +594,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 s_verts = 0;
                 s_act = 0;
             }
-            return step_barrier(st, out, &s_slot);
+            return step_barrier(st, out, &s_slot, arrived);
         };
         if (!dense) {
             const uint4* q = a.q[step & 1];
@@ -821,6 +824,7 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     BfsPersistState* h = reinterpret_cast<BfsPersistState*>(s.host_words);
     EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(BfsPersistState), g->stream));
     for (a.resume = 0;; a.resume = 1) {
+        if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
         void* kargs[] = {&a};
         {
             Timed t(&g->prof, g->stream, "bfs_persistent");
@@ -866,7 +870,7 @@ struct alignas(16) CcSlot {
     uint32_t pad[2];
 };
 struct CcState {
-    unsigned bar_count, bar_gen;
+    unsigned bar_count, bar_pad;
     int err;
     uint32_t pad;
     CcSlot slot;
@@ -927,6 +931,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         s_best = 0;
     }
     CcState* st = a.st;
+    unsigned arrived = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -940,17 +945,17 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
             if (b + k < e) p = min(p, __ldg(a.adj + b + k));
         a.comp[v] = p;
     }
-    if (!step_barrier(st, &st->slot, &s_slot)) return;
+    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
     cc_compress(a.comp, a.V, tid, stride);
-    if (!step_barrier(st, &st->slot, &s_slot)) return;
+    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
     for (uint32_t k = 0; k < kCcFirst; ++k) {
         for (uint64_t v = tid; v < a.V; v += stride) {
             const uint64_t b = __ldg(a.off + v) + k;
             if (b < __ldg(a.off + v + 1)) cc_unite(a.comp, (uint32_t)v, __ldg(a.adj + b));
         }
-        if (!step_barrier(st, &st->slot, &s_slot)) return;
+        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
         cc_compress(a.comp, a.V, tid, stride);
-        if (!step_barrier(st, &st->slot, &s_slot)) return;
+        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
     }
     // the component of most of a sample's vertices; one CTA decides for all
     if (blockIdx.x == 0) {
@@ -965,7 +970,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         __syncthreads();
         if (threadIdx.x == 0) st->slot.common = (uint32_t)s_best;
     }
-    if (!step_barrier(st, &st->slot, &s_slot)) return;
+    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
     const uint32_t common = s_slot.common;
     // the other components' lists, from the third neighbour on
     for (uint64_t base = tid & ~31ull; base < a.V; base += stride) {
@@ -980,7 +985,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         append_pieces<1>(lq, wb, vv, lb, le, a.q, &st->slot.n);
     }
     flush_pieces(lq, wb, a.q, &st->slot.n);
-    if (!step_barrier(st, &st->slot, &s_slot)) return;
+    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
     const uint32_t n = s_slot.n;
     if (n) {
         for (uint32_t base = 0; base < n; base += 32 * nwarps) {
@@ -1005,7 +1010,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
                 __syncwarp();
             }
         }
-        if (!step_barrier(st, &st->slot, &s_slot)) return;
+        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
         cc_compress(a.comp, a.V, tid, stride);
     }
 }

@@ -191,7 +191,8 @@ enum {
     EG_OPT_BFS_DIRECTION = 1,
     EG_OPT_DENSE_DIVISOR = 2,
     EG_OPT_CUDA_GRAPH = 3,
-    EG_OPT_PULL_BLOCKS_PER_SM = 4, /* pull-sweep CTAs per SM, 0 = occupancy limit */
+    EG_OPT_PULL_BLOCKS_PER_SM = 4, /* CTAs per SM of the chunked pull sweeps (CC propagation, one-seed
+                                      PPR, PageRank of several partitions), 0 = occupancy limit */
     EG_OPT_BATCH_WIDTH = 5,        /* roots per bit-parallel pass of eg_bfs_many, 1..64 */
     EG_OPT_SSSP_DELTA = 6,         /* eg_sssp near/far step in millionths of a weight unit; 0 = plain
                                       Bellman-Ford sweeps (the reference's order), -1 = automatic

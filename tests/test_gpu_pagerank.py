@@ -1,0 +1,55 @@
+"""GPU: the one-partition PageRank sweep on lists that end, begin and stay open at every edge of its
+blocking (lanes, blocks of 512 edges, runs of blocks), in the persistent launch and with one launch
+per sweep, with and without renumbered gathers."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import rel_l1
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(src, dst, V, iterations, relabels=(0, 1)):
+    """Relative L1 error against FP64 within 1e-6, the bound of the other PageRank comparisons."""
+    import endgraph_gb300 as eg
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    out, _ = oracle.degrees(src, dst, V)
+    csc = oracle.build_csc(src, dst, None, V, np.array([0, V], np.uint32))
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        for relabel in relabels:
+            g.set_option(eg.EG_OPT_PR_RELABEL, relabel)
+            for it in iterations:
+                ref = oracle.pagerank(csc["off"][0], csc["adj"], out, V, it, 0.85)
+                for _ in range(2):
+                    assert rel_l1(g.pagerank(it, 0.85), ref) <= 1e-6, (relabel, it)
+
+
+@pytest.mark.parametrize("length", [1, 2, 7, 8, 9, 16, 255, 256, 257, 511, 512, 513, 1024, 1025, 4096, 4097, 40_000])
+def test_pagerank_list_lengths(eg_lib, length):
+    """Every list has `length` in-edges (after one shorter list that shifts the others)."""
+    V = 50_000
+    rng = np.random.default_rng(length)
+    lists = max(2, min(V, 120_000 // length))
+    dst = np.concatenate([np.full(3, 0), np.repeat(np.arange(1, lists), length)])
+    src = rng.integers(0, V, len(dst))
+    _check(src, dst, V, (1, 2, 5))
+    _check(src[3:], dst[3:], V, (2,))  # not shifted: lists end on block edges
+
+
+@pytest.mark.parametrize("E", [1, 7, 8, 9, 31, 255, 256, 511, 512, 513, 1023, 1024, 1025, 16_384, 100_003])
+def test_pagerank_edge_counts(eg_lib, E):
+    rng = np.random.default_rng(E)
+    V = 777
+    _check(rng.integers(0, V, E), rng.integers(0, V, E), V, (1, 3))
+
+
+@pytest.mark.parametrize("E", [(1 << 22) + 1, 5_000_003, 13_000_001])
+def test_pagerank_one_launch_per_sweep(eg_lib, E):
+    """More edges than the persistent launch takes; a hub of a quarter of them, and short lists."""
+    V = 600_011
+    rng = np.random.default_rng(E)
+    dst = rng.integers(0, V, E)
+    dst[: E // 4] = 12_345
+    _check(rng.integers(0, V, E), dst, V, (1, 4))
