@@ -43,7 +43,7 @@ __device__ __forceinline__ bool bm_has(const unsigned long long* bm, uint32_t v)
     return (__ldcg(bm + (v >> 6)) >> (v & 63)) & 1ull;
 }
 
-struct MsBfsPullOp {  // k_pull_direct operator
+struct MsBfsPullOp {  // k_pull_direct operator (several partitions, and the persistent traversal)
     using Acc = unsigned long long;
     const unsigned long long* front;
     const unsigned long long* front_bm;  // 1 bit per vertex: front[v] != 0
@@ -71,6 +71,131 @@ struct MsBfsPullOp {  // k_pull_direct operator
         if (nb && atomicOr(next + v, nb) == 0ull) atomicOr(next_bm + (v >> 6), 1ull << (v & 63));
     }
 };
+
+// A dense level as a full sweep: the walk of the PageRank sweep (eg_pagerank.cu: list starts as one bit
+// per edge, 8 consecutive ids per lane, a segmented warp scan, lists finished one per lane) with OR in
+// the place of the sum.  A list that lies in one run is this warp's alone: its vertex's words are
+// stored plainly; pieces of longer lists are ORed in with atomics, each on its own.  64 roots at
+// 2^23 / 2^27: 0.59 ms a level at 3 to 6 CTAs per SM, 1.05 with a CTA per 4,096 edges, entry bounds in
+// shared memory and atomics for every list.
+constexpr uint32_t kMsBlock = 256;
+
+struct MsSweepArgs {
+    const uint32_t* adj;
+    const uint32_t* heads;    // bit e: edge e is the first of its list
+    const uint32_t* item_of;  // per kPrBlock edges: compressed entry that holds the first one
+    const uint32_t* cvert;
+    uint64_t E;
+    uint64_t nruns;           // runs of kPrBlock << shift edges
+    int shift;
+    const unsigned long long* front;
+    const unsigned long long* front_bm;  // 1 bit per vertex: front[v] != 0
+    int screen;                          // consult front_bm before gathering
+    unsigned long long* visit;
+    unsigned long long* next;
+    unsigned long long* next_bm;
+    const int* stop;  // captured level loops: set once a level found nothing new
+};
+
+__device__ __forceinline__ void ms_piece(const MsSweepArgs& a, uint32_t v, unsigned long long m) {
+    const unsigned long long fresh = m & ~__ldcg(a.visit + v);
+    if (!fresh) return;
+    const unsigned long long nb = fresh & ~atomicOr(a.visit + v, fresh);
+    if (nb && atomicOr(a.next + v, nb) == 0ull) atomicOr(a.next_bm + (v >> 6), 1ull << (v & 63));
+}
+__device__ __forceinline__ void ms_list(const MsSweepArgs& a, uint32_t v, unsigned long long m) {
+    const unsigned long long vis = __ldcg(a.visit + v), nb = m & ~vis;
+    if (!nb) return;
+    a.visit[v] = vis | nb;
+    a.next[v] = nb;
+    atomicOr(a.next_bm + (v >> 6), 1ull << (v & 63));
+}
+
+__global__ void __launch_bounds__(256, 5) k_ms_sweep(MsSweepArgs a) {
+    __shared__ unsigned long long s_or[8][kMsBlock];
+    if (a.stop && *(volatile const int*)a.stop) return;
+    constexpr int G = 8;
+    unsigned long long* s_list = s_or[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    const uint64_t run_edges = (uint64_t)kPrBlock << a.shift;
+    for (uint64_t run = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < a.nruns; run += (uint64_t)gridDim.x * 8) {
+        const uint64_t e_begin = run * run_edges, e_end = min(a.E, e_begin + run_edges);
+        uint32_t item = __ldg(a.item_of + (run << a.shift));
+        bool open_first = !(__ldg(a.heads + (e_begin >> 5)) & 1u);  // the first list began in an earlier run
+        unsigned long long carry = 0;                                // OR of the open list so far
+        for (uint64_t e0 = e_begin; e0 < e_end; e0 += kMsBlock) {
+            const uint64_t e = e0 + lane * G;
+            unsigned long long val[G];
+            uint32_t id[G];
+            uint32_t f = 0;
+            if (e + G <= a.E) {
+                const uint4 x = __ldcs(reinterpret_cast<const uint4*>(a.adj + e));
+                const uint4 y = __ldcs(reinterpret_cast<const uint4*>(a.adj + e) + 1);
+                id[0] = x.x; id[1] = x.y; id[2] = x.z; id[3] = x.w;
+                id[4] = y.x; id[5] = y.y; id[6] = y.z; id[7] = y.w;
+                if (a.screen) {
+#pragma unroll
+                    for (int j = 0; j < G; ++j) val[j] = bm_has(a.front_bm, id[j]) ? ld_keep(a.front + id[j]) : 0ull;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < G; ++j) val[j] = ld_keep(a.front + id[j]);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < G; ++j) val[j] = e + j < a.E ? ld_keep(a.front + a.adj[e + j]) : 0ull;
+            }
+            if (e < a.E) f = __ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8);
+            if (e == e_begin) f &= ~1u;  // the run's first edge opens nothing new
+            uint32_t rank = 0, closed = 0;  // lists that end in earlier lanes, and in the block
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const uint32_t b = __ballot_sync(0xffffffffu, (f >> j) & 1u);
+                rank += __popc(b & below);
+                closed += __popc(b);
+            }
+            const uint32_t v32 = lane < closed ? __ldg(a.cvert + item + lane) : 0u;
+            unsigned long long t = 0, first = 0;
+            uint32_t k = rank;
+            bool seen = false;
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if ((f >> j) & 1u) {
+                    if (seen) s_list[k] = t;
+                    else first = t;
+                    ++k;
+                    seen = true;
+                    t = 0;
+                }
+                t |= val[j];
+            }
+            // the open list along the lanes: t becomes its OR up to and including this lane
+            const uint32_t m = __ballot_sync(0xffffffffu, seen);
+            const int begin = 31 - __clz(m & (below | (1u << lane)));  // last lane that opened one, or -1
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, t, o);
+                if ((int)lane - o >= max(begin, 0)) t |= y;
+            }
+            if (begin < 0) t |= carry;
+            unsigned long long before = __shfl_up_sync(0xffffffffu, t, 1);
+            if (lane == 0) before = carry;
+            if (seen) s_list[rank] = before | first;
+            carry = __shfl_sync(0xffffffffu, t, 31);
+            __syncwarp();
+            for (uint32_t i = lane; i < closed; i += 32) {
+                const unsigned long long x = s_list[i];
+                if (!x) continue;
+                const uint32_t v = i < 32 ? v32 : __ldg(a.cvert + item + i);
+                if (i == 0 && open_first) ms_piece(a, v, x);
+                else ms_list(a, v, x);
+            }
+            __syncwarp();
+            if (closed) open_first = false;
+            item += closed;
+        }
+        if (lane == 0 && carry) ms_piece(a, __ldg(a.cvert + item), carry);
+    }
+}
 
 // Early-exit dense level: a destination stops reading in-edges as soon as its visited word holds
 // every root still running (nothing more can reach it in this level).  One thread per compressed
@@ -199,43 +324,42 @@ struct MsBfsPushOp {
     }
 };
 
-// level bytes of the queued vertices' new bits (row v of [V][64]: 2 threads, two 16-byte quarters
-// each, a quarter rewritten only where one of its roots is new) and the OR of their words, i.e.
-// the roots whose traversal is still running
-// With new_id, the words are also copied to renumbered positions (next_r[new_id[v]]) for the pull
-// gathers that go through the renumbered CSC sources.
+// A traversal keeps its levels as bit planes, [V][4] words for bits 0..3 of the level of each root and
+// [V][4] more for bits 4..7 (zeroed before the first level past 15): a vertex that new roots reach at
+// level l gets their bits ORed into the planes of l, or, when they are its first, its four words
+// written without a read (which is what clears them).  A level touches a sector per vertex where rows
+// of 64 level bytes took a read and a write of up to two; the bytes are made once, at the end.  64
+// roots at 2^23 / 2^27: vertex passes 0.76 -> 0.60 ms.
+// Also the OR of the queued vertices' words, i.e. the roots whose traversal is still running, and,
+// with new_id, the words copied to renumbered positions (next_r[new_id[v]]) for the pull gathers that
+// go through the renumbered CSC sources.
 __device__ __forceinline__ void queue_levels_work(const uint32_t* __restrict__ q, uint32_t n,
-                                                  const unsigned long long* __restrict__ next, uint8_t* levels,
-                                                  uint32_t lvl, unsigned long long* alive_out,
+                                                  const unsigned long long* __restrict__ next,
+                                                  const unsigned long long* visit, unsigned long long* planes,
+                                                  uint64_t V, uint32_t lvl, unsigned long long* alive_out,
                                                   const uint32_t* __restrict__ new_id,
                                                   unsigned long long* __restrict__ next_r) {
-    const uint32_t sub = threadIdx.x & 1u;
-    const uint32_t fill = (lvl & 0xFFu) * 0x01010101u;
     unsigned long long orr = 0;
-    for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1; i < n;
-         i += ((uint64_t)gridDim.x * blockDim.x) >> 1) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t v = q[i];
         const unsigned long long nb = next[v];
-        if (new_id && sub == 0) next_r[new_id[v]] = nb;
+        if (new_id) next_r[new_id[v]] = nb;
         orr |= nb;
+        if (!planes) continue;
+        unsigned long long* p = planes + (uint64_t)v * 4;
+        if (__ldcg(visit + v) == nb) {
+            ulonglong2* p2 = reinterpret_cast<ulonglong2*>(p);
+            p2[0] = make_ulonglong2(lvl & 1u ? nb : 0ull, lvl & 2u ? nb : 0ull);
+            p2[1] = make_ulonglong2(lvl & 4u ? nb : 0ull, lvl & 8u ? nb : 0ull);
+        } else {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const uint32_t quarter = sub * 2 + c;
-            const uint32_t h = (uint32_t)(nb >> (16 * quarter)) & 0xFFFFu;
-            if (levels && h) {
-                uint4* p = reinterpret_cast<uint4*>(levels + (uint64_t)v * 64) + quarter;
-                uint4 x = *p;
-                uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    // bit j of the nibble -> byte j all ones (the shifted copies never overlap)
-                    const uint32_t nib = (h >> (4 * k)) & 0xFu;
-                    const uint32_t m = ((nib * 0x00204081u) & 0x01010101u) * 0xFFu;
-                    w[k] = (w[k] & ~m) | (fill & m);
-                }
-                *p = make_uint4(w[0], w[1], w[2], w[3]);
-            }
+            for (int j = 0; j < 4; ++j)
+                if ((lvl >> j) & 1u) p[j] |= nb;
         }
+        if (lvl < 16) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if ((lvl >> (4 + j)) & 1u) p[4 * V + j] |= nb;
     }
     if (!alive_out) return;
 #pragma unroll
@@ -244,10 +368,47 @@ __device__ __forceinline__ void queue_levels_work(const uint32_t* __restrict__ q
 }
 
 __global__ void k_queue_levels(const uint32_t* __restrict__ q, const uint32_t* n_dev,
-                               const unsigned long long* __restrict__ next, uint8_t* levels, uint32_t lvl,
-                               unsigned long long* alive_out, const uint32_t* __restrict__ new_id,
-                               unsigned long long* __restrict__ next_r) {
-    queue_levels_work(q, __ldcg(n_dev), next, levels, lvl, alive_out, new_id, next_r);
+                               const unsigned long long* __restrict__ next, const unsigned long long* visit,
+                               unsigned long long* planes, uint64_t V, uint32_t lvl, unsigned long long* alive_out,
+                               const uint32_t* __restrict__ new_id, unsigned long long* __restrict__ next_r) {
+    queue_levels_work(q, __ldcg(n_dev), next, visit, planes, V, lvl, alive_out, new_id, next_r);
+}
+
+// level bytes of 16 roots (16 q .. 16 q + 15) of vertex v, 0xFF where the root never reached it
+__device__ __forceinline__ uint4 level_bytes(const unsigned long long* __restrict__ planes,
+                                             const unsigned long long* __restrict__ visit, uint64_t V, uint64_t v, int q,
+                                             int deep) {
+    uint32_t w[4] = {0, 0, 0, 0};
+    const uint32_t vis = (uint32_t)(__ldg(visit + v) >> (16 * q)) & 0xFFFFu;
+    if (vis) {
+        for (int h = 0; h <= deep; ++h) {
+            const ulonglong2* p = reinterpret_cast<const ulonglong2*>(planes + 4 * (h * V + v));
+            const ulonglong2 a = __ldg(p), b = __ldg(p + 1);
+            const unsigned long long pl[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t bits = (uint32_t)(pl[j] >> (16 * q)) & 0xFFFFu;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)  // bit i of the nibble -> byte i (the shifted copies never overlap)
+                    w[k] |= (((bits >> (4 * k)) & 0xFu) * (0x00204081u << (4 * h + j))) & (0x01010101u << (4 * h + j));
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t m = ((((vis >> (4 * k)) & 0xFu) * 0x00204081u) & 0x01010101u) * 0xFFu;
+        w[k] = (w[k] & m) | ~m;
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// level rows [V][64] of a graph batch (out: 16-byte aligned)
+__global__ void __launch_bounds__(256) k_level_rows(const unsigned long long* __restrict__ planes,
+                                                    const unsigned long long* __restrict__ visit, uint64_t V, int deep,
+                                                    uint4* __restrict__ out) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 4 * V; i += stride)
+        __stcs(out + i, level_bytes(planes, visit, V, i >> 2, (int)(i & 3), deep));
 }
 
 // zero the frontier words (and their renumbered copies) of the vertices a queue lists: the only
@@ -281,53 +442,65 @@ __global__ void k_reach_edges(const unsigned long long* __restrict__ visit, cons
     if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
 }
 
-// [V][64] level rows -> [n][V] root rows for the first n roots, 64 vertices per CTA: rows come in
-// as 16-byte loads, leave as 16-byte stores of 16 consecutive vertices (vec: V % 16 == 0 and out
-// 16-byte aligned; bytes otherwise).  A byte whose root never reached the vertex (its visited bit
-// is clear) becomes 0xFF, so the level rows need no initialisation.
-__global__ void __launch_bounds__(256) k_levels_out(const uint8_t* __restrict__ lev,
+// level planes -> [n][V] root rows for the first n roots, 256 vertices per CTA: 64 level bytes per vertex
+// into shared memory, 4 x 4 bytes at a time turned into 16 consecutive vertices of a root, and every
+// root's row stored in whole 16-byte pieces of the output whatever its alignment (V odd: each row
+// starts elsewhere), the row's first and last bytes one by one.  64 roots at 2^23: 0.30 ms (0.87 GB), and
+// 0.33 at 2^23 - 1; from level rows, with a byte per load and 16-byte stores only where V allows, 0.26 and 2.0.
+constexpr uint32_t kOutTile = 256;
+constexpr uint32_t kOutStride = kOutTile / 4 + 4;  // words per root row in shared memory
+__global__ void __launch_bounds__(256) k_levels_out(const unsigned long long* __restrict__ planes,
                                                     const unsigned long long* __restrict__ visit, uint32_t V, int n,
-                                                    uint8_t* __restrict__ out, int vec) {
-    __shared__ __align__(16) uint8_t t[64][68];  // 68-byte rows: column reads spread over banks
-    const uint64_t v0 = (uint64_t)blockIdx.x * 64;
-    {
-        const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
-        const uint64_t v = v0 + r;
-        uint32_t w[4] = {~0u, ~0u, ~0u, ~0u};
-        if (v < V) {
-            const uint4 x = *reinterpret_cast<const uint4*>(lev + v * 64 + 16 * q);
-            const unsigned long long vis = visit[v];
-            w[0] = x.x;
-            w[1] = x.y;
-            w[2] = x.z;
-            w[3] = x.w;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t nib = (uint32_t)(vis >> (16 * q + 4 * j)) & 0xFu;
-                const uint32_t m = ((nib * 0x00204081u) & 0x01010101u) * 0xFFu;  // bit k -> byte k
-                w[j] = (w[j] & m) | ~m;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint32_t*>(&t[r][16 * q + 4 * j]) = w[j];
+                                                    int deep, uint8_t* __restrict__ out) {
+    __shared__ uint32_t t[kOutTile][17];                      // [vertex][root / 4]
+    __shared__ __align__(16) uint32_t u[64][kOutStride];      // [root][vertex / 4]
+    const uint64_t v0 = (uint64_t)blockIdx.x * kOutTile;
+    for (uint32_t i = threadIdx.x; i < 4 * kOutTile; i += blockDim.x) {
+        const uint32_t r = i >> 2, q = i & 3;
+        const uint4 x = v0 + r < V ? level_bytes(planes, visit, V, v0 + r, (int)q, deep) : make_uint4(~0u, ~0u, ~0u, ~0u);
+        t[r][4 * q] = x.x;
+        t[r][4 * q + 1] = x.y;
+        t[r][4 * q + 2] = x.z;
+        t[r][4 * q + 3] = x.w;
     }
     __syncthreads();
-    const int s = threadIdx.x >> 2, k = threadIdx.x & 3;
-    if (s >= n) return;
-    const uint64_t vb = v0 + 16 * (uint64_t)k;
-    uint8_t* o = out + (uint64_t)s * V + vb;
-    if (vec && vb + 16 <= V) {
-        uint32_t w[4];
+    {
+        const uint32_t rq = threadIdx.x & 15, vg = threadIdx.x >> 4;  // roots 4 rq .. + 3, vertices 16 vg .. + 15
+        uint32_t row[4][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int b = 16 * k + 4 * j;
-            w[j] = (uint32_t)t[b][s] | ((uint32_t)t[b + 1][s] << 8) | ((uint32_t)t[b + 2][s] << 16) |
-                   ((uint32_t)t[b + 3][s] << 24);
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t a = t[16 * vg + 4 * k][rq], b = t[16 * vg + 4 * k + 1][rq];
+            const uint32_t c = t[16 * vg + 4 * k + 2][rq], d = t[16 * vg + 4 * k + 3][rq];
+            const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362);
+            const uint32_t cd0 = __byte_perm(c, d, 0x5140), cd1 = __byte_perm(c, d, 0x7362);
+            row[0][k] = __byte_perm(ab0, cd0, 0x5410);
+            row[1][k] = __byte_perm(ab0, cd0, 0x7632);
+            row[2][k] = __byte_perm(ab1, cd1, 0x5410);
+            row[3][k] = __byte_perm(ab1, cd1, 0x7632);
         }
-        *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
-    } else {
-        for (int j = 0; j < 16; ++j)
-            if (vb + j < V) o[j] = t[16 * k + j][s];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            *reinterpret_cast<uint4*>(&u[4 * rq + r][4 * vg]) = make_uint4(row[r][0], row[r][1], row[r][2], row[r][3]);
+    }
+    __syncthreads();
+    const uint32_t nv = V - v0 < kOutTile ? (uint32_t)(V - v0) : kOutTile;
+    const uint32_t c = threadIdx.x & 15;
+    for (uint32_t s = threadIdx.x >> 4; s < (uint32_t)n; s += 16) {
+        uint8_t* o = out + (uint64_t)s * V + v0;
+        const uint8_t* bytes = reinterpret_cast<const uint8_t*>(u[s]);
+        const uint32_t first = (uint32_t)(-(uintptr_t)o & 15u);  // bytes before the first whole piece
+        const uint32_t pieces = nv > first ? (nv - first) / 16 : 0u;
+        if (c < pieces) {
+            const uint32_t at = first + 16 * c, w = at >> 2, sh = (at & 3u) * 8;
+            uint32_t x[5];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) x[k] = u[s][w + k];
+            *reinterpret_cast<uint4*>(o + at) =
+                make_uint4(__funnelshift_r(x[0], x[1], sh), __funnelshift_r(x[1], x[2], sh), __funnelshift_r(x[2], x[3], sh),
+                           __funnelshift_r(x[3], x[4], sh));
+        }
+        if (c < first && c < nv) o[c] = bytes[c];
+        for (uint32_t i = first + 16 * pieces + c; i < nv; i += 16) o[i] = bytes[i];
     }
 }
 
@@ -909,19 +1082,22 @@ __global__ void k_root_entries_graphs(const uint32_t* roots, const uint64_t* vof
 }
 
 __global__ void k_msbfs_init_entries(const uint2* ent, const uint32_t* n_dev, unsigned long long* visit,
-                                     unsigned long long* front, unsigned long long* front_bm, uint8_t* levels,
-                                     uint32_t* q, uint32_t* nq, unsigned long long* act_edges, const uint32_t* deg) {
+                                     unsigned long long* front, unsigned long long* front_bm,
+                                     unsigned long long* planes, uint32_t* q, uint32_t* nq, unsigned long long* act_edges, const uint32_t* deg) {
     const uint32_t n = *n_dev;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t v = ent[i].x, s = ent[i].y;
         const unsigned long long bit = 1ull << s;
-        const unsigned long long old = atomicOr(visit + v, bit);
+        atomicOr(visit + v, bit);
         if (atomicOr(front + v, bit) == 0ull) {
             atomicOr(front_bm + (v >> 6), 1ull << (v & 63));
             q[atomicAdd(nq, 1u)] = v;
             atomicAdd(act_edges, (unsigned long long)deg[v]);
+            if (planes) {  // level 0
+                ulonglong2* p = reinterpret_cast<ulonglong2*>(planes + (uint64_t)v * 4);
+                p[0] = p[1] = make_ulonglong2(0ull, 0ull);
+            }
         }
-        if (!(old & bit) && levels) levels[(uint64_t)v * 64 + s] = 0;
     }
 }
 
@@ -1019,7 +1195,7 @@ struct MsPersistArgs {
     uint32_t* q0;
     uint32_t* q1;
     const unsigned long long* alive_all;
-    uint8_t* lev;
+    unsigned long long* lev;  // level planes
     unsigned long long* ms_seg;
     uint64_t* desc;
     uint64_t* ipref;
@@ -1108,7 +1284,7 @@ __global__ void __launch_bounds__(256, 4) k_msbfs_persistent(MsPersistArgs a) {
         n = __ldcg(&w->cnt[L]);
         act = __ldcg(&w->act[L]);
         if (dense) ++dense_count;
-        if (a.lev) queue_levels_work(q_next, n, next, a.lev, L + 1, nullptr, nullptr, nullptr);
+        if (a.lev) queue_levels_work(q_next, n, next, a.visit, a.lev, a.V, L + 1, nullptr, nullptr, nullptr);
         if (tid == 0) {
             w->levels = L + 1;
             w->pushes += dense ? 0u : 1u;
@@ -1116,11 +1292,41 @@ __global__ void __launch_bounds__(256, 4) k_msbfs_persistent(MsPersistArgs a) {
     }
 }
 
+// one dense level as a full sweep (k_ms_sweep)
+static int ms_sweep(eg_graph* g, const uint32_t* adj, const unsigned long long* front, const unsigned long long* front_bm,
+                    int screen, unsigned long long* visit, unsigned long long* next, unsigned long long* next_bm,
+                    const unsigned long long* alive, const int* stop) {
+    EngineState& s = g->eng;
+    if (!g->E) return EG_OK;
+    if (g->partitions > 1) {  // a vertex has a list per partition, and sentinel entries lie between them
+        MsBfsPullOp op{front, front_bm, screen, visit, next, next_bm, alive, stop};
+        return launch_pull_direct(g, op, "msbfs_pull", adj, stop ? (unsigned)g->num_sms * 128u : 0u);
+    }
+    MsSweepArgs a;
+    a.adj = adj;
+    a.heads = s.pr_heads.as<uint32_t>();
+    a.item_of = s.pr_item_of.as<uint32_t>();
+    a.cvert = g->cvert.as<uint32_t>();
+    a.E = g->E;
+    a.shift = list_run_shift(g->E);
+    a.nruns = (g->E + ((uint64_t)kPrBlock << a.shift) - 1) / ((uint64_t)kPrBlock << a.shift);
+    a.front = front;
+    a.front_bm = front_bm;
+    a.screen = screen;
+    a.visit = visit;
+    a.next = next;
+    a.next_bm = next_bm;
+    a.stop = stop;
+    Timed t(&g->prof, g->stream, "msbfs_pull");
+    k_ms_sweep<<<(unsigned)std::min<uint64_t>((a.nruns + 7) / 8, (uint64_t)g->num_sms * 64u), 256, 0, g->stream>>>(a);
+    EG_CHECK_LAUNCH("k_ms_sweep");
+    return EG_OK;
+}
+
 // MS-BFS over root entries already in b.entries (count in b.n_entries device word)
-// lev_filled: the level rows start as 0xFF (callers that hand them out as they are); otherwise
-// their unreached bytes are left as they are and masked by k_levels_out
-static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, uint64_t* reach_out, int* sweeps_out,
-                      int* pushes_out, bool lev_filled) {
+// lev: level planes (2 x [V][4] words) or null
+static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long long* lev, uint64_t* reach_out,
+                      int* sweeps_out, int* pushes_out) {
     BatchState& b = bstate(g);
     EngineState& s = g->eng;
     const uint64_t V = g->V;
@@ -1144,6 +1350,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
     // pull gathers through the CSC sources renumbered by out-degree class (hot frontier words share
     // cache lines), with a renumbered copy of each frontier; on one graph with the host-driven loop
     const bool renum = one_graph && !(g->use_cuda_graph & 1) && g->batch_launch != 1 && g->E > 0 && want_relabel(g);
+    if (g->E && g->partitions == 1) EG_TRY(setup_list_heads(g, renum));
     if (renum) {
         EG_TRY(setup_relabel(g));
         EG_TRY(b.wr0.reserve(8 * V + 8));
@@ -1161,7 +1368,9 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
         EG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (kGraphLevels + 2), g->stream));
         EG_CUDA(cudaMemcpyAsync(alive + 2, &full, 8, cudaMemcpyHostToDevice, g->stream));
         EG_CUDA(cudaMemcpyAsync(alive, &full, 8, cudaMemcpyHostToDevice, g->stream));
-        if (lev && lev_filled) EG_CUDA(cudaMemsetAsync(lev, 0xFF, 64 * V, g->stream));
+        // bits 4..7 of the levels: where the loop runs on the device, ahead of time
+        if (lev && (g->batch_launch == 1 || (g->use_cuda_graph & 1)))
+            EG_CUDA(cudaMemsetAsync(lev + 4 * V, 0, 32 * V, g->stream));
         k_msbfs_init_entries<<<init_grid, 256, 0, g->stream>>>(b.entries.as<uint2>(), b.n_entries.as<uint32_t>(), visit,
                                                                word[0], bm[0], lev, queue[0], d_nq, d_act, deg);
         EG_CHECK_LAUNCH("k_msbfs_init_entries");
@@ -1176,7 +1385,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
     // queue length lands in *count; captured loops (stop_flag set) pull every level and keep the
     // alive mask at "all roots".
     // The first dense level follows the frontier's explosion: most destinations miss most roots and
-    // read all their in-edges, which the balanced chunked sweep (k_pull_direct) does best.  Later
+    // read all their in-edges, which the full sweep (k_ms_sweep) does best.  Later
     // dense levels find most destinations nearly covered and use the early-exit pair -- on one
     // graph.  In a batch of graphs the running-root mask is shared by all graphs, so a vertex
     // waits for bits its own graph can never deliver, and every level keeps the chunked sweep.
@@ -1217,9 +1426,8 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
                 k_ms_tail<<<grid, 256, 0, g->stream>>>(ma);
                 EG_CHECK_LAUNCH("k_ms_tail");
             } else {
-                MsBfsPullOp op{gather_word, bm[c], screen ? 1 : 0, visit, word[x], bm[x],
-                               stop_flag ? alive + 2 : alive + c, stop_flag};
-                EG_TRY(launch_pull_direct(g, op, "msbfs_pull", gather_adj));
+                EG_TRY(ms_sweep(g, gather_adj, gather_word, bm[c], screen ? 1 : 0, visit, word[x], bm[x],
+                                stop_flag ? alive + 2 : alive + c, stop_flag));
             }
             Timed t(&g->prof, g->stream, "msbfs_vertex");
             k_bm_compact<<<grid_for(nwords, 256, grid), 256, 0, g->stream>>>(bm[x], nwords, queue[x], count,
@@ -1231,7 +1439,9 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
         }
         if (lev || alive_next || renum) {
             Timed t(&g->prof, g->stream, "msbfs_vertex");
-            k_queue_levels<<<grid, 256, 0, g->stream>>>(queue[x], count, word[x], lev, L + 1, alive_next,
+            if (lev && L + 1 == 16 && !(g->batch_launch == 1 || (g->use_cuda_graph & 1)))
+                EG_CUDA(cudaMemsetAsync(lev + 4 * V, 0, 32 * V, g->stream));
+            k_queue_levels<<<grid, 256, 0, g->stream>>>(queue[x], count, word[x], visit, lev, V, L + 1, alive_next,
                                                         renum ? new_id : nullptr, word_r[x]);
             EG_CHECK_LAUNCH("k_queue_levels");
         }
@@ -1388,8 +1598,9 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
                 ok(cudaMemsetAsync(bm[x], 0, bm_bytes, g->stream));
                 // pull: the chunked sweep or the early-exit pair, whichever the level armed
                 {
-                    MsBfsPullOp op{word[c], bm[c], 1, visit, word[x], bm[x], alive + 2, &cs->lv[L].skip_direct};
-                    if (st == EG_OK) st = launch_pull_direct(g, op, "msbfs_pull", gather_adj, 16 * grid);
+                    if (st == EG_OK)
+                        st = ms_sweep(g, gather_adj, word[c], bm[c], 1, visit, word[x], bm[x], alive + 2,
+                                      &cs->lv[L].skip_direct);
                     uint32_t* d_nseg = reinterpret_cast<uint32_t*>(cnt + kGraphLevels + 2);
                     ok(cudaMemsetAsync(d_nseg, 0, 4, g->stream));
                     MsBuArgs ma{gather_adj, g->cidx.as<uint64_t>(), g->cvert.as<uint32_t>(), g->ncompressed - 1,
@@ -1438,7 +1649,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, uint8_t* lev, 
                                                                                 cs->act + L, deg);
                 ok(cudaGetLastError());
                 if (lev) {
-                    k_queue_levels<<<grid, 256, 0, g->stream>>>(queue[x], cnt + L, word[x], lev, L + 1, nullptr,
+                    k_queue_levels<<<grid, 256, 0, g->stream>>>(queue[x], cnt + L, word[x], visit, lev, V, L + 1, nullptr,
                                                                 nullptr, nullptr);
                     ok(cudaGetLastError());
                 }
@@ -1541,10 +1752,10 @@ int run_msbfs(eg_graph* g, const uint32_t* roots, int n, uint8_t* levels, int wh
     EG_TRY(copy_small_in(g, b.seeds, roots, n, where));
     k_root_entries<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, 0, b.entries.as<uint2>());
     EG_CHECK_LAUNCH("k_root_entries");
-    uint8_t* lev = levels ? b.lev.as<uint8_t>() : nullptr;
+    unsigned long long* lev = levels ? b.lev.as<unsigned long long>() : nullptr;
     uint64_t reach = 0;
     int sweeps = 0, pushes = 0;
-    EG_TRY(msbfs_core(g, (uint32_t)n, n, lev, &reach, &sweeps, &pushes, false));
+    EG_TRY(msbfs_core(g, (uint32_t)n, n, lev, &reach, &sweeps, &pushes));
     if (levels) {
         uint8_t* out = levels;
         if (where != EG_DEVICE) {
@@ -1553,9 +1764,8 @@ int run_msbfs(eg_graph* g, const uint32_t* roots, int n, uint8_t* levels, int wh
         }
         {
             Timed t(&g->prof, g->stream, "msbfs_levels_out");
-            const int vec = (V % 16 == 0) && (((uintptr_t)out & 15u) == 0);
-            k_levels_out<<<(unsigned)((V + 63) / 64), 256, 0, g->stream>>>(lev, b.a64.as<unsigned long long>(),
-                                                                          (uint32_t)V, n, out, vec);
+            k_levels_out<<<(unsigned)((V + kOutTile - 1) / kOutTile), 256, 0, g->stream>>>(
+                lev, b.a64.as<unsigned long long>(), (uint32_t)V, n, sweeps >= 16 ? 1 : 0, out);
             EG_CHECK_LAUNCH("k_levels_out");
         }
         if (where != EG_DEVICE)
@@ -2057,10 +2267,26 @@ int run_msbfs_graphs(eg_graph* g, const uint32_t* roots, int nper, uint8_t* leve
     EG_CUDA(cudaMemcpyAsync(b.n_entries.ptr, &n, 4, cudaMemcpyHostToDevice, g->stream));
     uint64_t reach = 0;
     int sweeps = 0, pushes = 0;
-    EG_TRY(msbfs_core(g, n, nper, levels ? b.lev.as<uint8_t>() : nullptr, &reach, &sweeps, &pushes, true));
-    if (levels)
-        EG_CUDA(cudaMemcpyAsync(levels, b.lev.ptr, 64ull * g->V,
-                                where == EG_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, g->stream));
+    unsigned long long* lev = levels ? b.lev.as<unsigned long long>() : nullptr;
+    EG_TRY(msbfs_core(g, n, nper, lev, &reach, &sweeps, &pushes));
+    if (levels) {
+        const uint64_t V = g->V;
+        uint8_t* out = levels;
+        const bool direct = where == EG_DEVICE && ((uintptr_t)levels & 15u) == 0;
+        if (!direct) {
+            EG_TRY(b.tmp_out.reserve(64 * V + 64));
+            out = b.tmp_out.as<uint8_t>();
+        }
+        {
+            Timed t(&g->prof, g->stream, "msbfs_levels_out");
+            k_level_rows<<<grid_for(4 * V, 256, (unsigned)g->num_sms * 16u), 256, 0, g->stream>>>(
+                lev, b.a64.as<unsigned long long>(), V, sweeps >= 16 ? 1 : 0, reinterpret_cast<uint4*>(out));
+            EG_CHECK_LAUNCH("k_level_rows");
+        }
+        if (!direct)
+            EG_CUDA(cudaMemcpyAsync(levels, out, 64 * V, where == EG_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                                    g->stream));
+    }
     EG_CUDA(cudaStreamSynchronize(g->stream));
     if (edges) *edges = reach;
     g->last_edges_processed = reach;

@@ -256,6 +256,11 @@ int selftest_bounded_wait(eg_graph* g, uint32_t spin_cap);
 int selftest_grid_barrier(eg_graph* g, uint32_t spin_cap);
 int validate_edges(eg_graph* g, uint64_t E);
 int symmetrize_edges(eg_graph* g, uint64_t E);
+// list-start bits and block entries for sweeps by independent warps (eg_pagerank.cu), made once per
+// structure build: kPrBlock edges per block entry, runs of kPrBlock << list_run_shift(E) edges
+constexpr uint32_t kPrBlock = 512;
+int setup_list_heads(eg_graph* g, bool relabel);  // relabel: with places in renumbered order
+int list_run_shift(uint64_t E);
 int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, int where);
 int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where);
 // renumbering of the CSC sources by out-degree class (eng.pr_new_id / eng.pr_adj), built once per

@@ -18,7 +18,6 @@
 
 namespace eg {
 
-constexpr uint32_t kPrBlock = 512;  // edges per warp step
 constexpr uint32_t kNoBoundary = 0xFFFFFFFFu;
 constexpr int kPrGroup = 8;  // consecutive edges per lane: 4 or 16 were no faster (40.3 / 40.3 against 39.4 ms of sweeps)
 
@@ -258,7 +257,7 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
 
 // Blocks per run: few boundaries (sweeps at 2^25 / 2^29 with 1 / 4 / 8 blocks: 41.2 / 38.6 / 38.0 ms), but runs
 // enough for every resident warp several times (1 M / 16 M: 1.44 / 1.71 / 1.72).
-static int pr_shift(uint64_t E) {
+int list_run_shift(uint64_t E) {
     int s = 0;
     while (s < 3 && (E >> (10 + s)) >= 24000) ++s;
     return s;
@@ -269,7 +268,7 @@ static int pr_setup(eg_graph* g, const uint32_t* order) {
     if (s.pr_heads_ready && s.pr_heads_relabel == (order != nullptr)) return EG_OK;
     const uint64_t E = g->E, nitems = g->ncompressed - 1;
     const size_t words = E / 32 + 2;
-    const int shift = pr_shift(E);
+    const int shift = list_run_shift(E);
     EG_TRY(s.pr_heads.reserve(4 * words + 64));
     EG_TRY(s.pr_item_of.reserve(4 * (E / kPrBlock + 2)));
     EG_TRY(s.pr_split.reserve(4 * ((E / kPrBlock >> shift) + 3)));
@@ -287,15 +286,19 @@ static int pr_setup(eg_graph* g, const uint32_t* order) {
     return EG_OK;
 }
 
+int setup_list_heads(eg_graph* g, bool relabel) {
+    if (relabel) EG_TRY(setup_relabel(g));
+    return pr_setup(g, relabel ? g->eng.pr_new_id.as<uint32_t>() : nullptr);
+}
+
 int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, int where) {
     EngineState& s = g->eng;
     const uint64_t V = g->V, E = g->E;
     for (DevBuf* b : {&s.vals0, &s.vals1}) EG_TRY(b->reserve(4 * (V + 1)));
     // with renumbered gathers every vector but the final one is kept in class order
     const bool relabel = want_relabel(g);
-    if (relabel) EG_TRY(setup_relabel(g));
+    EG_TRY(setup_list_heads(g, relabel));
     const uint32_t* order = relabel ? s.pr_new_id.as<uint32_t>() : nullptr;
-    EG_TRY(pr_setup(g, order));
     float* vec[2] = {s.vals0.as<float>(), s.vals1.as<float>()};
     float* result = out && where == EG_DEVICE ? out : vec[iterations & 1];
     // every iteration in one launch up to here: 20 iterations take 0.26 / 0.35 ms (one launch / two per
@@ -308,7 +311,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     p.dst = relabel ? s.pr_place.as<uint32_t>() : g->cvert.as<uint32_t>();
     p.deg = s.pr_deg.as<uint32_t>();
     p.E = E;
-    p.shift = pr_shift(E);
+    p.shift = list_run_shift(E);
     p.nruns = (E + (kPrBlock << p.shift) - 1) / (kPrBlock << p.shift);
     EG_TRY(s.acc.reserve(4 * (p.nruns + 2)));
     p.acc = s.acc.as<float>();

@@ -283,3 +283,73 @@ def test_ppr_adjoint_against_fp64_autograd_and_finite_differences(eg_lib):
             fd[j] = (lp - lm) / (2 * h)
     err = np.linalg.norm(grad[idx] - fd) / np.linalg.norm(fd)
     assert err <= 1e-3, err
+
+
+@pytest.mark.parametrize("cuda_graph,persistent", [(0, 0), (1, 0), (0, 1)])
+def test_level_planes_shallow_and_deep(eg_lib, cuda_graph, persistent):
+    """Levels on both sides of every bit of their planes (a 250-vertex chain beside a random graph, in
+    one batch and as one graph), for roots that share vertices and for vertices that roots reach at
+    different levels; rows written to aligned and unaligned device memory and to the host."""
+    import torch
+
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(6)
+    n = 250
+    perm = rng.permutation(n).astype(np.uint32)
+    chain = (np.concatenate([perm[:-1], perm[1:16]]), np.concatenate([perm[1:], perm[:15]]))  # a stretch both ways
+    rs, rd = rng.integers(0, 400, 3000).astype(np.uint32), rng.integers(0, 400, 3000).astype(np.uint32)
+    graphs = [(chain[0], chain[1], n), (rs, rd, 400)]
+    per = 40
+    roots = np.concatenate([np.r_[perm[0], perm[:39]], rng.integers(0, 400, per)]).astype(np.uint32)
+    rec = np.concatenate([eg.pack_edges(s, d) for s, d, _ in graphs])
+    eoff = np.cumsum([0] + [len(s) for s, _, _ in graphs]).astype(np.uint64)
+    V = n + 400
+    want = np.full((V, 64), 255, np.uint8)
+    for k, (s, d, nv) in enumerate(graphs):
+        csr = oracle.build_csr(s, d, None, nv, np.array([0, nv], np.uint32))
+        for j in range(per):
+            ref = oracle.bfs_levels(csr["off"][0], csr["adj"], nv, int(roots[k * per + j]))
+            want[k * n:k * n + nv, j] = np.where(ref == oracle.UNREACHED, 255, ref).astype(np.uint8)
+    with eg.Graph() as g:
+        g.set_option(eg.EG_OPT_CUDA_GRAPH, cuda_graph)
+        g.set_option(eg.EG_OPT_BATCH_LAUNCH, persistent)
+        g.load_graph_batch(rec, eoff, np.array([n, 400], np.uint32))
+        for _ in range(2):
+            host, _ = g.msbfs_graphs(roots, per)
+            assert np.array_equal(host, want)
+        buf = torch.zeros(64 * V + 64, dtype=torch.uint8, device="cuda")
+        for skip in (0, 7, 16):
+            out = buf[skip:skip + 64 * V].view(V, 64)
+            g.msbfs_graphs(roots, per, levels=out)
+            assert np.array_equal(out.cpu().numpy(), want), skip
+        g.load_directed(eg.pack_edges(*chain), n)
+        for _ in range(2):
+            levels, _ = g.msbfs(roots[:per])
+            assert np.array_equal(levels, want[:n, :per].T)
+
+
+@pytest.mark.parametrize("V", [1, 3, 15, 16, 17, 255, 256, 257, 271, 1003, 4096])
+def test_msbfs_rows_of_any_alignment(eg_lib, V):
+    """Root rows of V bytes each, on the host and at any byte offset of device memory; bytes around the
+    rows stay as they were."""
+    import torch
+
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(V)
+    E = 4 * V
+    src, dst = rng.integers(0, V, E).astype(np.uint32), rng.integers(0, V, E).astype(np.uint32)
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    roots = rng.integers(0, V, 64).astype(np.uint32)
+    ref = np.stack([oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(r)) for r in roots])
+    want = np.where(ref == oracle.UNREACHED, 255, ref).astype(np.uint8)
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        for n in (1, 5, 17, 64):
+            levels, _ = g.msbfs(roots[:n])
+            assert np.array_equal(levels, want[:n])
+            for skip in (0, 1, 6, 13):
+                buf = torch.full((n * V + 64,), 77, dtype=torch.uint8, device="cuda")
+                g.msbfs(roots[:n], levels=buf[skip:skip + n * V].view(n, V))
+                h = buf.cpu().numpy()
+                assert np.array_equal(h[skip:skip + n * V].reshape(n, V), want[:n]), (n, skip)
+                assert (h[:skip] == 77).all() and (h[skip + n * V:] == 77).all()
