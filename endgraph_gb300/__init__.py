@@ -198,8 +198,11 @@ class Graph:
             return
         for x in values:
             if isinstance(x, torch.Tensor) and x.is_cuda:
+                current = torch.cuda.current_stream(x.device)
+                if current.query():  # nothing pending: nothing to wait for (3 us; the event takes 8)
+                    return
                 ev = torch.cuda.Event()
-                ev.record(torch.cuda.current_stream(x.device))
+                ev.record(current)
                 torch.cuda.ExternalStream(self.stream, device=x.device).wait_event(ev)
                 return
 

@@ -230,6 +230,8 @@ struct PrPersistArgs {
     float* out;             // the last vector
     int iterations;
     unsigned* words;        // barrier count, unused, error flag
+    void* words_next;       // the next launch's, zeroed by this one
+    uint32_t* finished;     // pinned: set when the last iteration is done
 };
 
 constexpr int kPrPersistThreads = 512, kPrPersistCtas = 2;
@@ -253,6 +255,8 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
         if (!barrier()) return;
         for (uint64_t r = tid; r < p.nruns; r += stride) pr_boundary(p, r);
     }
+    if (tid < 32) persist_clear(a.words_next);
+    if (tid == 0) *a.finished = 1;
 }
 
 // Blocks per run: few boundaries (sweeps at 2^25 / 2^29 with 1 / 4 / 8 blocks: 41.2 / 38.6 / 38.0 ms), but runs
@@ -320,9 +324,10 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     p.base = 1.0f - damping;
     p.d = damping;
     if (small) {
-        EG_TRY(s.persist.reserve(64));
-        EG_CUDA(cudaMemsetAsync(s.persist.ptr, 0, 16, g->stream));
-        PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations, s.persist.as<unsigned>()};
+        void *block = nullptr, *next = nullptr;
+        EG_TRY(persist_block(g, &block, &next));
+        PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations,
+                        static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words)};
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((uint64_t)g->num_sms * kPrPersistCtas, (p.nruns + kPrPersistThreads / 32 - 1) / (kPrPersistThreads / 32)));
         void* kargs[] = {&a};
@@ -331,8 +336,8 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
             EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_pr_persistent, dim3(grid), dim3(kPrPersistThreads), kargs, 0,
                                                 g->stream));
             EG_CHECK_LAUNCH("k_pr_persistent");
+            persist_launched(g);
         }
-        EG_CUDA(cudaMemcpyAsync(s.host_words, s.persist.ptr, 16, cudaMemcpyDeviceToHost, g->stream));
     } else {
         const unsigned gv = grid_for(V, 256, 152u * 16u);
         {
@@ -365,7 +370,8 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     if (out && where != EG_DEVICE)
         EG_CUDA(cudaMemcpyAsync(out, result, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
     EG_CUDA(cudaStreamSynchronize(g->stream));
-    if (small && reinterpret_cast<const int*>(s.host_words)[2]) {
+    if (small && !*reinterpret_cast<volatile uint32_t*>(s.host_words)) {
+        persist_reset(g);
         set_error("eg_pagerank: a bounded grid barrier gave up");
         return EG_ERR_TIMEOUT;
     }

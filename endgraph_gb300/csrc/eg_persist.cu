@@ -45,10 +45,17 @@ struct PersistState {
     StepSlot slot[4];    // step k reads slot k & 3, fills slot (k + 1) & 3 and clears slot (k + 2) & 3
     float thr, delta;    // SSSP near/far threshold and its step
     float weight_sum;    // sampled weights
-    uint32_t done;
+    uint32_t pushes;
     unsigned long long edges;  // edges of the pieces walked
-    uint32_t pushes, splits;
 };
+
+// what a launch tells the host, written to pinned memory by its first thread as it ends; `valid` stays
+// zero when a barrier gave up
+struct PersistResult {
+    uint32_t valid, done, step, pushes, pulls, pad;
+    unsigned long long reached, edges;
+};
+static_assert(sizeof(PersistResult) <= 256, "the results lie in the handle's pinned words");
 
 // one grid barrier; *s_slot gets the slot the finished step filled.  False: a wait gave up.
 template <class State, class Slot>
@@ -188,6 +195,8 @@ struct SsspPersistArgs {
     float delta;        // > 0: given; 0: plain sweeps; < 0: -delta x the sampled mean weight
     int resume;         // continue from the state an earlier launch left
     PersistState* st;
+    void* st_next;      // the next launch's state, zeroed by this one
+    PersistResult* result;
 };
 
 constexpr uint32_t kWeightSamples = 65536;
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint32_t warp = (uint32_t)(tid >> 5), nwarps = (uint32_t)(stride >> 5);
     unsigned long long my_edges = 0;
-    uint32_t step = 0, pushes = 0, splits = 0;
+    uint32_t step = 0, pushes = 0;
     float thr, delta;
     if (!a.resume) {
         for (uint64_t v = tid; v < a.V; v += stride) {
@@ -365,21 +374,22 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
                 atomicMin(&out->min_bits, mn);
                 atomicAdd(&out->parked, left);
             }
-            ++splits;
             last_kind = 1;
         }
         ++step;
         flush_pieces(lq, wb, q_out, &out->n);
         if (!step_barrier(st, out, &s_slot, arrived)) return;
     }
+    // every CTA leaves the loop at the same step; the edges walked are added up behind one more barrier
     if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
-    if (tid == 0) {  // every CTA leaves the loop at the same step
+    if (!step_barrier(st, &st->slot[step & 3], &s_slot, arrived)) return;
+    if (tid < 32) persist_clear(a.st_next);
+    if (tid == 0) {
         st->step = step;
         st->thr = thr;
         st->delta = delta;
-        st->done = done ? 1u : 0u;
         st->pushes += pushes;
-        st->splits += splits;
+        *a.result = PersistResult{1u, done ? 1u : 0u, step, st->pushes, 0u, 0u, 0ull, __ldcg(&st->edges)};
     }
 }
 
@@ -406,7 +416,6 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
     EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
     for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
-    EG_TRY(s.persist.reserve(sizeof(PersistState)));
     float* d_dist = dist;
     if (where != EG_DEVICE || !dist) {
         EG_TRY(s.vals0.reserve(sizeof(float) * (V + 1)));
@@ -426,13 +435,15 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     a.q[1] = s.pieces1.as<uint4>();
     a.root = root;
     a.delta = g->sssp_delta >= 0 ? (float)((double)g->sssp_delta * 1e-6) : -auto_delta(V, E);
-    a.st = s.persist.as<PersistState>();
+    static_assert(sizeof(PersistState) <= kPersistBytes, "one block of the state words");
+    void* block = nullptr;
+    EG_TRY(persist_block(g, &block, &a.st_next));
+    a.st = static_cast<PersistState*>(block);
+    a.result = reinterpret_cast<PersistResult*>(s.host_words);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
-    static_assert(sizeof(PersistState) <= 256, "the state is read back through the 256-byte pinned block");
-    PersistState* h = reinterpret_cast<PersistState*>(s.host_words);
-    EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(PersistState), g->stream));
+    volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
         void* kargs[] = {&a};
@@ -441,14 +452,16 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
             EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
                                                 g->stream));
             EG_CHECK_LAUNCH("k_sssp_persistent");
+            if (!a.resume) persist_launched(g);
         }
-        EG_CUDA(cudaMemcpyAsync(h, a.st, sizeof(PersistState), cudaMemcpyDeviceToHost, g->stream));
         EG_CUDA(cudaStreamSynchronize(g->stream));
-        if (h->err) {
+        if (!h->valid) {
+            persist_reset(g);
             set_error("eg_sssp: a bounded grid barrier gave up");
             return EG_ERR_TIMEOUT;
         }
         if (h->done) break;
+        h->valid = 0;
     }
     g->last_edges_processed = h->edges;
     g->last_iterations = (int)h->pushes;
@@ -487,7 +500,7 @@ struct alignas(16) BfsSlot {
 struct BfsPersistState {
     unsigned bar_count, bar_pad;
     int err;
-    uint32_t step, done, pushes, pulls, pad;
+    uint32_t step, pushes, pulls, pad[2];
     BfsSlot slot[4];  // as PersistState::slot
     unsigned long long reached, edges;
 };
@@ -508,6 +521,8 @@ struct BfsPersistArgs {
     unsigned long long dense_min;
     int resume;
     BfsPersistState* st;
+    void* st_next;  // the next launch's state, zeroed by this one
+    PersistResult* result;
 };
 
 __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persistent(BfsPersistArgs a) {
@@ -775,13 +790,14 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
         edges += s_slot.act;
         ++step;
     }
+    if (tid < 32) persist_clear(a.st_next);
     if (tid == 0) {  // every CTA leaves the loop at the same step
         st->step = step;
-        st->done = s_slot.verts == 0 ? 1u : 0u;
         st->reached = reached;
         st->edges = edges;
         st->pushes += pushes;
         st->pulls += pulls;
+        *a.result = PersistResult{1u, s_slot.verts == 0 ? 1u : 0u, step, st->pushes, st->pulls, 0u, reached, edges};
     }
 }
 
@@ -789,7 +805,6 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
     for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
-    EG_TRY(s.persist.reserve(sizeof(BfsPersistState)));
     BfsPersistArgs a;
     a.level = level;
     a.parent = parent;
@@ -816,13 +831,15 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     a.direction = g->bfs_direction;
     a.has_csc = g->built_csc ? 1 : 0;
     a.dense_min = E / (uint64_t)g->dense_div;
-    a.st = s.persist.as<BfsPersistState>();
+    static_assert(sizeof(BfsPersistState) <= kPersistBytes, "one block of the state words");
+    void* block = nullptr;
+    EG_TRY(persist_block(g, &block, &a.st_next));
+    a.st = static_cast<BfsPersistState*>(block);
+    a.result = reinterpret_cast<PersistResult*>(s.host_words);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
-    static_assert(sizeof(BfsPersistState) <= 256, "the state is read back through the 256-byte pinned block");
-    BfsPersistState* h = reinterpret_cast<BfsPersistState*>(s.host_words);
-    EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(BfsPersistState), g->stream));
+    volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
         void* kargs[] = {&a};
@@ -831,14 +848,16 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
             EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
                                                 g->stream));
             EG_CHECK_LAUNCH("k_bfs_persistent");
+            if (!a.resume) persist_launched(g);
         }
-        EG_CUDA(cudaMemcpyAsync(h, a.st, sizeof(BfsPersistState), cudaMemcpyDeviceToHost, g->stream));
         EG_CUDA(cudaStreamSynchronize(g->stream));
-        if (h->err) {
+        if (!h->valid) {
+            persist_reset(g);
             set_error("eg_bfs: a bounded grid barrier gave up");
             return EG_ERR_TIMEOUT;
         }
         if (h->done) break;
+        h->valid = 0;
     }
     g->last_edges_processed = h->edges;  // sum of out-degrees of the reached vertices
     g->last_iterations = (int)h->step;
@@ -882,6 +901,8 @@ struct CcArgs {
     uint32_t* comp;
     uint4* q;
     CcState* st;
+    void* st_next;  // the next launch's state, zeroed by this one
+    PersistResult* result;
 };
 constexpr uint32_t kCcFirst = 2;      // neighbours united before the common component is looked for
 constexpr int kCcSamples = 1024;
@@ -1013,37 +1034,41 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
         cc_compress(a.comp, a.V, tid, stride);
     }
+    if (tid < 32) persist_clear(a.st_next);
+    if (tid == 0) a.result->valid = 1;
 }
 
 int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
     EG_TRY(s.pieces0.reserve(sizeof(uint4) * queue_entries(g)));
-    EG_TRY(s.persist.reserve(sizeof(CcState)));
+    static_assert(sizeof(CcState) <= kPersistBytes, "one block of the state words");
+    void *block = nullptr, *next = nullptr;
+    EG_TRY(persist_block(g, &block, &next));
+    PersistResult* h = reinterpret_cast<PersistResult*>(s.host_words);
     uint32_t* comp = label;
     if (where != EG_DEVICE || !label) {
         EG_TRY(s.vals0.reserve(sizeof(uint32_t) * (V + 1)));
         comp = s.vals0.as<uint32_t>();
     }
-    CcArgs a{V, g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(), s.persist.as<CcState>()};
+    CcArgs a{V, g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(),
+             static_cast<CcState*>(block), next, h};
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_cc_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, (V + E / 16) / kEdgesPerCta));
-    static_assert(sizeof(CcState) <= 256, "the state is read back through the 256-byte pinned block");
-    CcState* h = reinterpret_cast<CcState*>(s.host_words);
-    EG_CUDA(cudaMemsetAsync(a.st, 0, sizeof(CcState), g->stream));
     void* kargs[] = {&a};
     {
         Timed t(&g->prof, g->stream, "cc_persistent");
         EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_cc_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
                                             g->stream));
         EG_CHECK_LAUNCH("k_cc_persistent");
+        persist_launched(g);
     }
-    EG_CUDA(cudaMemcpyAsync(h, a.st, sizeof(CcState), cudaMemcpyDeviceToHost, g->stream));
     if (label && where != EG_DEVICE)
         EG_CUDA(cudaMemcpyAsync(label, comp, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
     EG_CUDA(cudaStreamSynchronize(g->stream));
-    if (h->err) {
+    if (!*(volatile uint32_t*)&h->valid) {
+        persist_reset(g);
         set_error("eg_cc: a bounded grid barrier gave up");
         return EG_ERR_TIMEOUT;
     }

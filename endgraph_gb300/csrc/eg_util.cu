@@ -149,6 +149,24 @@ int selftest_bounded_wait(eg_graph* g, uint32_t spin_cap) {
     return check_device_error(g, "eg_selftest_bounded_wait");
 }
 
+int persist_block(eg_graph* g, void** mine, void** other) {
+    EngineState& s = g->eng;
+    if (!s.persist.ptr) {
+        EG_TRY(s.persist.reserve(2 * kPersistBytes));
+        EG_CUDA(cudaMemsetAsync(s.persist.ptr, 0, 2 * kPersistBytes, g->stream));
+    }
+    *mine = s.persist.as<uint8_t>() + s.persist_turn * kPersistBytes;
+    *other = s.persist.as<uint8_t>() + (s.persist_turn ^ 1) * kPersistBytes;
+    memset(s.host_words, 0, 256);  // a kernel that gives up writes nothing there
+    return EG_OK;
+}
+
+void persist_launched(eg_graph* g) { g->eng.persist_turn ^= 1; }
+
+void persist_reset(eg_graph* g) {
+    cudaMemsetAsync(g->eng.persist.ptr, 0, 2 * kPersistBytes, g->stream);
+}
+
 // The bounded grid barrier of the persistent kernels, exercised: a cooperative launch of four CTAs
 // in which CTA 0 never arrives, so the other three poll until spin_cap runs out, raise the error
 // flag and leave; the caller sees EG_ERR_TIMEOUT and the handle stays usable.

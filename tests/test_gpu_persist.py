@@ -184,3 +184,38 @@ def test_cc_grid_sizes(eg_lib, V, E):
     rng = np.random.default_rng(V)
     src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
     _check_cc(src, dst, V, rng.random(E).astype(np.float32))
+
+
+def test_launches_in_turn_on_one_handle(eg_lib):
+    """Every launch finds its state words zeroed by the launch before it, whichever traversal that was,
+    also across launches that continue (a chain deeper than one) and across loads."""
+    import torch
+
+    import endgraph_gb300 as eg
+    n = 4_500
+    rng = np.random.default_rng(11)
+    chain = np.arange(n, dtype=np.uint32)
+    src, dst = rng.integers(0, n, 30_000).astype(np.uint32), rng.integers(0, n, 30_000).astype(np.uint32)
+    with eg.Graph() as g:
+        for src, dst in ((chain[:-1], chain[1:]), (src, dst)):
+            w = rng.random(len(src)).astype(np.float32)
+            csr = oracle.build_csr(src, dst, w, n, np.array([0, n], np.uint32))
+            level = oracle.bfs_levels(csr["off"][0], csr["adj"], n, 0)
+            dist = oracle.sssp(csr["off"][0], csr["adj"], csr["w"], n, 0)
+            labels = oracle.cc_labels(src, dst, n)
+            lv = torch.empty(n, dtype=torch.int32, device="cuda")
+            for _ in range(2):
+                g.load_directed(eg.pack_edges(src, dst, w), n)
+                ranks = g.pagerank(3)
+                for call in (0, 1, 0, 0, 2, 1, 1, 2, 0):
+                    if call == 0:
+                        lv.fill_(-2)  # pending on torch's stream when the call is made
+                        g.bfs(0, level=lv, want_parent=False)
+                        assert np.array_equal(lv.cpu().numpy().view(np.uint32), level)
+                    elif call == 1:
+                        assert np.array_equal(g.sssp(0).view(np.uint32), dist.view(np.uint32))
+                    else:
+                        assert np.array_equal(g.pagerank(3), ranks)
+                g.load_undirected_from_directed(eg.pack_edges(src, dst, w), n)
+                assert np.array_equal(g.cc(), labels)
+                assert np.array_equal(g.cc(), labels)
