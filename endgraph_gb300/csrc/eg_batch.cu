@@ -575,10 +575,38 @@ __device__ __forceinline__ uint64_t task_begin(const uint4& t) { return ((uint64
 __device__ __forceinline__ uint32_t task_len(const uint4& t) { return t.y >> 8; }
 
 struct RowTasks {
-    DevBuf rec, heavy_vertex, counts;
+    DevBuf rec, heavy_vertex, counts, first;
     uint64_t ntasks = 0;
     uint32_t nheavy = 0;
+    uint32_t nbatches = 0;  // first: [nbatches + 1]
 };
+
+// Batches of consecutive tasks, one per warp of the row kernels: batch b holds the tasks that begin in edges
+// [b size, (b + 1) size).  Every warp is a CTA of its own, so the hardware hands batches to whichever SM
+// is free: with 32 warps per SM taking tasks by stride, SMs were idle for a quarter of a PPR sweep.
+__global__ void k_task_batches(const uint4* __restrict__ rec, uint64_t ntasks, uint32_t size, uint32_t nb,
+                               uint32_t* __restrict__ first) {
+    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t <= ntasks; t += (uint64_t)gridDim.x * blockDim.x) {
+        const int64_t lo = t ? (int64_t)(task_begin(rec[t - 1]) / size) : -1;
+        const int64_t hi = t < ntasks ? (int64_t)(task_begin(rec[t]) / size) : (int64_t)nb;
+        for (int64_t b = lo + 1; b <= hi; ++b) first[b] = (uint32_t)t;
+    }
+}
+
+// 512 edges a batch, fewer on graphs that would not give every resident warp one.  50 PPR iterations on
+// 1 M / 16 M: 35.8 ms with 256, 32.1 with 512, 31.0 with 1,024, whose batches come out as slow for the
+// adjoint (27.3 against 26.5) and SSSP; 20,000 / 100,000: 1.43 with 16, 1.31 with 32 or 64.
+constexpr uint64_t kBatchEdges = 512, kBatchEdgesMin = 32;
+static int make_batches(eg_graph* g, RowTasks& t) {
+    const uint64_t E = std::max<uint64_t>(g->E, 1), warps = g->num_sms * 32ull;
+    const uint64_t size = std::min(kBatchEdges, std::max(kBatchEdgesMin, (E + warps - 1) / warps));
+    t.nbatches = (uint32_t)((E + size - 1) / size);
+    EG_TRY(t.first.reserve(4ull * (t.nbatches + 1)));
+    k_task_batches<<<grid_for(t.ntasks + 1, 256), 256, 0, g->stream>>>(t.rec.as<uint4>(), t.ntasks, (uint32_t)size, t.nbatches,
+                                                                       t.first.as<uint32_t>());
+    EG_CHECK_LAUNCH("k_task_batches");
+    return EG_OK;
+}
 
 static int make_tasks(eg_graph* g, RowTasks& t, const uint64_t* begin, uint64_t nitems, const uint32_t* item_vertex) {
     // upper bound on tasks: non-empty items + E / kTaskEdges
@@ -596,115 +624,157 @@ static int make_tasks(eg_graph* g, RowTasks& t, const uint64_t* begin, uint64_t 
     EG_CUDA(cudaStreamSynchronize(g->stream));
     t.ntasks = nitems ? h[0] : 0;
     t.nheavy = (uint32_t)(h[1] & 0xFFFFFFFFu);
-    return EG_OK;
+    return make_batches(g, t);
 }
 
 // ---------------------------------------------------------------------------------------------
 // row kernels: one warp per task, 64-column rows of 256 bytes
 struct RowArgs {
     const uint4* rec;
-    uint64_t ntasks;
+    const uint32_t* first;        // first task of every batch
     const uint32_t* adj;
     const float* w;               // per-edge weight (normalised for PPR, raw for SSSP)
 };
 
-// The PPR sweeps read a 256-byte row per edge: one warp per task, the two half-warps take alternate
-// edges, lane c of a half owns columns 4c..4c+3 (one 16-byte load per row and lane).  A step is
-// 2 * kRowPairs edges: their ids and weights are loaded one edge per lane, while the previous step's
-// rows are reduced, and handed round by shuffles.
-// Both sweeps are bound by the row gathers (256 E bytes a sweep, mostly out of L2).  Rows are asked
-// to stay in L2 (half of them evict-last), ids, weights and results pass through evict-first.
-// 1 M vertices, 16 M edges: the forward sweep 0.61 ms with one 8-byte column pair per lane and
-// default caching, 0.66 ms with half-warp rows alone, 0.64 streaming ids and results, 0.53 ms with
-// the rows kept as well (7.8 TB/s of rows); the adjoint sweep 1.05 -> 0.76 ms.  8 rows per half-warp
-// at 4 CTAs per SM (64 registers): 4 rows 0.56, 16 rows 0.81 ms.
-constexpr int kRowPairs = 8;
-constexpr uint32_t kRowStep = 2 * kRowPairs;
+// The PPR sweeps read a 256-byte row per edge, 8 bytes per lane.  A warp walks the edges of its batch
+// without regard to where lists end: 16 rows are always on their way together, the next ids and
+// weights behind them, and a list's sum is stored when its last edge has been added.  (A warp per
+// task reads a list of three edges in a step for sixteen, and waits for a record, ids and rows each
+// time.)  Rows are asked to stay in L2 (half of them evict-last), ids, weights and results pass through
+// evict-first.  1 M vertices, 16 M edges, forward / adjoint sweep: a warp per task by stride, half a
+// warp per row 0.53 / 0.75 ms, the walk in CTAs of 8 warps 0.38 / -, of 2 0.35 / 0.61, of 1 0.32 /
+// 0.50 (12.9 / 8.2 TB/s of rows; random 256-byte rows out of 256 MB reach 10 TB/s, out of 64 MB 21).
+constexpr int kWalkRows = 16;
 
-__device__ __forceinline__ float4 half_sum(float4 v) {  // the two half-warps' partial rows
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
-    v.z += __shfl_xor_sync(0xffffffffu, v.z, 16);
-    v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
+__device__ __forceinline__ float2 ld_row(const float2* a, unsigned long long keep) {
+    float2 v;
+    asm volatile("ld.global.cg.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(a), "l"(keep));
     return v;
 }
 
-// a task's finished row: stored, or added to its list's accumulator when the list has several tasks
-__device__ __forceinline__ void row_out(const uint4& rec, float4 acc, uint32_t lane, float4* __restrict__ y,
-                                        float4* __restrict__ heavy_acc, float scale) {
-    acc = half_sum(acc);
-    if (lane >= 16) return;
-    if (rec.w == kNoSlot)
-        __stcs(y + (uint64_t)rec.z * 16 + lane, make_float4(scale * acc.x, scale * acc.y, scale * acc.z, scale * acc.w));
-    else
-        atomicAdd(heavy_acc + (uint64_t)rec.w * 16 + lane, acc);
+// acc plus four weighted rows, which are added up by themselves first: a long list's sum takes a quarter of
+// the roundings
+__device__ __forceinline__ float2 add_four(float2 acc, const float4& w, float2 a, float2 b, float2 c, float2 d) {
+    acc.x += fmaf(w.w, d.x, fmaf(w.z, c.x, fmaf(w.y, b.x, w.x * a.x)));
+    acc.y += fmaf(w.w, d.y, fmaf(w.z, c.y, fmaf(w.y, b.y, w.x * a.y)));
+    return acc;
 }
 
-// PPR forward: y[v] = (1-a) * sum_{u in in(v)} wn_uv * x[u]
-__global__ void __launch_bounds__(256, 4) k_row_spmm(RowArgs a, const float4* __restrict__ x, float4* __restrict__ y,
-                                                  float4* __restrict__ heavy_acc, float scale) {
-    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
-    for (; t < a.ntasks; t += nwarps) {
-        const uint4 rec = nxt;
-        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
-        const uint64_t e0 = task_begin(rec);
-        const uint32_t n = task_len(rec);
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t u = lane < n ? __ldcs(a.adj + e0 + lane) : 0u;
-        float w = lane < n ? __ldcs(a.w + e0 + lane) : 0.f;
-        for (uint32_t eb = 0; eb < n; eb += 32) {
-            const uint32_t k = eb + 32 + lane;
-            const uint32_t u2 = k < n ? __ldcs(a.adj + e0 + k) : 0u;
-            const float w2 = k < n ? __ldcs(a.w + e0 + k) : 0.f;
-            const uint32_t left = n - eb < 32 ? n - eb : 32;
-            for (uint32_t s = 0; s < left; s += kRowStep) {
-                float4 r[kRowPairs];
-                float wj[kRowPairs];
+__device__ __forceinline__ uint2 seeds_at(const uint32_t* seeds, int n, uint32_t lane) {  // of columns 2 lane, 2 lane + 1
+    return make_uint2(2 * lane < n ? __ldg(seeds + 2 * lane) : ~0u, 2 * lane + 1 < n ? __ldg(seeds + 2 * lane + 1) : ~0u);
+}
+__device__ __forceinline__ float2 ppr_row(float2 acc, uint32_t v, uint2 seed, float alpha) {
+    float2 r = make_float2((1.0f - alpha) * acc.x, (1.0f - alpha) * acc.y);
+    if (seed.x == v) r.x += alpha;
+    if (seed.y == v) r.y += alpha;
+    return r;
+}
+
+// PPR forward: y[v] = (1-a) * sum_{u in in(v)} wn_uv * x[u] + a * e_seed[v]
+__global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __restrict__ x, float2* __restrict__ y,
+                                                  float2* __restrict__ heavy_acc, const uint32_t* __restrict__ seeds, int n_seeds,
+                                                  float alpha) {
+    __shared__ __align__(16) uint32_t id[32];
+    __shared__ __align__(16) float wt[32];
+    __shared__ __align__(16) uint4 task[32];  // end (from the batch's first edge), vertex, slot
+    __shared__ __align__(8) uint2 s_seed[32];               // seeds of the lanes' columns
+    const uint32_t lane = threadIdx.x;
+    s_seed[lane] = seeds_at(seeds, n_seeds, lane);
+    unsigned long long keep;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
+    const uint32_t b = blockIdx.x;
+    uint32_t t = __ldg(a.first + b);
+    const uint32_t t1 = __ldg(a.first + b + 1);
+    if (t == t1) return;
+    const uint4 last = __ldg(a.rec + t1 - 1), tasks0 = t + lane < t1 ? __ldg(a.rec + t + lane) : last;
+    const uint64_t e0 = __shfl_sync(0xffffffffu, task_begin(tasks0), 0);
+    const uint32_t n = (uint32_t)(task_begin(last) - e0) + task_len(last);
+    auto stage = [&](const uint4& r) {  // 32 tasks of the batch
+        __syncwarp();
+        task[lane] = make_uint4((uint32_t)(task_begin(r) - e0) + task_len(r), r.z, r.w, 0u);
+        __syncwarp();
+        t += 32;
+    };
+    const uint32_t* adj = a.adj + e0 + lane;
+    const float* wts = a.w + e0 + lane;
+    x += lane;
+    uint32_t u = lane < n ? __ldcs(adj) : 0u;
+    float w = lane < n ? __ldcs(wts) : 0.f;
+    stage(tasks0);
+    uint32_t k = 0, lists = t1 - t + 32;  // of the batch (t is 32 tasks ahead)
+    uint32_t end = task[0].x;
+    float2 acc = make_float2(0.f, 0.f);
+    auto finish = [&]() {
+        const uint4 cur = task[k];
+        if (cur.z == kNoSlot) __stcs(y + (uint64_t)cur.y * 32 + lane, ppr_row(acc, cur.y, s_seed[lane], alpha));
+        else atomicAdd(heavy_acc + (uint64_t)cur.z * 32 + lane, acc);
+        acc = make_float2(0.f, 0.f);
+        if (++k == 32) {
+            stage(t + lane < t1 ? __ldg(a.rec + t + lane) : last);
+            k = 0;
+        }
+        end = --lists ? task[k].x : ~0u;
+    };
+    for (uint32_t c = 0; c < n; c += 32) {
+        __syncwarp();
+        id[lane] = u;
+        wt[lane] = w;
+        __syncwarp();
+        u = 0;
+        if (c + 32 + lane < n) {
+            u = __ldcs(adj + c + 32);
+            w = __ldcs(wts + c + 32);
+        }
+        const uint32_t left = n - c < 32 ? n - c : 32;
+        for (uint32_t s = 0; s < left; s += kWalkRows) {
+            float2 r[kWalkRows];
 #pragma unroll
-                for (int j = 0; j < kRowPairs; ++j) {
-                    const uint32_t i = s + 2 * j + half;
-                    const uint32_t uj = __shfl_sync(0xffffffffu, u, i & 31);
-                    wj[j] = __shfl_sync(0xffffffffu, w, i & 31);
-                    r[j] = i < left ? ld_keep(x + (uint64_t)uj * 16 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
+            for (int j = 0; j < kWalkRows; j += 4) {  // past the batch's last edge: row 0, not used
+                const uint4 q = *reinterpret_cast<const uint4*>(id + s + j);
+                r[j] = ld_row(x + (uint64_t)q.x * 32, keep);
+                r[j + 1] = ld_row(x + (uint64_t)q.y * 32, keep);
+                r[j + 2] = ld_row(x + (uint64_t)q.z * 32, keep);
+                r[j + 3] = ld_row(x + (uint64_t)q.w * 32, keep);
+            }
 #pragma unroll
-                for (int j = 0; j < kRowPairs; ++j) {
-                    acc.x = fmaf(wj[j], r[j].x, acc.x);
-                    acc.y = fmaf(wj[j], r[j].y, acc.y);
-                    acc.z = fmaf(wj[j], r[j].z, acc.z);
-                    acc.w = fmaf(wj[j], r[j].w, acc.w);
+            for (int j = 0; j < kWalkRows; j += 4) {
+                const float4 q = *reinterpret_cast<const float4*>(wt + s + j);
+                const uint32_t at = c + s + j;
+                if (at + 4 < end) {  // no list ends here
+                    acc = add_four(acc, q, r[j], r[j + 1], r[j + 2], r[j + 3]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float qi = i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w;
+                        acc.x = fmaf(qi, r[j + i].x, acc.x);
+                        acc.y = fmaf(qi, r[j + i].y, acc.y);
+                        if (at + i + 1 == end) finish();
+                    }
                 }
             }
-            u = u2;
-            w = w2;
         }
-        row_out(rec, acc, lane, y, heavy_acc, scale);
     }
 }
 
+// the rows of lists cut into several tasks (seeds null: no teleport), one warp each
 __global__ void k_row_heavy_finish(const uint32_t* __restrict__ heavy_vertex, uint32_t nheavy,
-                                   float4* __restrict__ heavy_acc, float4* __restrict__ y, float scale) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t slot = i >> 4;
-    const uint32_t c = threadIdx.x & 15;
+                                   float2* __restrict__ heavy_acc, float2* __restrict__ y, const uint32_t* __restrict__ seeds,
+                                   int n_seeds, float alpha) {
+    const uint32_t slot = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (slot >= nheavy) return;
     const uint32_t v = heavy_vertex[slot];
-    const float4 a = heavy_acc[slot * 16 + c];
-    heavy_acc[slot * 16 + c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    y[(uint64_t)v * 16 + c] = make_float4(scale * a.x, scale * a.y, scale * a.z, scale * a.w);
+    float2* p = heavy_acc + (uint64_t)slot * 32 + lane;
+    y[(uint64_t)v * 32 + lane] = ppr_row(*p, v, seeds_at(seeds, n_seeds, lane), alpha);
+    *p = make_float2(0.f, 0.f);
 }
 
-// y[seed_s][s] = (the sweep's value, 0 for a seed without in-edges) + a: the sweeps write only rows
-// with in-edges, so that a row without them keeps what the buffer held
-__global__ void k_ppr_teleport(const uint32_t* seeds, int n, const uint32_t* __restrict__ indeg, float* y, float alpha) {
-    const int s = threadIdx.x;
-    if (s >= n) return;
-    const uint32_t v = seeds[s];
-    float* p = y + (uint64_t)v * 64 + s;
-    *p = (indeg[v] ? *p : 0.f) + alpha;
+// Seeds without in-edges: the sweeps leave their rows as they are, a at the seed's column, in nbuf
+// consecutive row arrays.
+__global__ void k_ppr_lone_seeds(const uint32_t* __restrict__ seeds, int n, const uint32_t* __restrict__ indeg,
+                                 float* __restrict__ rows, uint64_t V, int nbuf, float alpha) {
+    const int s = threadIdx.x & 63;
+    if (s >= n || indeg[seeds[s]]) return;
+    for (int b = blockIdx.x; b < nbuf; b += gridDim.x) rows[((uint64_t)b * V + seeds[s]) * 64 + s] = alpha;
 }
 __global__ void k_ppr_init(const uint32_t* seeds, int n, float* x) {
     const int s = threadIdx.x;
@@ -779,83 +849,147 @@ __global__ void k_gather_norm_w(const uint32_t* __restrict__ nbr_is_src, const f
 // ---- adjoint sweep over the CSR: for a source row u,
 //   lam_out[u] = (1-a) * sum_{v in out(u)} wn_uv * lam_in[v]
 //   gA[e]     += (1-a) * <x_k[u], lam_in[v]>      (per CSR edge e = (u, v))
-// One step's dot products <x_k[u], lam[v]>, kRowPairs per half-warp, are summed over its 16 lanes by
-// halving: at each stage a lane hands half of its partial sums to its partner and keeps the other
-// half, so eight products take 8 shuffles (one at a time: 32); lanes with an even c end up with one
-// product each, in the order of dot_slot.
-__device__ __forceinline__ float dot_scatter(float (&d)[kRowPairs], uint32_t c) {
-    static_assert(kRowPairs == 8, "the three halving stages below leave one product of eight per lane pair");
+// The walk of k_row_spmm, with the source rows x_k[u] of the next 8 to 16 lists on their way to shared
+// memory.  A step's 16 dot products <x_k[u], lam[v]> are summed over the warp by halving: at each
+// stage a lane hands half of its partial sums to its partner and keeps the other half, so that 16
+// products take 16 shuffles (one at a time: 80); lane 2 j and its neighbour end up with product j.  gA is
+// kept in FP64: an edge's gradient is what is left of its gA minus the mean over the source's edges,
+// and the roundings of K steps were most of its error (K = 50, 1 M / 16 M, two seeds: 1.1e-6 and
+// 8.5e-7 with FP32 sums, 7.9e-7 and 5.4e-7 so, for 24.9 instead of 23.6 ms of sweeps).
+__device__ __forceinline__ float dot_scatter(float2 (&d)[kWalkRows], uint32_t lane) {
+    static_assert(kWalkRows == 16, "the four halving stages below leave one product of sixteen per lane pair");
 #pragma unroll
-    for (int o = 8, m = 4; o >= 2; o >>= 1, m >>= 1) {
-        const bool up = (c & o) != 0;
+    for (int o = 16, m = 8; o >= 2; o >>= 1, m >>= 1) {
+        const bool up = (lane & o) != 0;
 #pragma unroll
         for (int j = 0; j < m; ++j) {
-            const float give = up ? d[j] : d[j + m], keep = up ? d[j + m] : d[j];
-            d[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            const float give = up ? d[j].x : d[j + m].x, keep = up ? d[j + m].x : d[j].x;
+            d[j].x = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
     }
-    return d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+    return d[0].x + __shfl_xor_sync(0xffffffffu, d[0].x, 1);
 }
-__device__ __forceinline__ uint32_t dot_slot(uint32_t c) { return c >> 1; }  // which of the eight lane c holds
 
-__global__ void __launch_bounds__(256, 4) k_row_adjoint(RowArgs a, const float4* __restrict__ lam_in,
-                                                     const float4* __restrict__ xk, float4* __restrict__ lam_out,
-                                                     float4* __restrict__ heavy_acc, float* __restrict__ gA,
+// 28 warps per SM (72 registers): 32 (64, spilled) 28.5 ms for 50 sweeps, 24 27.5, 28 25.4.
+__global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2* __restrict__ lam_in,
+                                                     const float2* __restrict__ xk, float2* __restrict__ lam_out,
+                                                     float2* __restrict__ heavy_acc, double* __restrict__ gA,
                                                      float scale) {
-    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
-    for (; t < a.ntasks; t += nwarps) {
-        const uint4 rec = nxt;  // the task's vertex is the source u
-        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
-        const uint64_t e0 = task_begin(rec);
-        const uint32_t n = task_len(rec);
-        const float4 xu = __ldcg(xk + (uint64_t)rec.z * 16 + c);
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t v = lane < n ? __ldcs(a.adj + e0 + lane) : 0u;
-        float w = lane < n ? __ldcs(a.w + e0 + lane) : 0.f;
-        for (uint32_t eb = 0; eb < n; eb += 32) {
-            const uint32_t k = eb + 32 + lane;
-            const uint32_t v2 = k < n ? __ldcs(a.adj + e0 + k) : 0u;
-            const float w2 = k < n ? __ldcs(a.w + e0 + k) : 0.f;
-            const uint32_t left = n - eb < 32 ? n - eb : 32;
-            for (uint32_t s = 0; s < left; s += kRowStep) {
-                // the edge whose product this lane will hold, and its gA entry
-                const uint32_t mine = s + 2 * dot_slot(c) + half;
-                const bool have = !(c & 1) && mine < left;
-                float* g = gA + e0 + eb + mine;
-                const float g_old = have ? *g : 0.f;
-                float4 l[kRowPairs];
-                float wj[kRowPairs], d[kRowPairs];
+    __shared__ __align__(16) uint32_t id[32];
+    __shared__ __align__(16) float wt[32];
+    __shared__ __align__(16) uint4 task[16];      // ring of 16: end, vertex, slot
+    __shared__ __align__(16) float2 src[16][32];  // and their rows of x_k
+    const uint32_t lane = threadIdx.x & 31;
+    unsigned long long keep;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
+    const uint32_t b = blockIdx.x;
+    const uint32_t t0 = __ldg(a.first + b), lists = __ldg(a.first + b + 1) - t0;
+    if (!lists) return;
+    auto tasks_at = [&](uint32_t i) {
+        return lane < 8 && i + lane < lists ? __ldg(a.rec + t0 + i + lane) : make_uint4(0, 0, 0, 0);
+    };
+    const uint4 last = __ldg(a.rec + t0 + lists - 1), tasks0 = tasks_at(0), tasks8 = tasks_at(8);
+    uint4 ahead = tasks_at(16);
+    const uint64_t e0 = __shfl_sync(0xffffffffu, task_begin(tasks0), 0);
+    const uint32_t n = (uint32_t)(task_begin(last) - e0) + task_len(last);
+    auto stage = [&](const uint4& r, uint32_t slot) {  // 8 tasks (lanes 0..7) into the ring, their rows on the way
+        if (lane < 8) task[slot + lane] = make_uint4((uint32_t)(task_begin(r) - e0) + task_len(r), r.z, r.w, 0u);
 #pragma unroll
-                for (int j = 0; j < kRowPairs; ++j) {
-                    const uint32_t i = s + 2 * j + half;
-                    const uint32_t vj = __shfl_sync(0xffffffffu, v, i & 31);
-                    wj[j] = __shfl_sync(0xffffffffu, w, i & 31);
-                    l[j] = i < left ? ld_keep(lam_in + (uint64_t)vj * 16 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int j = 0; j < kRowPairs; ++j) {
-                    acc.x = fmaf(wj[j], l[j].x, acc.x);
-                    acc.y = fmaf(wj[j], l[j].y, acc.y);
-                    acc.z = fmaf(wj[j], l[j].z, acc.z);
-                    acc.w = fmaf(wj[j], l[j].w, acc.w);
-                    d[j] = fmaf(xu.x, l[j].x, xu.y * l[j].y) + fmaf(xu.z, l[j].z, xu.w * l[j].w);
-                }
-                const float dot = dot_scatter(d, c);
-                if (have) *g = fmaf(scale, dot, g_old);
-            }
-            v = v2;
-            w = w2;
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t q = 2 * i + (lane >> 4), v = __shfl_sync(0xffffffffu, r.z, q);
+            if (__shfl_sync(0xffffffffu, task_len(r), q))
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&src[slot + q][2 * (lane & 15)])),
+                             "l"(xk + (uint64_t)v * 32 + 2 * (lane & 15))
+                             : "memory");
         }
-        row_out(rec, acc, lane, lam_out, heavy_acc, scale);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const uint32_t* adj = a.adj + e0 + lane;
+    const float* wts = a.w + e0 + lane;
+    double* g = gA + e0 + (lane >> 1);
+    lam_in += lane;
+    uint32_t v = lane < n ? __ldcs(adj) : 0u;
+    float w = lane < n ? __ldcs(wts) : 0.f;
+    stage(tasks0, 0);
+    stage(tasks8, 8);
+    __syncwarp();
+    uint32_t k = 0, end = task[0].x;
+    float2 xu = make_float2(0.f, 0.f), acc = make_float2(0.f, 0.f);
+    auto finish = [&]() {
+        const uint4 cur = task[k & 15];
+        if (cur.z == kNoSlot) __stcs(lam_out + (uint64_t)cur.y * 32 + lane, make_float2(scale * acc.x, scale * acc.y));
+        else atomicAdd(heavy_acc + (uint64_t)cur.z * 32 + lane, acc);
+        acc = make_float2(0.f, 0.f);
+        ++k;
+        if (!(k & 7)) {  // the finished eight make room
+            __syncwarp();
+            stage(ahead, (k + 8) & 15);
+            ahead = tasks_at(k + 16);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+        }
+        end = k < lists ? task[k & 15].x : ~0u;
+        xu = src[k & 15][lane];
+    };
+    for (uint32_t c = 0; c < n; c += 32) {
+        __syncwarp();
+        id[lane] = v;
+        wt[lane] = w;
+        __syncwarp();
+        v = 0;
+        if (c + 32 + lane < n) {
+            v = __ldcs(adj + c + 32);
+            w = __ldcs(wts + c + 32);
+        }
+        const uint32_t left = n - c < 32 ? n - c : 32;
+        for (uint32_t s = 0; s < left; s += kWalkRows) {
+            const bool have = !(lane & 1) && s + (lane >> 1) < left;
+            const double g_old = have ? g[c + s] : 0.0;
+            float2 l[kWalkRows];
+#pragma unroll
+            for (int j = 0; j < kWalkRows; j += 4) {  // past the batch's last edge: row 0, not used
+                const uint4 q = *reinterpret_cast<const uint4*>(id + s + j);
+                l[j] = ld_row(lam_in + (uint64_t)q.x * 32, keep);
+                l[j + 1] = ld_row(lam_in + (uint64_t)q.y * 32, keep);
+                l[j + 2] = ld_row(lam_in + (uint64_t)q.z * 32, keep);
+                l[j + 3] = ld_row(lam_in + (uint64_t)q.w * 32, keep);
+            }
+            if (c + s == 0) {  // the first source rows
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                __syncwarp();
+                xu = src[0][lane];
+            }
+#pragma unroll
+            for (int j = 0; j < kWalkRows; j += 4) {
+                const float4 q = *reinterpret_cast<const float4*>(wt + s + j);
+                const uint32_t at = c + s + j;
+                if (at + 4 < end) {  // no list ends here
+                    acc = add_four(acc, q, l[j], l[j + 1], l[j + 2], l[j + 3]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) l[j + i].x = fmaf(xu.x, l[j + i].x, xu.y * l[j + i].y);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float qi = i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w;
+                        const float2 r = l[j + i];
+                        acc.x = fmaf(qi, r.x, acc.x);
+                        acc.y = fmaf(qi, r.y, acc.y);
+                        l[j + i].x = fmaf(xu.x, r.x, xu.y * r.y);
+                        if (at + i + 1 == end) finish();
+                    }
+                }
+            }
+            const float dot = dot_scatter(l, lane);
+            if (have) g[c + s] = fma((double)scale, (double)dot, g_old);
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // dL/dw_e = (gA_e - sum_{e' in row(u)} wn_e' gA_e') / s_u, scattered to the input edge order
 __global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ tasks, uint64_t ntasks,
-                                                     const float* __restrict__ wn, const float* __restrict__ gA,
+                                                     const float* __restrict__ wn, const double* __restrict__ gA,
                                                      const float* __restrict__ s, const float* __restrict__ eid,
                                                      float* __restrict__ dw, double* __restrict__ heavy,
                                                      int finish_heavy) {
@@ -870,7 +1004,7 @@ __global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ t
         if (finish_heavy) {
             dot = heavy[rec.w];
         } else {
-            for (uint32_t k = lane; k < n; k += 32) dot += (double)wn[e0 + k] * gA[e0 + k];
+            for (uint32_t k = lane; k < n; k += 32) dot += wn[e0 + k] * gA[e0 + k];
             dot = warp_sum_f64(dot);
             if (rec.w != kNoSlot) {
                 if (lane == 0) atomicAdd(heavy + rec.w, dot);
@@ -879,39 +1013,39 @@ __global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ t
         }
         const float inv = 1.0f / s[rec.z];
         for (uint32_t k = lane; k < n; k += 32)
-            dw[__float_as_uint(__ldg(eid + e0 + k))] = (float)(((double)gA[e0 + k] - dot) * inv);
+            dw[__float_as_uint(__ldg(eid + e0 + k))] = (float)((gA[e0 + k] - dot) * inv);
     }
 }
 
 // ---- batched SSSP: in place, skipping sources whose row did not change in the last sweep --------
-// One warp per task; the two half-warps take alternate edges and lane c of a half owns columns
-// 4c..4c+3 (one 16-byte load of a 256-byte row).  The sweep is bound by the latency of the chain
-// record -> ids -> changed bits -> rows, so the next task's record is loaded one task ahead, the
-// destination's row together with the ids, and up to kSsspRows rows are in flight per warp; sources
-// that did not change (one bit each, cached in L1: the bits do not change during a sweep) are
-// squeezed out first, their ids and weights queueing up in shared memory, so the row loads stay full
-// when few sources are active.  A destination with a single task is written by this warp alone and
-// stored plainly; cut lists (and items of several partitions that share a vertex) take the minimum
-// with atomics.  64 graphs of 1k-500k vertices, 93 M edges, 64 sources, 24 sweeps: 107 ms with one
-// row per warp load, byte flags and separate item / offset arrays, 47 ms so (10.8 E row gathers:
-// 5.5 TB/s); 6 CTAs per SM with 8 rows (40 registers) take 47.0 ms, 4 with 16 rows 47.5, 5 with 8
-// rows 52, 3 with 16 rows 53, 2 with 32 rows 72.
+// A warp takes the tasks of its batch one by one; the two half-warps take alternate edges and lane c of a
+// half owns columns 4c..4c+3 (one 16-byte load of a 256-byte row).  The sweep is bound by the latency
+// of the chain record -> ids -> changed bits -> rows, so the next task's record is loaded one task
+// ahead, the destination's row together with the ids, and up to kSsspRows rows are in flight per
+// warp; sources that did not change (one bit each, cached in L1: the bits do not change during a
+// sweep) are squeezed out first, their ids and weights queueing up in shared memory, so the row
+// loads stay full when few sources are active.  A destination with a single task is written by this
+// warp alone and stored plainly; cut lists (and items of several partitions that share a vertex) take
+// the minimum with atomics.  64 graphs of 1k-500k vertices, 93 M edges, 64 sources, 24 sweeps: 107 ms
+// with one row per warp load, byte flags and separate item / offset arrays; tasks by stride at 48
+// warps per SM (40 registers, spilled) 47.5 ms; batches in CTAs of 8 warps 44.4, of 2 45.2, of 2 at 40
+// / 32 warps per SM 42.2 / 40.5, of one warp at 32 (64 registers) 38.5 (10.8 E row gathers: 6.7
+// TB/s), there with 16 rows 41.0.
 constexpr int kSsspRows = 8;
 
-__global__ void __launch_bounds__(256, 6) k_row_sssp(RowArgs a, float4* __restrict__ dist,
+__global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float4* __restrict__ dist,
                                                   const uint32_t* __restrict__ changed_prev,
                                                   uint32_t* __restrict__ changed_next, int shared_vertex,
                                                   int* __restrict__ any) {
-    __shared__ uint2 s_act[8][64];
+    __shared__ uint2 act[64];
     const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
-    uint2* act = s_act[threadIdx.x >> 5];
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint4 nxt = t < a.ntasks ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
+    uint32_t t = __ldg(a.first + blockIdx.x);
+    const uint32_t t1 = __ldg(a.first + blockIdx.x + 1);
+    uint4 nxt = t < t1 ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
     bool any_lowered = false;
-    for (; t < a.ntasks; t += nwarps) {
+    for (; t < t1; ++t) {
         const uint4 rec = nxt;
-        if (t + nwarps < a.ntasks) nxt = __ldg(a.rec + t + nwarps);
+        if (t + 1 < t1) nxt = __ldg(a.rec + t + 1);
         const uint64_t e0 = task_begin(rec);
         const uint32_t n = task_len(rec), v = rec.z;
         const float4 dv = __ldcg(dist + (uint64_t)v * 16 + c);
@@ -1017,7 +1151,6 @@ struct BatchState {
     DevBuf persist;  // persistent traversal: per-level counts, barrier words, error flag
     DevBuf wr0, wr1;  // frontier words in renumbered order (pull gathers through renumbered sources)
     RowTasks csc_tasks, csr_tasks;
-    unsigned spmm_grid = 0;
     size_t device_bytes = 0;  // the GPU's memory
     bool csc_ready = false, csr_ready = false;
     // captured MS-BFS level loop and the shapes it was captured for
@@ -1795,16 +1928,8 @@ static int ensure_tasks(eg_graph* g, bool csr) {
     return EG_OK;
 }
 
-// resident CTAs of 256 threads of a row kernel over the whole GPU: its warps take tasks by stride
-static int resident_grid(eg_graph* g, const void* fn, unsigned* grid) {
-    int per_sm = 0;
-    EG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-    *grid = (unsigned)g->num_sms * (unsigned)std::max(per_sm, 1);
-    return EG_OK;
-}
-
 static RowArgs row_args(const RowTasks& t, const uint32_t* adj, const float* w) {
-    return RowArgs{t.rec.as<uint4>(), t.ntasks, adj, w};
+    return RowArgs{t.rec.as<uint4>(), t.first.as<uint32_t>(), adj, w};
 }
 
 // weights in CSC order (and, for the adjoint, in CSR order), row-normalised by the source's out-weight sum
@@ -1842,23 +1967,30 @@ static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev, bool want_csr
     return EG_OK;
 }
 
-// one forward step: y = a*e + (1-a) A^T x.  Rows of y without in-edges are zero already (the caller
-// cleared them once), except the seeds' entries, which k_ppr_teleport sets.
+// one forward step: y = a*e + (1-a) A^T x.  Rows of y without in-edges are as the caller left them: zero,
+// and `a` at a seed's own column (lone_seeds).
 static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
     BatchState& b = bstate(g);
     const RowTasks& t = b.csc_tasks;
     RowArgs a = row_args(t, g->csc_adj.as<uint32_t>(), b.wn_csc.as<float>());
     Timed tm(&g->prof, g->stream, "ppr_spmm");
-    k_row_spmm<<<b.spmm_grid, 256, 0, g->stream>>>(a, reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y),
-                                                  b.heavy.as<float4>(), 1.0f - alpha);
+    k_row_spmm<<<t.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<const float2*>(x), reinterpret_cast<float2*>(y),
+                                                  b.heavy.as<float2>(), b.seeds.as<uint32_t>(), n, alpha);
     EG_CHECK_LAUNCH("k_row_spmm");
     if (t.nheavy) {
-        k_row_heavy_finish<<<(unsigned)((t.nheavy * 16ull + 255) / 256), 256, 0, g->stream>>>(
-            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<float4>(), reinterpret_cast<float4*>(y), 1.0f - alpha);
+        k_row_heavy_finish<<<(unsigned)((t.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
+            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<float2>(), reinterpret_cast<float2*>(y),
+            b.seeds.as<uint32_t>(), n, alpha);
         EG_CHECK_LAUNCH("k_row_heavy_finish");
     }
-    k_ppr_teleport<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, g->indeg.as<uint32_t>(), y, alpha);
-    EG_CHECK_LAUNCH("k_ppr_teleport");
+    return EG_OK;
+}
+
+static int lone_seeds(eg_graph* g, float* rows, int nbuf, int n, float alpha) {
+    if (nbuf < 1) return EG_OK;
+    k_ppr_lone_seeds<<<std::min(nbuf, 64), 64, 0, g->stream>>>(bstate(g).seeds.as<uint32_t>(), n, g->indeg.as<uint32_t>(), rows,
+                                                               g->V, nbuf, alpha);
+    EG_CHECK_LAUNCH("k_ppr_lone_seeds");
     return EG_OK;
 }
 
@@ -1887,7 +2019,6 @@ static int ppr_common(eg_graph* g, const float* w_in, const uint32_t* seeds, int
     EG_CUDA(cudaMemsetAsync(b.heavy.ptr, 0, b.heavy.bytes, g->stream));
     EG_TRY(b.rows0.reserve(256 * V + 256));
     EG_TRY(b.rows1.reserve(256 * V + 256));
-    EG_TRY(resident_grid(g, (const void*)k_row_spmm, &b.spmm_grid));
     return prepare_ppr_weights(g, wd, adjoint);
 }
 
@@ -1980,6 +2111,7 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
     k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, x);
     EG_CHECK_LAUNCH("k_ppr_init");
     for (int k = 0; k < K; ++k) {
+        if (k < 2) EG_TRY(lone_seeds(g, y, 1, n, alpha));  // x_0 itself has 1 there
         EG_TRY(ppr_step(g, x, y, alpha, n));
         std::swap(x, y);
     }
@@ -2042,7 +2174,7 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
         if (C == most) return st;
         C = most;
     }
-    EG_TRY(b.gA.reserve(4 * E + 64));
+    EG_TRY(b.gA.reserve(8 * E + 64));
     // forward with checkpoints x_0, x_C, x_2C, ... up to the last one before x_K
     float* ck = b.ck.as<float>();
     float* seg = b.seg.as<float>();
@@ -2053,14 +2185,17 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     EG_CHECK_LAUNCH("k_ppr_init");
     if (C == 1) {
         EG_TRY(zero_rows(g, indeg, ck + 64 * V, K - 1));
+        EG_TRY(lone_seeds(g, ck + 64 * V, K - 1, n, alpha));
         for (int k = 0; k + 1 < K; ++k) EG_TRY(ppr_step(g, ck + 64 * V * k, ck + 64 * V * (k + 1), alpha, n));
     } else {
         EG_TRY(zero_rows(g, indeg, seg, C));
+        EG_TRY(lone_seeds(g, seg + 64 * V, C - 1, n, alpha));
         float* x = b.rows0.as<float>();
         float* y = b.rows1.as<float>();
         EG_CUDA(cudaMemcpyAsync(x, ck, row, cudaMemcpyDeviceToDevice, g->stream));
         EG_CUDA(cudaMemsetAsync(y, 0, row, g->stream));
         for (int k = 0; k < (K - 1) / C * C; ++k) {
+            if (k < 2) EG_TRY(lone_seeds(g, y, 1, n, alpha));
             EG_TRY(ppr_step(g, x, y, alpha, n));
             std::swap(x, y);
             if ((k + 1) % C == 0)
@@ -2082,10 +2217,8 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
         k_untranspose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(src, (uint32_t)V, n, lam);
         EG_CHECK_LAUNCH("k_untranspose_rows");
     }
-    EG_CUDA(cudaMemsetAsync(b.gA.ptr, 0, 4 * E, g->stream));
+    EG_CUDA(cudaMemsetAsync(b.gA.ptr, 0, 8 * E, g->stream));
     const RowTasks& tr = b.csr_tasks;
-    unsigned adjoint_grid = 0;
-    EG_TRY(resident_grid(g, (const void*)k_row_adjoint, &adjoint_grid));
     RowArgs ar = row_args(tr, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
     // the sweeps write only rows with out-edges; the others are zero from lambda_{K-1} on
     EG_TRY(zero_rows(g, outdeg, lam2, 1));
@@ -2102,15 +2235,15 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
             // lam holds lambda_{k+1}; gA += (1-a) <x_k[u], lam[v]>; lam2 = (1-a) A lam
             {
                 Timed tm(&g->prof, g->stream, "ppr_adjoint");
-                k_row_adjoint<<<adjoint_grid, 256, 0, g->stream>>>(
-                    ar, reinterpret_cast<const float4*>(lam), reinterpret_cast<const float4*>(xs + (size_t)(k - k0) * 64 * V),
-                    reinterpret_cast<float4*>(lam2), b.heavy.as<float4>(), b.gA.as<float>(), 1.0f - alpha);
+                k_row_adjoint<<<tr.nbatches, 32, 0, g->stream>>>(
+                    ar, reinterpret_cast<const float2*>(lam), reinterpret_cast<const float2*>(xs + (size_t)(k - k0) * 64 * V),
+                    reinterpret_cast<float2*>(lam2), b.heavy.as<float2>(), b.gA.as<double>(), 1.0f - alpha);
                 EG_CHECK_LAUNCH("k_row_adjoint");
             }
             if (tr.nheavy) {
-                k_row_heavy_finish<<<(unsigned)((tr.nheavy * 16ull + 255) / 256), 256, 0, g->stream>>>(
-                    tr.heavy_vertex.as<uint32_t>(), tr.nheavy, b.heavy.as<float4>(), reinterpret_cast<float4*>(lam2),
-                    1.0f - alpha);
+                k_row_heavy_finish<<<(unsigned)((tr.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
+                    tr.heavy_vertex.as<uint32_t>(), tr.nheavy, b.heavy.as<float2>(), reinterpret_cast<float2*>(lam2),
+                    nullptr, 0, alpha);
                 EG_CHECK_LAUNCH("k_row_heavy_finish");
             }
             if (k == K - 1) EG_TRY(zero_rows(g, outdeg, lam, 1));  // dL/dx_K itself is no longer needed
@@ -2130,7 +2263,7 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
         Timed tm(&g->prof, g->stream, "ppr_weight_grad");
         for (int heavy = 0; heavy <= (tr.nheavy ? 1 : 0); ++heavy) {
             k_weight_grad<<<(unsigned)g->num_sms * 8u, 256, 0, g->stream>>>(
-                tr.rec.as<uint4>(), tr.ntasks, b.wn_csr.as<float>(), b.gA.as<float>(), b.s_out.as<float>(),
+                tr.rec.as<uint4>(), tr.ntasks, b.wn_csr.as<float>(), b.gA.as<double>(), b.s_out.as<float>(),
                 g->csr_w.as<float>(), dw, b.heavy_sum.as<double>(), heavy);
             EG_CHECK_LAUNCH("k_weight_grad");
         }
@@ -2168,8 +2301,6 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
             b.entries.as<uint2>(), n_entries, dist, b.ch0.as<uint32_t>());
         EG_CHECK_LAUNCH("k_sssp_init_entries");
     }
-    unsigned grid = 0;
-    EG_TRY(resident_grid(g, (const void*)k_row_sssp, &grid));
     RowArgs a = row_args(b.csc_tasks, g->csc_adj.as<uint32_t>(), g->csc_w.as<float>());
     uint32_t* prev = b.ch0.as<uint32_t>();
     uint32_t* nxt = b.ch1.as<uint32_t>();
@@ -2179,7 +2310,7 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
         EG_CUDA(cudaMemsetAsync(b.flag.ptr, 0, 4, g->stream));
         {
             Timed t(&g->prof, g->stream, "sssp_batch_sweep");
-            k_row_sssp<<<grid, 256, 0, g->stream>>>(a, reinterpret_cast<float4*>(dist), prev, nxt,
+            k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<float4*>(dist), prev, nxt,
                                                           g->partitions > 1, b.flag.as<int>());
             EG_CHECK_LAUNCH("k_row_sssp");
         }

@@ -122,3 +122,58 @@ def test_ppr_adjoint_checkpoint_stride(eg_lib):
     dot = torch.zeros(V, dtype=torch.float64, device="cuda").index_add(0, s, a * ga)
     ref = (ga - dot[s]) / tot[s]
     assert float((dw.double() - ref).norm() / ref.norm()) <= 1e-4
+
+
+@pytest.mark.parametrize("V,E,longest", [(50, 1, 1), (3000, 31, 1), (40_000, 70_001, 1), (3_000_000, 2_900_003, 2),
+                                         (1_500_000, 4_000_037, 700)])
+def test_ppr_walk_over_lists(eg_lib, V, E, longest):
+    """Batches from one edge to a full one, with up to a few hundred lists of one or two edges in each (task
+    records and source rows come in groups of 8 and 32), and with lists longer than a batch.  Seeds
+    repeat and include vertices with and without in-edges."""
+    import torch
+
+    import endgraph_gb300 as eg
+    K, alpha, n = 4, 0.15, 5
+    gen = torch.Generator("cuda").manual_seed(V)
+    if longest == 1:      # a matching: every list has one edge
+        src, dst = torch.randperm(V, generator=gen, device="cuda")[:E], torch.randperm(V, generator=gen, device="cuda")[:E]
+        if E > V:
+            src, dst = torch.cat([src, src[: E - V]]), torch.cat([dst, dst[: E - V].flip(0)])
+    elif longest == 2:
+        src, dst = (torch.randperm(V, generator=gen, device="cuda")[torch.arange(E, device="cuda") // 2] for _ in range(2))
+        dst = dst[torch.randperm(E, generator=gen, device="cuda")]
+    else:
+        src, dst = (torch.randint(0, V, (E,), generator=gen, device="cuda") for _ in range(2))
+        src[: 700 * 30] = torch.arange(30, device="cuda").repeat(700)
+        dst[E - 700 * 30:] = torch.arange(40, 70, device="cuda").repeat(700)
+    src, dst = src[:E], dst[:E]
+    E = len(src)
+    rec = torch.stack([src, dst], 1).to(torch.int32).contiguous()
+    seeds = torch.stack([src[0], dst[0], dst[-1], dst[0], torch.tensor(V - 1, device="cuda")])
+    w = torch.rand(E, generator=gen, device="cuda") + 0.5
+    dl = torch.rand((n, V), generator=gen, device="cuda")
+    with eg.Graph() as g:
+        g.load_directed_with_ids(rec, V)
+        x = torch.empty((n, V), device="cuda")
+        dw = torch.empty(E, device="cuda")
+        sd = seeds.cpu().numpy().astype(np.uint32)
+        g.ppr(w, sd, alpha, K, out=x)
+        g.ppr_backward(w, sd, dl, alpha, K, dl_dw=dw)
+    s, d, wt = src.long(), dst.long(), w.double()
+    tot = torch.zeros(V, dtype=torch.float64, device="cuda").index_add(0, s, wt)
+    a = wt / tot[s]
+    e = torch.zeros((V, n), dtype=torch.float64, device="cuda")
+    e[seeds.long(), torch.arange(n, device="cuda")] = 1.0
+    xs = [e]
+    for _ in range(K):
+        xs.append(alpha * e + (1 - alpha) * torch.zeros_like(e).index_add(0, d, a[:, None] * xs[-1][s]))
+    lam = dl.double().t().contiguous()
+    ga = torch.zeros(E, dtype=torch.float64, device="cuda")
+    for k in range(K - 1, -1, -1):
+        ga += (1 - alpha) * (xs[k][s] * lam[d]).sum(1)
+        lam = (1 - alpha) * torch.zeros_like(lam).index_add(0, s, a[:, None] * lam[d])
+    dot = torch.zeros(V, dtype=torch.float64, device="cuda").index_add(0, s, a * ga)
+    ref = (ga - dot[s]) / tot[s]
+    assert float((x.double() - xs[K].t()).abs().sum() / xs[K].abs().sum()) <= 1e-6
+    # lists of one edge have no gradient: what is left are the roundings of terms of size |gA| / s
+    assert float((dw.double() - ref).norm()) <= 1e-4 * float(ref.norm()) + 1e-6 * float((ga / tot[s]).norm())
