@@ -1018,105 +1018,149 @@ __global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ t
 }
 
 // ---- batched SSSP: in place, skipping sources whose row did not change in the last sweep --------
-// A warp takes the tasks of its batch one by one; the two half-warps take alternate edges and lane c of a
-// half owns columns 4c..4c+3 (one 16-byte load of a 256-byte row).  The sweep is bound by the latency
-// of the chain record -> ids -> changed bits -> rows, so the next task's record is loaded one task
-// ahead, the destination's row together with the ids, and up to kSsspRows rows are in flight per
-// warp; sources that did not change (one bit each, cached in L1: the bits do not change during a
-// sweep) are squeezed out first, their ids and weights queueing up in shared memory, so the row
-// loads stay full when few sources are active.  A destination with a single task is written by this
-// warp alone and stored plainly; cut lists (and items of several partitions that share a vertex) take
-// the minimum with atomics.  64 graphs of 1k-500k vertices, 93 M edges, 64 sources, 24 sweeps: 107 ms
-// with one row per warp load, byte flags and separate item / offset arrays; tasks by stride at 48
-// warps per SM (40 registers, spilled) 47.5 ms; batches in CTAs of 8 warps 44.4, of 2 45.2, of 2 at 40
-// / 32 warps per SM 42.2 / 40.5, of one warp at 32 (64 registers) 38.5 (10.8 E row gathers: 6.7
-// TB/s), there with 16 rows 41.0.
-constexpr int kSsspRows = 8;
+// A warp walks the edges of its batch, 32 at a time: sources that did not change (one bit each, cached in
+// L1: the bits do not change during a sweep) are dropped, the others queue up in shared memory, the
+// sources of a list behind an entry for the list's own row.  16 queued rows are gathered together,
+// whatever lists they belong to; a list whose row was not lowered costs nothing more, one without
+// changed sources is never looked at.  Ids are on their way two steps ahead and bits one; the tasks are
+// read when the first changed source turns up.  A destination with a single task is written by this
+// warp alone and stored plainly; cut lists (and items of several partitions that share a vertex)
+// take the minimum with atomics.  The sweep is bound by the row gathers.  64 graphs of 1k-500k vertices,
+// 93 M edges, 64 sources, 24 sweeps: 107 ms with one row per warp load, byte flags and separate item /
+// offset arrays; a task at a time, rows by half-warps, tasks by stride 47.5 ms, in batches with a
+// warp per CTA 39.7; the walk 28.8 (10.8 E row gathers: 8.9 TB/s) at 32 warps per SM, 30.5 at 28,
+// 33.7 at 24.
+constexpr int kSsspRows = 16;
+constexpr uint32_t kDestRow = 1u << 31;  // queue entry: the list's own row
 
-__global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float4* __restrict__ dist,
-                                                  const uint32_t* __restrict__ changed_prev,
-                                                  uint32_t* __restrict__ changed_next, int shared_vertex,
-                                                  int* __restrict__ any) {
-    __shared__ uint2 act[64];
-    const uint32_t lane = threadIdx.x & 31, half = lane >> 4, c = lane & 15;
-    uint32_t t = __ldg(a.first + blockIdx.x);
-    const uint32_t t1 = __ldg(a.first + blockIdx.x + 1);
-    uint4 nxt = t < t1 ? __ldg(a.rec + t) : make_uint4(0, 0, 0, 0);
-    bool any_lowered = false;
-    for (; t < t1; ++t) {
-        const uint4 rec = nxt;
-        if (t + 1 < t1) nxt = __ldg(a.rec + t + 1);
-        const uint64_t e0 = task_begin(rec);
-        const uint32_t n = task_len(rec), v = rec.z;
-        const float4 dv = __ldcg(dist + (uint64_t)v * 16 + c);
-        float4 best = make_float4(1e9f, 1e9f, 1e9f, 1e9f);
-        uint32_t queued = 0;  // active sources waiting in act (the same in every lane)
-        for (uint32_t eb = 0; eb < n; eb += 32) {
-            const uint32_t k = eb + lane;
-            uint32_t u = 0;
-            bool ch = false;
-            if (k < n) {
-                u = __ldg(a.adj + e0 + k);
-                ch = (__ldg(changed_prev + (u >> 5)) >> (u & 31)) & 1u;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, ch);
-            if (ch) {
-                act[queued + __popc(m & ((1u << lane) - 1u))] =
-                    make_uint2(u, __float_as_uint(__ldg(a.w + e0 + k)));
-            }
-            queued += __popc(m);
-            if (queued <= 32 && eb + 32 < n) continue;  // room for another 32
-            __syncwarp();
-            for (uint32_t b = 0; b < queued; b += kSsspRows) {
-                float4 r[kSsspRows / 2];
-                float w[kSsspRows / 2];
+__global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float2* __restrict__ dist,
+                                                     const uint32_t* __restrict__ changed_prev,
+                                                     uint32_t* __restrict__ changed_next, int shared_vertex,
+                                                     int* __restrict__ any) {
+    static_assert(kBatchEdges + kTaskEdges <= 32 * 32, "a batch's list starts are one bit per edge in s_head");
+    __shared__ uint2 s_task[kBatchEdges];              // the batch's tasks: vertex, slot
+    __shared__ uint32_t s_head[32];                    // bit e: a task begins with edge e of the batch
+    __shared__ __align__(16) uint32_t q_row[kSsspRows + 64], q_edge[kSsspRows + 64];
+    const uint32_t lane = threadIdx.x, lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    const uint32_t t0 = __ldg(a.first + blockIdx.x), tasks = __ldg(a.first + blockIdx.x + 1) - t0;
+    if (!tasks) return;
+    const uint4 begin = __ldg(a.rec + t0), last = __ldg(a.rec + t0 + tasks - 1);
+    const uint64_t e0 = task_begin(begin);
+    const uint32_t n = (uint32_t)(task_begin(last) - e0) + task_len(last);
+    const uint32_t* adj = a.adj + e0 + lane;
+    const float* wts = a.w + e0;
+    dist += lane;
+    bool loaded = false, any_lowered = false;
+    uint32_t before = 0;       // tasks that begin before this chunk
+    uint32_t queued = 0;
+    uint32_t q_task = ~0u;     // task of the last queued source
+    uint32_t cur = ~0u;        // task whose row is being reduced
+    float2 dv = make_float2(0.f, 0.f), best = dv;
+    auto flush = [&]() {
+        bool low = best.x < dv.x || best.y < dv.y;
+        if (cur == ~0u || !__any_sync(0xffffffffu, low)) return;
+        const uint2 tk = s_task[cur];
+        float2* row = dist + (uint64_t)tk.x * 32;
+        if (tk.y == kNoSlot && !shared_vertex) {
+            if (low) __stcg(row, best);
+        } else {  // distances are >= 0: ordered like their bits
+            int* p = reinterpret_cast<int*>(row);
+            low = false;
+            if (best.x < dv.x) low |= best.x < __int_as_float(atomicMin(p, __float_as_int(best.x)));
+            if (best.y < dv.y) low |= best.y < __int_as_float(atomicMin(p + 1, __float_as_int(best.y)));
+            if (!__any_sync(0xffffffffu, low)) return;
+        }
+        if (lane == 0) atomicOr(changed_next + (tk.x >> 5), 1u << (tk.x & 31));
+        any_lowered = true;
+    };
+    auto reduce = [&](uint32_t base, uint32_t m) {  // entries [base, base + m) of the queue, m <= kSsspRows
+        const uint32_t qe = lane < m ? q_edge[base + lane] : kDestRow;
+        const float wl = qe & kDestRow ? 0.f : __ldg(wts + qe);
+        float2 r[kSsspRows];
 #pragma unroll
-                for (int j = 0; j < kSsspRows / 2; ++j) {
-                    const uint32_t i = b + 2 * j + half;
-                    if (i < queued) {
-                        const uint2 x = act[i];
-                        w[j] = __uint_as_float(x.y);
-                        r[j] = __ldcg(dist + (uint64_t)x.x * 16 + c);
-                    } else {
-                        w[j] = 0.f;
-                        r[j] = make_float4(1e9f, 1e9f, 1e9f, 1e9f);
+        for (int j = 0; j < kSsspRows; j += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(q_row + base + j);
+            if (j < m) r[j] = __ldcg(dist + (uint64_t)q.x * 32);
+            if (j + 1 < m) r[j + 1] = __ldcg(dist + (uint64_t)q.y * 32);
+            if (j + 2 < m) r[j + 2] = __ldcg(dist + (uint64_t)q.z * 32);
+            if (j + 3 < m) r[j + 3] = __ldcg(dist + (uint64_t)q.w * 32);
+        }
+#pragma unroll
+        for (int j = 0; j < kSsspRows; ++j) {
+            if (j >= m) break;
+            const uint32_t e = __shfl_sync(0xffffffffu, qe, j);
+            const float w = __shfl_sync(0xffffffffu, wl, j);
+            if (e & kDestRow) {
+                flush();
+                cur = e ^ kDestRow;
+                dv = best = r[j];
+            } else {  // toolkits/sssp.cpp:55: relax_dist = msg + w
+                best.x = fminf(best.x, r[j].x + w);
+                best.y = fminf(best.y, r[j].y + w);
+            }
+        }
+    };
+    uint32_t u0 = lane < n ? __ldg(adj) : 0u, u1 = lane + 32 < n ? __ldg(adj + 32) : 0u;
+    uint32_t b0 = lane < n ? __ldg(changed_prev + (u0 >> 5)) : 0u;
+    for (uint32_t c = 0; c < n; c += 32) {
+        const uint32_t u2 = c + 64 + lane < n ? __ldg(adj + c + 64) : 0u;
+        const uint32_t b1 = c + 32 + lane < n ? __ldg(changed_prev + (u1 >> 5)) : 0u;
+        const bool active = (b0 >> (u0 & 31)) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, active);
+        if (m && !loaded) {
+            loaded = true;
+            s_head[lane] = 0;
+            __syncwarp();
+            for (uint32_t i = lane; i < tasks; i += 32) {
+                const uint4 r = __ldg(a.rec + t0 + i);
+                s_task[i] = make_uint2(r.z, r.w);
+                const uint32_t at = (uint32_t)(task_begin(r) - e0);
+                atomicOr(s_head + (at >> 5), 1u << (at & 31));
+            }
+            __syncwarp();
+            before = __reduce_add_sync(0xffffffffu, lane < (c >> 5) ? __popc(s_head[lane]) : 0);
+        }
+        if (loaded) {
+            const uint32_t heads = s_head[c >> 5];
+            if (m) {
+                const uint32_t task = before + __popc(heads & le) - 1;
+                const uint32_t prev = m & lt;  // active sources before this one
+                const uint32_t since = prev ? (2u << (31 - __clz(prev))) - 1u : 0u;
+                const bool first = active && (prev ? (heads & le & ~since) != 0 : task != q_task);
+                const uint32_t f = __ballot_sync(0xffffffffu, first);
+                uint32_t at = queued + __popc(prev) + __popc(f & lt);
+                if (first) {
+                    q_row[at] = s_task[task].x;
+                    q_edge[at++] = kDestRow | task;
+                }
+                if (active) {
+                    q_row[at] = u0;
+                    q_edge[at] = c + lane;
+                }
+                q_task = __shfl_sync(0xffffffffu, task, 31 - __clz(m));
+                queued += __popc(m) + __popc(f);
+                __syncwarp();
+                uint32_t done = 0;
+                for (; queued - done >= kSsspRows; done += kSsspRows) reduce(done, kSsspRows);
+                if (done) {  // the rest to the front
+                    queued -= done;
+                    const uint32_t r = lane < queued ? q_row[done + lane] : 0u, e = lane < queued ? q_edge[done + lane] : 0u;
+                    __syncwarp();
+                    if (lane < queued) {
+                        q_row[lane] = r;
+                        q_edge[lane] = e;
                     }
-                }
-#pragma unroll
-                for (int j = 0; j < kSsspRows / 2; ++j) {  // toolkits/sssp.cpp:55: relax_dist = msg + w
-                    best.x = fminf(best.x, r[j].x + w[j]);
-                    best.y = fminf(best.y, r[j].y + w[j]);
-                    best.z = fminf(best.z, r[j].z + w[j]);
-                    best.w = fminf(best.w, r[j].w + w[j]);
+                    __syncwarp();
                 }
             }
-            queued = 0;
-            __syncwarp();
+            before += __popc(heads);
         }
-        best.x = fminf(best.x, __shfl_xor_sync(0xffffffffu, best.x, 16));
-        best.y = fminf(best.y, __shfl_xor_sync(0xffffffffu, best.y, 16));
-        best.z = fminf(best.z, __shfl_xor_sync(0xffffffffu, best.z, 16));
-        best.w = fminf(best.w, __shfl_xor_sync(0xffffffffu, best.w, 16));
-        bool lowered = best.x < dv.x || best.y < dv.y || best.z < dv.z || best.w < dv.w;
-        if (half == 0 && lowered) {
-            float4* row = dist + (uint64_t)v * 16 + c;
-            if (rec.w == kNoSlot && !shared_vertex) {
-                __stcg(row, make_float4(fminf(best.x, dv.x), fminf(best.y, dv.y), fminf(best.z, dv.z),
-                                        fminf(best.w, dv.w)));
-            } else {
-                int* p = reinterpret_cast<int*>(row);  // distances are >= 0: ordered like their bits
-                lowered = false;
-                if (best.x < dv.x) lowered |= best.x < __int_as_float(atomicMin(p, __float_as_int(best.x)));
-                if (best.y < dv.y) lowered |= best.y < __int_as_float(atomicMin(p + 1, __float_as_int(best.y)));
-                if (best.z < dv.z) lowered |= best.z < __int_as_float(atomicMin(p + 2, __float_as_int(best.z)));
-                if (best.w < dv.w) lowered |= best.w < __int_as_float(atomicMin(p + 3, __float_as_int(best.w)));
-            }
-        }
-        if (__any_sync(0xffffffffu, lowered && half == 0)) {
-            if (lane == 0) atomicOr(changed_next + (v >> 5), 1u << (v & 31));
-            any_lowered = true;
-        }
+        u0 = u1;
+        u1 = u2;
+        b0 = b1;
     }
+    if (queued) reduce(0, queued);
+    flush();
     if (any_lowered && lane == 0) *any = 1;
 }
 
@@ -2310,7 +2354,7 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
         EG_CUDA(cudaMemsetAsync(b.flag.ptr, 0, 4, g->stream));
         {
             Timed t(&g->prof, g->stream, "sssp_batch_sweep");
-            k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<float4*>(dist), prev, nxt,
+            k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<float2*>(dist), prev, nxt,
                                                           g->partitions > 1, b.flag.as<int>());
             EG_CHECK_LAUNCH("k_row_sssp");
         }

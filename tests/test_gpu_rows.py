@@ -177,3 +177,31 @@ def test_ppr_walk_over_lists(eg_lib, V, E, longest):
     assert float((x.double() - xs[K].t()).abs().sum() / xs[K].abs().sum()) <= 1e-6
     # lists of one edge have no gradient: what is left are the roundings of terms of size |gA| / s
     assert float((dw.double() - ref).norm()) <= 1e-4 * float(ref.norm()) + 1e-6 * float((ga / tot[s]).norm())
+
+
+@pytest.mark.parametrize("V,E,shape", [(40, 1, "one"), (5000, 5000, "one"), (3_000_000, 2_950_003, "two"),
+                                       (200_000, 3_000_001, "hubs")])
+def test_sssp_batch_walk_over_lists(eg_lib, V, E, shape):
+    """Batches of up to 512 lists, of which a few, all or none have a changed source in a sweep; chains, so
+    that a handful of sources changes at a time; lists longer than a batch between short ones."""
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(V)
+    perm = rng.permutation(V)
+    if shape == "one":      # a cycle: every list has one source
+        src, dst = perm[:E], np.roll(perm, 1)[:E]
+    elif shape == "two":    # up to two sources per list, a long chain among them
+        src, dst = perm[np.arange(E) // 2 % V], perm[(np.arange(E) + 1) % V]
+        src[:300], dst[:300] = perm[:300], perm[1:301]
+    else:
+        src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
+        dst[: 40 * 1500] = np.repeat(np.arange(40) * 7, 1500)
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    w = rng.random(E).astype(np.float32)
+    csr = oracle.build_csr(src, dst, w, V, np.array([0, V], np.uint32))
+    sources = np.array([src[0], src[E // 2], src[-1], dst[0]], np.uint32)
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst, w), V)
+        dist = g.sssp_batch(sources)
+    for s in range(len(sources)):
+        ref = oracle.sssp(csr["off"][0], csr["adj"], csr["w"], V, int(sources[s]))
+        assert np.array_equal(dist[s].view(np.uint32), ref.view(np.uint32)), s
