@@ -270,6 +270,9 @@ int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int whe
 // renumbering of the CSC sources by out-degree class (eng.pr_new_id / eng.pr_adj), built once per
 // structure build and shared by the PageRank and bit-parallel BFS pull gathers
 bool want_relabel(const eg_graph* g);
+// The renumbering spreads its first ranks over `lines` 128-byte lines (rank r < lines is id 32 r).
+constexpr uint32_t kRelabelHot = 1u << 21;
+inline uint32_t relabel_lines(uint32_t V) { return (V < kRelabelHot ? V : kRelabelHot) / 32u; }
 int setup_relabel(eg_graph* g);
 int run_bfs(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached);
 int run_sssp(eg_graph* g, uint32_t root, float* dist, int where);

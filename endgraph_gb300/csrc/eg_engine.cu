@@ -357,7 +357,6 @@ __global__ void k_pr_finish_all(const uint32_t* __restrict__ indeg, uint32_t V, 
 // vertices, classes counted per tile and scanned class-major), in any order inside a tile.
 constexpr uint32_t kRelabelTile = 8192;
 constexpr uint32_t kRelabelClasses = 33;
-constexpr uint32_t kRelabelHot = 1u << 21;  // ranks spread round-robin over the hot region's lines
 
 __global__ void __launch_bounds__(256) k_relabel_hist(const uint32_t* __restrict__ outdeg, uint32_t V, uint32_t ntiles,
                                                       uint32_t* __restrict__ cnt) {
@@ -441,7 +440,7 @@ int setup_relabel(eg_graph* g) {
     {
         Timed t(&g->prof, g->stream, "pr_relabel");
         if (ntiles) {
-            const uint32_t lines = std::min<uint32_t>(V, kRelabelHot) / 32u;
+            const uint32_t lines = relabel_lines(V);
             k_relabel_assign<<<ntiles, 256, 0, g->stream>>>(g->outdeg.as<uint32_t>(), V, ntiles, s.pr_off.as<uint64_t>(),
                                                             lines, s.pr_new_id.as<uint32_t>());
             EG_CHECK_LAUNCH("k_relabel_assign");

@@ -21,6 +21,8 @@ namespace eg {
 constexpr uint32_t kNoBoundary = 0xFFFFFFFFu;
 constexpr int kPrGroup = 8;  // consecutive edges per lane: 4 or 16 were no faster (40.3 / 40.3 against 39.4 ms of sweeps)
 
+constexpr uint32_t kPrSums = 32 * kPrGroup;  // lists that can end in a group of edges
+
 struct PrArgs {
     const uint32_t* adj;
     const uint32_t* heads;    // bit e: edge e is the first of its list (one word of zeros past E)
@@ -34,6 +36,8 @@ struct PrArgs {
     float* next;
     float* acc;               // per run boundary: the list that crosses it first there (split)
     const uint32_t* split;    // per run: boundary its first list's pieces meet at
+    uint32_t hot;             // ranks that k_pr_sweep keeps in shared memory
+    uint32_t* ticket;         // its next run
     float base, d;
     int divide;
 };
@@ -47,8 +51,9 @@ __device__ __forceinline__ void pr_write(const PrArgs& a, uint32_t item, float s
     a.next[to] = pr_value(a, sum, deg);
 }
 
-// one run of blocks by one warp; s_sum: kPrBlock floats of the warp's own
-__device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_sum) {
+// one run of blocks by one warp; s_sum: kPrSums floats of the warp's own
+template <class Gather>
+__device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_sum, Gather gather) {
     constexpr int G = kPrGroup, kGroups = (int)kPrBlock / (32 * G);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t below = (1u << lane) - 1u;
@@ -74,30 +79,31 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
                     id[4 * q + 3] = x.w;
                 }
 #pragma unroll
-                for (int j = 0; j < G; ++j) val[g][j] = ld_keep(a.curr + id[j]);
+                for (int j = 0; j < G; ++j) val[g][j] = gather(id[j]);
             } else {
 #pragma unroll
-                for (int j = 0; j < G; ++j) val[g][j] = e + j < a.E ? ld_keep(a.curr + a.adj[e + j]) : 0.f;
+                for (int j = 0; j < G; ++j) val[g][j] = e + j < a.E ? gather(a.adj[e + j]) : 0.f;
             }
             if (G == 16) head[g] = e < a.E ? __ldcs(reinterpret_cast<const uint16_t*>(a.heads) + e / 16) : 0u;
             else if (G == 8) head[g] = e < a.E ? __ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8) : 0u;
             else head[g] = e < a.E ? (__ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8) >> (e & 7)) & 0xFu : 0u;
             if (e == e_begin) head[g] &= ~1u;  // the run's first edge opens nothing new
         }
-        // lists that end in earlier lanes (rank, per group) and in the whole block
-        uint32_t rank[kGroups], closed = 0;
+        // lists that end in earlier lanes (rank) and in the whole group
+        uint32_t rank[kGroups], closed[kGroups], to[kGroups], deg[kGroups], at = item;
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
-            rank[g] = closed;
+            rank[g] = closed[g] = 0;
 #pragma unroll
             for (int j = 0; j < G; ++j) {
                 const uint32_t b = __ballot_sync(0xffffffffu, (head[g] >> j) & 1u);
                 rank[g] += __popc(b & below);
-                closed += __popc(b);
+                closed[g] += __popc(b);
             }
+            to[g] = lane < closed[g] ? __ldg(a.dst + at + lane) : 0u;
+            deg[g] = lane < closed[g] ? __ldg(a.deg + at + lane) : 0u;
+            at += closed[g];
         }
-        const uint32_t to = lane < closed ? __ldg(a.dst + item + lane) : 0u;
-        const uint32_t deg = lane < closed ? __ldg(a.deg + item + lane) : 0u;
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
             const uint32_t f = head[g];
@@ -128,17 +134,17 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
             if (lane == 0) before = carry;
             if (seen) s_sum[rank[g]] = before + first;
             carry = __shfl_sync(0xffffffffu, t, 31);
+            __syncwarp();
+            for (uint32_t i = lane; i < closed[g]; i += 32) {
+                const float sum = s_sum[i];
+                if (i == 0 && open_first) atomicAdd(a.acc + __ldg(a.split + run), sum);
+                else if (i < 32) a.next[to[g]] = pr_value(a, sum, deg[g]);
+                else pr_write(a, item + i, sum);
+            }
+            __syncwarp();
+            if (closed[g]) open_first = false;
+            item += closed[g];
         }
-        __syncwarp();
-        for (uint32_t k = lane; k < closed; k += 32) {
-            const float sum = s_sum[k];
-            if (k == 0 && open_first) atomicAdd(a.acc + __ldg(a.split + run), sum);
-            else if (k < 32) a.next[to] = pr_value(a, sum, deg);
-            else pr_write(a, item + k, sum);
-        }
-        __syncwarp();
-        if (closed) open_first = false;
-        item += closed;
     }
     if (lane == 0) {
         const bool ends = e_end == a.E || ((__ldg(a.heads + (e_end >> 5)) >> (e_end & 31)) & 1u);
@@ -156,15 +162,48 @@ __device__ __forceinline__ void pr_boundary(const PrArgs& a, uint64_t r) {
     pr_write(a, __ldg(a.item_of + (r << a.shift)), sum);
 }
 
-// 20 iterations at 2^25 / 2^29: 6 CTAs per SM (40 registers) 38.6 ms, 5 38.9, 4 39.5, 8 (32, spilled) 47;
-// 49.5 ms with 4,096-edge CTA chunks, entry bounds in shared memory and an accumulator per entry there
-__global__ void __launch_bounds__(256, 6) k_pr_sweep(PrArgs a) {
-    __shared__ float s_sum[8][kPrBlock];
-    const uint64_t run = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (run < a.nruns) pr_run(a, run, s_sum[threadIdx.x >> 5]);
+// The sweep of a large graph: one CTA of 32 warps per SM, runs by ticket.  With renumbered sources the
+// values of the first kPrHot ranks (rank r is id 32 r: see relabel_lines) are copied to shared memory
+// by every SM, where a warp's gathers take a few cycles instead of a lookup each: on a power law
+// a quarter of the gathers and more.  How many pays is set by the L1, whose lines hold the gathers in
+// flight and which gets what shared memory leaves: 20 iterations at 2^25 / 2^29, 2^23 / 2^27 and 5 M /
+// 40 M take 37.8 / 10.0 / 3.45 ms with none, 32.2 / 7.9 / - with 8,192, 29.8 / 7.3 / 2.65 with 16,384, 29.2 / 7.1
+// / 2.64 with 24,576, 29.4 / 6.9 / 2.64 with 32,768, 36.2 / 7.0 / 2.69 with 33,760 and 66 / 10.9 / 3.8 with
+// 40,960 (38.6 / 10.5 / 3.6 with CTAs of 8 warps, 48 warps per SM, a run per warp).
+constexpr uint32_t kPrHot = 24576, kPrSweepThreads = 1024;
+constexpr size_t kPrSweepSmem = sizeof(float) * (kPrHot + kPrSweepThreads / 32 * kPrSums);
+
+__global__ void __launch_bounds__(kPrSweepThreads, 1) k_pr_sweep(PrArgs a) {
+    extern __shared__ float s_dyn[];
+    float* s_hot = s_dyn + kPrSweepThreads / 32 * kPrSums;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t r = threadIdx.x; r < a.hot; r += kPrSweepThreads) s_hot[r] = __ldcg(a.curr + 32ull * r);
+    const uint32_t hot_addr = (uint32_t)__cvta_generic_to_shared(s_hot), hot = a.hot;
+    const float* curr = a.curr;
+    unsigned long long keep;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    while (true) {
+        const uint32_t run = __shfl_sync(0xffffffffu, next, 0);
+        if (run >= a.nruns) break;
+        if (lane == 0) next = atomicAdd(a.ticket, 1u);
+        pr_run(a, run, s_dyn + (threadIdx.x >> 5) * kPrSums, [&](uint32_t id) {
+            const uint32_t rank = __funnelshift_r(id, id, 5);  // ids that are no multiple of 32 come out large
+            float v;
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.lt.u32 p, %1, %2;\n@p ld.shared.f32 %0, [%3];\n"
+                "@!p ld.global.cg.L2::cache_hint.f32 %0, [%4], %5;\n}"
+                : "=f"(v)
+                : "r"(rank), "r"(hot), "r"(hot_addr + 4 * rank), "l"(curr + id), "l"(keep));
+            return v;
+        });
+    }
 }
 
 __global__ void k_pr_boundaries(PrArgs a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.ticket = 0;  // for the next sweep
     for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < a.nruns; r += (uint64_t)gridDim.x * blockDim.x)
         pr_boundary(a, r);
 }
@@ -237,7 +276,7 @@ struct PrPersistArgs {
 constexpr int kPrPersistThreads = 512, kPrPersistCtas = 2;
 
 __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persistent(PrPersistArgs a) {
-    __shared__ float s_sum[kPrPersistThreads / 32][kPrBlock];
+    __shared__ float s_sum[kPrPersistThreads / 32][kPrSums];
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     unsigned arrived = 0;
     auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), arrived); };
@@ -251,7 +290,7 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
         if (last) p.dst = a.cvert;
         p.divide = !last;
         if (it < 2 || last) pr_no_in(p.next, a.indeg, a.outdeg, a.V, p.base, p.divide, last ? nullptr : a.order, tid, stride);
-        for (uint64_t run = tid >> 5; run < p.nruns; run += stride >> 5) pr_run(p, run, s_sum[threadIdx.x >> 5]);
+        for (uint64_t run = tid >> 5; run < p.nruns; run += stride >> 5) pr_run(p, run, s_sum[threadIdx.x >> 5], [&](uint32_t id) { return ld_keep(p.curr + id); });
         if (!barrier()) return;
         for (uint64_t r = tid; r < p.nruns; r += stride) pr_boundary(p, r);
     }
@@ -300,14 +339,17 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     const uint64_t V = g->V, E = g->E;
     for (DevBuf* b : {&s.vals0, &s.vals1}) EG_TRY(b->reserve(4 * (V + 1)));
     // with renumbered gathers every vector but the final one is kept in class order
-    const bool relabel = want_relabel(g);
+    // Every iteration in one launch up to here: 20 iterations take 0.26 / 0.35 ms (one launch / sweeps) at
+    // 65,536 / 2^20, 0.62 / 0.67 at 300,000 / 5 M, 1.45 / 1.33 and 0.1 for the renumbering at 1 M / 16 M, 2.70
+    // / 1.91 at 2 M / 30 M.  Sweeps renumber by themselves when that comes back: 2^22 / 2^26 takes 0.30 ms to
+    // renumber and 0.18 instead of 0.26 a sweep; a GPU too full for the second list goes without.
+    const bool small = E <= (1ull << 24);
+    bool relabel = want_relabel(g);
+    if (!relabel && !small && g->pr_relabel < 0 && iterations >= 4) relabel = setup_list_heads(g, true) == EG_OK;
     EG_TRY(setup_list_heads(g, relabel));
     const uint32_t* order = relabel ? s.pr_new_id.as<uint32_t>() : nullptr;
     float* vec[2] = {s.vals0.as<float>(), s.vals1.as<float>()};
     float* result = out && where == EG_DEVICE ? out : vec[iterations & 1];
-    // every iteration in one launch up to here: 20 iterations take 0.26 / 0.35 ms (one launch / two per
-    // iteration) at 65,536 / 2^20, 1.45 / 1.54 at 1 M / 16 M, 5.29 / 5.17 at 2^22 / 2^26
-    const bool small = E <= (1ull << 25);
     PrArgs p;
     p.adj = relabel ? s.pr_adj.as<uint32_t>() : g->csc_adj.as<uint32_t>();
     p.heads = s.pr_heads.as<uint32_t>();
@@ -317,8 +359,10 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     p.E = E;
     p.shift = list_run_shift(E);
     p.nruns = (E + (kPrBlock << p.shift) - 1) / (kPrBlock << p.shift);
-    EG_TRY(s.acc.reserve(4 * (p.nruns + 2)));
+    EG_TRY(s.acc.reserve(4 * (p.nruns + 4)));
     p.acc = s.acc.as<float>();
+    p.ticket = s.acc.as<uint32_t>() + p.nruns + 3;
+    p.hot = relabel ? std::min(kPrHot, relabel_lines((uint32_t)V)) : 0;
     p.split = s.pr_split.as<uint32_t>();
     const uint32_t* outdeg = g->outdeg.as<uint32_t>();
     p.base = 1.0f - damping;
@@ -340,6 +384,8 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
         }
     } else {
         const unsigned gv = grid_for(V, 256, 152u * 16u);
+        EG_CUDA(cudaFuncSetAttribute(k_pr_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrSweepSmem));
+        EG_CUDA(cudaMemsetAsync(p.ticket, 0, 4, g->stream));
         {
             Timed t(&g->prof, g->stream, "pr_vertex");
             k_pr_start<<<gv, 256, 0, g->stream>>>(vec[0], outdeg, V, order, p.acc, p.nruns);
@@ -359,7 +405,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
             }
             {
                 Timed t(&g->prof, g->stream, "pr_pull");
-                k_pr_sweep<<<(unsigned)((p.nruns + 7) / 8), 256, 0, g->stream>>>(p);
+                k_pr_sweep<<<(unsigned)g->num_sms, kPrSweepThreads, kPrSweepSmem, g->stream>>>(p);
                 EG_CHECK_LAUNCH("k_pr_sweep");
             }
             Timed t(&g->prof, g->stream, "pr_finish");

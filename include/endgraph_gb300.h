@@ -202,7 +202,8 @@ enum {
                                       renumbered by out-degree class, high degrees first, so that
                                       the values most gathered share cache lines; the same values
                                       are summed per destination.  1 on, 0 off, -1 automatic (on
-                                      for V > 2^22; the default) */
+                                      for V > 2^22, and with one partition for E > 2^24 and
+                                      four or more iterations; the default) */
     EG_OPT_MAX_ITERATIONS = 8,     /* T of the CPBT page weight for the next build (the public
                                       max_iterations field of Graph, core/graph.hpp:733-738);
                                       eg_config.max_iterations sets it at creation */

@@ -53,3 +53,15 @@ def test_pagerank_one_launch_per_sweep(eg_lib, E):
     dst = rng.integers(0, V, E)
     dst[: E // 4] = 12_345
     _check(rng.integers(0, V, E), dst, V, (1, 4))
+
+
+@pytest.mark.parametrize("V,E", [(40, (1 << 24) + 5), (700_001, (1 << 24) + 1), (1_500_000, 17_000_003), (5_000_000, 17_000_000)])
+def test_pagerank_sweeps_with_hot_sources(eg_lib, V, E):
+    """Sweeps with a launch each, sources of very different out-degree (those of the first ranks are read from
+    shared memory: one, all that the first lines hold, a full table), hubs, lists of one edge and none."""
+    rng = np.random.default_rng(V)
+    src = (V * rng.random(E) ** 4).astype(np.int64)
+    dst = rng.integers(0, V, E)
+    dst[: E // 8] = V // 3
+    dst[E // 8: E // 4] //= 50
+    _check(src, dst, V, (1, 4), relabels=(-1, 0, 1))
