@@ -75,9 +75,12 @@ struct MsBfsPullOp {  // k_pull_direct operator (several partitions, and the per
 // A dense level as a full sweep: the walk of the PageRank sweep (eg_pagerank.cu: list starts as one bit
 // per edge, 8 consecutive ids per lane, a segmented warp scan, lists finished one per lane) with OR in
 // the place of the sum.  A list that lies in one run is this warp's alone: its vertex's words are
-// stored plainly; pieces of longer lists are ORed in with atomics, each on its own.  64 roots at
-// 2^23 / 2^27: 0.59 ms a level at 3 to 6 CTAs per SM, 1.05 with a CTA per 4,096 edges, entry bounds in
-// shared memory and atomics for every list.
+// stored plainly; pieces of longer lists are ORed in with atomics, each on its own.  As there, one CTA
+// of 32 warps per SM takes runs by ticket, and with renumbered sources the frontier words of the
+// hottest are kept in shared memory.  64 roots, 2^23 / 2^27 and 2^25 / 2^29: dense levels 1.47 / 5.8 ms with
+// CTAs of 8 warps at 5 per SM, 1.45 / 5.6 so without the table, 1.37 / 5.4 with 4,096 words, 1.34 / 5.5 with
+// 8,192, 1.34 / 5.7 with 12,288.  (At 2^23 a level had taken 1.05 ms with a CTA per 4,096 edges, entry
+// bounds in shared memory and atomics for every list, 0.59 with the walk.)
 constexpr uint32_t kMsBlock = 256;
 
 struct MsSweepArgs {
@@ -95,6 +98,8 @@ struct MsSweepArgs {
     unsigned long long* next;
     unsigned long long* next_bm;
     const int* stop;  // captured level loops: set once a level found nothing new
+    uint32_t hot;     // ranks of the renumbering (rank r is id 32 r) whose words are kept in shared memory
+    uint32_t* ticket; // the sweep's next run, zero before it
 };
 
 __device__ __forceinline__ void ms_piece(const MsSweepArgs& a, uint32_t v, unsigned long long m) {
@@ -111,14 +116,38 @@ __device__ __forceinline__ void ms_list(const MsSweepArgs& a, uint32_t v, unsign
     atomicOr(a.next_bm + (v >> 6), 1ull << (v & 63));
 }
 
-__global__ void __launch_bounds__(256, 5) k_ms_sweep(MsSweepArgs a) {
-    __shared__ unsigned long long s_or[8][kMsBlock];
+constexpr uint32_t kMsHot = 8192, kMsThreads = 1024;
+constexpr size_t kMsSmem = 8ull * (kMsHot + kMsThreads / 32 * kMsBlock);
+
+__global__ void __launch_bounds__(kMsThreads, 1) k_ms_sweep(MsSweepArgs a) {
+    extern __shared__ unsigned long long s_or[];
     if (a.stop && *(volatile const int*)a.stop) return;
     constexpr int G = 8;
-    unsigned long long* s_list = s_or[threadIdx.x >> 5];
+    unsigned long long* s_list = s_or + (threadIdx.x >> 5) * kMsBlock;
+    unsigned long long* s_hot = s_or + kMsThreads / 32 * kMsBlock;
     const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    for (uint32_t r = threadIdx.x; r < a.hot; r += kMsThreads) s_hot[r] = __ldcg(a.front + 32ull * r);
+    const uint32_t hot_addr = (uint32_t)__cvta_generic_to_shared(s_hot), hot = a.hot;
+    unsigned long long keep;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
+    auto gather = [&](uint32_t id) {
+        const uint32_t rank = __funnelshift_r(id, id, 5);  // ids that are no multiple of 32 come out large
+        unsigned long long v;
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.lt.u32 p, %1, %2;\n@p ld.shared.u64 %0, [%3];\n"
+            "@!p ld.global.cg.L2::cache_hint.u64 %0, [%4], %5;\n}"
+            : "=l"(v)
+            : "r"(rank), "r"(hot), "r"(hot_addr + 8 * rank), "l"(a.front + id), "l"(keep));
+        return v;
+    };
     const uint64_t run_edges = (uint64_t)kPrBlock << a.shift;
-    for (uint64_t run = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5); run < a.nruns; run += (uint64_t)gridDim.x * 8) {
+    uint32_t ticket = 0;
+    if (lane == 0) ticket = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    while (true) {
+        const uint64_t run = __shfl_sync(0xffffffffu, ticket, 0);
+        if (run >= a.nruns) break;
+        if (lane == 0) ticket = atomicAdd(a.ticket, 1u);
         const uint64_t e_begin = run * run_edges, e_end = min(a.E, e_begin + run_edges);
         uint32_t item = __ldg(a.item_of + (run << a.shift));
         bool open_first = !(__ldg(a.heads + (e_begin >> 5)) & 1u);  // the first list began in an earlier run
@@ -135,14 +164,14 @@ __global__ void __launch_bounds__(256, 5) k_ms_sweep(MsSweepArgs a) {
                 id[4] = y.x; id[5] = y.y; id[6] = y.z; id[7] = y.w;
                 if (a.screen) {
 #pragma unroll
-                    for (int j = 0; j < G; ++j) val[j] = bm_has(a.front_bm, id[j]) ? ld_keep(a.front + id[j]) : 0ull;
+                    for (int j = 0; j < G; ++j) val[j] = bm_has(a.front_bm, id[j]) ? gather(id[j]) : 0ull;
                 } else {
 #pragma unroll
-                    for (int j = 0; j < G; ++j) val[j] = ld_keep(a.front + id[j]);
+                    for (int j = 0; j < G; ++j) val[j] = gather(id[j]);
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < G; ++j) val[j] = e + j < a.E ? ld_keep(a.front + a.adj[e + j]) : 0ull;
+                for (int j = 0; j < G; ++j) val[j] = e + j < a.E ? gather(a.adj[e + j]) : 0ull;
             }
             if (e < a.E) f = __ldcs(reinterpret_cast<const uint8_t*>(a.heads) + e / 8);
             if (e == e_begin) f &= ~1u;  // the run's first edge opens nothing new
@@ -1189,7 +1218,7 @@ int expand_with_ids(eg_graph* g, const uint8_t* rec8_dev, uint64_t E) {
 
 // ---------------------------------------------------------------------------------------------
 struct BatchState {
-    DevBuf a64, b64, c64, lev, rows0, rows1, heavy, tmp_out, seeds, wn_csc, wn_csr, s_out, gA, heavy_sum, ck, seg;
+    DevBuf ticket, a64, b64, c64, lev, rows0, rows1, heavy, tmp_out, seeds, wn_csc, wn_csr, s_out, gA, heavy_sum, ck, seg;
     DevBuf ch0, ch1, flag, level_cnt, entries, n_entries, bm0, bm1, alive, ms_seg;
     DevBuf cap;      // captured level loop: per-level direction decisions and frontier edge counts
     DevBuf persist;  // persistent traversal: per-level counts, barrier words, error flag
@@ -1472,8 +1501,9 @@ __global__ void __launch_bounds__(256, 4) k_msbfs_persistent(MsPersistArgs a) {
 // one dense level as a full sweep (k_ms_sweep)
 static int ms_sweep(eg_graph* g, const uint32_t* adj, const unsigned long long* front, const unsigned long long* front_bm,
                     int screen, unsigned long long* visit, unsigned long long* next, unsigned long long* next_bm,
-                    const unsigned long long* alive, const int* stop) {
+                    const unsigned long long* alive, const int* stop, bool renumbered) {
     EngineState& s = g->eng;
+    BatchState& b = bstate(g);
     if (!g->E) return EG_OK;
     if (g->partitions > 1) {  // a vertex has a list per partition, and sentinel entries lie between them
         MsBfsPullOp op{front, front_bm, screen, visit, next, next_bm, alive, stop};
@@ -1494,8 +1524,12 @@ static int ms_sweep(eg_graph* g, const uint32_t* adj, const unsigned long long* 
     a.next = next;
     a.next_bm = next_bm;
     a.stop = stop;
+    a.hot = renumbered ? std::min(kMsHot, relabel_lines((uint32_t)g->V)) : 0;
+    a.ticket = b.ticket.as<uint32_t>();
     Timed t(&g->prof, g->stream, "msbfs_pull");
-    k_ms_sweep<<<(unsigned)std::min<uint64_t>((a.nruns + 7) / 8, (uint64_t)g->num_sms * 64u), 256, 0, g->stream>>>(a);
+    EG_CUDA(cudaMemsetAsync(a.ticket, 0, 4, g->stream));
+    k_ms_sweep<<<(unsigned)std::min<uint64_t>((a.nruns + kMsThreads / 32 - 1) / (kMsThreads / 32), (uint64_t)g->num_sms),
+                 kMsThreads, kMsSmem, g->stream>>>(a);
     EG_CHECK_LAUNCH("k_ms_sweep");
     return EG_OK;
 }
@@ -1527,7 +1561,11 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
     // pull gathers through the CSC sources renumbered by out-degree class (hot frontier words share
     // cache lines), with a renumbered copy of each frontier; on one graph with the host-driven loop
     const bool renum = one_graph && !(g->use_cuda_graph & 1) && g->batch_launch != 1 && g->E > 0 && want_relabel(g);
-    if (g->E && g->partitions == 1) EG_TRY(setup_list_heads(g, renum));
+    if (g->E && g->partitions == 1) {
+        EG_TRY(setup_list_heads(g, renum));
+        EG_TRY(b.ticket.reserve(16));
+        EG_CUDA(cudaFuncSetAttribute(k_ms_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMsSmem));
+    }
     if (renum) {
         EG_TRY(setup_relabel(g));
         EG_TRY(b.wr0.reserve(8 * V + 8));
@@ -1604,7 +1642,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
                 EG_CHECK_LAUNCH("k_ms_tail");
             } else {
                 EG_TRY(ms_sweep(g, gather_adj, gather_word, bm[c], screen ? 1 : 0, visit, word[x], bm[x],
-                                stop_flag ? alive + 2 : alive + c, stop_flag));
+                                stop_flag ? alive + 2 : alive + c, stop_flag, renum));
             }
             Timed t(&g->prof, g->stream, "msbfs_vertex");
             k_bm_compact<<<grid_for(nwords, 256, grid), 256, 0, g->stream>>>(bm[x], nwords, queue[x], count,
@@ -1777,7 +1815,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
                 {
                     if (st == EG_OK)
                         st = ms_sweep(g, gather_adj, word[c], bm[c], 1, visit, word[x], bm[x], alive + 2,
-                                      &cs->lv[L].skip_direct);
+                                      &cs->lv[L].skip_direct, false);
                     uint32_t* d_nseg = reinterpret_cast<uint32_t*>(cnt + kGraphLevels + 2);
                     ok(cudaMemsetAsync(d_nseg, 0, 4, g->stream));
                     MsBuArgs ma{gather_adj, g->cidx.as<uint64_t>(), g->cvert.as<uint32_t>(), g->ncompressed - 1,

@@ -353,3 +353,28 @@ def test_msbfs_rows_of_any_alignment(eg_lib, V):
                 h = buf.cpu().numpy()
                 assert np.array_equal(h[skip:skip + n * V].reshape(n, V), want[:n]), (n, skip)
                 assert (h[:skip] == 77).all() and (h[skip + n * V:] == 77).all()
+
+
+@pytest.mark.parametrize("V,E", [(31, 400), (64, 900), (3000, 50_000), (300_007, 2_000_003)])
+def test_msbfs_dense_levels_with_hot_sources(eg_lib, V, E):
+    """Dense levels through renumbered sources of very different out-degree: the words of the first ranks
+    come out of shared memory (none, one line's, a table cut short, a full one)."""
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(V)
+    src = (V * rng.random(E) ** 3).astype(np.uint32)
+    dst = rng.integers(0, V, E).astype(np.uint32)
+    dst[: E // 6] = V // 2
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    roots = rng.choice(src, 64).astype(np.uint32)
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        g.set_option(eg.EG_OPT_DENSE_DIVISOR, 1 << 30)
+        levels = {}
+        for relabel in (0, 1, 0):
+            g.set_option(eg.EG_OPT_PR_RELABEL, relabel)
+            levels[relabel], _ = g.msbfs(roots)
+        assert np.array_equal(levels[0], levels[1])
+    for k in (0, 13, 63):
+        ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(roots[k]))
+        got = levels[1][k].astype(np.uint32)
+        assert np.array_equal(np.where(ref == oracle.UNREACHED, 255, ref), got), k
