@@ -115,7 +115,7 @@ int eg_autotune(eg_graph* g, const uint32_t* sample_roots, int nroots, eg_tuning
     out->dense_divisor = best_div;
     out->bfs_ms = best / nb;
 
-    // 2. pull-sweep grid: CTAs per SM (0 = occupancy limit)
+    // 2. pull-sweep grid: CTAs per SM (0 = occupancy limit); the sweeps of one partition do not use it
     const int blocks[] = {0, 1, 2, 3, 4};
     best = 1e30;
     int best_blocks = 0;

@@ -239,8 +239,8 @@ int eg_load_directed_with_ids(eg_graph* g, const void* edges, uint64_t E, uint32
 int eg_ppr(eg_graph* g, const float* weights, const uint32_t* seeds, int nseeds, float alpha, int iterations,
            float* out, int where);
 /* Adjoint of eg_ppr: given dL/dx_iterations (dl_dx[n][V]) writes dL/dw (dl_dw[E], input edge
- * order).  The transposed iteration runs over the CSR; iterates are recomputed from checkpoints
- * stored every ceil(sqrt(iterations)) steps. */
+ * order).  The transposed iteration runs over the CSR; the iterates are kept while they fit an eighth
+ * of the GPU's memory, else recomputed from checkpoints at most ceil(sqrt(iterations)) steps apart. */
 int eg_ppr_backward(eg_graph* g, const float* weights, const uint32_t* seeds, int nseeds, float alpha, int iterations,
                     const float* dl_dx, float* dl_dw, int where);
 
