@@ -534,12 +534,12 @@ __global__ void __launch_bounds__(256) k_levels_out(const unsigned long long* __
 }
 
 template <typename T>
-__global__ void k_transpose_rows(const T* __restrict__ in, uint32_t V, int n, T* __restrict__ out) {
+__global__ void k_transpose_rows(const T* __restrict__ in, uint32_t V, int n, T* __restrict__ out, int width = 64) {
     __shared__ T t[64][33];
     const uint64_t v0 = (uint64_t)blockIdx.x * 32;
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         const uint64_t v = v0 + i;
-        for (int s = threadIdx.x; s < 64; s += blockDim.x) t[s][i] = v < V ? in[v * 64 + s] : T(0);
+        for (int s = threadIdx.x; s < width; s += blockDim.x) t[s][i] = v < V ? in[v * width + s] : T(0);
     }
     __syncthreads();
     for (int s = threadIdx.y; s < n; s += blockDim.y) {
@@ -549,18 +549,18 @@ __global__ void k_transpose_rows(const T* __restrict__ in, uint32_t V, int n, T*
 }
 
 template <typename T>
-__global__ void k_untranspose_rows(const T* __restrict__ in, uint32_t V, int n, T* __restrict__ out) {
+__global__ void k_untranspose_rows(const T* __restrict__ in, uint32_t V, int n, T* __restrict__ out, int width) {
     __shared__ T t[64][33];
     const uint64_t v0 = (uint64_t)blockIdx.x * 32;
-    for (int s = threadIdx.y; s < 64; s += blockDim.y) {
+    for (int s = threadIdx.y; s < width; s += blockDim.y) {
         const uint64_t v = v0 + threadIdx.x;
         t[s][threadIdx.x] = (s < n && v < V) ? in[(uint64_t)s * V + v] : T(0);
     }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         const uint64_t v = v0 + i;
-        for (int s = threadIdx.x; s < 64; s += blockDim.x)
-            if (v < V) out[v * 64 + s] = t[s][i];
+        for (int s = threadIdx.x; s < width; s += blockDim.x)
+            if (v < V) out[v * width + s] = t[s][i];
     }
 }
 
@@ -675,40 +675,66 @@ struct RowArgs {
 // 0.50 (12.9 / 8.2 TB/s of rows; random 256-byte rows out of 256 MB reach 10 TB/s, out of 64 MB 21).
 constexpr int kWalkRows = 16;
 
+// A lane's part of a row: two columns of 64 (float2), one of 32 (float)
 __device__ __forceinline__ float2 ld_row(const float2* a, unsigned long long keep) {
     float2 v;
     asm volatile("ld.global.cg.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(a), "l"(keep));
     return v;
 }
+__device__ __forceinline__ float ld_row(const float* a, unsigned long long keep) {
+    float v;
+    asm volatile("ld.global.cg.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(a), "l"(keep));
+    return v;
+}
+__device__ __forceinline__ void row_zero(float2& a) { a = make_float2(0.f, 0.f); }
+__device__ __forceinline__ void row_zero(float& a) { a = 0.f; }
+__device__ __forceinline__ float2 row_scale(float f, float2 a) { return make_float2(f * a.x, f * a.y); }
+__device__ __forceinline__ float row_scale(float f, float a) { return f * a; }
+__device__ __forceinline__ float2 row_add(float2 acc, float w, float2 a) {
+    return make_float2(fmaf(w, a.x, acc.x), fmaf(w, a.y, acc.y));
+}
+__device__ __forceinline__ float row_add(float acc, float w, float a) { return fmaf(w, a, acc); }
+__device__ __forceinline__ float row_dot(float2 a, float2 b) { return fmaf(a.x, b.x, a.y * b.y); }
+__device__ __forceinline__ float row_dot(float a, float b) { return a * b; }
 
 // acc plus four weighted rows, which are added up by themselves first: a long list's sum takes a quarter of
 // the roundings
+__device__ __forceinline__ float add_four(float acc, const float4& w, float a, float b, float c, float d) {
+    return acc + fmaf(w.w, d, fmaf(w.z, c, fmaf(w.y, b, w.x * a)));
+}
 __device__ __forceinline__ float2 add_four(float2 acc, const float4& w, float2 a, float2 b, float2 c, float2 d) {
-    acc.x += fmaf(w.w, d.x, fmaf(w.z, c.x, fmaf(w.y, b.x, w.x * a.x)));
-    acc.y += fmaf(w.w, d.y, fmaf(w.z, c.y, fmaf(w.y, b.y, w.x * a.y)));
-    return acc;
+    return make_float2(add_four(acc.x, w, a.x, b.x, c.x, d.x), add_four(acc.y, w, a.y, b.y, c.y, d.y));
 }
 
-__device__ __forceinline__ uint2 seeds_at(const uint32_t* seeds, int n, uint32_t lane) {  // of columns 2 lane, 2 lane + 1
+// the seeds of a lane's columns
+__device__ __forceinline__ uint2 seeds_at(const uint32_t* seeds, int n, uint32_t lane, float2) {
     return make_uint2(2 * lane < n ? __ldg(seeds + 2 * lane) : ~0u, 2 * lane + 1 < n ? __ldg(seeds + 2 * lane + 1) : ~0u);
 }
+__device__ __forceinline__ uint2 seeds_at(const uint32_t* seeds, int n, uint32_t lane, float) {
+    return make_uint2(lane < n ? __ldg(seeds + lane) : ~0u, ~0u);
+}
 __device__ __forceinline__ float2 ppr_row(float2 acc, uint32_t v, uint2 seed, float alpha) {
-    float2 r = make_float2((1.0f - alpha) * acc.x, (1.0f - alpha) * acc.y);
+    float2 r = row_scale(1.0f - alpha, acc);
     if (seed.x == v) r.x += alpha;
     if (seed.y == v) r.y += alpha;
     return r;
 }
+__device__ __forceinline__ float ppr_row(float acc, uint32_t v, uint2 seed, float alpha) {
+    const float r = row_scale(1.0f - alpha, acc);
+    return seed.x == v ? r + alpha : r;
+}
 
 // PPR forward: y[v] = (1-a) * sum_{u in in(v)} wn_uv * x[u] + a * e_seed[v]
-__global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __restrict__ x, float2* __restrict__ y,
-                                                  float2* __restrict__ heavy_acc, const uint32_t* __restrict__ seeds, int n_seeds,
+template <class Row>
+__global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const Row* __restrict__ x, Row* __restrict__ y,
+                                                  Row* __restrict__ heavy_acc, const uint32_t* __restrict__ seeds, int n_seeds,
                                                   float alpha) {
     __shared__ __align__(16) uint32_t id[32];
     __shared__ __align__(16) float wt[32];
     __shared__ __align__(16) uint4 task[32];  // end (from the batch's first edge), vertex, slot
     __shared__ __align__(8) uint2 s_seed[32];               // seeds of the lanes' columns
     const uint32_t lane = threadIdx.x;
-    s_seed[lane] = seeds_at(seeds, n_seeds, lane);
+    s_seed[lane] = seeds_at(seeds, n_seeds, lane, Row());
     unsigned long long keep;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
     const uint32_t b = blockIdx.x;
@@ -732,12 +758,13 @@ __global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __
     stage(tasks0);
     uint32_t k = 0, lists = t1 - t + 32;  // of the batch (t is 32 tasks ahead)
     uint32_t end = task[0].x;
-    float2 acc = make_float2(0.f, 0.f);
+    Row acc;
+    row_zero(acc);
     auto finish = [&]() {
         const uint4 cur = task[k];
         if (cur.z == kNoSlot) __stcs(y + (uint64_t)cur.y * 32 + lane, ppr_row(acc, cur.y, s_seed[lane], alpha));
         else atomicAdd(heavy_acc + (uint64_t)cur.z * 32 + lane, acc);
-        acc = make_float2(0.f, 0.f);
+        row_zero(acc);
         if (++k == 32) {
             stage(t + lane < t1 ? __ldg(a.rec + t + lane) : last);
             k = 0;
@@ -756,7 +783,7 @@ __global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __
         }
         const uint32_t left = n - c < 32 ? n - c : 32;
         for (uint32_t s = 0; s < left; s += kWalkRows) {
-            float2 r[kWalkRows];
+            Row r[kWalkRows];
 #pragma unroll
             for (int j = 0; j < kWalkRows; j += 4) {  // past the batch's last edge: row 0, not used
                 const uint4 q = *reinterpret_cast<const uint4*>(id + s + j);
@@ -775,8 +802,7 @@ __global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float qi = i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w;
-                        acc.x = fmaf(qi, r[j + i].x, acc.x);
-                        acc.y = fmaf(qi, r[j + i].y, acc.y);
+                        acc = row_add(acc, qi, r[j + i]);
                         if (at + i + 1 == end) finish();
                     }
                 }
@@ -786,36 +812,37 @@ __global__ void __launch_bounds__(32, 32) k_row_spmm(RowArgs a, const float2* __
 }
 
 // the rows of lists cut into several tasks (seeds null: no teleport), one warp each
+template <class Row>
 __global__ void k_row_heavy_finish(const uint32_t* __restrict__ heavy_vertex, uint32_t nheavy,
-                                   float2* __restrict__ heavy_acc, float2* __restrict__ y, const uint32_t* __restrict__ seeds,
+                                   Row* __restrict__ heavy_acc, Row* __restrict__ y, const uint32_t* __restrict__ seeds,
                                    int n_seeds, float alpha) {
     const uint32_t slot = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (slot >= nheavy) return;
     const uint32_t v = heavy_vertex[slot];
-    float2* p = heavy_acc + (uint64_t)slot * 32 + lane;
-    y[(uint64_t)v * 32 + lane] = ppr_row(*p, v, seeds_at(seeds, n_seeds, lane), alpha);
-    *p = make_float2(0.f, 0.f);
+    Row* p = heavy_acc + (uint64_t)slot * 32 + lane;
+    y[(uint64_t)v * 32 + lane] = ppr_row(*p, v, seeds_at(seeds, n_seeds, lane, Row()), alpha);
+    row_zero(*p);
 }
 
 // Seeds without in-edges: the sweeps leave their rows as they are, a at the seed's column, in nbuf
 // consecutive row arrays.
 __global__ void k_ppr_lone_seeds(const uint32_t* __restrict__ seeds, int n, const uint32_t* __restrict__ indeg,
-                                 float* __restrict__ rows, uint64_t V, int nbuf, float alpha) {
+                                 float* __restrict__ rows, uint64_t V, int nbuf, float alpha, int width) {
     const int s = threadIdx.x & 63;
     if (s >= n || indeg[seeds[s]]) return;
-    for (int b = blockIdx.x; b < nbuf; b += gridDim.x) rows[((uint64_t)b * V + seeds[s]) * 64 + s] = alpha;
+    for (int b = blockIdx.x; b < nbuf; b += gridDim.x) rows[((uint64_t)b * V + seeds[s]) * width + s] = alpha;
 }
-__global__ void k_ppr_init(const uint32_t* seeds, int n, float* x) {
+__global__ void k_ppr_init(const uint32_t* seeds, int n, float* x, int width) {
     const int s = threadIdx.x;
-    if (s < n) x[(uint64_t)seeds[s] * 64 + s] = 1.0f;
+    if (s < n) x[(uint64_t)seeds[s] * width + s] = 1.0f;
 }
 // zero the rows that no sweep writes (deg = 0) in nbuf consecutive row arrays
 __global__ void __launch_bounds__(256) k_zero_rows(const uint32_t* __restrict__ deg, uint64_t V, float4* __restrict__ rows,
-                                                   int nbuf) {
+                                                   int nbuf, int parts) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V * 16; i += stride) {
-        if (deg[i >> 4]) continue;
-        for (int b = 0; b < nbuf; ++b) __stcs(rows + (uint64_t)b * V * 16 + i, make_float4(0.f, 0.f, 0.f, 0.f));
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V * parts; i += stride) {
+        if (deg[i / (uint32_t)parts]) continue;
+        for (int b = 0; b < nbuf; ++b) __stcs(rows + (uint64_t)b * V * parts + i, make_float4(0.f, 0.f, 0.f, 0.f));
     }
 }
 
@@ -885,29 +912,30 @@ __global__ void k_gather_norm_w(const uint32_t* __restrict__ nbr_is_src, const f
 // kept in FP64: an edge's gradient is what is left of its gA minus the mean over the source's edges,
 // and the roundings of K steps were most of its error (K = 50, 1 M / 16 M, two seeds: 1.1e-6 and
 // 8.5e-7 with FP32 sums, 7.9e-7 and 5.4e-7 so, for 24.9 instead of 23.6 ms of sweeps).
-__device__ __forceinline__ float dot_scatter(float2 (&d)[kWalkRows], uint32_t lane) {
+__device__ __forceinline__ float dot_scatter(float (&d)[kWalkRows], uint32_t lane) {
     static_assert(kWalkRows == 16, "the four halving stages below leave one product of sixteen per lane pair");
 #pragma unroll
     for (int o = 16, m = 8; o >= 2; o >>= 1, m >>= 1) {
         const bool up = (lane & o) != 0;
 #pragma unroll
         for (int j = 0; j < m; ++j) {
-            const float give = up ? d[j].x : d[j + m].x, keep = up ? d[j + m].x : d[j].x;
-            d[j].x = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            const float give = up ? d[j] : d[j + m], keep = up ? d[j + m] : d[j];
+            d[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
     }
-    return d[0].x + __shfl_xor_sync(0xffffffffu, d[0].x, 1);
+    return d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
 }
 
 // 28 warps per SM (72 registers): 32 (64, spilled) 28.5 ms for 50 sweeps, 24 27.5, 28 25.4.
-__global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2* __restrict__ lam_in,
-                                                     const float2* __restrict__ xk, float2* __restrict__ lam_out,
-                                                     float2* __restrict__ heavy_acc, double* __restrict__ gA,
+template <class Row>
+__global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const Row* __restrict__ lam_in,
+                                                     const Row* __restrict__ xk, Row* __restrict__ lam_out,
+                                                     Row* __restrict__ heavy_acc, double* __restrict__ gA,
                                                      float scale) {
     __shared__ __align__(16) uint32_t id[32];
     __shared__ __align__(16) float wt[32];
     __shared__ __align__(16) uint4 task[16];      // ring of 16: end, vertex, slot
-    __shared__ __align__(16) float2 src[16][32];  // and their rows of x_k
+    __shared__ __align__(16) Row src[16][32];  // and their rows of x_k
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long keep;
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 0.5;" : "=l"(keep));
@@ -923,13 +951,14 @@ __global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2*
     const uint32_t n = (uint32_t)(task_begin(last) - e0) + task_len(last);
     auto stage = [&](const uint4& r, uint32_t slot) {  // 8 tasks (lanes 0..7) into the ring, their rows on the way
         if (lane < 8) task[slot + lane] = make_uint4((uint32_t)(task_begin(r) - e0) + task_len(r), r.z, r.w, 0u);
+        constexpr uint32_t kLanes = 2 * sizeof(Row), kPart = 16 / sizeof(Row);  // lanes per row, 16 bytes each
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t q = 2 * i + (lane >> 4), v = __shfl_sync(0xffffffffu, r.z, q);
+        for (int i = 0; i < 8 * kLanes / 32; ++i) {
+            const uint32_t q = 32 / kLanes * i + lane / kLanes, v = __shfl_sync(0xffffffffu, r.z, q);
             if (__shfl_sync(0xffffffffu, task_len(r), q))
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(&src[slot + q][2 * (lane & 15)])),
-                             "l"(xk + (uint64_t)v * 32 + 2 * (lane & 15))
+                                 (uint32_t)__cvta_generic_to_shared(&src[slot + q][kPart * (lane % kLanes)])),
+                             "l"(xk + (uint64_t)v * 32 + kPart * (lane % kLanes))
                              : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -944,12 +973,14 @@ __global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2*
     stage(tasks8, 8);
     __syncwarp();
     uint32_t k = 0, end = task[0].x;
-    float2 xu = make_float2(0.f, 0.f), acc = make_float2(0.f, 0.f);
+    Row xu, acc;
+    row_zero(xu);
+    row_zero(acc);
     auto finish = [&]() {
         const uint4 cur = task[k & 15];
-        if (cur.z == kNoSlot) __stcs(lam_out + (uint64_t)cur.y * 32 + lane, make_float2(scale * acc.x, scale * acc.y));
+        if (cur.z == kNoSlot) __stcs(lam_out + (uint64_t)cur.y * 32 + lane, row_scale(scale, acc));
         else atomicAdd(heavy_acc + (uint64_t)cur.z * 32 + lane, acc);
-        acc = make_float2(0.f, 0.f);
+        row_zero(acc);
         ++k;
         if (!(k & 7)) {  // the finished eight make room
             __syncwarp();
@@ -975,7 +1006,8 @@ __global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2*
         for (uint32_t s = 0; s < left; s += kWalkRows) {
             const bool have = !(lane & 1) && s + (lane >> 1) < left;
             const double g_old = have ? g[c + s] : 0.0;
-            float2 l[kWalkRows];
+            Row l[kWalkRows];
+            float d[kWalkRows];
 #pragma unroll
             for (int j = 0; j < kWalkRows; j += 4) {  // past the batch's last edge: row 0, not used
                 const uint4 q = *reinterpret_cast<const uint4*>(id + s + j);
@@ -996,20 +1028,18 @@ __global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const float2*
                 if (at + 4 < end) {  // no list ends here
                     acc = add_four(acc, q, l[j], l[j + 1], l[j + 2], l[j + 3]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) l[j + i].x = fmaf(xu.x, l[j + i].x, xu.y * l[j + i].y);
+                    for (int i = 0; i < 4; ++i) d[j + i] = row_dot(xu, l[j + i]);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float qi = i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w;
-                        const float2 r = l[j + i];
-                        acc.x = fmaf(qi, r.x, acc.x);
-                        acc.y = fmaf(qi, r.y, acc.y);
-                        l[j + i].x = fmaf(xu.x, r.x, xu.y * r.y);
+                        acc = row_add(acc, qi, l[j + i]);
+                        d[j + i] = row_dot(xu, l[j + i]);
                         if (at + i + 1 == end) finish();
                     }
                 }
             }
-            const float dot = dot_scatter(l, lane);
+            const float dot = dot_scatter(d, lane);
             if (have) g[c + s] = fma((double)scale, (double)dot, g_old);
         }
     }
@@ -2051,18 +2081,44 @@ static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev, bool want_csr
 
 // one forward step: y = a*e + (1-a) A^T x.  Rows of y without in-edges are as the caller left them: zero,
 // and `a` at a seed's own column (lone_seeds).
-static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
+template <class Row>
+static int ppr_step_as(eg_graph* g, const float* x, float* y, float alpha, int n) {
     BatchState& b = bstate(g);
     const RowTasks& t = b.csc_tasks;
     RowArgs a = row_args(t, g->csc_adj.as<uint32_t>(), b.wn_csc.as<float>());
     Timed tm(&g->prof, g->stream, "ppr_spmm");
-    k_row_spmm<<<t.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<const float2*>(x), reinterpret_cast<float2*>(y),
-                                                  b.heavy.as<float2>(), b.seeds.as<uint32_t>(), n, alpha);
+    k_row_spmm<Row><<<t.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<const Row*>(x), reinterpret_cast<Row*>(y),
+                                                  b.heavy.as<Row>(), b.seeds.as<uint32_t>(), n, alpha);
     EG_CHECK_LAUNCH("k_row_spmm");
     if (t.nheavy) {
-        k_row_heavy_finish<<<(unsigned)((t.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
-            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<float2>(), reinterpret_cast<float2*>(y),
+        k_row_heavy_finish<Row><<<(unsigned)((t.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
+            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<Row>(), reinterpret_cast<Row*>(y),
             b.seeds.as<uint32_t>(), n, alpha);
+        EG_CHECK_LAUNCH("k_row_heavy_finish");
+    }
+    return EG_OK;
+}
+// Columns of a row: 32 for up to 32 seeds, which halves what the sweeps gather, else 64.  A step of 20
+// iterations on 1 M / 16 M: 25.3 -> 20.5 ms with 32 seeds, 20.9 -> 17.5 with one.
+static int row_width(int n) { return n <= 32 ? 32 : 64; }
+static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
+    return row_width(n) == 32 ? ppr_step_as<float>(g, x, y, alpha, n) : ppr_step_as<float2>(g, x, y, alpha, n);
+}
+template <class Row>
+static int adjoint_step(eg_graph* g, const float* lam, const float* xk, float* lam2, float alpha) {
+    BatchState& b = bstate(g);
+    const RowTasks& t = b.csr_tasks;
+    RowArgs a = row_args(t, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
+    {
+        Timed tm(&g->prof, g->stream, "ppr_adjoint");
+        k_row_adjoint<Row><<<t.nbatches, 32, 0, g->stream>>>(
+            a, reinterpret_cast<const Row*>(lam), reinterpret_cast<const Row*>(xk), reinterpret_cast<Row*>(lam2),
+            b.heavy.as<Row>(), b.gA.as<double>(), 1.0f - alpha);
+        EG_CHECK_LAUNCH("k_row_adjoint");
+    }
+    if (t.nheavy) {
+        k_row_heavy_finish<Row><<<(unsigned)((t.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
+            t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy.as<Row>(), reinterpret_cast<Row*>(lam2), nullptr, 0, alpha);
         EG_CHECK_LAUNCH("k_row_heavy_finish");
     }
     return EG_OK;
@@ -2071,7 +2127,7 @@ static int ppr_step(eg_graph* g, const float* x, float* y, float alpha, int n) {
 static int lone_seeds(eg_graph* g, float* rows, int nbuf, int n, float alpha) {
     if (nbuf < 1) return EG_OK;
     k_ppr_lone_seeds<<<std::min(nbuf, 64), 64, 0, g->stream>>>(bstate(g).seeds.as<uint32_t>(), n, g->indeg.as<uint32_t>(), rows,
-                                                               g->V, nbuf, alpha);
+                                                               g->V, nbuf, alpha, row_width(n));
     EG_CHECK_LAUNCH("k_ppr_lone_seeds");
     return EG_OK;
 }
@@ -2186,11 +2242,12 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
         EG_CUDA(cudaStreamSynchronize(g->stream));
         return run_ppr_single(g, seed, alpha, K, out, where);
     }
+    const int W = row_width(n);
     float* x = b.rows0.as<float>();
     float* y = b.rows1.as<float>();
-    EG_CUDA(cudaMemsetAsync(x, 0, 256 * V, g->stream));
-    EG_CUDA(cudaMemsetAsync(y, 0, 256 * V, g->stream));
-    k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, x);
+    EG_CUDA(cudaMemsetAsync(x, 0, 4ull * W * V, g->stream));
+    EG_CUDA(cudaMemsetAsync(y, 0, 4ull * W * V, g->stream));
+    k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, x, W);
     EG_CHECK_LAUNCH("k_ppr_init");
     for (int k = 0; k < K; ++k) {
         if (k < 2) EG_TRY(lone_seeds(g, y, 1, n, alpha));  // x_0 itself has 1 there
@@ -2204,7 +2261,7 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
             dst = b.tmp_out.as<float>();
         }
         dim3 blk(32, 8);
-        k_transpose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(x, (uint32_t)V, n, dst);
+        k_transpose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(x, (uint32_t)V, n, dst, W);
         EG_CHECK_LAUNCH("k_transpose_rows");
         if (where != EG_DEVICE) EG_CUDA(cudaMemcpyAsync(out, dst, 4ull * n * V, cudaMemcpyDeviceToHost, g->stream));
     }
@@ -2226,10 +2283,10 @@ static int ppr_stride(int K, uint64_t row, uint64_t budget) {
     return C;
 }
 
-static int zero_rows(eg_graph* g, const uint32_t* deg, float* rows, int nbuf) {
+static int zero_rows(eg_graph* g, const uint32_t* deg, float* rows, int nbuf, int width) {
     if (nbuf < 1) return EG_OK;
-    k_zero_rows<<<grid_for(16ull * g->V, 256, (unsigned)g->num_sms * 16u), 256, 0, g->stream>>>(
-        deg, g->V, reinterpret_cast<float4*>(rows), nbuf);
+    k_zero_rows<<<grid_for(width / 4 * (uint64_t)g->V, 256, (unsigned)g->num_sms * 16u), 256, 0, g->stream>>>(
+        deg, g->V, reinterpret_cast<float4*>(rows), nbuf, width / 4);
     EG_CHECK_LAUNCH("k_zero_rows");
     return EG_OK;
 }
@@ -2242,7 +2299,8 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     if (!dl_dx || !dl_dw) { set_error("eg_ppr_backward: need dL/dx and the dL/dw output"); return EG_ERR_INVALID; }
     BatchState& b = bstate(g);
     const uint64_t V = g->V, E = g->E, Ein = g->E_input;
-    const size_t row = 256 * V;
+    const int W = row_width(n);
+    const size_t row = 4ull * W * V;
     if (!b.device_bytes) {
         size_t free_bytes = 0;
         EG_CUDA(cudaMemGetInfo(&free_bytes, &b.device_bytes));
@@ -2263,15 +2321,15 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     const uint32_t* indeg = g->indeg.as<uint32_t>();
     const uint32_t* outdeg = g->outdeg.as<uint32_t>();
     EG_CUDA(cudaMemsetAsync(ck, 0, row, g->stream));
-    k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, ck);
+    k_ppr_init<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, ck, W);
     EG_CHECK_LAUNCH("k_ppr_init");
     if (C == 1) {
-        EG_TRY(zero_rows(g, indeg, ck + 64 * V, K - 1));
-        EG_TRY(lone_seeds(g, ck + 64 * V, K - 1, n, alpha));
-        for (int k = 0; k + 1 < K; ++k) EG_TRY(ppr_step(g, ck + 64 * V * k, ck + 64 * V * (k + 1), alpha, n));
+        EG_TRY(zero_rows(g, indeg, ck + W * V, K - 1, W));
+        EG_TRY(lone_seeds(g, ck + W * V, K - 1, n, alpha));
+        for (int k = 0; k + 1 < K; ++k) EG_TRY(ppr_step(g, ck + W * V * k, ck + W * V * (k + 1), alpha, n));
     } else {
-        EG_TRY(zero_rows(g, indeg, seg, C));
-        EG_TRY(lone_seeds(g, seg + 64 * V, C - 1, n, alpha));
+        EG_TRY(zero_rows(g, indeg, seg, C, W));
+        EG_TRY(lone_seeds(g, seg + W * V, C - 1, n, alpha));
         float* x = b.rows0.as<float>();
         float* y = b.rows1.as<float>();
         EG_CUDA(cudaMemcpyAsync(x, ck, row, cudaMemcpyDeviceToDevice, g->stream));
@@ -2296,39 +2354,27 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
             src = b.tmp_out.as<float>();
         }
         dim3 blk(32, 8);
-        k_untranspose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(src, (uint32_t)V, n, lam);
+        k_untranspose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(src, (uint32_t)V, n, lam, W);
         EG_CHECK_LAUNCH("k_untranspose_rows");
     }
     EG_CUDA(cudaMemsetAsync(b.gA.ptr, 0, 8 * E, g->stream));
     const RowTasks& tr = b.csr_tasks;
-    RowArgs ar = row_args(tr, g->csr_adj.as<uint32_t>(), b.wn_csr.as<float>());
     // the sweeps write only rows with out-edges; the others are zero from lambda_{K-1} on
-    EG_TRY(zero_rows(g, outdeg, lam2, 1));
+    EG_TRY(zero_rows(g, outdeg, lam2, 1, W));
     for (int cp = (K - 1) / C; cp >= 0 && K > 0; --cp) {
         const int k0 = cp * C, k1 = std::min(K, k0 + C);
-        const float* xs = ck + 64 * V * cp;  // x_k0 .. x_{k1-1}
+        const float* xs = ck + W * V * cp;  // x_k0 .. x_{k1-1}
         if (C > 1) {  // recomputed into the segment buffer
             EG_CUDA(cudaMemcpyAsync(seg, xs, row, cudaMemcpyDeviceToDevice, g->stream));
             for (int k = k0 + 1; k < k1; ++k)
-                EG_TRY(ppr_step(g, seg + (size_t)(k - 1 - k0) * 64 * V, seg + (size_t)(k - k0) * 64 * V, alpha, n));
+                EG_TRY(ppr_step(g, seg + (size_t)(k - 1 - k0) * W * V, seg + (size_t)(k - k0) * W * V, alpha, n));
             xs = seg;
         }
         for (int k = k1 - 1; k >= k0; --k) {
             // lam holds lambda_{k+1}; gA += (1-a) <x_k[u], lam[v]>; lam2 = (1-a) A lam
-            {
-                Timed tm(&g->prof, g->stream, "ppr_adjoint");
-                k_row_adjoint<<<tr.nbatches, 32, 0, g->stream>>>(
-                    ar, reinterpret_cast<const float2*>(lam), reinterpret_cast<const float2*>(xs + (size_t)(k - k0) * 64 * V),
-                    reinterpret_cast<float2*>(lam2), b.heavy.as<float2>(), b.gA.as<double>(), 1.0f - alpha);
-                EG_CHECK_LAUNCH("k_row_adjoint");
-            }
-            if (tr.nheavy) {
-                k_row_heavy_finish<<<(unsigned)((tr.nheavy * 32ull + 255) / 256), 256, 0, g->stream>>>(
-                    tr.heavy_vertex.as<uint32_t>(), tr.nheavy, b.heavy.as<float2>(), reinterpret_cast<float2*>(lam2),
-                    nullptr, 0, alpha);
-                EG_CHECK_LAUNCH("k_row_heavy_finish");
-            }
-            if (k == K - 1) EG_TRY(zero_rows(g, outdeg, lam, 1));  // dL/dx_K itself is no longer needed
+            const float* xk = xs + (size_t)(k - k0) * W * V;
+            EG_TRY(W == 32 ? adjoint_step<float>(g, lam, xk, lam2, alpha) : adjoint_step<float2>(g, lam, xk, lam2, alpha));
+            if (k == K - 1) EG_TRY(zero_rows(g, outdeg, lam, 1, W));  // dL/dx_K itself is no longer needed
             std::swap(lam, lam2);
         }
     }

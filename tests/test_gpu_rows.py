@@ -205,3 +205,9 @@ def test_sssp_batch_walk_over_lists(eg_lib, V, E, shape):
     for s in range(len(sources)):
         ref = oracle.sssp(csr["off"][0], csr["adj"], csr["w"], V, int(sources[s]))
         assert np.array_equal(dist[s].view(np.uint32), ref.view(np.uint32)), s
+
+
+@pytest.mark.parametrize("n", [31, 32, 33])
+def test_ppr_row_widths(eg_lib, n):
+    """Rows of 32 columns for up to 32 seeds, of 64 for more."""
+    test_ppr_and_adjoint_list_lengths(eg_lib, n, 3)
