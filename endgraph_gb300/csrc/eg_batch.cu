@@ -1089,10 +1089,26 @@ __global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ t
 // offset arrays; a task at a time, rows by half-warps, tasks by stride 47.5 ms, in batches with a
 // warp per CTA 39.7; the walk 28.8 (10.8 E row gathers: 8.9 TB/s) at 32 warps per SM, 30.5 at 28,
 // 33.7 at 24.
+__device__ __forceinline__ float relaxed(float best, float msg, float w) { return fminf(best, msg + w); }  // toolkits/sssp.cpp:55
+__device__ __forceinline__ float2 relaxed(float2 best, float2 msg, float w) {
+    return make_float2(relaxed(best.x, msg.x, w), relaxed(best.y, msg.y, w));
+}
+__device__ __forceinline__ bool lower(float a, float b) { return a < b; }
+__device__ __forceinline__ bool lower(float2 a, float2 b) { return a.x < b.x || a.y < b.y; }
+// distances are >= 0: ordered like their bits
+__device__ __forceinline__ bool lower_atomic(float* p, float a, float b) {
+    return a < b && a < __int_as_float(atomicMin(reinterpret_cast<int*>(p), __float_as_int(a)));
+}
+__device__ __forceinline__ bool lower_atomic(float2* p, float2 a, float2 b) {
+    const bool x = lower_atomic(&p->x, a.x, b.x), y = lower_atomic(&p->y, a.y, b.y);
+    return x || y;
+}
+
 constexpr int kSsspRows = 16;
 constexpr uint32_t kDestRow = 1u << 31;  // queue entry: the list's own row
 
-__global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float2* __restrict__ dist,
+template <class Row>
+__global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, Row* __restrict__ dist,
                                                      const uint32_t* __restrict__ changed_prev,
                                                      uint32_t* __restrict__ changed_next, int shared_vertex,
                                                      int* __restrict__ any) {
@@ -1114,19 +1130,18 @@ __global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float2* __restri
     uint32_t queued = 0;
     uint32_t q_task = ~0u;     // task of the last queued source
     uint32_t cur = ~0u;        // task whose row is being reduced
-    float2 dv = make_float2(0.f, 0.f), best = dv;
+    Row dv, best;
+    row_zero(dv);
+    row_zero(best);
     auto flush = [&]() {
-        bool low = best.x < dv.x || best.y < dv.y;
+        bool low = lower(best, dv);
         if (cur == ~0u || !__any_sync(0xffffffffu, low)) return;
         const uint2 tk = s_task[cur];
-        float2* row = dist + (uint64_t)tk.x * 32;
+        Row* row = dist + (uint64_t)tk.x * 32;
         if (tk.y == kNoSlot && !shared_vertex) {
             if (low) __stcg(row, best);
-        } else {  // distances are >= 0: ordered like their bits
-            int* p = reinterpret_cast<int*>(row);
-            low = false;
-            if (best.x < dv.x) low |= best.x < __int_as_float(atomicMin(p, __float_as_int(best.x)));
-            if (best.y < dv.y) low |= best.y < __int_as_float(atomicMin(p + 1, __float_as_int(best.y)));
+        } else {
+            low = lower_atomic(row, best, dv);
             if (!__any_sync(0xffffffffu, low)) return;
         }
         if (lane == 0) atomicOr(changed_next + (tk.x >> 5), 1u << (tk.x & 31));
@@ -1135,7 +1150,7 @@ __global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float2* __restri
     auto reduce = [&](uint32_t base, uint32_t m) {  // entries [base, base + m) of the queue, m <= kSsspRows
         const uint32_t qe = lane < m ? q_edge[base + lane] : kDestRow;
         const float wl = qe & kDestRow ? 0.f : __ldg(wts + qe);
-        float2 r[kSsspRows];
+        Row r[kSsspRows];
 #pragma unroll
         for (int j = 0; j < kSsspRows; j += 4) {
             const uint4 q = *reinterpret_cast<const uint4*>(q_row + base + j);
@@ -1153,9 +1168,8 @@ __global__ void __launch_bounds__(32, 32) k_row_sssp(RowArgs a, float2* __restri
                 flush();
                 cur = e ^ kDestRow;
                 dv = best = r[j];
-            } else {  // toolkits/sssp.cpp:55: relax_dist = msg + w
-                best.x = fminf(best.x, r[j].x + w);
-                best.y = fminf(best.y, r[j].y + w);
+            } else {
+                best = relaxed(best, r[j], w);
             }
         }
     };
@@ -2402,19 +2416,27 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-__global__ void k_sssp_init_entries(const uint2* ent, uint32_t n, float* dist, uint32_t* changed) {
+__global__ void k_sssp_init_entries(const uint2* ent, uint32_t n, float* dist, int width, uint32_t* changed) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        dist[(uint64_t)ent[i].x * 64 + ent[i].y] = 0.f;
+        dist[(uint64_t)ent[i].x * width + ent[i].y] = 0.f;
         atomicOr(changed + (ent[i].x >> 5), 1u << (ent[i].x & 31));
     }
 }
 
-// Bellman-Ford sweeps from the root entries in b.entries; leaves dist [V][64] in b.rows0
-static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
+// Bellman-Ford sweeps from the root entries in b.entries; leaves dist [V][row_width(n)] in b.rows0
+// [V][32] rows -> [V][64], the columns past 32 unreached
+__global__ void __launch_bounds__(256) k_widen_rows(const float* __restrict__ in, uint64_t V, float* __restrict__ out) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 64 * V; i += (uint64_t)gridDim.x * blockDim.x)
+        out[i] = i & 32 ? 1e9f : __ldcs(in + (i >> 6) * 32 + (i & 31));
+}
+
+// n: sources per row (32 columns for up to 32, which halves what the sweeps gather, else 64)
+static int sssp_core(eg_graph* g, int n, uint32_t n_entries, int* sweeps_out) {
+    const int W = row_width(n);
     EG_TRY(ensure_tasks(g, false));
     BatchState& b = bstate(g);
     const uint64_t V = g->V;
-    EG_TRY(b.rows0.reserve(256 * V + 256));
+    EG_TRY(b.rows0.reserve(4ull * W * V + 256));
     const size_t ch_bytes = 4 * (V / 32 + 1);  // one bit per vertex: changed in the last sweep
     EG_TRY(b.ch0.reserve(ch_bytes));
     EG_TRY(b.ch1.reserve(ch_bytes));
@@ -2422,11 +2444,11 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
     float* dist = b.rows0.as<float>();
     {
         Timed t(&g->prof, g->stream, "sssp_batch_init");
-        k_fill_f32_rows<<<grid_for(64 * V, 256, 152u * 16u), 256, 0, g->stream>>>(dist, 64 * V, 1e9f);
+        k_fill_f32_rows<<<grid_for(W * V, 256, 152u * 16u), 256, 0, g->stream>>>(dist, W * V, 1e9f);
         EG_CHECK_LAUNCH("k_fill_f32_rows");
         EG_CUDA(cudaMemsetAsync(b.ch0.ptr, 0, ch_bytes, g->stream));
         k_sssp_init_entries<<<std::max(1u, std::min<unsigned>((n_entries + 255) / 256, 4096u)), 256, 0, g->stream>>>(
-            b.entries.as<uint2>(), n_entries, dist, b.ch0.as<uint32_t>());
+            b.entries.as<uint2>(), n_entries, dist, W, b.ch0.as<uint32_t>());
         EG_CHECK_LAUNCH("k_sssp_init_entries");
     }
     RowArgs a = row_args(b.csc_tasks, g->csc_adj.as<uint32_t>(), g->csc_w.as<float>());
@@ -2438,8 +2460,11 @@ static int sssp_core(eg_graph* g, uint32_t n_entries, int* sweeps_out) {
         EG_CUDA(cudaMemsetAsync(b.flag.ptr, 0, 4, g->stream));
         {
             Timed t(&g->prof, g->stream, "sssp_batch_sweep");
-            k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<float2*>(dist), prev, nxt,
-                                                          g->partitions > 1, b.flag.as<int>());
+            if (W == 32)
+                k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, dist, prev, nxt, g->partitions > 1, b.flag.as<int>());
+            else
+                k_row_sssp<<<b.csc_tasks.nbatches, 32, 0, g->stream>>>(a, reinterpret_cast<float2*>(dist), prev, nxt,
+                                                                      g->partitions > 1, b.flag.as<int>());
             EG_CHECK_LAUNCH("k_row_sssp");
         }
         ++sweeps;
@@ -2469,7 +2494,7 @@ int run_sssp_batch(eg_graph* g, const uint32_t* srcs, int n, float* out, int whe
     k_root_entries<<<1, 64, 0, g->stream>>>(b.seeds.as<uint32_t>(), n, 0, b.entries.as<uint2>());
     EG_CHECK_LAUNCH("k_root_entries");
     int sweeps = 0;
-    EG_TRY(sssp_core(g, (uint32_t)n, &sweeps));
+    EG_TRY(sssp_core(g, n, (uint32_t)n, &sweeps));
     if (out) {
         float* dst = out;
         if (where != EG_DEVICE) {
@@ -2477,7 +2502,8 @@ int run_sssp_batch(eg_graph* g, const uint32_t* srcs, int n, float* out, int whe
             dst = b.tmp_out.as<float>();
         }
         dim3 blk(32, 8);
-        k_transpose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(b.rows0.as<float>(), (uint32_t)V, n, dst);
+        k_transpose_rows<float><<<(unsigned)((V + 31) / 32), blk, 0, g->stream>>>(b.rows0.as<float>(), (uint32_t)V, n, dst,
+                                                                                  row_width(n));
         EG_CHECK_LAUNCH("k_transpose_rows");
         if (where != EG_DEVICE) EG_CUDA(cudaMemcpyAsync(out, dst, 4ull * n * V, cudaMemcpyDeviceToHost, g->stream));
     }
@@ -2560,9 +2586,21 @@ int run_sssp_graphs(eg_graph* g, const uint32_t* sources, int nper, float* dist,
     uint32_t n = 0;
     EG_TRY(graph_roots(g, sources, nper, where, "eg_sssp_graphs", &n));
     int sweeps = 0;
-    EG_TRY(sssp_core(g, n, &sweeps));
-    if (dist)
-        EG_CUDA(cudaMemcpyAsync(dist, bstate(g).rows0.ptr, 256ull * g->V,
+    EG_TRY(sssp_core(g, nper, n, &sweeps));
+    BatchState& b = bstate(g);
+    const float* rows = b.rows0.as<float>();
+    if (dist && row_width(nper) == 32) {
+        float* wide = dist;
+        if (where != EG_DEVICE) {
+            EG_TRY(b.tmp_out.reserve(256ull * g->V + 64));
+            wide = b.tmp_out.as<float>();
+        }
+        k_widen_rows<<<grid_for(64ull * g->V, 256, 152u * 32u), 256, 0, g->stream>>>(rows, g->V, wide);
+        EG_CHECK_LAUNCH("k_widen_rows");
+        rows = wide;
+    }
+    if (dist && rows != dist)
+        EG_CUDA(cudaMemcpyAsync(dist, rows, 256ull * g->V,
                                 where == EG_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, g->stream));
     EG_CUDA(cudaStreamSynchronize(g->stream));
     g->last_iterations = sweeps;

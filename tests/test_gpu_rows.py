@@ -211,3 +211,35 @@ def test_sssp_batch_walk_over_lists(eg_lib, V, E, shape):
 def test_ppr_row_widths(eg_lib, n):
     """Rows of 32 columns for up to 32 seeds, of 64 for more."""
     test_ppr_and_adjoint_list_lengths(eg_lib, n, 3)
+
+
+@pytest.mark.parametrize("per", [1, 31, 32, 33])
+def test_sssp_graphs_row_widths(eg_lib, per):
+    """Distances of a batch come as rows of 64 columns whatever width the sweeps used, on the host and on the
+    device; columns past the last source are unreached."""
+    import torch
+
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(per)
+    sizes, edges = [700, 33, 2000], [5000, 40, 30_000]
+    graphs = [(rng.integers(0, v, e).astype(np.uint32), rng.integers(0, v, e).astype(np.uint32),
+               rng.random(e).astype(np.float32)) for v, e in zip(sizes, edges)]
+    rec = np.concatenate([eg.pack_edges(s, d, w) for s, d, w in graphs])
+    eoff = np.cumsum([0] + edges).astype(np.uint64)
+    V = sum(sizes)
+    sources = np.concatenate([rng.integers(0, v, per) for v in sizes]).astype(np.uint32)
+    want = np.full((V, 64), 1e9, np.float32)
+    at = 0
+    for k, (s, d, w) in enumerate(graphs):
+        csr = oracle.build_csr(s, d, w, sizes[k], np.array([0, sizes[k]], np.uint32))
+        for j in range(per):
+            want[at:at + sizes[k], j] = oracle.sssp(csr["off"][0], csr["adj"], csr["w"], sizes[k], int(sources[k * per + j]))
+        at += sizes[k]
+    with eg.Graph() as g:
+        g.load_graph_batch(rec, eoff, np.array(sizes, np.uint32))
+        assert np.array_equal(g.sssp_graphs(sources, per), want)
+        buf = torch.zeros(64 * V + 3, device="cuda")
+        for skip in (0, 1, 3):
+            out = buf[skip:skip + 64 * V].view(V, 64)
+            g.sssp_graphs(sources, per, dist=out)
+            assert np.array_equal(out.cpu().numpy(), want), skip
