@@ -3,18 +3,18 @@
 //
 //  * eg_msbfs: bit-parallel BFS from up to 64 roots.  Every vertex keeps a u64 of the roots that
 //    reached it and a u64 of the roots whose frontier it is in; a level either pushes the queued
-//    frontier's words along the CSR or is one chunked pull over the CSC that ORs the
-//    in-neighbours' frontier words (exact integer work, levels identical to 64 separate BFS runs).
-//  * 64-column row engine: a destination's 64 values (one per seed / source) sit in one 256-byte
-//    row; one warp reduces a task of <= kTaskEdges in-edges, each lane owning two columns, so every
-//    gathered row is a single coalesced 256-byte read.  Lists longer than a task are split and
-//    their partial rows combined in a small per-heavy-vertex buffer.  Used by
+//    frontier's words along the CSR or is one sweep over the CSC that ORs the in-neighbours'
+//    frontier words (exact integer work, levels identical to 64 separate BFS runs).
+//  * row engine: a destination's 64 values (one per seed / source) sit in one 256-byte row, up to 32
+//    in one of 128; a warp walks the edges of a batch of lists and reads a whole row per edge, each
+//    lane owning its columns.  Lists longer than a task (kTaskEdges) are split and their partial
+//    rows combined in a small per-heavy-vertex buffer.  Used by
 //      - eg_ppr: personalised PageRank x_{k+1} = a*e_seed + (1-a) * A^T x_k, A = row-normalised
 //        edge weights, FP32;
 //      - eg_ppr_backward: the adjoint of K unrolled iterations.  lambda_k = (1-a) A lambda_{k+1} is
 //        a pull over the CSR (the transpose of the forward CSC); the same sweep accumulates
-//        dL/dA_uv = (1-a) sum_k <x_k[u], lambda_{k+1}[v]>; iterates x_k are recomputed from
-//        checkpoints kept every ceil(sqrt(K)) steps;
+//        dL/dA_uv = (1-a) sum_k <x_k[u], lambda_{k+1}[v]>; the iterates x_k are kept while they fit
+//        an eighth of the GPU's memory, else recomputed from checkpoints;
 //      - eg_sssp_batch: Bellman-Ford from up to 64 sources, in place, skipping sources whose
 //        distance did not change in the previous sweep (bit-exact least fixpoint).
 #include <math.h>
