@@ -18,16 +18,11 @@
 #include <algorithm>
 
 #include "eg_pull.cuh"
+#include "eg_queue.cuh"
 
 namespace eg {
 
-constexpr uint32_t kPiece = 256;          // edges per queue entry
 constexpr int kIlp = 4;
-// two CTAs of 512 threads at 64 registers: a BFS of 2^25 / 2^29 takes 1.61 ms (mean of 16 roots)
-// against 1.66 with one CTA of 1,024, 1.70 with three of 512 (42 registers), 1.75 with two of 768 and
-// 1.87 with two of 1,024; one of 2^22 / 2^26 0.29 against 0.30 / 0.28 / 0.29 / 0.32
-constexpr int kPersistThreads = 512;
-constexpr int kPersistCtas = 2;
 constexpr uint32_t kStepsPerLaunch = 4096;  // then the host launches again: a kernel always ends
 
 // what one step left behind, read by every CTA after the barrier that ends the step
@@ -88,22 +83,13 @@ __device__ __forceinline__ uint32_t warp_owner(uint32_t incl, uint32_t r) {
     return o;
 }
 
-// The CTA's share of the next queue: entries gather in shared memory and go out together (flush).
-// What does not fit goes to the global queue in blocks of kQueueBlock entries that one warp reserves
-// at a time (a reservation per warp and 128 edges made a push level of 2.7 M activations 0.38 ms
-// long); the rest of a warp's last block is filled with empty pieces.
-constexpr uint32_t kLocalQueue = 2048;
-constexpr uint32_t kQueueBlock = 256;
+// The CTA's share of the next queue (eg_queue.cuh)
 struct LocalQueue {
     uint4 e[kLocalQueue];
     uint32_t n;      // reserved
     uint32_t valid;  // reservations from here on did not fit
     uint32_t base;
 };
-struct WarpBlock {  // the warp's block of the global queue, the same in every lane
-    uint32_t pos = 0, end = 0;
-};
-
 __device__ __forceinline__ uint4 piece(uint32_t v, uint64_t beg, uint64_t end) {
     const uint32_t len = (uint32_t)(end - beg < kPiece ? end - beg : kPiece);
     return make_uint4(v, (uint32_t)beg, (uint32_t)(beg >> 32), len);
@@ -136,10 +122,9 @@ __device__ __forceinline__ void append_pieces(LocalQueue& lq, WarpBlock& wb, con
             for (uint64_t b = beg[j]; b < end[j]; b += kPiece) lq.e[at + k++] = piece(v[j], b, end[j]);
         return;
     }
-    const uint32_t room = wb.end - wb.pos;
-    uint32_t fresh = 0, block = 0;
-    if (tot > room) {
-        block = tot - room > kQueueBlock ? tot - room : kQueueBlock;
+    const uint32_t room = wb.end - wb.pos, block = wb.wants(tot);
+    uint32_t fresh = 0;
+    if (block) {
         if ((threadIdx.x & 31) == 31) fresh = atomicAdd(n_out, block);
         fresh = __shfl_sync(0xffffffffu, fresh, 31);
     }
@@ -147,18 +132,15 @@ __device__ __forceinline__ void append_pieces(LocalQueue& lq, WarpBlock& wb, con
     for (int j = 0; j < K; ++j)
         for (uint64_t b = beg[j]; b < end[j]; b += kPiece, ++k)
             q_out[k < room ? wb.pos + k : fresh + (k - room)] = piece(v[j], b, end[j]);
-    if (tot > room) {
-        wb.pos = fresh + (tot - room);
-        wb.end = fresh + block;
-    } else {
-        wb.pos += tot;
-    }
+    wb.took(tot, fresh, block);
 }
 
-// by the whole CTA, before the barrier that ends the step
-__device__ __forceinline__ void flush_pieces(LocalQueue& lq, WarpBlock& wb, uint4* q_out, uint32_t* n_out) {
+// By the whole CTA, before the barrier that ends a phase.  What a warp has left of its block is filled with
+// empty pieces, which a later phase of the step (behind that barrier) may overwrite.
+__device__ __forceinline__ void flush_pieces(LocalQueue& lq, WarpBlock& wb, uint4* q_out, uint32_t* n_out,
+                                             bool step_done = true) {
     for (uint32_t i = wb.pos + (threadIdx.x & 31); i < wb.end; i += 32) q_out[i] = make_uint4(0, 0, 0, 0);
-    wb.pos = wb.end = 0;
+    wb.phase_done(step_done);
     __syncthreads();
     const uint32_t n = min(lq.n, lq.valid);
     if (threadIdx.x == 0) lq.base = n ? atomicAdd(n_out, n) : 0u;
@@ -168,12 +150,6 @@ __device__ __forceinline__ void flush_pieces(LocalQueue& lq, WarpBlock& wb, uint
         lq.n = 0;
         lq.valid = 0xFFFFFFFFu;
     }
-}
-
-// entries a queue has to hold: every vertex's pieces and the blocks' empty ends
-static uint64_t queue_entries(const eg_graph* g) {
-    return std::min<uint64_t>(g->V, g->E) + g->E / kPiece +
-           (uint64_t)g->num_sms * kPersistCtas * (kPersistThreads / 32) * kQueueBlock + 64;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -415,7 +391,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EngineState& s = g->eng;
     EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
     EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
-    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
     float* d_dist = dist;
     if (where != EG_DEVICE || !dist) {
         EG_TRY(s.vals0.reserve(sizeof(float) * (V + 1)));
@@ -590,7 +566,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
             clear->act = 0;
         }
         // hand the step's totals and the gathered queue entries over; false: a barrier gave up
-        auto end_phase = [&]() -> bool {
+        auto end_phase = [&](bool step_done) -> bool {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 my_verts += __shfl_xor_sync(0xffffffffu, my_verts, o);
@@ -602,7 +578,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
             }
             my_verts = 0;
             my_act = 0;
-            flush_pieces(lq, wb, q_out, &out->n);
+            flush_pieces(lq, wb, q_out, &out->n, step_done);
             if (threadIdx.x == 0 && s_verts) {
                 atomicAdd(&out->verts, s_verts);
                 atomicAdd(&out->act, s_act);
@@ -659,7 +635,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 }
             }
             ++pushes;
-            if (!end_phase()) return;
+            if (!end_phase(true)) return;
         } else {
             // a list's vertex is loaded two rounds ahead, its level and bounds one round ahead
             uint64_t i = tid;
@@ -747,8 +723,9 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 append_pieces<1>(lq, wb, vv, lb, le, q_out, &out->n);
             }
             ++pulls;
-            if (!end_phase()) return;
+            if (!end_phase(false)) return;  // whether there are segments is known behind the barrier
             const uint32_t nseg = s_slot.nseg;
+            if (!nseg) wb.phase_done(true);
             if (nseg) {  // long lists, a warp per segment; the first segment to find a parent claims
                 __syncthreads();  // s_slot has been read
                 for (uint32_t t = warp; t < nseg; t += nwarps) {
@@ -783,7 +760,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                     }
                     append_pieces<1>(lq, wb, vv, lb, le, q_out, &out->n);
                 }
-                if (!end_phase()) return;
+                if (!end_phase(true)) return;
             }
         }
         reached += s_slot.verts;
@@ -804,7 +781,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
 int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
-    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g)));
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
     BfsPersistArgs a;
     a.level = level;
     a.parent = parent;
@@ -1041,7 +1018,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
 int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
-    EG_TRY(s.pieces0.reserve(sizeof(uint4) * queue_entries(g)));
+    EG_TRY(s.pieces0.reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
     static_assert(sizeof(CcState) <= kPersistBytes, "one block of the state words");
     void *block = nullptr, *next = nullptr;
     EG_TRY(persist_block(g, &block, &next));
