@@ -200,13 +200,17 @@ int load_edges_impl(eg_graph* g, const void* edges, uint64_t E, uint32_t V, int 
     return EG_OK;
 }
 
-bool direct_records(const eg_graph* g, const void* edges, int where) {
-    if (where != EG_DEVICE || ((uintptr_t)edges & 15u)) return false;
+bool plain_device(const eg_graph* g, const void* p, size_t align) {
+    if (!p || ((uintptr_t)p & (align - 1))) return false;
     cudaPointerAttributes at{};
-    const bool ok = cudaPointerGetAttributes(&at, edges) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+    const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
                     at.device == g->device;
     cudaGetLastError();
     return ok;
+}
+
+bool direct_records(const eg_graph* g, const void* edges, int where) {
+    return where == EG_DEVICE && plain_device(g, edges, 16);
 }
 
 // argument checks, state reset and the record buffer of a new edge list

@@ -2557,7 +2557,7 @@ int run_msbfs_graphs(eg_graph* g, const uint32_t* roots, int nper, uint8_t* leve
     if (levels) {
         const uint64_t V = g->V;
         uint8_t* out = levels;
-        const bool direct = where == EG_DEVICE && ((uintptr_t)levels & 15u) == 0;
+        const bool direct = where == EG_DEVICE && plain_device(g, levels, 16);
         if (!direct) {
             EG_TRY(b.tmp_out.reserve(64 * V + 64));
             out = b.tmp_out.as<uint8_t>();
@@ -2591,7 +2591,7 @@ int run_sssp_graphs(eg_graph* g, const uint32_t* sources, int nper, float* dist,
     const float* rows = b.rows0.as<float>();
     if (dist && row_width(nper) == 32) {
         float* wide = dist;
-        if (where != EG_DEVICE) {
+        if (where != EG_DEVICE || !plain_device(g, dist, 4)) {
             EG_TRY(b.tmp_out.reserve(256ull * g->V + 64));
             wide = b.tmp_out.as<float>();
         }

@@ -243,7 +243,10 @@ bool persistent_build_fits(const eg_graph* g);
 // src (optional): device records, 16-byte aligned, read where they are; with g->symmetric they are the
 // E / 2 records before symmetrisation
 int build_persistent(eg_graph* g, const uint64_t* eoff, const uint64_t* voff, uint32_t G, const void* src);
-// whether pass A may read the caller's records itself: plain device memory of this GPU, 16-byte aligned
+// Whether kernels may work on a caller's array itself: plain memory of this GPU, aligned.  Anything else that
+// a copy serves (another GPU's memory, managed or mapped host memory, any alignment) gets a copy.
+bool plain_device(const eg_graph* g, const void* p, size_t align);
+// whether pass A may read the caller's records itself
 bool direct_records(const eg_graph* g, const void* edges, int where);
 int prepare_load(eg_graph* g, uint64_t E, uint32_t V, int edge_bytes, int symmetric, bool keep_list = true);
 int ensure_list(eg_graph* g);  // g->edges holds the list again

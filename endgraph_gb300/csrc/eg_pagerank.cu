@@ -349,7 +349,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     EG_TRY(setup_list_heads(g, relabel));
     const uint32_t* order = relabel ? s.pr_new_id.as<uint32_t>() : nullptr;
     float* vec[2] = {s.vals0.as<float>(), s.vals1.as<float>()};
-    float* result = out && where == EG_DEVICE ? out : vec[iterations & 1];
+    float* result = where == EG_DEVICE && plain_device(g, out, 4) ? out : vec[iterations & 1];
     PrArgs p;
     p.adj = relabel ? s.pr_adj.as<uint32_t>() : g->csc_adj.as<uint32_t>();
     p.heads = s.pr_heads.as<uint32_t>();
@@ -413,8 +413,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
             EG_CHECK_LAUNCH("k_pr_boundaries");
         }
     }
-    if (out && where != EG_DEVICE)
-        EG_CUDA(cudaMemcpyAsync(out, result, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
+    if (result != out) EG_TRY(copy_out(g, out, result, sizeof(float) * V, where));
     EG_CUDA(cudaStreamSynchronize(g->stream));
     if (small && !*reinterpret_cast<volatile uint32_t*>(s.host_words)) {
         persist_reset(g);

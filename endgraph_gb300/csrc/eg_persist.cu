@@ -393,7 +393,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
     for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
     float* d_dist = dist;
-    if (where != EG_DEVICE || !dist) {
+    if (where != EG_DEVICE || !plain_device(g, dist, 4)) {
         EG_TRY(s.vals0.reserve(sizeof(float) * (V + 1)));
         d_dist = s.vals0.as<float>();
     }
@@ -443,8 +443,8 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     g->last_iterations = (int)h->pushes;
     g->last_pushes = (int)h->pushes;
     g->last_pulls = 0;
-    if (dist && where != EG_DEVICE) {
-        EG_CUDA(cudaMemcpyAsync(dist, d_dist, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream));
+    if (dist && d_dist != dist) {
+        EG_TRY(copy_out(g, dist, d_dist, sizeof(float) * V, where));
         EG_CUDA(cudaStreamSynchronize(g->stream));
     }
     return EG_OK;
@@ -785,11 +785,11 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     BfsPersistArgs a;
     a.level = level;
     a.parent = parent;
-    if (where != EG_DEVICE || !level) {
+    if (where != EG_DEVICE || !plain_device(g, level, 4)) {
         EG_TRY(s.vals0.reserve(sizeof(uint32_t) * (V + 1)));
         a.level = s.vals0.as<uint32_t>();
     }
-    if (where != EG_DEVICE && parent) {
+    if (parent && (where != EG_DEVICE || !plain_device(g, parent, 4))) {
         EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
         a.parent = s.vals1.as<uint32_t>();
     }
@@ -841,9 +841,9 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     g->last_pushes = (int)h->pushes;
     g->last_pulls = (int)h->pulls;
     if (reached) *reached = h->reached;
-    if (where != EG_DEVICE) {
-        if (level) EG_CUDA(cudaMemcpyAsync(level, a.level, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
-        if (parent) EG_CUDA(cudaMemcpyAsync(parent, a.parent, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
+    if ((level && a.level != level) || a.parent != parent) {
+        if (a.level != level) EG_TRY(copy_out(g, level, a.level, sizeof(uint32_t) * V, where));
+        if (a.parent != parent) EG_TRY(copy_out(g, parent, a.parent, sizeof(uint32_t) * V, where));
         EG_CUDA(cudaStreamSynchronize(g->stream));
     }
     return EG_OK;
@@ -1024,7 +1024,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     EG_TRY(persist_block(g, &block, &next));
     PersistResult* h = reinterpret_cast<PersistResult*>(s.host_words);
     uint32_t* comp = label;
-    if (where != EG_DEVICE || !label) {
+    if (where != EG_DEVICE || !plain_device(g, label, 4)) {
         EG_TRY(s.vals0.reserve(sizeof(uint32_t) * (V + 1)));
         comp = s.vals0.as<uint32_t>();
     }
@@ -1041,8 +1041,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
         EG_CHECK_LAUNCH("k_cc_persistent");
         persist_launched(g);
     }
-    if (label && where != EG_DEVICE)
-        EG_CUDA(cudaMemcpyAsync(label, comp, sizeof(uint32_t) * V, cudaMemcpyDeviceToHost, g->stream));
+    if (comp != label) EG_TRY(copy_out(g, label, comp, sizeof(uint32_t) * V, where));
     EG_CUDA(cudaStreamSynchronize(g->stream));
     if (!*(volatile uint32_t*)&h->valid) {
         persist_reset(g);

@@ -161,6 +161,8 @@ int eg_cpbt_partition_noalloc(const uint32_t* deg, uint32_t V, int P, int S, uin
                               int dense, uint32_t* partition_offset, uint32_t* local_offset, void* stream);
 
 /* ---- toolkits: process_edges / process_vertices core/graph.hpp:1376-1817 ------------------ */
+/* Output arrays with EG_DEVICE: whatever a device copy can write.  Arrays in this GPU's memory, aligned
+ * for their type, are worked on in place; after an error they hold unspecified values. */
 /* Gemini PageRank (toolkits/pagerank.cpp:26-98): dense pull every iteration, FP32 ranks.
  * out[V] receives the final curr array. */
 int eg_pagerank(eg_graph* g, int iterations, float damping, float* out, int where);
