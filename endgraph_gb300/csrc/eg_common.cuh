@@ -285,7 +285,12 @@ int run_sssp(eg_graph* g, uint32_t root, float* dist, int where);
 constexpr size_t kPersistBytes = 256;
 int persist_block(eg_graph* g, void** mine, void** other);
 void persist_launched(eg_graph* g);
-void persist_reset(eg_graph* g);
+// After the stream is done: EG_OK if the launch set the first of the handle's pinned words (by its first thread,
+// at its end) and no CTA gave up at a barrier.  A CTA says so itself (grid_sync_growing): it may have
+// given up as the barrier completed for the others.
+int persist_finish(eg_graph* g, const char* what);
+constexpr int kPersistGaveUp = 63;  // index of that word among the pinned u32 words
+inline uint32_t* persist_gave_up(const eg_graph* g) { return reinterpret_cast<uint32_t*>(g->eng.host_words) + kPersistGaveUp; }
 __device__ __forceinline__ void persist_clear(void* other) {  // by one warp
     if ((threadIdx.x & 31) < kPersistBytes / 16)
         reinterpret_cast<uint4*>(other)[threadIdx.x & 31] = make_uint4(0, 0, 0, 0);
@@ -348,7 +353,8 @@ __device__ __forceinline__ bool grid_sync_bounded(unsigned* count, unsigned* gen
 // The same for kernels whose steps are a few microseconds: one counter that only grows, so that no
 // CTA resets it and advances a generation before the others can go on (40 barriers of 128 CTAs in a
 // PageRank of 65,536 / 2^20: 0.23 instead of 0.27 ms).  *count is zero at launch; `target` starts at zero in every CTA.
-__device__ __forceinline__ bool grid_sync_growing(unsigned* count, int* err, unsigned& target,
+// A CTA that gives up also sets *gave_up (pinned host memory).
+__device__ __forceinline__ bool grid_sync_growing(unsigned* count, int* err, uint32_t* gave_up, unsigned& target,
                                                   uint32_t spin_cap = kBarrierSpinCap) {
     __shared__ int s_ok;
     __syncthreads();
@@ -363,6 +369,7 @@ __device__ __forceinline__ bool grid_sync_growing(unsigned* count, int* err, uns
             if ((int)(x - target) >= 0) break;
             if (spins > spin_cap || ((spins & 63u) == 0 && *(volatile int*)err)) {
                 atomicExch(err, 1);
+                *(volatile uint32_t*)gave_up = 1;
                 ok = 0;
                 break;
             }

@@ -271,6 +271,7 @@ struct PrPersistArgs {
     unsigned* words;        // barrier count, unused, error flag
     void* words_next;       // the next launch's, zeroed by this one
     uint32_t* finished;     // pinned: set when the last iteration is done
+    uint32_t* gave_up;
 };
 
 constexpr int kPrPersistThreads = 512, kPrPersistCtas = 2;
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
     __shared__ float s_sum[kPrPersistThreads / 32][kPrSums];
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     unsigned arrived = 0;
-    auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), arrived); };
+    auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), a.gave_up, arrived); };
     pr_start(a.vec[0], a.outdeg, a.V, a.order, a.pr.acc, a.pr.nruns, tid, stride);
     for (int it = 0; it < a.iterations; ++it) {
         if (!barrier()) return;
@@ -371,7 +372,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
         void *block = nullptr, *next = nullptr;
         EG_TRY(persist_block(g, &block, &next));
         PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations,
-                        static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words)};
+                        static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words), persist_gave_up(g)};
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((uint64_t)g->num_sms * kPrPersistCtas, (p.nruns + kPrPersistThreads / 32 - 1) / (kPrPersistThreads / 32)));
         void* kargs[] = {&a};
@@ -415,11 +416,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     }
     if (result != out) EG_TRY(copy_out(g, out, result, sizeof(float) * V, where));
     EG_CUDA(cudaStreamSynchronize(g->stream));
-    if (small && !*reinterpret_cast<volatile uint32_t*>(s.host_words)) {
-        persist_reset(g);
-        set_error("eg_pagerank: a bounded grid barrier gave up");
-        return EG_ERR_TIMEOUT;
-    }
+    if (small) EG_TRY(persist_finish(g, "eg_pagerank"));
     g->last_edges_processed = E * (uint64_t)iterations;
     g->last_iterations = iterations;
     g->last_pushes = 0;

@@ -44,18 +44,17 @@ struct PersistState {
     unsigned long long edges;  // edges of the pieces walked
 };
 
-// what a launch tells the host, written to pinned memory by its first thread as it ends; `valid` stays
-// zero when a barrier gave up
+// what a launch tells the host, written to pinned memory by its first thread as it ends (persist_finish)
 struct PersistResult {
     uint32_t valid, done, step, pushes, pulls, pad;
     unsigned long long reached, edges;
 };
-static_assert(sizeof(PersistResult) <= 256, "the results lie in the handle's pinned words");
+static_assert(sizeof(PersistResult) <= 4 * kPersistGaveUp, "the results lie in the handle's pinned words");
 
 // one grid barrier; *s_slot gets the slot the finished step filled.  False: a wait gave up.
 template <class State, class Slot>
-__device__ __forceinline__ bool step_barrier(State* st, const Slot* slot, Slot* s_slot, unsigned& arrived) {
-    if (!grid_sync_growing(&st->bar_count, &st->err, arrived)) return false;
+__device__ __forceinline__ bool step_barrier(State* st, uint32_t* gave_up, const Slot* slot, Slot* s_slot, unsigned& arrived) {
+    if (!grid_sync_growing(&st->bar_count, &st->err, gave_up, arrived)) return false;
     if (threadIdx.x < sizeof(Slot) / 16)
         reinterpret_cast<uint4*>(s_slot)[threadIdx.x] = __ldcg(reinterpret_cast<const uint4*>(slot) + threadIdx.x);
     __syncthreads();
@@ -173,6 +172,7 @@ struct SsspPersistArgs {
     PersistState* st;
     void* st_next;      // the next launch's state, zeroed by this one
     PersistResult* result;
+    uint32_t* gave_up;
 };
 
 constexpr uint32_t kWeightSamples = 65536;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
             for (uint32_t p = lane; p < np; p += 32) a.q[0][p] = piece(a.root, b + (uint64_t)p * kPiece, z);
             if (lane == 0) st->slot[0].n = np;
         }
-        if (!step_barrier(st, &st->slot[0], &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, &st->slot[0], &s_slot, arrived)) return;
         delta = a.delta;
         if (delta < 0.f) {
             const uint64_t every = max(a.E / kWeightSamples, (uint64_t)1);
@@ -354,11 +354,11 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
         }
         ++step;
         flush_pieces(lq, wb, q_out, &out->n);
-        if (!step_barrier(st, out, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, out, &s_slot, arrived)) return;
     }
     // every CTA leaves the loop at the same step; the edges walked are added up behind one more barrier
     if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
-    if (!step_barrier(st, &st->slot[step & 3], &s_slot, arrived)) return;
+    if (!step_barrier(st, a.gave_up, &st->slot[step & 3], &s_slot, arrived)) return;
     if (tid < 32) persist_clear(a.st_next);
     if (tid == 0) {
         st->step = step;
@@ -416,6 +416,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EG_TRY(persist_block(g, &block, &a.st_next));
     a.st = static_cast<PersistState*>(block);
     a.result = reinterpret_cast<PersistResult*>(s.host_words);
+    a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
@@ -431,11 +432,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
             if (!a.resume) persist_launched(g);
         }
         EG_CUDA(cudaStreamSynchronize(g->stream));
-        if (!h->valid) {
-            persist_reset(g);
-            set_error("eg_sssp: a bounded grid barrier gave up");
-            return EG_ERR_TIMEOUT;
-        }
+        EG_TRY(persist_finish(g, "eg_sssp"));
         if (h->done) break;
         h->valid = 0;
     }
@@ -499,6 +496,7 @@ struct BfsPersistArgs {
     BfsPersistState* st;
     void* st_next;  // the next launch's state, zeroed by this one
     PersistResult* result;
+    uint32_t* gave_up;
 };
 
 __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persistent(BfsPersistArgs a) {
@@ -538,7 +536,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 st->slot[0].act = z - b;
             }
         }
-        if (!step_barrier(st, &st->slot[0], &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, &st->slot[0], &s_slot, arrived)) return;
         reached = 1;
         edges = s_slot.act;
     } else {
@@ -585,7 +583,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 s_verts = 0;
                 s_act = 0;
             }
-            return step_barrier(st, out, &s_slot, arrived);
+            return step_barrier(st, a.gave_up, out, &s_slot, arrived);
         };
         if (!dense) {
             const uint4* q = a.q[step & 1];
@@ -813,6 +811,7 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     EG_TRY(persist_block(g, &block, &a.st_next));
     a.st = static_cast<BfsPersistState*>(block);
     a.result = reinterpret_cast<PersistResult*>(s.host_words);
+    a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
@@ -828,11 +827,7 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
             if (!a.resume) persist_launched(g);
         }
         EG_CUDA(cudaStreamSynchronize(g->stream));
-        if (!h->valid) {
-            persist_reset(g);
-            set_error("eg_bfs: a bounded grid barrier gave up");
-            return EG_ERR_TIMEOUT;
-        }
+        EG_TRY(persist_finish(g, "eg_bfs"));
         if (h->done) break;
         h->valid = 0;
     }
@@ -880,6 +875,7 @@ struct CcArgs {
     CcState* st;
     void* st_next;  // the next launch's state, zeroed by this one
     PersistResult* result;
+    uint32_t* gave_up;
 };
 constexpr uint32_t kCcFirst = 2;      // neighbours united before the common component is looked for
 constexpr int kCcSamples = 1024;
@@ -943,17 +939,17 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
             if (b + k < e) p = min(p, __ldg(a.adj + b + k));
         a.comp[v] = p;
     }
-    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     cc_compress(a.comp, a.V, tid, stride);
-    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     for (uint32_t k = 0; k < kCcFirst; ++k) {
         for (uint64_t v = tid; v < a.V; v += stride) {
             const uint64_t b = __ldg(a.off + v) + k;
             if (b < __ldg(a.off + v + 1)) cc_unite(a.comp, (uint32_t)v, __ldg(a.adj + b));
         }
-        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
         cc_compress(a.comp, a.V, tid, stride);
-        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     }
     // the component of most of a sample's vertices; one CTA decides for all
     if (blockIdx.x == 0) {
@@ -968,7 +964,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         __syncthreads();
         if (threadIdx.x == 0) st->slot.common = (uint32_t)s_best;
     }
-    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     const uint32_t common = s_slot.common;
     // the other components' lists, from the third neighbour on
     for (uint64_t base = tid & ~31ull; base < a.V; base += stride) {
@@ -983,7 +979,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         append_pieces<1>(lq, wb, vv, lb, le, a.q, &st->slot.n);
     }
     flush_pieces(lq, wb, a.q, &st->slot.n);
-    if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     const uint32_t n = s_slot.n;
     if (n) {
         for (uint32_t base = 0; base < n; base += 32 * nwarps) {
@@ -1008,7 +1004,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
                 __syncwarp();
             }
         }
-        if (!step_barrier(st, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
         cc_compress(a.comp, a.V, tid, stride);
     }
     if (tid < 32) persist_clear(a.st_next);
@@ -1029,7 +1025,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
         comp = s.vals0.as<uint32_t>();
     }
     CcArgs a{V, g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(),
-             static_cast<CcState*>(block), next, h};
+             static_cast<CcState*>(block), next, h, persist_gave_up(g)};
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_cc_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, (V + E / 16) / kEdgesPerCta));
@@ -1043,11 +1039,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     }
     if (comp != label) EG_TRY(copy_out(g, label, comp, sizeof(uint32_t) * V, where));
     EG_CUDA(cudaStreamSynchronize(g->stream));
-    if (!*(volatile uint32_t*)&h->valid) {
-        persist_reset(g);
-        set_error("eg_cc: a bounded grid barrier gave up");
-        return EG_ERR_TIMEOUT;
-    }
+    EG_TRY(persist_finish(g, "eg_cc"));
     g->last_edges_processed = E;  // united once, or skipped because both ends were
     g->last_iterations = 1;
     g->last_pushes = 0;

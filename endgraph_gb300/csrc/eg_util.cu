@@ -163,8 +163,36 @@ int persist_block(eg_graph* g, void** mine, void** other) {
 
 void persist_launched(eg_graph* g) { g->eng.persist_turn ^= 1; }
 
-void persist_reset(eg_graph* g) {
+int persist_finish(eg_graph* g, const char* what) {
+    const volatile uint32_t* h = reinterpret_cast<const uint32_t*>(g->eng.host_words);
+    if (h[0] && !h[kPersistGaveUp]) return EG_OK;
     cudaMemsetAsync(g->eng.persist.ptr, 0, 2 * kPersistBytes, g->stream);
+    set_error("%s: a bounded grid barrier gave up", what);
+    return EG_ERR_TIMEOUT;
+}
+
+// The barrier of the traversals, exercised: CTA 0 arrives only when another has given up (or its own wait for
+// that has run out).  All have arrived then, so it passes and reports success; the call has to fail.
+__global__ void k_late_barrier_selftest(unsigned* words, uint32_t* host, uint32_t spin_cap) {
+    int* err = reinterpret_cast<int*>(words + 2);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        for (uint32_t i = 0; i < 2 * kBarrierSpinCap && !*(volatile int*)err; ++i) __nanosleep(100);
+    unsigned arrived = 0;
+    if (!grid_sync_growing(words, err, host + kPersistGaveUp, arrived, blockIdx.x ? spin_cap : kBarrierSpinCap)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *host = 1;
+}
+
+static int selftest_late_barrier(eg_graph* g, uint32_t spin_cap) {
+    void *block = nullptr, *next = nullptr;
+    EG_TRY(persist_block(g, &block, &next));
+    unsigned* words = static_cast<unsigned*>(block);
+    uint32_t* host = reinterpret_cast<uint32_t*>(g->eng.host_words);
+    void* kargs[] = {&words, &host, &spin_cap};
+    EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_late_barrier_selftest, dim3(4), dim3(32), kargs, 0, g->stream));
+    EG_CHECK_LAUNCH("k_late_barrier_selftest");
+    persist_launched(g);
+    EG_CUDA(cudaStreamSynchronize(g->stream));
+    return persist_finish(g, "eg_selftest_grid_barrier");
 }
 
 // The bounded grid barrier of the persistent kernels, exercised: a cooperative launch of four CTAs
@@ -176,6 +204,8 @@ __global__ void k_grid_barrier_selftest(unsigned* words, int* err, uint32_t spin
 }
 
 int selftest_grid_barrier(eg_graph* g, uint32_t spin_cap) {
+    const int late = selftest_late_barrier(g, spin_cap);
+    if (late != EG_ERR_TIMEOUT) return late;
     EG_TRY(g->tmp64.reserve(16));
     unsigned* words = reinterpret_cast<unsigned*>(g->tmp64.ptr);
     EG_CUDA(cudaMemsetAsync(words, 0, 16, g->stream));

@@ -219,3 +219,19 @@ def test_launches_in_turn_on_one_handle(eg_lib):
                 g.load_undirected_from_directed(eg.pack_edges(src, dst, w), n)
                 assert np.array_equal(g.cc(), labels)
                 assert np.array_equal(g.cc(), labels)
+
+
+@pytest.mark.parametrize("spin_cap", [1, 200, 20_000])
+def test_barrier_given_up_as_it_completes(eg_lib, spin_cap):
+    """A CTA that gives up at a barrier which then completes for the others (the self-test's first launch) makes
+    the call fail, and the state words are clean for the launches after it."""
+    import endgraph_gb300 as eg
+    n = 600
+    i = np.arange(n - 1, dtype=np.uint32)
+    with eg.Graph() as g:
+        g.load_undirected_from_directed(eg.pack_edges(i, i + 1, np.ones(n - 1, np.float32)), n)
+        for _ in range(2):
+            assert g.selftest_grid_barrier(spin_cap) == 5  # EG_ERR_TIMEOUT
+            assert np.array_equal(g.bfs(0)[0], np.arange(n))
+            assert np.array_equal(g.sssp(0), np.arange(n, dtype=np.float32))
+            assert not g.cc().any()
