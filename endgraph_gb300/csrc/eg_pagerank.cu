@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "eg_pull.cuh"
+#include "eg_queue.cuh"
 
 namespace eg {
 
@@ -343,8 +344,10 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     // Every iteration in one launch up to here: 20 iterations take 0.26 / 0.35 ms (one launch / sweeps) at
     // 65,536 / 2^20, 0.62 / 0.67 at 300,000 / 5 M, 1.45 / 1.33 and 0.1 for the renumbering at 1 M / 16 M, 2.70
     // / 1.91 at 2 M / 30 M.  Sweeps renumber by themselves when that comes back: 2^22 / 2^26 takes 0.30 ms to
-    // renumber and 0.18 instead of 0.26 a sweep; a GPU too full for the second list goes without.
-    const bool small = E <= (1ull << 24);
+    // renumber and 0.18 instead of 0.26 a sweep; a GPU too full for the second list goes without.  Passes over
+    // many vertices want more threads than the one launch has: 3 iterations at 2^26 vertices take 2.23 / 1.33
+    // with 1,000 edges, 2.86 / 1.96 with 2^24; 20 at 2^23 0.52 / 0.81 and 2.48 / 2.78.
+    const bool small = E <= (1ull << 24) && V <= (1ull << 24);
     bool relabel = want_relabel(g);
     if (!relabel && !small && g->pr_relabel < 0 && iterations >= 4) relabel = setup_list_heads(g, true) == EG_OK;
     EG_TRY(setup_list_heads(g, relabel));
@@ -363,7 +366,8 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     EG_TRY(s.acc.reserve(4 * (p.nruns + 4)));
     p.acc = s.acc.as<float>();
     p.ticket = s.acc.as<uint32_t>() + p.nruns + 3;
-    p.hot = relabel ? std::min(kPrHot, relabel_lines((uint32_t)V)) : 0;
+    // no more hot ranks than a quarter of an SM's edges: every SM copies them for every sweep
+    p.hot = relabel ? (uint32_t)std::min<uint64_t>({kPrHot, relabel_lines((uint32_t)V), E / (4 * (uint64_t)g->num_sms)}) : 0;
     p.split = s.pr_split.as<uint32_t>();
     const uint32_t* outdeg = g->outdeg.as<uint32_t>();
     p.base = 1.0f - damping;
@@ -373,8 +377,12 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
         EG_TRY(persist_block(g, &block, &next));
         PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations,
                         static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words), persist_gave_up(g)};
-        const unsigned grid = (unsigned)std::max<uint64_t>(
-            1, std::min<uint64_t>((uint64_t)g->num_sms * kPrPersistCtas, (p.nruns + kPrPersistThreads / 32 - 1) / (kPrPersistThreads / 32)));
+        // A warp per run, or what the vertices' values want where they are more: 20 iterations at 2^20 vertices
+        // with 1,000 edges take 0.23 ms so and 2.7 by the one CTA that the runs want; the sum of both is
+        // slower where the barriers dominate (0.41 instead of 0.32 ms at 2^20 / 2^20).
+        const uint64_t warps = kPrPersistThreads / 32;
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)g->num_sms * kPrPersistCtas,
+                                                           std::max((p.nruns + warps - 1) / warps, V / kVerticesPerCta));
         void* kargs[] = {&a};
         {
             Timed t(&g->prof, g->stream, "pr_persistent");

@@ -382,10 +382,6 @@ static float auto_delta(uint64_t V, uint64_t E) {
     return 0.7f / deg;
 }
 
-// one CTA per this many edges, up to one per SM: fewer CTAs meet sooner at a barrier, but 2,048 was
-// no slower than 4,096 or 8,192 from 20 k edges on (0.134 / 0.142 / 0.159 ms at 2 k vertices, 20 k edges)
-constexpr uint64_t kEdgesPerCta = 2048;
-
 int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
@@ -419,7 +415,7 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
+    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
     volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
@@ -814,7 +810,7 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, E / kEdgesPerCta));
+    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
     volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
@@ -1028,7 +1024,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
              static_cast<CcState*>(block), next, h, persist_gave_up(g)};
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_cc_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms * kPersistCtas, (V + E / 16) / kEdgesPerCta));
+    const unsigned grid = (unsigned)persist_ctas(4 * V, E / 16, (uint64_t)g->num_sms);
     void* kargs[] = {&a};
     {
         Timed t(&g->prof, g->stream, "cc_persistent");

@@ -25,6 +25,16 @@ constexpr int kPersistCtas = 2;
 constexpr uint32_t kLocalQueue = 2048;
 constexpr uint32_t kQueueBlock = 256;
 
+// CTAs of a launch: one per kEdgesPerCta edges and per kVerticesPerCta vertices, whose values it sets up,
+// up to the GPU's.  Fewer CTAs meet sooner at a barrier, but 2,048 edges were no slower than 4,096 or 8,192
+// from 20 k edges on (0.134 / 0.142 / 0.159 ms at 2 k vertices, 20 k edges).  Without a share for
+// the vertices an SSSP of 2^26 with 1,000 edges had one CTA to set them up and took 9.4 ms.
+constexpr uint64_t kEdgesPerCta = 2048, kVerticesPerCta = 8192;
+inline uint64_t persist_ctas(uint64_t V, uint64_t E, uint64_t num_sms) {
+    const uint64_t want = E / kEdgesPerCta + V / kVerticesPerCta, most = num_sms * kPersistCtas;
+    return want < 1 ? 1 : want < most ? want : most;
+}
+
 struct WarpBlock {  // the warp's block of the global queue, the same in every lane
     uint32_t pos = 0, end = 0;
 
