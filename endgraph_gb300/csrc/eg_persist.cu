@@ -863,7 +863,9 @@ struct CcState {
     CcSlot slot;
 };
 struct CcArgs {
-    uint64_t V;
+    uint64_t V, nlists;
+    const uint32_t* deg;
+    const uint32_t* vert;  // kIndex: the vertices with neighbours (the compressed index); else list i is vertex i's
     const uint64_t* off;
     const uint32_t* adj;
     uint32_t* comp;
@@ -901,13 +903,19 @@ __device__ __forceinline__ void cc_unite(uint32_t* comp, uint32_t u, uint32_t v)
     }
 }
 
-__device__ __forceinline__ void cc_compress(uint32_t* comp, uint64_t V, uint64_t tid, uint64_t stride) {
-    for (uint64_t v = tid; v < V; v += stride) {
-        const uint32_t p = __ldca(comp + v), r = cc_root(comp, p);
+template <bool kIndex>
+__device__ __forceinline__ uint32_t cc_vertex(const uint32_t* vert, uint64_t i) { return kIndex ? __ldg(vert + i) : (uint32_t)i; }
+
+template <bool kIndex>
+__device__ __forceinline__ void cc_compress(uint32_t* comp, const uint32_t* __restrict__ vert, uint64_t n, uint64_t tid,
+                                            uint64_t stride) {
+    for (uint64_t i = tid; i < n; i += stride) {
+        const uint32_t v = cc_vertex<kIndex>(vert, i), p = __ldca(comp + v), r = cc_root(comp, p);
         if (r != p) comp[v] = r;
     }
 }
 
+template <bool kIndex>
 __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent(CcArgs a) {
     __shared__ CcSlot s_slot;
     __shared__ uint32_t s_sample[kCcSamples];
@@ -926,31 +934,35 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint32_t warp = (uint32_t)(tid >> 5), nwarps = (uint32_t)(stride >> 5);
-    // every vertex starts under the smallest of itself and its first neighbours
-    for (uint64_t v = tid; v < a.V; v += stride) {
-        const uint64_t b = __ldg(a.off + v), e = __ldg(a.off + v + 1);
-        uint32_t p = (uint32_t)v;
+    // A vertex with neighbours starts under the smallest of itself and its first ones.  The others are done: what
+    // follows passes over the compressed index (over all vertices, the 2^26 of a graph with 2^21 edges took 3.8 ms).
+    for (uint64_t v = tid; v < a.V; v += stride)
+        if (!__ldg(a.deg + v)) a.comp[v] = (uint32_t)v;
+    for (uint64_t i = tid; i < a.nlists; i += stride) {
+        const uint64_t b = __ldg(a.off + i), e = __ldg(a.off + i + 1);
+        const uint32_t v = cc_vertex<kIndex>(a.vert, i);
+        uint32_t p = v;
 #pragma unroll
         for (uint32_t k = 0; k < kCcFirst; ++k)
             if (b + k < e) p = min(p, __ldg(a.adj + b + k));
         a.comp[v] = p;
     }
     if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
-    cc_compress(a.comp, a.V, tid, stride);
+    cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
     if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     for (uint32_t k = 0; k < kCcFirst; ++k) {
-        for (uint64_t v = tid; v < a.V; v += stride) {
-            const uint64_t b = __ldg(a.off + v) + k;
-            if (b < __ldg(a.off + v + 1)) cc_unite(a.comp, (uint32_t)v, __ldg(a.adj + b));
+        for (uint64_t i = tid; i < a.nlists; i += stride) {
+            const uint64_t b = __ldg(a.off + i) + k;
+            if (b < __ldg(a.off + i + 1)) cc_unite(a.comp, cc_vertex<kIndex>(a.vert, i), __ldg(a.adj + b));
         }
         if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
-        cc_compress(a.comp, a.V, tid, stride);
+        cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
         if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     }
     // the component of most of a sample's vertices; one CTA decides for all
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < kCcSamples; i += blockDim.x)
-            s_sample[i] = __ldcg(a.comp + (uint64_t)(i * 2654435761u) * a.V / (1ull << 32));
+            s_sample[i] = a.nlists ? __ldcg(a.comp + cc_vertex<kIndex>(a.vert, (uint64_t)(i * 2654435761u) * a.nlists / (1ull << 32))) : 0u;
         __syncthreads();
         for (int i = threadIdx.x; i < kCcSamples; i += blockDim.x) {
             uint32_t same = 0;
@@ -963,13 +975,13 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
     if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
     const uint32_t common = s_slot.common;
     // the other components' lists, from the third neighbour on
-    for (uint64_t base = tid & ~31ull; base < a.V; base += stride) {
-        const uint64_t v = base + lane;
-        const uint32_t vv[1] = {(uint32_t)v};
+    for (uint64_t base = tid & ~31ull; base < a.nlists; base += stride) {
+        const uint64_t i = base + lane;
+        const uint32_t vv[1] = {i < a.nlists ? cc_vertex<kIndex>(a.vert, i) : 0u};
         uint64_t lb[1] = {0}, le[1] = {0};
-        if (v < a.V && __ldcg(a.comp + v) != common) {
-            lb[0] = __ldg(a.off + v) + kCcFirst;
-            le[0] = __ldg(a.off + v + 1);
+        if (i < a.nlists && __ldcg(a.comp + vv[0]) != common) {
+            lb[0] = __ldg(a.off + i) + kCcFirst;
+            le[0] = __ldg(a.off + i + 1);
             if (lb[0] >= le[0]) lb[0] = le[0] = 0;
         }
         append_pieces<1>(lq, wb, vv, lb, le, a.q, &st->slot.n);
@@ -1001,7 +1013,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
             }
         }
         if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
-        cc_compress(a.comp, a.V, tid, stride);
+        cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
     }
     if (tid < 32) persist_clear(a.st_next);
     if (tid == 0) a.result->valid = 1;
@@ -1020,15 +1032,24 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
         EG_TRY(s.vals0.reserve(sizeof(uint32_t) * (V + 1)));
         comp = s.vals0.as<uint32_t>();
     }
-    CcArgs a{V, g->csr_off.as<uint64_t>(), g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(),
+    // The passes go over the compressed index where a quarter of the vertices and more have no neighbours: 2^26 with
+    // 2,000 / 2^21 / 2^26 list entries take 1.84 / 3.8 / 10.0 ms over all vertices and 0.29 / 0.61 / 8.4 so, an
+    // R-MAT of 2^23 / 2^27 1.10 and 0.93.  With next to none the index is 12 bytes a vertex for nothing: uniform
+    // graphs of 2^26 / 2^28 take 14.8 and 17.0, of 2^23 / 2^25 1.45 and 1.65.
+    const uint64_t nitems = g->ncompressed - 1;
+    const bool index = nitems < V - V / 4;
+    CcArgs a{V, index ? nitems : V, g->outdeg.as<uint32_t>(), index ? g->cvert.as<uint32_t>() : nullptr,
+             index ? g->cidx.as<uint64_t>() : g->csr_off.as<uint64_t>(),
+             index ? g->csc_adj.as<uint32_t>() : g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(),
              static_cast<CcState*>(block), next, h, persist_gave_up(g)};
     const size_t smem = sizeof(LocalQueue);
-    EG_CUDA(cudaFuncSetAttribute(k_cc_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const void* fn = index ? (const void*)k_cc_persistent<true> : (const void*)k_cc_persistent<false>;
+    EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)persist_ctas(4 * V, E / 16, (uint64_t)g->num_sms);
     void* kargs[] = {&a};
     {
         Timed t(&g->prof, g->stream, "cc_persistent");
-        EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_cc_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
+        EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPersistThreads), kargs, smem,
                                             g->stream));
         EG_CHECK_LAUNCH("k_cc_persistent");
         persist_launched(g);
