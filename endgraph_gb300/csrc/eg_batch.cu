@@ -852,22 +852,49 @@ __device__ __forceinline__ double warp_sum_f64(double v) {
     return v;
 }
 
-// Row normalisation and its gradient: one warp per CSR task (<= 512 edges of one source), so that a
-// hub's list is spread over warps.  A list of one task is finished by its warp; of a longer one the
-// FP64 partial sums meet in heavy[slot] and its tasks are finished by a second pass (heavy = 1).
-// Bound by the random 4-byte reads of the input-ordered weights; one thread per source took 10.5 ms
-// for 1 M sources and 16 M edges (a hub's list in one thread), a warp per task 0.3 ms.
-//
+// Row normalisation and its gradient over the CSR tasks (<= 512 edges of one source), a batch of them per warp:
+// 32 tasks at a time, each lane those of up to kLane edges by itself (if a few of them are), the warp together the
+// longer ones, so that neither a hub's list nor a graph of short lists leaves lanes idle.  A list of one task
+// is finished here; of a longer one the FP64 partial sums meet in heavy[slot] and its tasks are finished by a
+// second pass (finish_heavy).  Bound by the random 4-byte reads of the input-ordered weights.  Weights of the
+// forward, with one thread per source / a warp per task by stride / so: 1 M R-MAT sources, 16 M edges
+// 7.9 / 0.49 / 0.34 ms; 1 M uniform, 16 M 0.46 / 0.70 / 0.28; 8 M uniform, 8 M 0.34 / 2.8 / 0.24.
+constexpr int kTaskThreads = 64;  // two batches per CTA, 64 warps per SM
+constexpr int kLaneTasks = 4;
+// Uniform lists of 32 edges: weights 0.25 ms with lists of up to 32 edges by a lane, 0.25 up to 16; gradients, with
+// two FP64 reads per edge, 0.34 and 0.27.  Of 16 edges: 0.28 and 0.48; 0.38 and 0.52, as up to 24.
+constexpr uint32_t kLaneWeights = 32, kLaneGrad = 24;
+
+// f(task, k0, step): a lane's own short task with 0, 1; a long one with lane, 32, all lanes together
+template <uint32_t kLane, class F>
+__device__ __forceinline__ void each_task(const uint4* __restrict__ tasks, const uint32_t* __restrict__ first,
+                                          uint32_t nbatches, F f) {
+    const uint32_t lane = threadIdx.x & 31, b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b >= nbatches) return;
+    const uint32_t t1 = __ldg(first + b + 1);
+    for (uint32_t t = __ldg(first + b); t < t1; t += 32) {
+        const uint4 own = t + lane < t1 ? __ldg(tasks + t + lane) : make_uint4(0, 0, 0, kNoSlot);
+        const uint32_t n = task_len(own);
+        const uint32_t some = __ballot_sync(0xffffffffu, n != 0), lng = __ballot_sync(0xffffffffu, n > kLane);
+        const bool lanes = __popc(some & ~lng) >= kLaneTasks;
+        if (lanes && n && n <= kLane) f(own, 0u, 1u);
+        for (uint32_t m = lanes ? lng : some; m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const uint4 rec = make_uint4(__shfl_sync(0xffffffffu, own.x, l), __shfl_sync(0xffffffffu, own.y, l),
+                                         __shfl_sync(0xffffffffu, own.z, l), __shfl_sync(0xffffffffu, own.w, l));
+            f(rec, lane, 32u);
+        }
+    }
+}
+
 // s[u] = sum of u's out-weights; wn[e] = w[eid[e]] / s[u] (null: not wanted)
-__global__ void __launch_bounds__(256) k_out_weights(const uint4* __restrict__ tasks, uint64_t ntasks,
+__global__ void __launch_bounds__(kTaskThreads, 32) k_out_weights(const uint4* __restrict__ tasks,
+                                                     const uint32_t* __restrict__ first, uint32_t nbatches,
                                                      const float* __restrict__ eid, const float* __restrict__ w_in,
                                                      float* __restrict__ s, float* __restrict__ wn,
                                                      double* __restrict__ heavy, int finish_heavy) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
-        const uint4 rec = __ldg(tasks + t);
-        if (finish_heavy && rec.w == kNoSlot) continue;
+    each_task<kLaneWeights>(tasks, first, nbatches, [&](const uint4& rec, uint32_t k0, uint32_t step) {
+        if (finish_heavy && rec.w == kNoSlot) return;
         const uint64_t e0 = task_begin(rec);
         const uint32_t n = task_len(rec);
         float sum;
@@ -875,18 +902,20 @@ __global__ void __launch_bounds__(256) k_out_weights(const uint4* __restrict__ t
             sum = s[rec.z];
         } else {
             double acc = 0;
-            for (uint32_t k = lane; k < n; k += 32) acc += w_in[__float_as_uint(__ldg(eid + e0 + k))];
-            acc = warp_sum_f64(acc);
+#pragma unroll 4
+            for (uint32_t k = k0; k < n; k += step) acc += w_in[__float_as_uint(__ldg(eid + e0 + k))];
+            if (step > 1) acc = warp_sum_f64(acc);
             sum = (float)acc;
-            if (lane == 0) {
+            if (k0 == 0) {
                 if (rec.w == kNoSlot) s[rec.z] = sum;
                 else atomicAdd(heavy + rec.w, acc);
             }
-            if (rec.w != kNoSlot) continue;
+            if (rec.w != kNoSlot) return;
         }
         if (wn)
-            for (uint32_t k = lane; k < n; k += 32) wn[e0 + k] = w_in[__float_as_uint(__ldg(eid + e0 + k))] / sum;
-    }
+#pragma unroll 4
+            for (uint32_t k = k0; k < n; k += step) wn[e0 + k] = w_in[__float_as_uint(__ldg(eid + e0 + k))] / sum;
+    });
 }
 __global__ void k_heavy_out_sums(const uint32_t* __restrict__ heavy_vertex, uint32_t nheavy,
                                  const double* __restrict__ heavy, float* __restrict__ s) {
@@ -1047,33 +1076,33 @@ __global__ void __launch_bounds__(32, 28) k_row_adjoint(RowArgs a, const Row* __
 }
 
 // dL/dw_e = (gA_e - sum_{e' in row(u)} wn_e' gA_e') / s_u, scattered to the input edge order
-__global__ void __launch_bounds__(256) k_weight_grad(const uint4* __restrict__ tasks, uint64_t ntasks,
+__global__ void __launch_bounds__(kTaskThreads, 32) k_weight_grad(const uint4* __restrict__ tasks,
+                                                     const uint32_t* __restrict__ first, uint32_t nbatches,
                                                      const float* __restrict__ wn, const double* __restrict__ gA,
                                                      const float* __restrict__ s, const float* __restrict__ eid,
                                                      float* __restrict__ dw, double* __restrict__ heavy,
                                                      int finish_heavy) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
-        const uint4 rec = __ldg(tasks + t);
-        if (finish_heavy && rec.w == kNoSlot) continue;
+    each_task<kLaneGrad>(tasks, first, nbatches, [&](const uint4& rec, uint32_t k0, uint32_t step) {
+        if (finish_heavy && rec.w == kNoSlot) return;
         const uint64_t e0 = task_begin(rec);
         const uint32_t n = task_len(rec);
         double dot = 0;
         if (finish_heavy) {
             dot = heavy[rec.w];
         } else {
-            for (uint32_t k = lane; k < n; k += 32) dot += wn[e0 + k] * gA[e0 + k];
-            dot = warp_sum_f64(dot);
+#pragma unroll 4
+            for (uint32_t k = k0; k < n; k += step) dot += wn[e0 + k] * gA[e0 + k];
+            if (step > 1) dot = warp_sum_f64(dot);
             if (rec.w != kNoSlot) {
-                if (lane == 0) atomicAdd(heavy + rec.w, dot);
-                continue;
+                if (k0 == 0) atomicAdd(heavy + rec.w, dot);
+                return;
             }
         }
         const float inv = 1.0f / s[rec.z];
-        for (uint32_t k = lane; k < n; k += 32)
+#pragma unroll 4
+        for (uint32_t k = k0; k < n; k += step)
             dw[__float_as_uint(__ldg(eid + e0 + k))] = (float)((gA[e0 + k] - dot) * inv);
-    }
+    });
 }
 
 // ---- batched SSSP: in place, skipping sources whose row did not change in the last sweep --------
@@ -2067,13 +2096,13 @@ static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev, bool want_csr
     if (want_csr) EG_TRY(b.wn_csr.reserve(4 * E + 64));
     EG_TRY(b.s_out.reserve(4 * V + 64));
     EG_TRY(b.heavy_sum.reserve(8ull * t.nheavy + 64));
-    const unsigned grid = (unsigned)g->num_sms * 8u;
+    const unsigned grid = (t.nbatches + kTaskThreads / 32 - 1) / (kTaskThreads / 32);
     const float* eid = g->csr_w.as<float>();
     float* wn = want_csr ? b.wn_csr.as<float>() : nullptr;
     Timed tm(&g->prof, g->stream, "ppr_weights");
     if (t.nheavy) EG_CUDA(cudaMemsetAsync(b.heavy_sum.ptr, 0, 8ull * t.nheavy, g->stream));
     if (g->partitions > 1) EG_CUDA(cudaMemsetAsync(b.s_out.ptr, 0, 4 * V, g->stream));  // sources without a task
-    k_out_weights<<<grid, 256, 0, g->stream>>>(t.rec.as<uint4>(), t.ntasks, eid, w_in_dev, b.s_out.as<float>(), wn,
+    k_out_weights<<<grid, kTaskThreads, 0, g->stream>>>(t.rec.as<uint4>(), t.first.as<uint32_t>(), t.nbatches, eid, w_in_dev, b.s_out.as<float>(), wn,
                                                b.heavy_sum.as<double>(), 0);
     EG_CHECK_LAUNCH("k_out_weights");
     if (t.nheavy) {
@@ -2081,7 +2110,7 @@ static int prepare_ppr_weights(eg_graph* g, const float* w_in_dev, bool want_csr
             t.heavy_vertex.as<uint32_t>(), t.nheavy, b.heavy_sum.as<double>(), b.s_out.as<float>());
         EG_CHECK_LAUNCH("k_heavy_out_sums");
         if (wn) {
-            k_out_weights<<<grid, 256, 0, g->stream>>>(t.rec.as<uint4>(), t.ntasks, eid, w_in_dev, b.s_out.as<float>(),
+            k_out_weights<<<grid, kTaskThreads, 0, g->stream>>>(t.rec.as<uint4>(), t.first.as<uint32_t>(), t.nbatches, eid, w_in_dev, b.s_out.as<float>(),
                                                        wn, nullptr, 1);
             EG_CHECK_LAUNCH("k_out_weights");
         }
@@ -2404,8 +2433,8 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     {
         Timed tm(&g->prof, g->stream, "ppr_weight_grad");
         for (int heavy = 0; heavy <= (tr.nheavy ? 1 : 0); ++heavy) {
-            k_weight_grad<<<(unsigned)g->num_sms * 8u, 256, 0, g->stream>>>(
-                tr.rec.as<uint4>(), tr.ntasks, b.wn_csr.as<float>(), b.gA.as<double>(), b.s_out.as<float>(),
+            k_weight_grad<<<(tr.nbatches + kTaskThreads / 32 - 1) / (kTaskThreads / 32), kTaskThreads, 0, g->stream>>>(
+                tr.rec.as<uint4>(), tr.first.as<uint32_t>(), tr.nbatches, b.wn_csr.as<float>(), b.gA.as<double>(), b.s_out.as<float>(),
                 g->csr_w.as<float>(), dw, b.heavy_sum.as<double>(), heavy);
             EG_CHECK_LAUNCH("k_weight_grad");
         }
