@@ -91,6 +91,9 @@ struct MsSweepArgs {
     uint64_t E;
     uint64_t nruns;           // runs of kPrBlock << shift edges
     int shift;
+    uint32_t nitems;
+    const unsigned long long* alive;     // roots still running: a vertex that has them all gains nothing (null: not
+                                         // looked at; in a graph batch no vertex has the roots of all graphs)
     const unsigned long long* front;
     const unsigned long long* front_bm;  // 1 bit per vertex: front[v] != 0
     int screen;                          // consult front_bm before gathering
@@ -141,6 +144,7 @@ __global__ void __launch_bounds__(kMsThreads, 1) k_ms_sweep(MsSweepArgs a) {
         return v;
     };
     const uint64_t run_edges = (uint64_t)kPrBlock << a.shift;
+    const unsigned long long al = a.alive ? __ldg(a.alive) : 0ull;
     uint32_t ticket = 0;
     if (lane == 0) ticket = atomicAdd(a.ticket, 1u);
     __syncthreads();
@@ -150,6 +154,15 @@ __global__ void __launch_bounds__(kMsThreads, 1) k_ms_sweep(MsSweepArgs a) {
         if (lane == 0) ticket = atomicAdd(a.ticket, 1u);
         const uint64_t e_begin = run * run_edges, e_end = min(a.E, e_begin + run_edges);
         uint32_t item = __ldg(a.item_of + (run << a.shift));
+        // Few lists, all of whose vertices have every running root: nothing to read.  With few roots the first dense
+        // level of a dense graph finds most vertices so (1,000 vertices, 2^26 edges, 3 roots: 1.42 -> 0.03 ms).
+        if (al) {
+            const uint32_t last_item = run + 1 < a.nruns ? __ldg(a.item_of + ((run + 1) << a.shift)) : a.nitems - 1;
+            if (last_item - item < 32) {
+                const bool idle = lane > last_item - item || !(al & ~__ldcg(a.visit + __ldg(a.cvert + item + lane)));
+                if (__all_sync(0xffffffffu, idle)) continue;
+            }
+        }
         bool open_first = !(__ldg(a.heads + (e_begin >> 5)) & 1u);  // the first list began in an earlier run
         unsigned long long carry = 0;                                // OR of the open list so far
         for (uint64_t e0 = e_begin; e0 < e_end; e0 += kMsBlock) {
@@ -1590,6 +1603,8 @@ static int ms_sweep(eg_graph* g, const uint32_t* adj, const unsigned long long* 
     a.E = g->E;
     a.shift = list_run_shift(g->E);
     a.nruns = (g->E + ((uint64_t)kPrBlock << a.shift) - 1) / ((uint64_t)kPrBlock << a.shift);
+    a.nitems = (uint32_t)(g->ncompressed - 1);
+    a.alive = g->batch_voff.empty() ? alive : nullptr;
     a.front = front;
     a.front_bm = front_bm;
     a.screen = screen;

@@ -378,3 +378,40 @@ def test_msbfs_dense_levels_with_hot_sources(eg_lib, V, E):
         ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(roots[k]))
         got = levels[1][k].astype(np.uint32)
         assert np.array_equal(np.where(ref == oracle.UNREACHED, 255, ref), got), k
+
+
+@pytest.mark.parametrize("V,E", [(40, 1 << 15), (1000, 1 << 20), (1000, 1 << 25), (3000, 400_000)])
+@pytest.mark.parametrize("n", [1, 3, 64])
+def test_msbfs_dense_level_of_covered_vertices(eg_lib, V, E, n):
+    """Graphs so dense that a level pushed from the roots reaches (nearly) every vertex: the dense level after it
+    finds whole runs of lists that have every root, next to vertices without in-edges from there, and
+    a component that none of the roots reaches."""
+    import torch
+
+    import endgraph_gb300 as eg
+    gen = torch.Generator("cuda").manual_seed(V + n)
+    a = V - V // 10
+    rec = torch.randint(0, a, (E, 2), generator=gen, device="cuda", dtype=torch.int32)
+    rec[: E // 16] = torch.randint(a, V, (E // 16, 2), generator=gen, device="cuda", dtype=torch.int32)
+    rec[E // 16: E // 16 + 5, 1] = a  # one edge and a few from the first component into the second
+    rec = rec.contiguous()
+    roots = torch.randint(0, a, (n,), generator=gen, device="cuda").cpu().numpy().astype(np.uint32)
+    e = rec.cpu().numpy().view(np.uint32)
+    csr = oracle.build_csr(e[:, 0].copy(), e[:, 1].copy(), None, V, np.array([0, V], np.uint32))
+    with eg.Graph() as g:
+        g.load_directed(rec, V)
+        for div in (20, 1, 1 << 30):
+            g.set_option(eg.EG_OPT_BATCH_DIVISOR, div)
+            levels, _ = g.msbfs(roots)
+            for s, r in enumerate(roots):
+                ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(r))
+                assert np.array_equal(levels[s], np.where(ref == oracle.UNREACHED, 255, ref).astype(np.uint8)), (div, s)
+        if E >= 1 << 25 and n == 3:
+            g.set_option(eg.EG_OPT_BATCH_DIVISOR, 20)
+            g.profile(True)
+            best = 1e9
+            for _ in range(4):
+                g.profile_reset()
+                g.msbfs(roots)
+                best = min(best, g.profile_read()["msbfs_pull"][1])
+            assert best <= 0.2, best  # 2^25 ids read in vain take 0.7
