@@ -487,8 +487,9 @@ __global__ void k_reach_edges(const unsigned long long* __restrict__ visit, cons
 // level planes -> [n][V] root rows for the first n roots, 256 vertices per CTA: 64 level bytes per vertex
 // into shared memory, 4 x 4 bytes at a time turned into 16 consecutive vertices of a root, and every
 // root's row stored in whole 16-byte pieces of the output whatever its alignment (V odd: each row
-// starts elsewhere), the row's first and last bytes one by one.  64 roots at 2^23: 0.30 ms (0.87 GB), and
-// 0.33 at 2^23 - 1; from level rows, with a byte per load and 16-byte stores only where V allows, 0.26 and 2.0.
+// starts elsewhere), the row's first and last bytes one by one.  64 roots at 2^23: 0.28 ms (0.87 GB), one
+// root 0.09 (0.24 with all columns made); from level rows, with a byte per load and 16-byte stores only where V allows,
+// 0.26, and 2.0 at 2^23 - 1.
 constexpr uint32_t kOutTile = 256;
 constexpr uint32_t kOutStride = kOutTile / 4 + 4;  // words per root row in shared memory
 __global__ void __launch_bounds__(256) k_levels_out(const unsigned long long* __restrict__ planes,
@@ -497,8 +498,9 @@ __global__ void __launch_bounds__(256) k_levels_out(const unsigned long long* __
     __shared__ uint32_t t[kOutTile][17];                      // [vertex][root / 4]
     __shared__ __align__(16) uint32_t u[64][kOutStride];      // [root][vertex / 4]
     const uint64_t v0 = (uint64_t)blockIdx.x * kOutTile;
-    for (uint32_t i = threadIdx.x; i < 4 * kOutTile; i += blockDim.x) {
-        const uint32_t r = i >> 2, q = i & 3;
+    const uint32_t quads = ((uint32_t)n + 15) / 16;  // of 16 columns that the call has
+    for (uint32_t i = threadIdx.x; i < quads * kOutTile; i += blockDim.x) {
+        const uint32_t r = i % kOutTile, q = i / kOutTile;
         const uint4 x = v0 + r < V ? level_bytes(planes, visit, V, v0 + r, (int)q, deep) : make_uint4(~0u, ~0u, ~0u, ~0u);
         t[r][4 * q] = x.x;
         t[r][4 * q + 1] = x.y;
@@ -506,8 +508,8 @@ __global__ void __launch_bounds__(256) k_levels_out(const unsigned long long* __
         t[r][4 * q + 3] = x.w;
     }
     __syncthreads();
-    {
-        const uint32_t rq = threadIdx.x & 15, vg = threadIdx.x >> 4;  // roots 4 rq .. + 3, vertices 16 vg .. + 15
+    const uint32_t rq = threadIdx.x & 15, vg = threadIdx.x >> 4;  // roots 4 rq .. + 3, vertices 16 vg .. + 15
+    if (4 * rq < (uint32_t)n) {
         uint32_t row[4][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {

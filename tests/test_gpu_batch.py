@@ -415,3 +415,24 @@ def test_msbfs_dense_level_of_covered_vertices(eg_lib, V, E, n):
                 g.msbfs(roots)
                 best = min(best, g.profile_read()["msbfs_pull"][1])
             assert best <= 0.2, best  # 2^25 ids read in vain take 0.7
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 15, 16, 17, 20, 31, 32, 33, 47, 48, 49, 63, 64])
+@pytest.mark.parametrize("V", [255, 1021])
+def test_level_rows_of_some_columns(eg_lib, n, V):
+    import torch
+
+    import endgraph_gb300 as eg
+    rng = np.random.default_rng(n)
+    src, dst = rng.integers(0, V, 4 * V).astype(np.uint32), rng.integers(0, V, 4 * V).astype(np.uint32)
+    roots = rng.integers(0, V, n).astype(np.uint32)
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        buf = torch.full((n * V + 32,), 0x77, dtype=torch.uint8, device="cuda")
+        g.msbfs(roots, levels=buf[7:7 + n * V].view(n, V))
+        got = buf.cpu().numpy()
+    assert (got[:7] == 0x77).all() and (got[7 + n * V:] == 0x77).all()
+    for s, r in enumerate(roots):
+        ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(r))
+        assert np.array_equal(got[7 + s * V: 7 + (s + 1) * V], np.where(ref == oracle.UNREACHED, 255, ref).astype(np.uint8)), s
