@@ -367,7 +367,7 @@ struct MsBfsPushOp {
 };
 
 // A traversal keeps its levels as bit planes, [V][4] words for bits 0..3 of the level of each root and
-// [V][4] more for bits 4..7 (zeroed before the first level past 15): a vertex that new roots reach at
+// [V][4] more for bits 4..7 (zeroed before the first level past 15: kHighPlanes): a vertex that new roots reach at
 // level l gets their bits ORed into the planes of l, or, when they are its first, its four words
 // written without a read (which is what clears them).  A level touches a sector per vertex where rows
 // of 64 level bytes took a read and a write of up to two; the bytes are made once, at the end.  64
@@ -414,6 +414,14 @@ __global__ void k_queue_levels(const uint32_t* __restrict__ q, const uint32_t* n
                                unsigned long long* planes, uint64_t V, uint32_t lvl, unsigned long long* alive_out,
                                const uint32_t* __restrict__ new_id, unsigned long long* __restrict__ next_r) {
     queue_levels_work(q, __ldcg(n_dev), next, visit, planes, V, lvl, alive_out, new_id, next_r);
+}
+
+// The upper planes (bits 4..7) are zeroed as this level begins, whose vertices are the first to have level 16: not
+// ahead of time for traversals that hardly ever get there.
+constexpr uint32_t kHighPlanes = 15;
+__global__ void k_zero_planes(unsigned long long* __restrict__ planes, uint64_t n, const uint32_t* frontier) {
+    if (!*frontier) return;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) planes[i] = 0ull;
 }
 
 // level bytes of 16 roots (16 q .. 16 q + 15) of vertex v, 0xFF where the root never reached it
@@ -1534,6 +1542,8 @@ __global__ void __launch_bounds__(256, 4) k_msbfs_persistent(MsPersistArgs a) {
                 for (uint64_t i = tid; i < n_old; i += stride) next[q_next[i]] = 0ull;
             }
             for (uint64_t i = tid; i < a.nwords; i += stride) next_bm[i] = 0ull;
+            if (a.lev && L == kHighPlanes)
+                for (uint64_t i = tid; i < 4 * a.V; i += stride) a.lev[4 * a.V + i] = 0ull;
             if (!dense) {
                 const uint64_t tiles = ((uint64_t)n * a.P + kScanTile - 1) / kScanTile + 1;
                 for (uint64_t i = tid; i < tiles; i += stride) a.desc[i] = 0ull;
@@ -1673,9 +1683,6 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
         EG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (kGraphLevels + 2), g->stream));
         EG_CUDA(cudaMemcpyAsync(alive + 2, &full, 8, cudaMemcpyHostToDevice, g->stream));
         EG_CUDA(cudaMemcpyAsync(alive, &full, 8, cudaMemcpyHostToDevice, g->stream));
-        // bits 4..7 of the levels: where the loop runs on the device, ahead of time
-        if (lev && (g->batch_launch == 1 || (g->use_cuda_graph & 1)))
-            EG_CUDA(cudaMemsetAsync(lev + 4 * V, 0, 32 * V, g->stream));
         k_msbfs_init_entries<<<init_grid, 256, 0, g->stream>>>(b.entries.as<uint2>(), b.n_entries.as<uint32_t>(), visit,
                                                                word[0], bm[0], lev, queue[0], d_nq, d_act, deg);
         EG_CHECK_LAUNCH("k_msbfs_init_entries");
@@ -1744,7 +1751,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
         }
         if (lev || alive_next || renum) {
             Timed t(&g->prof, g->stream, "msbfs_vertex");
-            if (lev && L + 1 == 16 && !(g->batch_launch == 1 || (g->use_cuda_graph & 1)))
+            if (lev && L == kHighPlanes)
                 EG_CUDA(cudaMemsetAsync(lev + 4 * V, 0, 32 * V, g->stream));
             k_queue_levels<<<grid, 256, 0, g->stream>>>(queue[x], count, word[x], visit, lev, V, L + 1, alive_next,
                                                         renum ? new_id : nullptr, word_r[x]);
@@ -1895,6 +1902,10 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
                 k_cap_decide<<<1, 1, 0, g->stream>>>(cs, (int)L, n_cur, act_cur, dense_min, one_graph ? 1 : 0,
                                                      g->built_csr ? 1 : 0);
                 ok(cudaGetLastError());
+                if (lev && L == kHighPlanes) {
+                    k_zero_planes<<<grid, 256, 0, g->stream>>>(lev + 4 * V, 4 * V, n_cur);
+                    ok(cudaGetLastError());
+                }
                 if (L >= 1) {  // the frontier words written two levels back (level 1: the roots)
                     const uint32_t* n_old = L == 1 ? d_nq : cnt + L - 2;
                     k_clear_front_dev<<<grid, 256, 0, g->stream>>>(queue[x], n_old, word[x], V, cs);

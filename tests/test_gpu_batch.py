@@ -417,6 +417,37 @@ def test_msbfs_dense_level_of_covered_vertices(eg_lib, V, E, n):
             assert best <= 0.2, best  # 2^25 ids read in vain take 0.7
 
 
+@pytest.mark.parametrize("cuda_graph,persistent", [(0, 0), (1, 0), (0, 1)])
+def test_level_planes_from_dirty_memory(eg_lib, cuda_graph, persistent):
+    """Traversals that end just before, at and after the level that needs the upper planes, in turn with deep ones
+    that leave them full."""
+    import endgraph_gb300 as eg
+    n = 300
+    i = np.arange(n - 1, dtype=np.uint32)
+    # tails of 13 to 20 vertices, and one chain of 250: every vertex of a tail is as deep as its place
+    src, dst, starts, at = [i[:249]], [i[:249] + 1], [0], 260
+    with eg.Graph() as g:
+        for length in range(13, 21):
+            c = np.arange(at, at + length, dtype=np.uint32)
+            src.append(c[:-1])
+            dst.append(c[1:])
+            starts.append(at)
+            at += length
+        V = at + 100
+        src, dst = np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+        csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+        refs = {r: oracle.bfs_levels(csr["off"][0], csr["adj"], V, r) for r in starts}
+        refs = {r: np.where(x == oracle.UNREACHED, 255, x).astype(np.uint8) for r, x in refs.items()}
+        g.load_directed(eg.pack_edges(src, dst), V)
+        g.set_option(eg.EG_OPT_CUDA_GRAPH, cuda_graph)
+        g.set_option(eg.EG_OPT_BATCH_LAUNCH, persistent)
+        for r in starts + starts[::-1]:
+            for roots in ([r], [0, r], [r, r, r], [starts[1]] * 17 + [r]):
+                levels, _ = g.msbfs(np.array(roots, np.uint32))
+                for s, root in enumerate(roots):
+                    assert np.array_equal(levels[s], refs[root]), (r, s)
+
+
 @pytest.mark.parametrize("n", [1, 2, 4, 5, 15, 16, 17, 20, 31, 32, 33, 47, 48, 49, 63, 64])
 @pytest.mark.parametrize("V", [255, 1021])
 def test_level_rows_of_some_columns(eg_lib, n, V):
