@@ -483,6 +483,9 @@ struct BfsPersistArgs {
     const uint32_t* cvert;
     uint32_t* level;
     uint32_t* parent;  // null: not wanted
+    unsigned long long* vis;   // kBits: reached vertices, and those of before the dense level
+    unsigned long long* snap;
+    uint64_t nwords;
     uint4* q[2];
     unsigned long long* seg;  // (segment << 32) | compressed entry
     uint32_t root;
@@ -495,6 +498,14 @@ struct BfsPersistArgs {
     uint32_t* gave_up;
 };
 
+// Levels as the only record of what is reached are gathered from L2 while they fit it.  Past that (kBits) one bit per
+// vertex says that it is reached (the level is stored before the bit may be seen; a bit that comes late costs a
+// compare-and-swap that fails), and a dense level looks for parents in a copy of the bits from before it: a
+// reached in-neighbour of an unreached vertex is in the frontier, or the vertex would have been reached with it.
+__device__ __forceinline__ bool bit_at(const unsigned long long* w, uint32_t v) { return (__ldcg(w + (v >> 6)) >> (v & 63)) & 1ull; }
+__device__ __forceinline__ void set_bit(unsigned long long* w, uint32_t v) { atomicOr(w + (v >> 6), 1ull << (v & 63)); }
+
+template <bool kBits>
 __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persistent(BfsPersistArgs a) {
     __shared__ BfsSlot s_slot;
     __shared__ uint32_t s_verts;
@@ -522,6 +533,8 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
             a.level[v] = v == a.root ? 0u : kUnreached;
             if (a.parent) a.parent[v] = v == a.root ? (uint32_t)v : (uint32_t)a.V;
         }
+        if (kBits)
+            for (uint64_t i = tid; i < a.nwords; i += stride) a.vis[i] = i == a.root >> 6 ? 1ull << (a.root & 63) : 0ull;
         if (tid < 32) {  // the root's pieces
             const uint64_t b = a.off[a.root], z = a.off[(uint64_t)a.root + 1];
             const uint32_t np = (uint32_t)((z - b + kPiece - 1) / kPiece);
@@ -609,7 +622,8 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                         x[j] = r < total ? __ldg(a.adj + pos) : a.root;
                     }
 #pragma unroll
-                    for (int j = 0; j < kIlp; ++j) open[j] = __ldcg(a.level + x[j]) == kUnreached;
+                    for (int j = 0; j < kIlp; ++j)
+                        open[j] = kBits ? !bit_at(a.vis, x[j]) : __ldcg(a.level + x[j]) == kUnreached;
 #pragma unroll
                     for (int j = 0; j < kIlp; ++j) {
                         lb[j] = le[j] = 0;
@@ -617,6 +631,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                             const uint32_t old = atomicCAS(a.level + x[j], kUnreached, lvl + 1);
                             const uint64_t b = __ldg(a.off + x[j]), z = __ldg(a.off + (uint64_t)x[j] + 1);
                             if (old == kUnreached) {
+                                if (kBits) set_bit(a.vis, x[j]);
                                 if (a.parent) a.parent[x[j]] = par[j];
                                 lb[j] = b;
                                 le[j] = z;
@@ -631,11 +646,17 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
             ++pushes;
             if (!end_phase(true)) return;
         } else {
+            if (kBits) {
+                for (uint64_t i = tid; i < a.nwords; i += stride) a.snap[i] = __ldcg(a.vis + i);
+                if (!step_barrier(st, a.gave_up, &st->slot[step & 3], &s_slot, arrived)) return;
+            }
+            auto unreached = [&](uint32_t v) { return kBits ? !bit_at(a.vis, v) : __ldcg(a.level + v) == kUnreached; };
+            auto in_front = [&](uint32_t u) { return kBits ? bit_at(a.snap, u) : __ldcg(a.level + u) == lvl; };
             // a list's vertex is loaded two rounds ahead, its level and bounds one round ahead
             uint64_t i = tid;
             uint32_t v1 = i < a.nitems ? __ldg(a.cvert + i) : kUnreached;
             uint32_t v2 = i + stride < a.nitems ? __ldg(a.cvert + i + stride) : kUnreached;
-            bool open1 = v1 < a.V && __ldcg(a.level + v1) == kUnreached;
+            bool open1 = v1 < a.V && unreached(v1);
             uint64_t p1 = i < a.nitems ? __ldg(a.cidx + i) : 0, e1 = i < a.nitems ? __ldg(a.cidx + i + 1) : 0;
             for (uint64_t base = tid & ~31ull; base < a.nitems; base += stride, i += stride) {
                 const uint32_t v = v1;
@@ -645,7 +666,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 uint32_t par = kUnreached, len = 0, nsg = 0;
                 v1 = v2;
                 v2 = i + 2 * stride < a.nitems ? __ldg(a.cvert + i + 2 * stride) : kUnreached;
-                open1 = v1 < a.V && __ldcg(a.level + v1) == kUnreached;
+                open1 = v1 < a.V && unreached(v1);
                 if (i + stride < a.nitems) {
                     p1 = __ldg(a.cidx + i + stride);
                     e1 = __ldg(a.cidx + i + stride + 1);
@@ -658,7 +679,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
 #pragma unroll
                         for (int j = 0; j < 4; ++j) u[j] = x + j < h ? __ldg(a.csc_adj + x + j) : a.root;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) hit[j] = x + j < h && __ldcg(a.level + u[j]) == lvl;
+                        for (int j = 0; j < 4; ++j) hit[j] = x + j < h && in_front(u[j]);
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
                             if (hit[j]) par = u[j];
@@ -690,7 +711,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                         }
 #pragma unroll
                         for (int j = 0; j < kIlp; ++j)
-                            if (want[j] && __ldcg(a.level + u[j]) == lvl) *(volatile uint32_t*)(found + o[j]) = u[j];
+                            if (want[j] && in_front(u[j])) *(volatile uint32_t*)(found + o[j]) = u[j];
                     }
                     __syncwarp();
                     if (len) par = found[lane];
@@ -708,6 +729,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 uint64_t lb[1] = {0}, le[1] = {0};
                 if (open && par != kUnreached) {  // this lane owns v's only list
                     a.level[v] = lvl + 1;
+                    if (kBits) set_bit(a.vis, v);
                     if (a.parent) a.parent[v] = par;
                     lb[0] = __ldg(a.off + v);
                     le[0] = __ldg(a.off + (uint64_t)v + 1);
@@ -738,12 +760,13 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                         for (int j = 0; j < kIlp; ++j) {
                             const uint64_t x = p + 32 * j + lane;
                             const uint32_t u = x < pe ? __ldg(a.csc_adj + x) : a.root;
-                            if (x < pe && __ldcg(a.level + u) == lvl) cand = u;
+                            if (x < pe && in_front(u)) cand = u;
                         }
                         const unsigned m = __ballot_sync(0xffffffffu, cand != kUnreached);
                         if (!m) continue;
                         const uint32_t par = __shfl_sync(0xffffffffu, cand, __ffs(m) - 1);
                         if (lane == 0 && atomicCAS(a.level + v, kUnreached, lvl + 1) == kUnreached) {
+                            if (kBits) set_bit(a.vis, v);
                             if (a.parent) a.parent[v] = par;
                             lb[0] = __ldg(a.off + v);
                             le[0] = __ldg(a.off + (uint64_t)v + 1);
@@ -771,6 +794,12 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
         *a.result = PersistResult{1u, s_slot.verts == 0 ? 1u : 0u, step, st->pushes, st->pulls, 0u, reached, edges};
     }
 }
+
+// Bits from more than this many vertices on.  Means of four roots, levels alone / host-driven levels with bitmaps
+// before them / bits, in ms: R-MAT 2^22 / 2^26 0.21 / 0.52 / 0.22, 2^23 / 2^27 0.33 / 0.63 / 0.33, 2^24 / 2^28 0.59 / 0.88 /
+// 0.55, 2^25 / 2^29 1.08 / 1.33 / 0.92, 2^27 / 2^30 3.91 / 3.54 / 2.47; uniform 2^20 / 2^24 0.17 / 1.00 / 0.19, 2^23 / 2^24
+// 1.22 / 3.03 / 1.21, 2^26 / 2^27 10.6 / 9.8 / 8.1, 2^27 / 2^28 23.3 / 18.3 / 16.6.
+constexpr uint64_t kBfsBits = 1ull << 23;
 
 int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached) {
     const uint64_t V = g->V, E = g->E;
@@ -808,8 +837,15 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     a.st = static_cast<BfsPersistState*>(block);
     a.result = reinterpret_cast<PersistResult*>(s.host_words);
     a.gave_up = persist_gave_up(g);
+    const bool bits = V > kBfsBits;
+    a.nwords = V / 64 + 1;
+    if (bits)
+        for (DevBuf* w : {&s.bm_visit, &s.bm_front}) EG_TRY(w->reserve(sizeof(uint64_t) * a.nwords));
+    a.vis = s.bm_visit.as<unsigned long long>();
+    a.snap = s.bm_front.as<unsigned long long>();
+    const void* fn = bits ? (const void*)k_bfs_persistent<true> : (const void*)k_bfs_persistent<false>;
     const size_t smem = sizeof(LocalQueue);
-    EG_CUDA(cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
     volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
@@ -817,7 +853,7 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
         void* kargs[] = {&a};
         {
             Timed t(&g->prof, g->stream, "bfs_persistent");
-            EG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_persistent, dim3(grid), dim3(kPersistThreads), kargs, smem,
+            EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPersistThreads), kargs, smem,
                                                 g->stream));
             EG_CHECK_LAUNCH("k_bfs_persistent");
             if (!a.resume) persist_launched(g);

@@ -235,3 +235,40 @@ def test_barrier_given_up_as_it_completes(eg_lib, spin_cap):
             assert np.array_equal(g.bfs(0)[0], np.arange(n))
             assert np.array_equal(g.sssp(0), np.arange(n, dtype=np.float32))
             assert not g.cc().any()
+
+
+def _spread(src, dst, n, V, seed):
+    """A graph over n vertices moved to random ids of V."""
+    ids = np.random.default_rng(seed).choice(V, n, replace=False)
+    return ids[src], ids[dst], ids
+
+
+@pytest.mark.parametrize("deg", [1, 13, 257, 1036, 1037, 5000])
+def test_bfs_bits_list_edges(eg_lib, deg):
+    """More vertices than the traversal keeps levels alone for: reached vertices are bits as well, copied before
+    each dense level.  Lists at the edges of a dense level's phases, half of them read in vain."""
+    V, n = (1 << 23) + 1, 40_000
+    rng = np.random.default_rng(deg)
+    nbr, back = rng.choice(n - 10, deg, replace=False) + 10, rng.choice(n - 10, deg, replace=False) + 10
+    src = np.concatenate([np.full(deg, 7), back, rng.integers(10, n // 2, 60_000)])
+    dst = np.concatenate([nbr, np.full(deg, 7), rng.integers(10, n // 2, 60_000)])
+    s, d, ids = _spread(src, dst, n, V, deg)
+    _check_bfs(s, d, V, [int(ids[7]), int(s[-1])], divisors=(1, 20))
+
+
+def test_bfs_bits_sizes(eg_lib):
+    """On both sides of the switch, and a vertex count that fills its last word of bits."""
+    rng = np.random.default_rng(3)
+    src, dst = rng.integers(0, 30_000, 200_000), rng.integers(0, 30_000, 200_000)
+    for V in (1 << 23, (1 << 23) + 1, (1 << 23) + 63, (1 << 23) + 64):
+        s, d, ids = _spread(src, dst, 30_000, V, V & 7)
+        s[0], d[0], s[1], d[1] = ids[0], V - 1, V - 1, 0
+        _check_bfs(s, d, V, [int(ids[0]), V - 1, 0])
+
+
+def test_bfs_bits_deeper_than_one_launch(eg_lib):
+    n, V = 9_000, (1 << 23) + 100
+    i = np.arange(n - 1)
+    s, d, ids = _spread(i, i + 1, n, V, 8)
+    _check_bfs(s, d, V, [int(ids[0])], directions=(0, 1))
+    _check_bfs(s, d, V, [int(ids[n - 300])])
