@@ -374,11 +374,13 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
 // that R-MAT distances need one or two phases; larger ones gain more from relaxing less.  Times in
 // ms with 0.7 / 3 / 100 x mean weight / mean degree: 20 k vertices, 300 k edges 1.14 / 0.51 / 0.28; 200 k,
 // 4 M 1.99 / 0.87 / 0.56; 1 M, 8 M 1.42 / 1.07 / 0.88; 2 M, 64 M 4.4 / 2.9 / 3.7; 4 M, 20 M 1.8 / 2.4 / 3.1; 4 M,
-// 67 M 3.8 / 3.8 / 5.4 (a tenth of the mean weight is 1.6 to 3.2 of these units there).
+// 67 M 3.8 / 3.8 / 5.4 (a tenth of the mean weight is 1.6 to 3.2 of these units there, and less than 0.7 of them on
+// sparser graphs, which then take as many phases for nothing: with 0.1 / 0.7 / deg of the mean weight 4 M vertices,
+// 8 M edges 5.7 / 2.5, a star of 4 M 0.57 / 0.17, a grid of 2000 x 2000 233 / 161).
 static float auto_delta(uint64_t V, uint64_t E) {
     const float deg = (float)std::max((double)E / (double)V, 1.0);
     if (V <= (1u << 20)) return 100.f / deg;
-    if (V <= (1u << 23)) return 0.1f;
+    if (V <= (1u << 23)) return std::max(0.1f, 0.7f / deg);
     return 0.7f / deg;
 }
 
