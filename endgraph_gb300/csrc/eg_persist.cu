@@ -389,7 +389,8 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EngineState& s = g->eng;
     EG_TRY(s.vals1.reserve(sizeof(uint32_t) * (V + 1)));
     EG_TRY(s.bm_visit.reserve(sizeof(uint64_t) * (V / 64 + 1)));
-    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
+    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(V, E, grid)));
     float* d_dist = dist;
     if (where != EG_DEVICE || !plain_device(g, dist, 4)) {
         EG_TRY(s.vals0.reserve(sizeof(float) * (V + 1)));
@@ -417,7 +418,6 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
     volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
@@ -806,7 +806,8 @@ constexpr uint64_t kBfsBits = 1ull << 23;
 int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* parent, int where, uint64_t* reached) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
-    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
+    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
+    for (DevBuf* q : {&s.pieces0, &s.pieces1}) EG_TRY(q->reserve(sizeof(uint4) * queue_entries(V, E, grid)));
     BfsPersistArgs a;
     a.level = level;
     a.parent = parent;
@@ -848,7 +849,6 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     const void* fn = bits ? (const void*)k_bfs_persistent<true> : (const void*)k_bfs_persistent<false>;
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)persist_ctas(V, E, (uint64_t)g->num_sms);
     volatile PersistResult* h = a.result;
     for (a.resume = 0;; a.resume = 1) {
         if (a.resume) EG_CUDA(cudaMemsetAsync(&a.st->bar_count, 0, sizeof(unsigned), g->stream));
@@ -1060,7 +1060,8 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
 int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     const uint64_t V = g->V, E = g->E;
     EngineState& s = g->eng;
-    EG_TRY(s.pieces0.reserve(sizeof(uint4) * queue_entries(g->V, g->E, (uint64_t)g->num_sms)));
+    const unsigned grid = (unsigned)persist_ctas(4 * V, E / 16, (uint64_t)g->num_sms);
+    EG_TRY(s.pieces0.reserve(sizeof(uint4) * queue_entries(V, E, grid)));
     static_assert(sizeof(CcState) <= kPersistBytes, "one block of the state words");
     void *block = nullptr, *next = nullptr;
     EG_TRY(persist_block(g, &block, &next));
@@ -1083,7 +1084,6 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     const size_t smem = sizeof(LocalQueue);
     const void* fn = index ? (const void*)k_cc_persistent<true> : (const void*)k_cc_persistent<false>;
     EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)persist_ctas(4 * V, E / 16, (uint64_t)g->num_sms);
     void* kargs[] = {&a};
     {
         Timed t(&g->prof, g->stream, "cc_persistent");

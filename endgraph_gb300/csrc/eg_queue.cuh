@@ -63,10 +63,10 @@ struct WarpBlock {  // the warp's block of the global queue, the same in every l
 };
 
 // Entries of one step's queue: the pieces (a vertex's list is queued at most once per step) and the
-// unfinished blocks.
-inline uint64_t queue_entries(uint64_t V, uint64_t E, uint64_t num_sms) {
-    const uint64_t pieces = (V < E ? V : E) + E / kPiece;
-    return pieces + num_sms * kPersistCtas * (kPersistThreads / 32) * kQueueBlock + 64;
+// unfinished blocks of the warps of CTAs that can fill their shared part at all.
+inline uint64_t queue_entries(uint64_t V, uint64_t E, uint64_t ctas) {
+    const uint64_t pieces = (V < E ? V : E) + E / kPiece, full = pieces / kLocalQueue;
+    return pieces + (ctas < full ? ctas : full) * (kPersistThreads / 32) * kQueueBlock + 64;
 }
 
 }  // namespace eg

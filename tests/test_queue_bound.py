@@ -15,8 +15,8 @@ def count(tmp_path_factory):
                         os.path.join(ROOT, "tests", "queue", "queue_bound.cpp"), "-o", exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
 
-    def run(V, E, phases, sms=152, ctas=None, seed=1, keep=1):
-        args = [V, E, sms, ctas if ctas is not None else 2 * sms, seed, keep, *phases]
+    def run(V, E, phases, ctas=304, seed=1, keep=1, few=0):
+        args = [V, E, ctas, seed, keep, few, *phases]
         r = subprocess.run([exe, *map(str, args)], capture_output=True, text=True)
         assert r.returncode == 0
         return [int(x) for x in r.stdout.split()]
@@ -42,3 +42,23 @@ def test_dense_level_of_two_phases(count, seed):
     # with a block left open per warp and phase the same level would not fit
     used, reserved, _ = count(V, E, phases, seed=seed, keep=0)
     assert used > reserved
+
+
+@pytest.mark.parametrize("few", [0, 1])
+@pytest.mark.parametrize("ctas", [1, 2, 9, 50, 304])
+@pytest.mark.parametrize("per", [1, 3, 32, 100, 257, 2048, 2049])
+@pytest.mark.parametrize("vertices", [100, 2049, 5000, 40_000, 300_000])
+def test_levels_of_any_size(count, few, ctas, per, vertices):
+    """Levels that reach every vertex, in one phase and in two, appended in equal parts: from queues that no CTA's
+    shared part overflows to ones where all do."""
+    appends = -(-vertices // per)
+    for phases in ([f"{appends}:{per}"], [f"{appends // 2}:{per}", f"{appends - appends // 2}:{per}"]):
+        used, reserved, pieces = count(appends * per, appends * per, phases, ctas=ctas, seed=per, few=few)
+        assert pieces == appends * per and pieces <= used <= reserved
+
+
+def test_small_graphs_reserve_what_they_can_use(count):
+    """1,000 vertices and 8,000 edges fit one CTA's shared part: nothing for unfinished blocks (1.2 M entries, 19 MB a
+    queue, when every warp of the GPU counted)."""
+    assert count(1000, 8000, ["1000:1"], ctas=3)[1] <= 1000 + 8000 // 256 + 64
+    assert count(100_003, 1_000_003, ["103909:1"], ctas=304)[1] <= 310_000
