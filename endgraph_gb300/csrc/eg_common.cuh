@@ -269,7 +269,8 @@ constexpr uint32_t kPrBlock = 512;
 int setup_list_heads(eg_graph* g, bool relabel);  // relabel: with places in renumbered order
 int list_run_shift(uint64_t E);
 int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, int where);
-int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where);
+// chunked: with the chunked pull sweep of several partitions also on one (what eg_autotune sizes a grid for)
+int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where, bool chunked = false);
 // renumbering of the CSC sources by out-degree class (eng.pr_new_id / eng.pr_adj), built once per
 // structure build and shared by the PageRank and bit-parallel BFS pull gathers
 bool want_relabel(const eg_graph* g);

@@ -681,10 +681,10 @@ static int build_bfs_graph(eg_graph* g) {
 }
 
 // ---------------------------------------------------------------------------------------------
-int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where) {
+int run_pagerank(eg_graph* g, int iterations, float damping, float* out, int where, bool chunked) {
     if (!g->built_csc) { set_error("eg_pagerank: CSC not built"); return EG_ERR_STATE; }
     if (iterations < 0) { set_error("eg_pagerank: iterations must be >= 0"); return EG_ERR_INVALID; }
-    if (g->partitions == 1 && iterations > 0 && g->E > 0) return run_pagerank_single(g, iterations, damping, out, where);
+    if (g->partitions == 1 && iterations > 0 && g->E > 0 && !chunked) return run_pagerank_single(g, iterations, damping, out, where);
     EG_TRY(ensure_engine(g));
     EG_TRY(setup_pull(g));
     const uint32_t V = g->V;

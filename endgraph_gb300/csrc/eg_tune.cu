@@ -115,14 +115,15 @@ int eg_autotune(eg_graph* g, const uint32_t* sample_roots, int nroots, eg_tuning
     out->dense_divisor = best_div;
     out->bfs_ms = best / nb;
 
-    // 2. pull-sweep grid: CTAs per SM (0 = occupancy limit); the sweeps of one partition do not use it
+    // 2. grid of the chunked pull sweeps, CTAs per SM (0 = occupancy limit), on the sweep with the least work beside
+    // it.  PageRank itself takes the chunked sweep with several partitions only; CC and one-seed PPR with one too.
     const int blocks[] = {0, 1, 2, 3, 4};
     best = 1e30;
     int best_blocks = 0;
     for (int bps : blocks) {
         g->pull_blocks_per_sm = bps;
         double ms = 0;
-        EG_TRY(time_median([&]() { return run_pagerank(g, 2, 0.85f, nullptr, EG_HOST); }, &ms));
+        EG_TRY(time_median([&]() { return run_pagerank(g, 2, 0.85f, nullptr, EG_HOST, true); }, &ms));
         if (ms < best * kTuneMargin) {
             best = ms;
             best_blocks = bps;

@@ -277,7 +277,7 @@ typedef struct eg_tuning {
     int32_t batch_width;        /* EG_OPT_BATCH_WIDTH chosen */
     int32_t batch_divisor;      /* EG_OPT_BATCH_DIVISOR chosen */
     double bfs_ms;              /* best single-root BFS time */
-    double pull_sweep_ms;       /* best pull-sweep time (one PageRank iteration) */
+    double pull_sweep_ms;       /* best time of a chunked pull sweep (one iteration of PageRank by it) */
     double msbfs_ms_per_root;   /* best batched BFS time per root */
 } eg_tuning;
 int eg_autotune(eg_graph* g, const uint32_t* sample_roots, int nroots, eg_tuning* out);

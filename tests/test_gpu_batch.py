@@ -467,3 +467,22 @@ def test_level_rows_of_some_columns(eg_lib, n, V):
     for s, r in enumerate(roots):
         ref = oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(r))
         assert np.array_equal(got[7 + s * V: 7 + (s + 1) * V], np.where(ref == oracle.UNREACHED, 255, ref).astype(np.uint8)), s
+
+
+@pytest.mark.parametrize("partitions", [1, 2])
+def test_autotune_times_the_sweeps_it_sizes(eg_lib, partitions):
+    """The grid that is tuned is the chunked pull sweep's: every candidate runs that sweep (five candidates, five
+    times two iterations), also where PageRank itself takes another one."""
+    import endgraph_gb300 as eg
+    V, E = 1 << 13, 1 << 17
+    src, dst, _ = rmat_graph(V, E, 97)
+    with eg.Graph(partitions=partitions) as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        before = g.pagerank(10)
+        g.profile(True)
+        t = g.autotune(src[:8])
+        ran = g.profile_read()
+        g.profile(False)
+        assert ran["pr_pull"][0] == 50 and "pr_persistent" not in ran
+        assert 0 <= t["pull_blocks_per_sm"] <= 4 and t["pull_sweep_ms"] > 0
+        assert rel_l1(g.pagerank(10), before) <= 1e-6
