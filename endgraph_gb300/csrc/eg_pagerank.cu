@@ -310,7 +310,8 @@ int list_run_shift(uint64_t E) {
 
 static int pr_setup(eg_graph* g, const uint32_t* order) {
     EngineState& s = g->eng;
-    if (s.pr_heads_ready && s.pr_heads_relabel == (order != nullptr)) return EG_OK;
+    // with places it serves sweeps in vertex order too, so that calls of both kinds in turn make it once
+    if (s.pr_heads_ready && (s.pr_heads_relabel || !order)) return EG_OK;
     const uint64_t E = g->E, nitems = g->ncompressed - 1;
     const size_t words = E / 32 + 2;
     const int shift = list_run_shift(E);

@@ -65,3 +65,31 @@ def test_pagerank_sweeps_with_hot_sources(eg_lib, V, E):
     dst[: E // 8] = V // 3
     dst[E // 8: E // 4] //= 50
     _check(src, dst, V, (1, 4), relabels=(-1, 0, 1))
+
+
+def test_list_starts_made_once(eg_lib):
+    """Sweeps with and without renumbered sources in turn, and batched BFS between them, share one table of list
+    starts: it is made anew only when the first sweep that wants places comes."""
+    import endgraph_gb300 as eg
+    V, E = 30_000, 400_000
+    rng = np.random.default_rng(3)
+    src, dst = rng.integers(0, V, E), rng.integers(0, V, E)
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    out, _ = oracle.degrees(src, dst, V)
+    csc = oracle.build_csc(src, dst, None, V, np.array([0, V], np.uint32))
+    ref = oracle.pagerank(csc["off"][0], csc["adj"], out, V, 5, 0.85)
+    csr = oracle.build_csr(src, dst, None, V, np.array([0, V], np.uint32))
+    roots = src[:40]
+    levels = [oracle.bfs_levels(csr["off"][0], csr["adj"], V, int(r)) for r in roots]
+    with eg.Graph() as g:
+        for load in range(2):
+            g.load_directed(eg.pack_edges(src, dst), V)
+            g.profile(True)
+            g.profile_reset()
+            for relabel in (0, 1, 0, 1, 1, 0):
+                g.set_option(eg.EG_OPT_PR_RELABEL, relabel)
+                assert rel_l1(g.pagerank(5), ref) <= 1e-6
+                lv, _ = g.msbfs(roots)
+                for s in range(len(roots)):
+                    assert np.array_equal(lv[s], np.where(levels[s] == oracle.UNREACHED, 255, levels[s]).astype(np.uint8))
+            assert g.profile_read()["pr_setup"][0] == 2
