@@ -1025,6 +1025,10 @@ int eg_set_option(eg_graph* g, int option, int64_t value) {
             if (value < 0 || value > INT32_MAX) break;
             g->max_iterations = (int)value;
             return EG_OK;
+        case EG_OPT_PPR_KEEP_MIB:
+            if (value < -1 || value > (1ll << 30)) break;
+            g->ppr_keep_mib = value;
+            return EG_OK;
         case EG_OPT_BUILD_LAUNCH:
             if (value != 0 && value != 1) break;
             g->build_launch = (int)value;

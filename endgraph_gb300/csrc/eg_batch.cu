@@ -1320,7 +1320,6 @@ struct BatchState {
     DevBuf persist;  // persistent traversal: per-level counts, barrier words, error flag
     DevBuf wr0, wr1;  // frontier words in renumbered order (pull gathers through renumbered sources)
     RowTasks csc_tasks, csr_tasks;
-    size_t device_bytes = 0;  // the GPU's memory
     bool csc_ready = false, csr_ready = false;
     // captured MS-BFS level loop and the shapes it was captured for
     void* graph_exec = nullptr;
@@ -2342,7 +2341,7 @@ int run_ppr(eg_graph* g, const float* w_in, const uint32_t* seeds, int n, float 
     return EG_OK;
 }
 
-// Checkpoint stride of the adjoint: the smallest one whose iterates fit an eighth of the GPU's memory
+// Checkpoint stride of the adjoint: the smallest one whose iterates fit EG_OPT_PPR_KEEP_MIB
 // (all of x_0 .. x_{K-1} at stride 1, which recomputes nothing; else K / C checkpoints and a segment
 // of C), at most ceil(sqrt(K)).  1 M vertices, K = 50: stride 1 keeps 12.8 GB and runs 99 forward
 // sweeps in a forward and an adjoint, stride 8 keeps 4 GB and runs 143.
@@ -2372,14 +2371,25 @@ int run_ppr_backward(eg_graph* g, const float* w_in, const uint32_t* seeds, int 
     const uint64_t V = g->V, E = g->E, Ein = g->E_input;
     const int W = row_width(n);
     const size_t row = 4ull * W * V;
-    if (!b.device_bytes) {
-        size_t free_bytes = 0;
-        EG_CUDA(cudaMemGetInfo(&free_bytes, &b.device_bytes));
+    uint64_t budget = 0;
+    if (g->ppr_keep_mib >= 0) {
+        budget = (uint64_t)g->ppr_keep_mib << 20;
+    } else if (ppr_rows_kept(K, 1) * row <= (1ull << 30)) {
+        budget = 1ull << 30;  // not worth a look at what is free
+    } else {
+        size_t free_bytes = 0, total_bytes = 0;
+        EG_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        budget = std::min<uint64_t>(total_bytes / 8, (free_bytes + b.ck.bytes + b.seg.bytes) / 2);
     }
-    int C = ppr_stride(K, row, b.device_bytes / 8);
+    int C = ppr_stride(K, row, budget);
     while (true) {
-        int st = b.ck.reserve(row * ((std::max(K, 1) + C - 1) / C) + 256);
-        if (st == EG_OK && C > 1) st = b.seg.reserve(row * C + 256);
+        const size_t ck = row * ((std::max(K, 1) + C - 1) / C) + 256, seg = C > 1 ? row * C + 256 : 0;
+        if (b.ck.bytes + b.seg.bytes > budget) {  // an earlier call was allowed more
+            if (b.ck.bytes > ck) b.ck.release();
+            if (b.seg.bytes > seg) b.seg.release();
+        }
+        int st = b.ck.reserve(ck);
+        if (st == EG_OK && C > 1) st = b.seg.reserve(seg);
         if (st == EG_OK) break;
         const int most = ppr_stride(K, row, 0);  // the GPU is fuller than that: the fewest rows
         if (C == most) return st;

@@ -209,6 +209,7 @@ struct eg_graph {
     int pull_blocks_per_sm = 0;  // pull-sweep grid; 0 = occupancy limit
     int batch_width = 64;        // roots per bit-parallel pass (eg_bfs_many)
     int pr_relabel = -1;         // PageRank gathers through renumbered sources: 1 on, 0 off, -1 automatic
+    int64_t ppr_keep_mib = -1;   // memory for the adjoint's iterates; -1 = automatic
     int64_t sssp_delta = -1;     // SSSP near/far step in millionths; 0 = Bellman-Ford, -1 = automatic
     // many small graphs in one handle (eg_load_graph_batch): per-graph vertex / edge offsets
     std::vector<uint64_t> batch_voff, batch_eoff;

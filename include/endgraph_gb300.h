@@ -216,11 +216,16 @@ enum {
                                       with EG_OPT_CUDA_GRAPH, the captured one */
     EG_OPT_BATCH_DIVISOR = 10,     /* the switch of the batched BFS (push iff the union frontier's
                                       out-edges < E / divisor); 0 (the default): EG_OPT_DENSE_DIVISOR */
-    EG_OPT_BUILD_LAUNCH = 11       /* the next one-partition, one-sub-partition build from device
+    EG_OPT_BUILD_LAUNCH = 11,      /* the next one-partition, one-sub-partition build from device
                                       records (eg_build, eg_load_graph_batch): 1 runs it as one
                                       persistent cooperative launch (the default: batch id relabel,
                                       the three bucket passes, bitmap and compressed index between
                                       bounded grid barriers); 0: one launch per pass */
+    EG_OPT_PPR_KEEP_MIB = 12       /* device memory that eg_ppr_backward may keep iterates in, in MiB;
+                                      what they do not fit in is recomputed from checkpoints, at 0
+                                      from the fewest (every ceil(sqrt(iterations)) steps).  -1
+                                      automatic: an eighth of the GPU's memory, and no more than
+                                      half of what is free (the default) */
 };
 int eg_set_option(eg_graph* g, int option, int64_t value);
 
@@ -241,8 +246,9 @@ int eg_load_directed_with_ids(eg_graph* g, const void* edges, uint64_t E, uint32
 int eg_ppr(eg_graph* g, const float* weights, const uint32_t* seeds, int nseeds, float alpha, int iterations,
            float* out, int where);
 /* Adjoint of eg_ppr: given dL/dx_iterations (dl_dx[n][V]) writes dL/dw (dl_dw[E], input edge
- * order).  The transposed iteration runs over the CSR; the iterates are kept while they fit an eighth
- * of the GPU's memory, else recomputed from checkpoints at most ceil(sqrt(iterations)) steps apart. */
+ * order).  The transposed iteration runs over the CSR; the iterates are kept while they fit
+ * EG_OPT_PPR_KEEP_MIB, else recomputed from checkpoints at most ceil(sqrt(iterations)) steps apart.
+ * The memory stays with the handle until the next load. */
 int eg_ppr_backward(eg_graph* g, const float* weights, const uint32_t* seeds, int nseeds, float alpha, int iterations,
                     const float* dl_dx, float* dl_dw, int where);
 

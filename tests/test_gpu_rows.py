@@ -298,3 +298,66 @@ def test_ppr_weights_of_short_lists_in_time(eg_lib):
             for k, (_, ms) in g.profile_read().items():
                 best[k] = min(best.get(k, 1e9), ms)
     assert best["ppr_weights"] <= 1.0 and best["ppr_weight_grad"] <= 1.2, best
+
+
+def _spmm_launches(K, C):
+    """Forward sweeps of an adjoint of K steps at stride C: up to the last checkpoint, then in each segment."""
+    return K - 1 if C == 1 else (K - 1) // C * C + sum(min(C, K - k) - 1 for k in range(0, K, C))
+
+
+@pytest.mark.parametrize("n", [5, 32, 33, 64])
+@pytest.mark.parametrize("K", [1, 2, 23])
+def test_ppr_adjoint_strides(eg_lib, n, K):
+    """The adjoint with all iterates kept and with checkpoints every 2, 3, 4 and ceil(sqrt(K)) steps (the last segment
+    full or not), chosen by the memory it may keep; the stride shows in the number of forward sweeps.  Rows of
+    both widths, seeds without in-edges and without any; the tolerance is that of the other comparisons."""
+    import torch
+
+    import endgraph_gb300 as eg
+    src, dst, V0 = _fans(n + K)
+    V = 8192  # a row array is 1 MiB (32 columns) or 2 (64)
+    assert V0 <= V
+    no_in = np.setdiff1d(src, dst)
+    seeds = np.concatenate([[no_in[0], V - 1, 0, 1000], src[:60]]).astype(np.uint32)[:n]
+    rng = np.random.default_rng(K)
+    w = rng.uniform(0.5, 1.5, len(src)).astype(np.float32)
+    dl = rng.random((n, V)).astype(np.float32) / V
+    alpha, mib = 0.15, 1 if n <= 32 else 2
+    wt = torch.tensor(w, dtype=torch.float64, requires_grad=True)
+    _ppr64(src, dst, wt, V, seeds, alpha, K).backward(torch.from_numpy(dl.astype(np.float64)))
+    ref = wt.grad.numpy()
+    # rows kept at each stride for K = 23: 23, 12 + 2, 8 + 3, 6 + 4, 5 + 5
+    strides = {-1: 1, 23 * mib: 1, 14 * mib: 2, 11 * mib: 3, 10 * mib: 4, 0: 5} if K == 23 else {-1: 1, 2 * mib: 1, 0: min(K, 2)}
+    with eg.Graph() as g:
+        g.load_directed_with_ids(eg.pack_edges(src, dst), V)
+        g.profile(True)
+        for keep in list(strides) + list(strides)[::-1]:
+            g.set_option(eg.EG_OPT_PPR_KEEP_MIB, keep)
+            g.profile_reset()
+            dw = g.ppr_backward(w, seeds, dl, alpha, K)
+            assert g.profile_read().get("ppr_spmm", (0, 0))[0] == _spmm_launches(K, strides[keep]), keep
+            assert np.linalg.norm(dw - ref) / np.linalg.norm(ref) <= 1e-4, keep
+
+
+def test_ppr_adjoint_gives_memory_back(eg_lib):
+    """Iterates kept by an earlier call are freed when less is allowed."""
+    import torch
+
+    import endgraph_gb300 as eg
+    V, E, K = 1 << 20, 1 << 20, 20  # 128 MiB a row array: 2.5 GiB of iterates, 9 arrays at the widest stride
+    gen = torch.Generator("cuda").manual_seed(4)
+    rec = torch.randint(0, V, (E, 2), generator=gen, device="cuda", dtype=torch.int32)
+    w, dl = torch.rand(E, generator=gen, device="cuda") + 0.5, torch.rand((2, V), generator=gen, device="cuda")
+    seeds = rec[:2, 0].cpu().numpy().astype(np.uint32)
+    with eg.Graph() as g:
+        g.load_directed_with_ids(rec, V)
+        out = []
+        for keep in (-1, 0, 1 << 20):
+            g.set_option(eg.EG_OPT_PPR_KEEP_MIB, keep)
+            dw = torch.empty(E, device="cuda")
+            g.ppr_backward(w, seeds, dl, 0.15, K, dl_dw=dw)
+            torch.cuda.synchronize()
+            out.append((torch.cuda.mem_get_info()[0], dw))
+    assert out[1][0] - out[0][0] >= 1 << 30 and out[1][0] - out[2][0] >= 1 << 30
+    for _, dw in out[1:]:
+        assert float((dw - out[0][1]).norm() / out[0][1].norm()) <= 1e-5
