@@ -292,7 +292,6 @@ void persist_launched(eg_graph* g);
 // given up as the barrier completed for the others.
 int persist_finish(eg_graph* g, const char* what);
 constexpr int kPersistGaveUp = 63;  // index of that word among the pinned u32 words
-inline uint32_t* persist_gave_up(const eg_graph* g) { return reinterpret_cast<uint32_t*>(g->eng.host_words) + kPersistGaveUp; }
 __device__ __forceinline__ void persist_clear(void* other) {  // by one warp
     if ((threadIdx.x & 31) < kPersistBytes / 16)
         reinterpret_cast<uint4*>(other)[threadIdx.x & 31] = make_uint4(0, 0, 0, 0);

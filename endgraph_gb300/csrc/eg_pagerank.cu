@@ -271,8 +271,7 @@ struct PrPersistArgs {
     int iterations;
     unsigned* words;        // barrier count, unused, error flag
     void* words_next;       // the next launch's, zeroed by this one
-    uint32_t* finished;     // pinned: set when the last iteration is done
-    uint32_t* gave_up;
+    uint32_t* finished;     // the pinned words: set when the last iteration is done
 };
 
 constexpr int kPrPersistThreads = 512, kPrPersistCtas = 2;
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
     __shared__ float s_sum[kPrPersistThreads / 32][kPrSums];
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     unsigned arrived = 0;
-    auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), a.gave_up, arrived); };
+    auto barrier = [&]() { return grid_sync_growing(a.words, reinterpret_cast<int*>(a.words + 2), a.finished + kPersistGaveUp, arrived); };
     pr_start(a.vec[0], a.outdeg, a.V, a.order, a.pr.acc, a.pr.nruns, tid, stride);
     for (int it = 0; it < a.iterations; ++it) {
         if (!barrier()) return;
@@ -377,7 +376,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
         void *block = nullptr, *next = nullptr;
         EG_TRY(persist_block(g, &block, &next));
         PrPersistArgs a{p, V, g->indeg.as<uint32_t>(), outdeg, g->cvert.as<uint32_t>(), order, {vec[0], vec[1]}, result, iterations,
-                        static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words), persist_gave_up(g)};
+                        static_cast<unsigned*>(block), next, reinterpret_cast<uint32_t*>(s.host_words)};
         // A warp per run, or what the vertices' values want where they are more: 20 iterations at 2^20 vertices
         // with 1,000 edges take 0.23 ms so and 2.7 by the one CTA that the runs want; the sum of both is
         // slower where the barriers dominate (0.41 instead of 0.32 ms at 2^20 / 2^20).

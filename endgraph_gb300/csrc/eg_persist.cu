@@ -53,8 +53,8 @@ static_assert(sizeof(PersistResult) <= 4 * kPersistGaveUp, "the results lie in t
 
 // one grid barrier; *s_slot gets the slot the finished step filled.  False: a wait gave up.
 template <class State, class Slot>
-__device__ __forceinline__ bool step_barrier(State* st, uint32_t* gave_up, const Slot* slot, Slot* s_slot, unsigned& arrived) {
-    if (!grid_sync_growing(&st->bar_count, &st->err, gave_up, arrived)) return false;
+__device__ __forceinline__ bool step_barrier(State* st, PersistResult* result, const Slot* slot, Slot* s_slot, unsigned& arrived) {
+    if (!grid_sync_growing(&st->bar_count, &st->err, reinterpret_cast<uint32_t*>(result) + kPersistGaveUp, arrived)) return false;
     if (threadIdx.x < sizeof(Slot) / 16)
         reinterpret_cast<uint4*>(s_slot)[threadIdx.x] = __ldcg(reinterpret_cast<const uint4*>(slot) + threadIdx.x);
     __syncthreads();
@@ -172,7 +172,6 @@ struct SsspPersistArgs {
     PersistState* st;
     void* st_next;      // the next launch's state, zeroed by this one
     PersistResult* result;
-    uint32_t* gave_up;
 };
 
 constexpr uint32_t kWeightSamples = 65536;
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
             for (uint32_t p = lane; p < np; p += 32) a.q[0][p] = piece(a.root, b + (uint64_t)p * kPiece, z);
             if (lane == 0) st->slot[0].n = np;
         }
-        if (!step_barrier(st, a.gave_up, &st->slot[0], &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, &st->slot[0], &s_slot, arrived)) return;
         delta = a.delta;
         if (delta < 0.f) {
             const uint64_t every = max(a.E / kWeightSamples, (uint64_t)1);
@@ -354,11 +353,11 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
         }
         ++step;
         flush_pieces(lq, wb, q_out, &out->n);
-        if (!step_barrier(st, a.gave_up, out, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, out, &s_slot, arrived)) return;
     }
     // every CTA leaves the loop at the same step; the edges walked are added up behind one more barrier
     if (lane == 0 && my_edges) atomicAdd(&st->edges, my_edges);
-    if (!step_barrier(st, a.gave_up, &st->slot[step & 3], &s_slot, arrived)) return;
+    if (!step_barrier(st, a.result, &st->slot[step & 3], &s_slot, arrived)) return;
     if (tid < 32) persist_clear(a.st_next);
     if (tid == 0) {
         st->step = step;
@@ -418,7 +417,6 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
     EG_TRY(persist_block(g, &block, &a.st_next));
     a.st = static_cast<PersistState*>(block);
     a.result = reinterpret_cast<PersistResult*>(s.host_words);
-    a.gave_up = persist_gave_up(g);
     const size_t smem = sizeof(LocalQueue);
     EG_CUDA(cudaFuncSetAttribute(k_sssp_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     volatile PersistResult* h = a.result;
@@ -500,7 +498,6 @@ struct BfsPersistArgs {
     BfsPersistState* st;
     void* st_next;  // the next launch's state, zeroed by this one
     PersistResult* result;
-    uint32_t* gave_up;
 };
 
 // Levels as the only record of what is reached are gathered from L2 while they fit it.  Past that (kBits) one bit per
@@ -550,7 +547,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 st->slot[0].act = z - b;
             }
         }
-        if (!step_barrier(st, a.gave_up, &st->slot[0], &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, &st->slot[0], &s_slot, arrived)) return;
         reached = 1;
         edges = s_slot.act;
     } else {
@@ -597,7 +594,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
                 s_verts = 0;
                 s_act = 0;
             }
-            return step_barrier(st, a.gave_up, out, &s_slot, arrived);
+            return step_barrier(st, a.result, out, &s_slot, arrived);
         };
         if (!dense) {
             const uint4* q = a.q[step & 1];
@@ -653,7 +650,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_bfs_persisten
         } else {
             if (kBits) {
                 for (uint64_t i = tid; i < a.nwords; i += stride) a.snap[i] = __ldcg(a.vis + i);
-                if (!step_barrier(st, a.gave_up, &st->slot[step & 3], &s_slot, arrived)) return;
+                if (!step_barrier(st, a.result, &st->slot[step & 3], &s_slot, arrived)) return;
             }
             auto unreached = [&](uint32_t v) { return kBits ? !bit_at(a.vis, v) : __ldcg(a.level + v) == kUnreached; };
             auto in_front = [&](uint32_t u) { return kBits ? bit_at(a.snap, u) : __ldcg(a.level + u) == lvl; };
@@ -842,7 +839,6 @@ int run_bfs_persistent(eg_graph* g, uint32_t root, uint32_t* level, uint32_t* pa
     EG_TRY(persist_block(g, &block, &a.st_next));
     a.st = static_cast<BfsPersistState*>(block);
     a.result = reinterpret_cast<PersistResult*>(s.host_words);
-    a.gave_up = persist_gave_up(g);
     const bool bits = V > kBfsBits;
     a.nwords = V / 64 + 1;
     if (bits)
@@ -914,7 +910,6 @@ struct CcArgs {
     CcState* st;
     void* st_next;  // the next launch's state, zeroed by this one
     PersistResult* result;
-    uint32_t* gave_up;
 };
 constexpr uint32_t kCcFirst = 2;      // neighbours united before the common component is looked for
 constexpr int kCcSamples = 1024;
@@ -988,17 +983,17 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
             if (b + k < e) p = min(p, __ldg(a.adj + b + k));
         a.comp[v] = p;
     }
-    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
     cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
-    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
     for (uint32_t k = 0; k < kCcFirst; ++k) {
         for (uint64_t i = tid; i < a.nlists; i += stride) {
             const uint64_t b = __ldg(a.off + i) + k;
             if (b < __ldg(a.off + i + 1)) cc_unite(a.comp, cc_vertex<kIndex>(a.vert, i), __ldg(a.adj + b));
         }
-        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
         cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
-        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
     }
     // the component of most of a sample's vertices; one CTA decides for all
     if (blockIdx.x == 0) {
@@ -1013,7 +1008,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         __syncthreads();
         if (threadIdx.x == 0) st->slot.common = (uint32_t)s_best;
     }
-    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
     const uint32_t common = s_slot.common;
     // the other components' lists, from the third neighbour on
     for (uint64_t base = tid & ~31ull; base < a.nlists; base += stride) {
@@ -1028,7 +1023,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
         append_pieces<1>(lq, wb, vv, lb, le, a.q, &st->slot.n);
     }
     flush_pieces(lq, wb, a.q, &st->slot.n);
-    if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+    if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
     const uint32_t n = s_slot.n;
     if (n) {
         for (uint32_t base = 0; base < n; base += 32 * nwarps) {
@@ -1053,7 +1048,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_cc_persistent
                 __syncwarp();
             }
         }
-        if (!step_barrier(st, a.gave_up, &st->slot, &s_slot, arrived)) return;
+        if (!step_barrier(st, a.result, &st->slot, &s_slot, arrived)) return;
         cc_compress<kIndex>(a.comp, a.vert, a.nlists, tid, stride);
     }
     if (tid < 32) persist_clear(a.st_next);
@@ -1083,7 +1078,7 @@ int run_cc_symmetric(eg_graph* g, uint32_t* label, int where) {
     CcArgs a{V, index ? nitems : V, g->outdeg.as<uint32_t>(), index ? g->cvert.as<uint32_t>() : nullptr,
              index ? g->cidx.as<uint64_t>() : g->csr_off.as<uint64_t>(),
              index ? g->csc_adj.as<uint32_t>() : g->csr_adj.as<uint32_t>(), comp, s.pieces0.as<uint4>(),
-             static_cast<CcState*>(block), next, h, persist_gave_up(g)};
+             static_cast<CcState*>(block), next, h};
     const size_t smem = sizeof(LocalQueue);
     const void* fn = index ? (const void*)k_cc_persistent<true> : (const void*)k_cc_persistent<false>;
     EG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
