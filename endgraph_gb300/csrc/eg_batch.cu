@@ -14,7 +14,7 @@
 //      - eg_ppr_backward: the adjoint of K unrolled iterations.  lambda_k = (1-a) A lambda_{k+1} is
 //        a pull over the CSR (the transpose of the forward CSC); the same sweep accumulates
 //        dL/dA_uv = (1-a) sum_k <x_k[u], lambda_{k+1}[v]>; the iterates x_k are kept while they fit
-//        an eighth of the GPU's memory, else recomputed from checkpoints;
+//        EG_OPT_PPR_KEEP_MIB, else recomputed from checkpoints;
 //      - eg_sssp_batch: Bellman-Ford from up to 64 sources, in place, skipping sources whose
 //        distance did not change in the previous sweep (bit-exact least fixpoint).
 #include <math.h>
@@ -680,7 +680,7 @@ static int make_tasks(eg_graph* g, RowTasks& t, const uint64_t* begin, uint64_t 
 }
 
 // ---------------------------------------------------------------------------------------------
-// row kernels: one warp per task, 64-column rows of 256 bytes
+// row kernels: a warp per batch of tasks, rows of 64 columns (256 bytes) or 32
 struct RowArgs {
     const uint4* rec;
     const uint32_t* first;        // first task of every batch
@@ -1406,7 +1406,7 @@ constexpr int kGraphLevels = 16;
 
 // The captured level loop makes, on the device, the choice the host loop makes per level: each
 // level's first kernel reads the frontier's length and out-edges and arms either the pull kernels
-// (the chunked sweep for the first dense level, the early-exit pair after it on one graph) or the
+// (the full sweep for the first dense level, the early-exit pair after it on one graph) or the
 // push (a scan and expansion whose item count it sets); the kernels of the other path find
 // nothing to do.  After an empty frontier every later level is disarmed.
 struct CapLevel {
@@ -1699,7 +1699,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
     // read all their in-edges, which the full sweep (k_ms_sweep) does best.  Later
     // dense levels find most destinations nearly covered and use the early-exit pair -- on one
     // graph.  In a batch of graphs the running-root mask is shared by all graphs, so a vertex
-    // waits for bits its own graph can never deliver, and every level keeps the chunked sweep.
+    // waits for bits its own graph can never deliver, and every level keeps the full sweep.
     // clear_n: how many vertices queue[x] lists from two levels back (the non-zero words of
     // word[x]); kUnknownQueue when not known on the host, and the arrays are cleared whole
     auto enqueue_level = [&](uint32_t L, uint64_t n_host, bool dense, bool screen, uint32_t* count, const int* stop_flag,
@@ -1911,7 +1911,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
                     ok(cudaGetLastError());
                 }
                 ok(cudaMemsetAsync(bm[x], 0, bm_bytes, g->stream));
-                // pull: the chunked sweep or the early-exit pair, whichever the level armed
+                // pull: the full sweep or the early-exit pair, whichever the level armed
                 {
                     if (st == EG_OK)
                         st = ms_sweep(g, gather_adj, word[c], bm[c], 1, visit, word[x], bm[x], alive + 2,
@@ -2002,7 +2002,7 @@ static int msbfs_core(eg_graph* g, uint32_t n_entries, int nbits, unsigned long 
         }
         if (!done) {
             // deeper than the captured levels: the host-driven loop takes over at level
-            // kGraphLevels (queue[0] lists level 31's output, queue[1] level 30's); the captured
+            // kGraphLevels (queue[0] lists the last captured level's output, queue[1] the one's before); the captured
             // levels kept no running-root masks, so every root counts as running
             lvl = kGraphLevels;
             EG_CUDA(cudaMemcpyAsync(alive + (lvl & 1), &full, 8, cudaMemcpyHostToDevice, g->stream));
@@ -2490,13 +2490,13 @@ __global__ void k_sssp_init_entries(const uint2* ent, uint32_t n, float* dist, i
     }
 }
 
-// Bellman-Ford sweeps from the root entries in b.entries; leaves dist [V][row_width(n)] in b.rows0
 // [V][32] rows -> [V][64], the columns past 32 unreached
 __global__ void __launch_bounds__(256) k_widen_rows(const float* __restrict__ in, uint64_t V, float* __restrict__ out) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 64 * V; i += (uint64_t)gridDim.x * blockDim.x)
         out[i] = i & 32 ? 1e9f : __ldcs(in + (i >> 6) * 32 + (i & 31));
 }
 
+// Bellman-Ford sweeps from the root entries in b.entries; leaves dist [V][row_width(n)] in b.rows0.
 // n: sources per row (32 columns for up to 32, which halves what the sweeps gather, else 64)
 static int sssp_core(eg_graph* g, int n, uint32_t n_entries, int* sweeps_out) {
     const int W = row_width(n);

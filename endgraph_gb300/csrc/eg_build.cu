@@ -879,7 +879,7 @@ static int build_single(eg_graph* g, const UploadParts* up) {
 // ---------------------------------------------------------------------------------------------
 // The one-partition bucketed build in one cooperative launch: every phase of build_single and of
 // the index kernels of build_structures, separated by bounded grid barriers (grid_sync_bounded),
-// with one 1,024-thread CTA per SM taking pass-A and pass-B blocks by stride, pass-C buckets by
+// with one 1,024-thread CTA per SM taking pass-A blocks and pass-B tiles by stride, pass-C buckets by
 // ticket and the scans as contiguous ranges.  A graph batch's ids are moved to the union in pass A.
 constexpr int kPersistBuildMaxCtas = 1024;
 
@@ -1095,7 +1095,7 @@ template <int REC>
 __global__ void __launch_bounds__(kBucketThreads, 1) k_build_persistent(PersistBuildArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     BuildWords* w = a.w;
-    // A: the records in, bucket counts per (half, bucket, block)
+    // A: the records in, bucket totals per (half, bucket)
     for (uint32_t blk = blockIdx.x; blk < a.nblk; blk += gridDim.x) {
         load_count_block<REC>(a.src, a.E, a.chunk, a.shift, a.nb, a.tot, a.V, &w->bad, blk,
                               reinterpret_cast<uint32_t*>(s_raw));

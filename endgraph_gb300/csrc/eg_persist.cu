@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistCtas) k_sssp_persiste
 }
 
 // The automatic threshold step, in mean weights.  A step costs a barrier and some L2 round trips
-// (6.5 us) however few edges it relaxes, so graphs whose vertex arrays sit in L2 take steps so wide
+// (3.6 us with one CTA, 3.9 with 304) however few edges it relaxes, so graphs whose vertex arrays sit in L2 take steps so wide
 // that R-MAT distances need one or two phases; larger ones gain more from relaxing less.  Times in
 // ms with 0.7 / 3 / 100 x mean weight / mean degree: 20 k vertices, 300 k edges 1.14 / 0.51 / 0.28; 200 k,
 // 4 M 1.99 / 0.87 / 0.56; 1 M, 8 M 1.42 / 1.07 / 0.88; 2 M, 64 M 4.4 / 2.9 / 3.7; 4 M, 20 M 1.8 / 2.4 / 3.1; 4 M,
@@ -451,11 +451,11 @@ int run_sssp_persistent(eg_graph* g, uint32_t root, float* dist, int where) {
 // dense level gives every compressed in-list of an unreached vertex a thread that looks at its first
 // kBfsHead in-edges, then the warp walks what its 32 lists have left together, and lists longer than
 // that are cut into segments that a second half of the level spreads over the GPU.  The frontier is
-// "level == this level": no bitmaps to keep or clear.  Means of 16 roots, against the level loop driven
+// "level == this level", or past 2^23 vertices the bits of kBits below.  Means of 16 roots, against the level loop driven
 // from the host that it replaces (kernels per level, bitmaps, counters read back): 100,003 vertices,
-// 1,000,003 edges 0.33 -> 0.09 ms; 2^22, 2^26 0.41 -> 0.26; 2^25, 2^29 2.11 -> 1.29, most of it where the
-// first dense level finds few parents in the lists' heads (5.04 -> 1.89 ms: the rest of a list was one
-// warp's).  A dense level is bound by its gathers: rounds of four in-edges, up to 12, take 1.29 ms, up
+// 1,000,003 edges 0.33 -> 0.08 ms; 2^22, 2^26 0.41 -> 0.26; 2^25, 2^29 2.11 -> 0.97 (1.29 by levels), most of it where the
+// first dense level finds few parents in the lists' heads (5.04 -> 1.89 ms by levels: the rest of a list was one
+// warp's).  A dense level is bound by its gathers: by levels, rounds of four in-edges, up to 12, took 1.29 ms, up
 // to 8 1.34, up to 4 1.44, eight at once 1.54.
 constexpr uint32_t kBfsHead = 12;
 constexpr uint32_t kBfsSeg = 1024;

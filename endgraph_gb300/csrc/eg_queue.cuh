@@ -14,9 +14,10 @@
 namespace eg {
 
 constexpr uint32_t kPiece = 256;  // edges per queue entry
-// two CTAs of 512 threads per SM at 64 registers: a BFS of 2^25 / 2^29 took 1.61 ms (mean of 16 roots)
-// against 1.66 with one CTA of 1,024, 1.70 with three of 512 (42 registers), 1.75 with two of 768 and
-// 1.87 with two of 1,024; one of 2^22 / 2^26 0.29 against 0.30 / 0.28 / 0.29 / 0.32
+// Two CTAs of 512 threads per SM at 64 registers.  Measured on the first BFS kernel (levels alone, the rest of a long list
+// walked by one thread): 2^25 / 2^29 1.61 ms (mean of 16 roots) against 1.66 with one CTA of 1,024, 1.70 with
+// three of 512 (42 registers), 1.75 with two of 768 and 1.87 with two of 1,024; 2^22 / 2^26 0.29 against 0.30 / 0.28 /
+// 0.29 / 0.32.
 constexpr int kPersistThreads = 512;
 constexpr int kPersistCtas = 2;
 // A CTA's share of the next queue gathers in shared memory and goes out with one reservation.  What does
