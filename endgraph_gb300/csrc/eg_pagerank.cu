@@ -14,6 +14,8 @@
 // a list's pieces, so that the last warp finishes it, made the sweep wait for the counters of the
 // hubs: 2.7 instead of 1.95 ms at 2^25 / 2^29, 2.8 with fences.)  Small graphs run every iteration in one
 // persistent launch between grid barriers.
+#include <math.h>
+
 #include <algorithm>
 
 #include "eg_pull.cuh"
@@ -54,6 +56,12 @@ __device__ __forceinline__ void pr_write(const PrArgs& a, uint32_t item, float s
     a.next[to] = pr_value(a, sum, deg);
 }
 
+// what a + b = s loses by rounding (Knuth's two-sum); nothing once the sum is infinite
+__device__ __forceinline__ float sum_lost(float a, float b, float s) {
+    const float v = s - a;
+    return fabsf(s) < INFINITY ? (a - (s - v)) + (b - v) : 0.f;
+}
+
 // one run of blocks by one warp; s_sum: kPrSums floats of the warp's own
 template <class Gather>
 __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_sum, Gather gather) {
@@ -64,11 +72,7 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
     const uint64_t e_end = min(a.E, ((run + 1) << a.shift) * kPrBlock);
     uint32_t item = __ldg(a.item_of + (run << a.shift));
     bool open_first = !(__ldg(a.heads + (e_begin >> 5)) & 1u);  // the first list began in an earlier run
-    float carry = 0.f, carry_low = 0.f;  // sum of the open list so far, and what its roundings lost (Knuth's two-sum)
-    auto plus_carry = [&](float x) {     // carry + x, rounded once
-        const float s = carry + x, v = s - carry;
-        return s + (((carry - (s - v)) + (x - v)) + carry_low);
-    };
+    float carry = 0.f, carry_low = 0.f;  // sum of the open list so far, and what its roundings lost
     for (uint64_t e0 = e_begin; e0 < e_end; e0 += kPrBlock) {
         float val[kGroups][G];
         uint32_t head[kGroups];
@@ -138,14 +142,17 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
             }
             float before = __shfl_up_sync(0xffffffffu, t, 1);
             if (lane == 0) before = 0.f;
-            if (seen) s_sum[rank[g]] = m & below ? before + first : plus_carry(before + first);
+            if (seen) {
+                const float x = before + first, s = carry + x;
+                s_sum[rank[g]] = m & below ? x : s + (sum_lost(carry, x, s) + carry_low);
+            }
             const float rest = __shfl_sync(0xffffffffu, t, 31);
             if (m) {
                 carry = rest;
                 carry_low = 0.f;
             } else {
-                const float s = carry + rest, v = s - carry;
-                carry_low += (carry - (s - v)) + (rest - v);
+                const float s = carry + rest;
+                carry_low += sum_lost(carry, rest, s);
                 carry = s;
             }
             __syncwarp();

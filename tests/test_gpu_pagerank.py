@@ -121,3 +121,16 @@ def test_pagerank_of_a_hub(eg_lib, E):
                 g.set_option(eg.EG_OPT_PR_RELABEL, relabel)
                 got = g.pagerank(it, 0.85)
                 assert abs(float(got[1234]) - float(cur[1234])) <= 4 * 2.0**-24 * float(cur[1234]), (it, relabel)
+
+
+def test_pagerank_that_overflows(eg_lib):
+    """Values past the largest float become infinite, as in a plain sum, and not NaN."""
+    import endgraph_gb300 as eg
+    V, E = 2000, 300_000
+    rng = np.random.default_rng(4)
+    src, dst = rng.integers(0, V, E).astype(np.uint32), rng.integers(0, V, E).astype(np.uint32)
+    dst[:100_000] = 7
+    with eg.Graph() as g:
+        g.load_directed(eg.pack_edges(src, dst), V)
+        x = g.pagerank(2, -1e35)  # the second sweep sums values of 1e33 and more
+        assert not np.isnan(x).any() and np.isinf(x[7])
