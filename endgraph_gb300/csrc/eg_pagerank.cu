@@ -63,7 +63,8 @@ __device__ __forceinline__ float sum_lost(float a, float b, float s) {
 }
 
 // one run of blocks by one warp; s_sum: kPrSums floats of the warp's own
-template <class Gather>
+// kLong: runs of several blocks, whose carry is compensated (one block adds its two groups plainly)
+template <bool kLong, class Gather>
 __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_sum, Gather gather) {
     constexpr int G = kPrGroup, kGroups = (int)kPrBlock / (32 * G);
     const uint32_t lane = threadIdx.x & 31;
@@ -144,7 +145,7 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
             if (lane == 0) before = 0.f;
             if (seen) {
                 const float x = before + first, s = carry + x;
-                s_sum[rank[g]] = m & below ? x : s + (sum_lost(carry, x, s) + carry_low);
+                s_sum[rank[g]] = m & below ? x : kLong ? s + (sum_lost(carry, x, s) + carry_low) : s;
             }
             const float rest = __shfl_sync(0xffffffffu, t, 31);
             if (m) {
@@ -152,7 +153,7 @@ __device__ __forceinline__ void pr_run(const PrArgs& a, uint64_t run, float* s_s
                 carry_low = 0.f;
             } else {
                 const float s = carry + rest;
-                carry_low += sum_lost(carry, rest, s);
+                if (kLong) carry_low += sum_lost(carry, rest, s);
                 carry = s;
             }
             __syncwarp();
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(kPrSweepThreads, 1) k_pr_sweep(PrArgs a) {
         const uint32_t run = __shfl_sync(0xffffffffu, next, 0);
         if (run >= a.nruns) break;
         if (lane == 0) next = atomicAdd(a.ticket, 1u);
-        pr_run(a, run, s_dyn + (threadIdx.x >> 5) * kPrSums, [&](uint32_t id) {
+        pr_run<true>(a, run, s_dyn + (threadIdx.x >> 5) * kPrSums, [&](uint32_t id) {
             const uint32_t rank = __funnelshift_r(id, id, 5);  // ids that are no multiple of 32 come out large
             float v;
             asm volatile(
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(kPrPersistThreads, kPrPersistCtas) k_pr_persis
         if (last) p.dst = a.cvert;
         p.divide = !last;
         if (it < 2 || last) pr_no_in(p.next, a.indeg, a.outdeg, a.V, p.base, p.divide, last ? nullptr : a.order, tid, stride);
-        for (uint64_t run = tid >> 5; run < p.nruns; run += stride >> 5) pr_run(p, run, s_sum[threadIdx.x >> 5], [&](uint32_t id) { return ld_keep(p.curr + id); });
+        for (uint64_t run = tid >> 5; run < p.nruns; run += stride >> 5) pr_run<false>(p, run, s_sum[threadIdx.x >> 5], [&](uint32_t id) { return ld_keep(p.curr + id); });
         if (!barrier()) return;
         for (uint64_t r = tid; r < p.nruns; r += stride) pr_boundary(p, r);
     }
@@ -367,7 +368,7 @@ int run_pagerank_single(eg_graph* g, int iterations, float damping, float* out, 
     // renumber and 0.18 instead of 0.26 a sweep; a GPU too full for the second list goes without.  Passes over
     // many vertices want more threads than the one launch has: 3 iterations at 2^26 vertices take 2.23 / 1.33
     // with 1,000 edges, 2.86 / 1.96 with 2^24; 20 at 2^23 0.52 / 0.81 and 2.48 / 2.78.
-    const bool small = E <= (1ull << 24) && V <= (1ull << 24);
+    const bool small = E <= (1ull << 24) && V <= (1ull << 24) && list_run_shift(E) == 0;
     bool relabel = want_relabel(g);
     if (!relabel && !small && g->pr_relabel < 0 && iterations >= 4) relabel = setup_list_heads(g, true) == EG_OK;
     EG_TRY(setup_list_heads(g, relabel));
